@@ -181,6 +181,86 @@ __device__ __forceinline__ void gauge_values(const ScenarioDev &s, int parity, i
     }
 }
 
+// The control of one scenario after a step (src/GPU/ShallowWater.cu:397-450
+// loop body after the step; src/GPU/Timestep.cu:35-68 dt truncation to fault
+// times): time, next dt (dmin: the step's CFL minimum), status and events in
+// c.  Returns the ring slot of a gauge sample to take at this step (at c.t), or -1.
+__device__ __forceinline__ int advance_scenario(ScenarioCtl &c, const ScenarioDev &s, float dmin, unsigned errs)
+{
+    int sample = -1;
+    c.t += c.dt;
+    double dt = (double)dmin;
+    // truncation so that t lands on the next fault time
+    const int nf = c.nfaults;
+    const int f = c.fault_next;
+    const double *tf = c.fault_times;
+    if (!c.jumping) {
+        if (f < nf && (c.t + dt) * c.T > tf[f]) {
+            dt = tf[f] / c.T - c.t;
+            c.jumping = 1;
+        }
+    } else {
+        c.jumping = 0;
+        if (f < nf) {
+            int i = f + 1;
+            while (i < nf && !(fabs(tf[i] - tf[f]) > 2.220446049250313e-16)) i++;
+            if (i < nf && (c.t + dt) * c.T > tf[i]) {
+                dt = tf[i] / c.T - c.t;
+                c.jumping = 1;
+            }
+        }
+    }
+    c.dt = dt;
+    c.step += 1;
+    c.parity ^= 1;
+    c.dt_bits = 0x7f7fffffu;
+    c.tiles_done = 0u;
+    int ev = 0;
+    if (errs || !(dmin > 0.f) || isnan(dmin)) {
+        c.status = kFailed;
+    } else if (!(c.t < c.t_end)) {
+        c.status = kDone;
+    } else if (c.max_steps >= 0 && c.step >= c.max_steps) {
+        c.events = kEvStepBudget;
+        c.status = kDone;
+    } else {
+        if (f < nf && c.t * c.T >= tf[f]) ev |= kEvFault;
+        if (c.save_nc >= 0.0 && c.t >= c.next_nc) ev |= kEvSnapshot;
+        if (c.save_ts >= 0.0 && c.t >= c.next_ts) {
+            if (s.ngauges > 0 && !(ev & kEvFault)) {
+                // the loop's gauge event on the device: same time test
+                // and interval update as the host's
+                sample = (int)(c.gauge_count % kGaugeRing);
+                c.next_ts += c.save_ts;
+                c.gauge_count += 1;
+            } else {
+                ev |= kEvSeries;
+            }
+        }
+        if (ev) {
+            c.events = ev;
+            c.status = kPaused;
+        }
+    }
+    return sample;
+}
+
+// the fields advance_scenario changes, back to the scenario's control block
+__device__ __forceinline__ void store_advanced(ScenarioCtl *cp, const ScenarioCtl &c)
+{
+    cp->t = c.t;
+    cp->dt = c.dt;
+    cp->step = c.step;
+    cp->parity = c.parity;
+    cp->jumping = c.jumping;
+    cp->dt_bits = c.dt_bits;
+    cp->tiles_done = c.tiles_done;
+    cp->events = c.events;
+    cp->status = c.status;
+    cp->next_ts = c.next_ts;
+    cp->gauge_count = c.gauge_count;
+}
+
 __host__ __device__ inline float fmax_(float a, float b) { return (a < b) ? b : a; }
 __host__ __device__ inline float fmin_(float a, float b) { return (b < a) ? b : a; }
 
@@ -213,21 +293,6 @@ __device__ __forceinline__ float inv_depth(float h, float eps)
     return kSqrt2 * h * rsqrt_ap(pow4f(h) + pow4f(eps));
 }
 
-// Monotone limiter of the WAF correction (src/GPU/Arista_kernel.cu:45-68).
-__device__ __forceinline__ float monotone_limiter(float pm, float p0, float p1, float pp, float wave)
-{
-    float d_mid = p1 - p0;
-    float d_up = (wave < 0.f) ? (pp - p1) : ((wave > 0.f) ? (p0 - pm) : 0.5f * (pp - pm));
-    float same = (d_mid * d_up >= 0.f) ? 1.f : 0.f;
-    d_mid = fabsf(d_mid);
-    d_up = fabsf(d_up);
-    if (d_mid < kEps) return 1.f;
-    float a = fabsf(__fdividef(d_up - d_mid, d_up + d_mid));
-    d_up = 0.5f * (d_up + d_mid) * (1.f - a * a * a);
-    float r = (d_mid > d_up) ? __fdividef(d_up, d_mid + kEps) : __fdividef(d_mid, d_up + kEps);
-    return same * r * __fdividef(1.f + r, 1.f + r * r);
-}
-
 // Limits a mass flux so that neither side loses more than 1/4 of its water in
 // one step (src/GPU/Arista_kernel.cu:79-114; c0/c1 = cos(lat) for y edges).
 // dt > dt0 = cap / (|F| + eps) is tested as dt (|F| + eps) > cap, so the
@@ -238,14 +303,6 @@ __device__ __forceinline__ float limit_outflow(float F, float h0, float h1, floa
     const float aF = fabsf(F) + kEps;
     if (dt * aF > cap) F *= (cap / aF) / (dt + kEps);
     return F;
-}
-
-// Blend weight of the 2s flux against the WAF flux (src/GPU/Arista_kernel.cu:208).
-__device__ __forceinline__ float blend_2s(float hij, float hpos, bool no_lim)
-{
-    if (no_lim) return 0.f;
-    if (hij < hpos) return __frcp_rn(1.f + __expf(-15.f * (1.f - 0.5f * hpos / (hij + kEps))));
-    return 1.f;
 }
 
 // Surface-gradient term max(eta1+Hm,0) - max(eta0+Hm,0) with Hm = min(D0,D1),
@@ -261,45 +318,15 @@ __device__ __forceinline__ float surface_jump(float e0, float e1, float D0, floa
     return fmax_(a, 0.f) - fmax_(b, 0.f);
 }
 
-// One edge: four stencil cells along the edge normal.  "u" is the momentum
-// component normal to the edge, "v" the tangential one.
-struct Edge {
-    float h0m, h0, h1, h1p;
-    float e0m, e0, e1, e1p;
-    float D0, D1;
-    float u0m, u0, u1, u1p;
-    float v0m, v0, v1, v1p;
-    float area0, area1, cos0, cos1;
-    float len;      // x edges: len/cos (ilcos); y edges: len
-    float normal;
-    bool front;     // ghost on the low side: sides swapped, flux computed mirrored
-    bool no_lim;    // within two cells of a boundary: first order, no 2s blend
-};
-
 __device__ __forceinline__ void swapf(float &a, float &b) { float t = a; a = b; b = t; }
-
-__device__ __forceinline__ void swap_sides(Edge &e)
-{
-    swapf(e.h0m, e.h1p); swapf(e.h0, e.h1);
-    swapf(e.e0m, e.e1p); swapf(e.e0, e.e1);
-    swapf(e.D0, e.D1);
-    swapf(e.u0m, e.u1p); swapf(e.u0, e.u1);
-    swapf(e.v0m, e.v1p); swapf(e.v0, e.v1);
-    swapf(e.area0, e.area1); swapf(e.cos0, e.cos1);
-}
-
-__device__ __forceinline__ bool all_deep(const Edge &e, float hpos)
-{
-    return (e.h0 > hpos) && (e.h1 > hpos) && (e.h0m > hpos) && (e.h1p > hpos) && !e.no_lim;
-}
 
 // ---------------------------------------------------------------------------
 // Edges whose four stencil cells are all deeper than hpos and which lie at
 // least two cells from a boundary: the 2s blend weight is exactly 1, so the
 // flux is the 2s flux alone (the WAF part, the wet/dry tests and the limiter
-// drop out).  The general functions below and deep phase 1 call these; deep
-// phase 2 evaluates the same formulas two edges at a time in packed FP32x2
-// arithmetic (step.cu), which can round its last bit differently.
+// drop out).  The general units and deep phase 1 call the mass fluxes; deep
+// phase 2 evaluates the momentum formulas two edges at a time in packed FP32x2
+// arithmetic (step_parts.cuh), which can round its last bit differently.
 // ---------------------------------------------------------------------------
 
 // x edge: F = q0 len, outflow-limited (src/GPU/Arista_kernel.cu:118-219, alfa = 1)
@@ -314,15 +341,6 @@ __device__ __forceinline__ float mass_2s_y(float q0, float len, float cos0, floa
 {
     return limit_outflow(len * q0 * cos0, h0, h1, cos0, cos1, dt, a0, a1);
 }
-
-// Result of a momentum flux: contributions to the two cells (already with
-// the "acc -= F" sign applied) and the wave-speed term for the time step.
-struct MomFlux {
-    float m_x, m_y;   // to cell0: subtract
-    float p_x, p_y;   // to cell1: subtract
-    float lam;        // edge length * max wave speed (added to both)
-    bool active;
-};
 
 // Per-cell factors of the 2s fluxes, computed once per cell and shared by
 // its four edges: 1/h (approximate reciprocal) and sqrt(h).
@@ -368,296 +386,252 @@ __device__ __forceinline__ YRowK make_yrow(float cos0, float cos1, float icos0, 
     return k;
 }
 
-// x edge, components (qx, qy); u = qx normal, v = qy tangential, rh = 1/h,
-// sh = sqrt(h) of each side, jump = the surface jump, k = the row's constants
-// (src/GPU/Arista_kernel.cu:221-464, alfa = 1)
-__device__ __forceinline__ void momentum_2s_x(MomFlux &r, float h0, float h1, float rh0, float rh1, float s0, float s1,
-                                              float u0, float u1, float v0, float v1, float jump, const XRowK &k)
+// ---------------------------------------------------------------------------
+// Roundings.  The edge fluxes below and the cell updates are written with
+// explicit operations (add, sub, mul, fma2p, ...), never left to the
+// compiler's contraction: the same cell is stepped by code copies in several
+// kernels (tilings, launched and resident steps), and every copy must round
+// alike.  Which products are fused is part of the formula.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float sub(float a, float b) { return __fadd_rn(a, -b); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+// a b + c d and a b - c d, the second product rounded first (fma2p, fma2m) or
+// the first one (fma2q, fma2n)
+__device__ __forceinline__ float fma2p(float a, float b, float c, float d) { return fma_(a, b, mul(c, d)); }
+__device__ __forceinline__ float fma2m(float a, float b, float c, float d) { return fma_(a, b, -mul(c, d)); }
+__device__ __forceinline__ float fma2q(float a, float b, float c, float d) { return fma_(c, d, mul(a, b)); }
+__device__ __forceinline__ float fma2n(float a, float b, float c, float d) { return fma_(-c, d, mul(a, b)); }
+
+// Desingularised 1/h (src/GPU/Arista_kernel.cu:164): sqrt2 h / sqrt(h^4 + max(h,eps)^4),
+// which is exactly 1/h for h >= eps.
+__device__ __forceinline__ float inv_depth_x(float h, float eps)
 {
-    const float ilcos = k.ilcos;
-    const float hij = 0.5f * (h0 + h1);
-    const float u0n = u0 * rh0, u1n = u1 * rh1;
-    const float uijn = __fdividef(s0 * u0n + s1 * u1n, s0 + s1 + kEps);
-    const float maxa = fabsf(uijn) + sqrt_ap(hij);
-    float mx, my, px, py;
-    if (uijn < 0.f) {
-        mx = u1n * u1 * ilcos; px = -mx; mx += hij * jump * ilcos;
-        my = u1n * v1 * ilcos; py = -my;
-    } else {
-        mx = u0n * u0 * ilcos; px = -mx; mx += hij * jump * ilcos;
-        my = u0n * v0 * ilcos; py = -my;
-    }
-    const float des = k.kdes * (maxa * maxa) * (u1 - u0);
-    r.m_x = mx - des; r.m_y = my;
-    r.p_x = px + des; r.p_y = py;
-    r.lam = ilcos * maxa;
-    r.active = true;
+    if (h >= eps) return __frcp_rn(h);
+    const float h2 = mul(h, h), e2 = mul(eps, eps);
+    return mul(mul(kSqrt2, h), rsqrt_ap(fma2p(h2, h2, e2, e2)));
 }
 
-// y edge, components (qx, qy); u = qy normal, v = qx tangential; k = the
-// constants of the edge's row pair (src/GPU/Arista_kernel.cu:780-1026, alfa = 1)
-__device__ __forceinline__ void momentum_2s_y(MomFlux &r, float h0, float h1, float rh0, float rh1, float s0, float s1,
-                                              float u0, float u1, float v0, float v1, float jump, const YRowK &k)
+// Monotone limiter of the WAF correction from the difference across the edge
+// and the one upwind of it (src/GPU/Arista_kernel.cu:45-68)
+__device__ __forceinline__ float limiter_of(float d_mid, float d_up)
 {
-    const float hij = 0.5f * (h0 + h1);
-    const float u0n = u0 * rh0, u1n = u1 * rh1;
-    const float uijn = __fdividef(s0 * u0n + s1 * u1n, s0 + s1 + kEps);
-    const float maxa = fabsf(uijn) + sqrt_ap(hij);
-    const float deta = k.cmid * jump - uijn * uijn * k.cdiff;
-    float fym, fyp, fxm, fxp;
-    if (uijn < 0.f) {
-        fym = u1n * u1 * k.len; fyp = -fym; fym *= k.c10; fym += hij * deta * k.li0;
-        fxm = u1n * v1 * k.len; fxp = -fxm;
-    } else {
-        fym = u0n * u0 * k.len; fyp = -fym * k.c01; fym += hij * deta * k.li0;
-        fxm = u0n * v0 * k.len; fxp = -fxm;
-    }
-    const float m2 = (maxa * maxa) * (u1 * k.cos1 - u0 * k.cos0);
-    r.m_x = fxm; r.m_y = fym - k.kdes0 * m2;
-    r.p_x = fxp; r.p_y = fyp + k.kdes1 * m2;
-    r.lam = k.len * maxa;
-    r.active = true;
+    const float same = (mul(d_mid, d_up) >= 0.f) ? 1.f : 0.f;
+    const float m = fabsf(d_mid), u = fabsf(d_up);
+    const float a = fabsf(__fdividef(sub(u, m), add(u, m)));
+    const float v = mul(mul(0.5f, add(u, m)), fma_(-mul(a, a), a, 1.f));
+    const bool big = m > v;
+    const float r = __fdividef(big ? v : m, add(big ? m : v, kEps));
+    const float x = mul(mul(same, r), __fdividef(add(1.f, r), fma_(r, r, 1.f)));
+    return m < kEps ? 1.f : x;
+}
+
+// Blend weight of the 2s flux against the WAF flux (src/GPU/Arista_kernel.cu:208).
+__device__ __forceinline__ float blend_weight(float hij, float hpos, bool no_lim)
+{
+    const float x = __frcp_rn(add(1.f, __expf(mul(-15.f, fma_(-mul(0.5f, hpos), __fdividef(1.f, add(hij, kEps)), 1.f)))));
+    return no_lim ? 0.f : (hij < hpos) ? x : 1.f;
+}
+
+// The two sides of an edge along its normal, low side 0 and high side 1: depth,
+// surface, still-water depth, sqrt(h), discharge and velocity along the normal
+// (velocity: desingularised discharge / h).  A ghost side repeats the cell's
+// with the discharge times the border value; where the ghost is on the low side
+// the edge is computed mirrored: side 0 is the cell, normal -1.
+struct Sides {
+    float h0, h1, e0, e1, D0, D1, s0, s1, u0, u1, t0, t1;
+    float em, ep;          // surface of the cells next to sides 0 and 1
+    float area0, area1, cos0, cos1, len;   // len: x edges len / cos
+    float normal;
+    bool no_lim;           // within two cells of a boundary: first order, no 2s blend
+};
+
+// What both phases form of an edge first: the velocities and discharges without
+// flow into a dry cell above the wet neighbour's surface, the Roe velocity, the
+// wave speeds and the WAF coefficients' limiters.
+struct EdgeWaves {
+    float t0, t1, uij, val, lo, hi, maxa, alr, blr, jump, hij;
+    bool z0, z1, split;
+};
+template <bool X_FUSED>   // the mass flux of x edges fuses the Roe velocity's quotient into the wave speeds
+__device__ __forceinline__ EdgeWaves edge_waves(const Sides &e, float dt, float eps_h)
+{
+    EdgeWaves w;
+    w.z1 = (e.h0 < eps_h) && (-e.e1 > e.D0);
+    w.z0 = (e.h1 < eps_h) && (-e.e0 > e.D1);
+    w.t0 = w.z0 ? 0.f : mul(e.t0, e.normal);
+    w.t1 = w.z1 ? 0.f : mul(e.t1, e.normal);
+    w.hij = mul(0.5f, add(e.h0, e.h1));
+    const float c = sqrt_ap(w.hij);
+    const float num = fma2p(e.s0, w.t0, e.s1, w.t1), den = add(add(e.s0, e.s1), kEps);
+    w.uij = __fdividef(num, den);
+    const float rden = __fdividef(1.f, den);
+    w.val = __fdividef(mul(mul(2.f, e.len), dt), add(e.area0, e.area1));
+    w.lo = fmin_(X_FUSED ? fma_(num, rden, -c) : sub(w.uij, c), sub(w.t0, e.s0));
+    w.hi = fmax_(X_FUSED ? fma_(num, rden, c) : add(w.uij, c), add(w.t1, e.s1));
+    w.maxa = fmax_(fabsf(w.hi), fabsf(w.lo));
+    const float mid = sub(e.e1, e.e0), below = sub(e.e0, e.em), above = sub(e.ep, e.e1), both = mul(0.5f, sub(e.ep, e.em));
+    float xl = limiter_of(mid, (w.lo < 0.f) ? above : (w.lo > 0.f) ? below : both);
+    float xr = limiter_of(mid, (w.hi < 0.f) ? above : (w.hi > 0.f) ? below : both);
+    xl = e.no_lim ? 0.f : xl;
+    xr = e.no_lim ? 0.f : xr;
+    w.split = fabsf(sub(w.lo, w.hi)) >= kEps;
+    w.alr = fma_(mul(w.val, w.lo), xl, mul(sgnf(w.lo), sub(1.f, xl)));
+    w.blr = fma_(mul(w.val, w.hi), xr, mul(sgnf(w.hi), sub(1.f, xr)));
+    w.jump = surface_jump(e.e0, e.e1, e.D0, e.D1);
+    return w;
 }
 
 // ---------------------------------------------------------------------------
-// phase 1: mass flux through one edge (src/GPU/Arista_kernel.cu:118-219 for
-// x edges, 674-778 for y edges).  Returns F; the caller applies it as
-// cell0 -= F (/cos0 for y), cell1 += F (/cos1).
+// phase 1: mass flux through one edge that is not all deep
+// (src/GPU/Arista_kernel.cu:118-219 for x edges, 674-778 for y edges).  Returns
+// F; the caller applies it as cell0 -= F (/cos0 for y), cell1 += F (/cos1).
 // ---------------------------------------------------------------------------
 template <bool LAT>
-__device__ __forceinline__ float mass_flux(Edge &e, const ScenarioDev &s, float dt)
+__device__ __forceinline__ float mass_waf(const Sides &e, float dt, float eps_h, float hpos)
 {
-    if (all_deep(e, s.hpos)) {
-        if (!LAT) return mass_2s_x(e.u0, e.len, e.h0, e.h1, dt, e.area0, e.area1);
-        return mass_2s_y(e.u0, e.len, e.cos0, e.cos1, e.h0, e.h1, dt, e.area0, e.area1);
-    }
-    if (e.front) swap_sides(e);
-    const float h0 = e.h0, h1 = e.h1;
-    if (!((h0 > kEps) || (h1 > kEps))) return 0.f;
-    float q0n = e.u0 * e.normal, q1n = e.u1 * e.normal;
-    const float hij = 0.5f * (h0 + h1);
-    const float c0 = sqrt_ap(hij);
-    if ((h0 < s.eps_h) && (-e.e1 > e.D0)) q1n = 0.f;
-    if ((h1 < s.eps_h) && (-e.e0 > e.D1)) q0n = 0.f;
-    const float u0n = inv_depth(h0, s.eps_h) * q0n;
-    const float u1n = inv_depth(h1, s.eps_h) * q1n;
-    q0n = u0n * h0;
-    q1n = u1n * h1;
-    const float F2s = LAT ? e.len * q0n * e.cos0 * e.normal : e.len * q0n * e.normal;
-    const float s0 = sqrt_ap(h0), s1 = sqrt_ap(h1);
-    const float uijn = (s0 * u0n + s1 * u1n) / (s0 + s1 + kEps);
-    const float val = (2.f * e.len * dt) / (e.area0 + e.area1);
-    const float aut1 = fmin_(uijn - c0, u0n - s0);
-    const float aut2 = fmax_(uijn + c0, u1n + s1);
-    const float maxa = fmax_(fabsf(aut2), fabsf(aut1));
-    float xiL = 0.f, xiR = 0.f;
-    if (!e.no_lim) {
-        xiL = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut1);
-        xiR = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut2);
-    }
-    float a0;
-    if (fabsf(aut1 - aut2) >= kEps) {
-        const float alr = sgnf(aut1) * (1.f - xiL) + val * aut1 * xiL;
-        const float blr = sgnf(aut2) * (1.f - xiR) + val * aut2 * xiR;
-        a0 = (alr - blr) * (aut1 * aut2) / (aut2 - aut1);
-    } else {
-        a0 = maxa;
-    }
-    const float jump = surface_jump(e.e0, e.e1, e.D0, e.D1);
+    const EdgeWaves w = edge_waves<!LAT>(e, dt, eps_h);
+    const float q0 = mul(w.t0, e.h0), q1 = mul(w.t1, e.h1);
+    const float F2s = LAT ? mul(mul(mul(e.len, q0), e.cos0), e.normal) : mul(mul(e.len, q0), e.normal);
+    const float a0 = w.split ? __fdividef(mul(sub(w.alr, w.blr), mul(w.lo, w.hi)), sub(w.hi, w.lo)) : w.maxa;
     float Fwaf;
     if (!LAT) {
-        Fwaf = 0.5f * (q1n + q0n - a0 * jump) * e.len;
+        Fwaf = mul(mul(0.5f, fma_(-a0, w.jump, fma_(w.t1, e.h1, q0))), e.len);
     } else {
-        const float deta = 0.5f * (e.cos0 + e.cos1) * jump - uijn * uijn * (e.cos1 - e.cos0);
-        Fwaf = 0.5f * (q0n * e.cos0 + q1n * e.cos1 - a0 * deta) * e.len;
+        const float deta = fma2m(mul(0.5f, add(e.cos0, e.cos1)), w.jump, mul(w.uij, w.uij), sub(e.cos1, e.cos0));
+        Fwaf = mul(mul(0.5f, fma_(-a0, deta, fma2p(q0, e.cos0, q1, e.cos1))), e.len);
     }
-    const float alfa = blend_2s(hij, s.hpos, e.no_lim);
-    const float F = alfa * F2s + (1.f - alfa) * Fwaf;
-    if (!LAT) return limit_outflow(F, h0, h1, 1.f, 1.f, dt, e.area0, e.area1);
-    return limit_outflow(F, h0, h1, e.cos0, e.cos1, dt, e.area0, e.area1);
+    const float alfa = blend_weight(w.hij, hpos, e.no_lim);
+    const float F = fma2p(alfa, F2s, sub(1.f, alfa), Fwaf);
+    const float Fl = limit_outflow(F, e.h0, e.h1, LAT ? e.cos0 : 1.f, LAT ? e.cos1 : 1.f, dt, e.area0, e.area1);
+    return ((e.h0 > kEps) || (e.h1 > kEps)) ? Fl : 0.f;
 }
 
-// ---------------------------------------------------------------------------
-// phase 2: momentum flux of an x edge (src/GPU/Arista_kernel.cu:221-464).
-// Components are (qx, qy).
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ MomFlux momentum_flux_x(Edge &e, const ScenarioDev &s, float dt)
+// Result of a momentum flux, to be subtracted: components along the normal (n)
+// and the tangent (t) for side 0 and side 1, and the wave-speed term for the
+// time step (added to both).
+struct MomFlux {
+    float n0, t0, n1, t1, lam;
+};
+
+// Edges whose four stencil cells are all deeper than hpos and which lie at
+// least two cells from a boundary: the 2s flux alone (alfa = 1).
+// x edge (src/GPU/Arista_kernel.cu:221-280); rh = 1/h (approximate), sh = sqrt(h),
+// u normal and v tangential discharge, k = the row's constants
+__device__ __forceinline__ MomFlux momentum_2s_x(float h0, float h1, float rh0, float rh1, float s0, float s1, float u0,
+                                                 float u1, float v0, float v1, float jump, const XRowK &k)
 {
     MomFlux r;
-    r.active = true;
-    const float ilcos = e.len;
-    if (all_deep(e, s.hpos)) {
-        momentum_2s_x(r, e.h0, e.h1, rcp_depth(e.h0), rcp_depth(e.h1), sqrt_ap(e.h0), sqrt_ap(e.h1), e.u0, e.u1, e.v0,
-                      e.v1, surface_jump(e.e0, e.e1, e.D0, e.D1), make_xrow(ilcos, e.area0 + e.area1, dt, s.cvis));
-        return r;
-    }
-    if (e.front) swap_sides(e);
-    const float h0 = e.h0, h1 = e.h1;
-    if (!((h0 > kEps) || (h1 > kEps))) { r.active = false; return r; }
-    float w0 = e.u0 * e.normal, w1 = e.u1 * e.normal;
-    const float hij = 0.5f * (h0 + h1);
-    if ((h0 < s.eps_h) && (-e.e1 > e.D0)) w1 = 0.f;
-    if ((h1 < s.eps_h) && (-e.e0 > e.D1)) w0 = 0.f;
-    const float h0rg = inv_depth(h0, s.eps_h), h1rg = inv_depth(h1, s.eps_h);
-    float u0n = h0rg * w0, u1n = h1rg * w1;
-    w0 = u0n * h0;
-    w1 = u1n * h1;
-    const float s0 = sqrt_ap(h0), s1 = sqrt_ap(h1);
-    float uijn = (s0 * u0n + s1 * u1n) / (s0 + s1 + kEps);
-    const float val = (2.f * ilcos * dt) / (e.area0 + e.area1);
-    const float c0 = sqrt_ap(hij);
-    const float aut1 = fmin_(uijn - c0, u0n - s0);
-    const float aut2 = fmax_(uijn + c0, u1n + s1);
-    float maxa = fmax_(fabsf(aut2), fabsf(aut1));
-    const float fl1x = w1, fl1y = u1n * w1, fl0x = w0, fl0y = u0n * w0;
-    const float dq = fl1x - fl0x;
-    const float deta = surface_jump(e.e0, e.e1, e.D0, e.D1);
-    float s_my, s_py, s_mz, s_pz;
-    if (uijn < 0.f) {
-        s_my = u1n * w1 * ilcos * e.normal; s_py = -s_my; s_my += hij * deta * ilcos;
-        s_mz = u1n * e.v1 * ilcos; s_pz = -s_mz;
-    } else {
-        s_my = u0n * w0 * ilcos * e.normal; s_py = -s_my; s_my += hij * deta * ilcos;
-        s_mz = u0n * e.v0 * ilcos; s_pz = -s_mz;
-    }
-    const float cd = 0.5f * (1.f - s.cvis / (1.f + __expf(-20.f * (1.f - s.hpos / hij))));
-    const float des = cd * val * maxa * maxa * dq * ilcos * e.normal;
-    s_my -= des;
-    s_py += des;
-    float xiL = 0.f, xiR = 0.f;
-    if (!e.no_lim) {
-        xiL = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut1);
-        xiR = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut2);
-    }
-    float a0, a1;
-    if (fabsf(aut1 - aut2) >= kEps) {
-        const float alr = sgnf(aut1) * (1.f - xiL) + val * aut1 * xiL;
-        const float blr = sgnf(aut2) * (1.f - xiR) + val * aut2 * xiR;
-        const float aux = 1.f / (aut2 - aut1);
-        a0 = (alr - blr) * (aut1 * aut2) * aux;
-        a1 = (blr * aut2 - alr * aut1) * aux;
-    } else {
-        a0 = maxa;
-        a1 = 0.f;
-    }
-    float mx = 0.5f * dq, px = mx;
-    float my = 0.5f * (fl1y - fl0y + hij * deta), py = my;
-    const float desx = 0.5f * a0 * deta, desy = 0.5f * a0 * dq + a1 * my;
-    mx += fl0x - desx; my += fl0y - desy;
-    px += desx - fl1x; py += desy - fl1y;
-    mx *= ilcos; my *= ilcos; px *= ilcos; py *= ilcos;
-    // transverse momentum carried with a limited tangential velocity
-    const float q0mt = e.v0m * e.normal, q0t = e.v0 * e.normal, q1t = e.v1 * e.normal, q1pt = e.v1p * e.normal;
-    const float p0m = inv_depth(e.h0m, s.eps_h) * q0mt;
-    const float p1p = inv_depth(e.h1p, s.eps_h) * q1pt;
-    u0n = h0rg * q0t;
-    u1n = h1rg * q1t;
-    const float sg = -1.f * (mx < 0.f) + 1.f * (mx > 0.f);
-    uijn = fabsf(uijn) * sg;
-    const float xit = e.no_lim ? 0.f : monotone_limiter(p0m, u0n, u1n, p1p, uijn);
-    const float uijt = 0.5f * (u0n + u1n) - 0.5f * ((1.f - xit) * sg + xit * uijn * val) * (u1n - u0n);
-    const float aux = mx * uijt;
-    const float t_py = py * e.normal, t_pz = -aux * e.normal, t_my = my * e.normal, t_mz = aux * e.normal;
-    const float alfa = blend_2s(hij, s.hpos, e.no_lim);
-    r.m_x = alfa * s_my + (1.f - alfa) * t_my;
-    r.m_y = alfa * s_mz + (1.f - alfa) * t_mz;
-    r.p_x = alfa * s_py + (1.f - alfa) * t_py;
-    r.p_y = alfa * s_pz + (1.f - alfa) * t_pz;
-    if (maxa < s.eps_h) maxa += s.eps_h;
-    r.lam = ilcos * maxa;
+    const float hij = mul(0.5f, add(h0, h1));
+    const float u0n = mul(u0, rh0), u1n = mul(u1, rh1);
+    const float uij = __fdividef(fma2p(s0, u0n, s1, u1n), add(add(s0, s1), kEps));
+    const float maxa = add(fabsf(uij), sqrt_ap(hij));
+    const bool neg = uij < 0.f;
+    const float un = neg ? u1n : u0n, uu = neg ? u1 : u0, vv = neg ? v1 : v0;
+    const float m = mul(mul(un, uu), k.ilcos);
+    const float c = mul(k.kdes, mul(maxa, maxa)), du = sub(u1, u0);
+    r.n0 = fma_(-c, du, fma_(mul(hij, jump), k.ilcos, m));
+    r.n1 = fma_(c, du, -m);
+    r.t0 = mul(mul(un, vv), k.ilcos);
+    r.t1 = -r.t0;
+    r.lam = mul(k.ilcos, maxa);
+    return r;
+}
+
+// y edge (src/GPU/Arista_kernel.cu:780-843); k = the constants of its row pair
+__device__ __forceinline__ MomFlux momentum_2s_y(float h0, float h1, float rh0, float rh1, float s0, float s1, float u0,
+                                                 float u1, float v0, float v1, float jump, const YRowK &k)
+{
+    MomFlux r;
+    const float hij = mul(0.5f, add(h0, h1));
+    const float u0n = mul(u0, rh0), u1n = mul(u1, rh1);
+    const float uij = __fdividef(fma2p(s0, u0n, s1, u1n), add(add(s0, s1), kEps));
+    const float maxa = add(fabsf(uij), sqrt_ap(hij));
+    const float deta = fma2m(k.cmid, jump, mul(uij, uij), k.cdiff);
+    const float g = mul(hij, deta);
+    const float m2 = mul(mul(maxa, maxa), fma2m(u1, k.cos1, u0, k.cos0));
+    const bool neg = uij < 0.f;
+    const float un = neg ? u1n : u0n, uu = neg ? u1 : u0, vv = neg ? v1 : v0;
+    const float f = mul(mul(un, uu), k.len);
+    // (a factor 1 leaves a product as it is)
+    r.n0 = fma_(-k.kdes0, m2, fma2p(g, k.li0, f, neg ? k.c10 : 1.f));
+    r.n1 = fma2p(k.kdes1, m2, -f, neg ? 1.f : k.c01);
+    r.t0 = mul(mul(un, vv), k.len);
+    r.t1 = -r.t0;
+    r.lam = mul(k.len, maxa);
     return r;
 }
 
 // ---------------------------------------------------------------------------
-// phase 2: momentum flux of a y edge (src/GPU/Arista_kernel.cu:780-1026).
-// Edge "u" is qy, "v" is qx; components returned as (qx, qy).
+// phase 2: momentum flux of an edge that is not all deep
+// (src/GPU/Arista_kernel.cu:282-464 for x edges, 845-1026 for y edges).  v0, v1:
+// tangential discharges; pm, p0, p1, pp: tangential velocities of the four
+// stencil cells.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ MomFlux momentum_flux_y(Edge &e, const ScenarioDev &s, float dt)
+template <bool LAT>
+__device__ __forceinline__ MomFlux momentum_waf(const Sides &e, float v0, float v1, float pm, float p0, float p1, float pp,
+                                                float icos0, float icos1, float dt, float eps_h, float hpos, float cvis)
 {
     MomFlux r;
-    r.active = true;
-    const float len = e.len;
-    if (all_deep(e, s.hpos)) {
-        momentum_2s_y(r, e.h0, e.h1, rcp_depth(e.h0), rcp_depth(e.h1), sqrt_ap(e.h0), sqrt_ap(e.h1), e.u0, e.u1, e.v0,
-                      e.v1, surface_jump(e.e0, e.e1, e.D0, e.D1),
-                      make_yrow(e.cos0, e.cos1, __frcp_rn(e.cos0), __frcp_rn(e.cos1), len, e.area0 + e.area1, dt,
-                                s.cvis));
-        return r;
-    }
-    if (e.front) swap_sides(e);
-    const float h0 = e.h0, h1 = e.h1;
-    if (!((h0 > kEps) || (h1 > kEps))) { r.active = false; return r; }
-    const float icos0 = __frcp_rn(e.cos0), icos1 = __frcp_rn(e.cos1);
-    float w0 = e.u0 * e.normal, w1 = e.u1 * e.normal;
-    const float hij = 0.5f * (h0 + h1);
-    const float c0 = sqrt_ap(hij);
-    if ((h0 < s.eps_h) && (-e.e1 > e.D0)) w1 = 0.f;
-    if ((h1 < s.eps_h) && (-e.e0 > e.D1)) w0 = 0.f;
-    const float h0rg = inv_depth(h0, s.eps_h), h1rg = inv_depth(h1, s.eps_h);
-    float u0n = h0rg * w0, u1n = h1rg * w1;
-    const float s0 = sqrt_ap(h0), s1 = sqrt_ap(h1);
-    float uijn = (s0 * u0n + s1 * u1n) / (s0 + s1 + kEps);
-    const float val = (2.f * len * dt) / (e.area0 + e.area1);
-    const float aut1 = fmin_(uijn - c0, u0n - s0);
-    const float aut2 = fmax_(uijn + c0, u1n + s1);
-    float maxa = fmax_(fabsf(aut2), fabsf(aut1));
-    const float deta = 0.5f * (e.cos0 + e.cos1) * surface_jump(e.e0, e.e1, e.D0, e.D1) - uijn * uijn * (e.cos1 - e.cos0);
-    float s_mz, s_pz, s_my, s_py;
-    if (uijn < 0.f) {
-        s_mz = u1n * w1 * len * e.normal; s_pz = -s_mz; s_mz *= e.cos1 * icos0; s_mz += hij * deta * len * icos0;
-        s_my = u1n * e.v1 * len; s_py = -s_my;
+    const EdgeWaves w = edge_waves<false>(e, dt, eps_h);
+    const float n = e.normal;
+    const float w0 = LAT ? (w.z0 ? 0.f : mul(e.u0, n)) : mul(w.t0, e.h0);
+    const float w1 = LAT ? (w.z1 ? 0.f : mul(e.u1, n)) : mul(w.t1, e.h1);
+    const float deta = LAT ? fma2m(mul(0.5f, add(e.cos0, e.cos1)), w.jump, mul(w.uij, w.uij), sub(e.cos1, e.cos0)) : w.jump;
+    const bool neg = w.uij < 0.f;
+    const float un = neg ? w.t1 : w.t0;
+    const float s = mul(mul(mul(un, neg ? w1 : w0), e.len), n);
+    const float f0 = LAT ? mul(w0, e.cos0) : w0, f1 = LAT ? mul(w1, e.cos1) : w1;
+    const float g0 = mul(w.t0, f0), g1 = mul(w.t1, f1);
+    const float dq = sub(f1, f0);
+    const float ex = add(1.f, __expf(mul(-20.f, fma_(-hpos, __fdividef(1.f, w.hij), 1.f))));
+    const float cd = mul(0.5f, fma_(-cvis, __fdividef(1.f, ex), 1.f));
+    const float des = mul(mul(mul(mul(mul(cd, w.val), w.maxa), w.maxa), dq), e.len);
+    float sn0, sn1;
+    if (!LAT) {
+        sn0 = sub(fma_(mul(w.hij, deta), e.len, s), mul(des, n));
+        sn1 = add(-s, mul(des, n));
     } else {
-        s_mz = u0n * w0 * len * e.normal; s_pz = -s_mz * e.cos0 * icos1; s_mz += hij * deta * len * icos0;
-        s_my = u0n * e.v0 * len; s_py = -s_my;
+        const float grav = mul(mul(w.hij, deta), e.len);
+        sn0 = fma_(-des, icos0, fma_(grav, icos0, neg ? mul(s, mul(e.cos1, icos0)) : s));
+        sn1 = fma_(des, icos1, neg ? -s : mul(mul(-s, e.cos0), icos1));
     }
-    const float cd = 0.5f * (1.f - s.cvis / (1.f + __expf(-20.f * (1.f - s.hpos / hij))));
-    const float fl1x = w1 * e.cos1, fl1y = u1n * fl1x, fl0x = w0 * e.cos0, fl0y = u0n * fl0x;
-    const float dq = fl1x - fl0x;
-    const float des = cd * val * maxa * maxa * dq * len;
-    s_mz -= des * icos0;
-    s_pz += des * icos1;
-    float xiL = 0.f, xiR = 0.f;
-    if (!e.no_lim) {
-        xiL = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut1);
-        xiR = monotone_limiter(e.e0m, e.e0, e.e1, e.e1p, aut2);
-    }
-    float a0, a1;
-    if (fabsf(aut1 - aut2) >= kEps) {
-        const float alr = sgnf(aut1) * (1.f - xiL) + val * aut1 * xiL;
-        const float blr = sgnf(aut2) * (1.f - xiR) + val * aut2 * xiR;
-        const float aux = 1.f / (aut2 - aut1);
-        a0 = (alr - blr) * (aut1 * aut2) * aux;
-        a1 = (blr * aut2 - alr * aut1) * aux;
-    } else {
-        a0 = maxa;
-        a1 = 0.f;
-    }
-    float mx = 0.5f * dq, px = mx;
-    float my = 0.5f * (fl1y - fl0y + hij * deta), py = my;
-    const float desx = 0.5f * a0 * deta, desy = 0.5f * a0 * dq + a1 * my;
-    mx += fl0x - desx; my += fl0y - desy;
-    px += desx - fl1x; py += desy - fl1y;
-    mx *= len; my *= len; px *= len; py *= len;
-    const float q0mt = -e.v0m * e.normal, q0t = -e.v0 * e.normal, q1t = -e.v1 * e.normal, q1pt = -e.v1p * e.normal;
-    const float p0m = inv_depth(e.h0m, s.eps_h) * q0mt;
-    const float p1p = inv_depth(e.h1p, s.eps_h) * q1pt;
-    u0n = h0rg * q0t;
-    u1n = h1rg * q1t;
-    const float sg = -1.f * (mx < 0.f) + 1.f * (mx > 0.f);
-    uijn = fabsf(uijn) * sg;
-    const float xit = e.no_lim ? 0.f : monotone_limiter(p0m, u0n, u1n, p1p, uijn);
-    const float uijt = 0.5f * (u0n * icos0 + u1n * icos1) -
-                       0.5f * ((1.f - xit) * sg + xit * uijn * val) * (u1n * icos1 - u0n * icos0);
-    const float aux = mx * uijt;
-    const float t_py = aux * e.normal, t_pz = py * e.normal * icos1;
-    const float t_my = -aux * e.normal, t_mz = my * e.normal * icos0;
-    if (maxa < s.eps_h) maxa += s.eps_h;
-    const float alfa = blend_2s(hij, s.hpos, e.no_lim);
-    r.m_x = alfa * s_my + (1.f - alfa) * t_my;
-    r.m_y = alfa * s_mz + (1.f - alfa) * t_mz;
-    r.p_x = alfa * s_py + (1.f - alfa) * t_py;
-    r.p_y = alfa * s_pz + (1.f - alfa) * t_pz;
-    r.lam = len * maxa;
+    const float st = mul(mul(un, neg ? v1 : v0), e.len);
+    const float aux = __fdividef(1.f, sub(w.hi, w.lo));
+    const float a0 = w.split ? mul(mul(sub(w.alr, w.blr), mul(w.lo, w.hi)), aux) : w.maxa;
+    const float a1 = w.split ? mul(fma2m(w.blr, w.hi, w.alr, w.lo), aux) : 0.f;
+    const float hm = mul(0.5f, dq), hn = mul(0.5f, add(sub(g1, g0), mul(w.hij, deta)));
+    const float ha = mul(0.5f, a0);
+    const float dn = fma2p(ha, dq, a1, hn);
+    const float mx = mul(add(hm, fma_(-ha, deta, f0)), e.len);
+    const float my = mul(add(hn, sub(g0, dn)), e.len);
+    const float py = mul(add(hn, sub(dn, g1)), e.len);
+    // transverse momentum carried with a limited tangential velocity
+    const float sg = LAT ? -n : n;
+    const float ym = mul(pm, sg), y0 = mul(p0, sg), y1 = mul(p1, sg), yp = mul(pp, sg);
+    const float side = sgnf(mx);
+    const float speed = mul(fabsf(w.uij), side);
+    const float up = (speed < 0.f) ? sub(yp, y1) : (speed > 0.f) ? sub(y0, ym) : mul(0.5f, sub(yp, ym));
+    const float xi = e.no_lim ? 0.f : limiter_of(sub(y1, y0), up);
+    const float coef = add(mul(sub(1.f, xi), side), mul(mul(xi, speed), w.val));
+    const float sum = LAT ? fma2p(y0, icos0, y1, icos1) : add(y0, y1);
+    const float dif = LAT ? fma2n(y1, icos1, y0, icos0) : sub(y1, y0);
+    const float ut = sub(mul(0.5f, sum), mul(mul(0.5f, coef), dif));
+    const float tt = mul(mul(mx, ut), sg);
+    const float alfa = blend_weight(w.hij, hpos, e.no_lim), be = sub(1.f, alfa);
+    const float tn0 = LAT ? mul(mul(my, n), icos0) : mul(my, n), tn1 = LAT ? mul(mul(py, n), icos1) : mul(py, n);
+    r.n0 = fma2p(alfa, sn0, be, tn0);
+    r.n1 = fma2p(alfa, sn1, be, tn1);
+    r.t0 = fma2q(alfa, st, be, tt);
+    r.t1 = -r.t0;
+    r.lam = mul(e.len, (w.maxa < eps_h) ? add(w.maxa, eps_h) : w.maxa);
+    const bool wet = (e.h0 > kEps) || (e.h1 > kEps);
+    r.n0 = wet ? r.n0 : 0.f;
+    r.n1 = wet ? r.n1 : 0.f;
+    r.t0 = wet ? r.t0 : 0.f;
+    r.t1 = wet ? r.t1 : 0.f;
+    r.lam = wet ? r.lam : 0.f;
     return r;
 }
 

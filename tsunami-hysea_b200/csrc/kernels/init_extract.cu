@@ -135,74 +135,9 @@ __global__ void __launch_bounds__(kControllerThreads) controller_kernel(const Sc
         ScenarioCtl *cp = s.ctl;
         if (cp && cp->status == kRunning) {
             ScenarioCtl c = *cp;
-            const float dmin = __uint_as_float(c.dt_bits);
-            const unsigned errs = c.errors;
-            c.t += c.dt;
-            double dt = (double)dmin;
-            // truncation so that t lands on the next fault time
-            const int nf = c.nfaults;
-            const int f = c.fault_next;
-            const double *tf = c.fault_times;
-            if (!c.jumping) {
-                if (f < nf && (c.t + dt) * c.T > tf[f]) {
-                    dt = tf[f] / c.T - c.t;
-                    c.jumping = 1;
-                }
-            } else {
-                c.jumping = 0;
-                if (f < nf) {
-                    int i = f + 1;
-                    while (i < nf && !(fabs(tf[i] - tf[f]) > 2.220446049250313e-16)) i++;
-                    if (i < nf && (c.t + dt) * c.T > tf[i]) {
-                        dt = tf[i] / c.T - c.t;
-                        c.jumping = 1;
-                    }
-                }
-            }
-            c.dt = dt;
-            c.step += 1;
-            c.parity ^= 1;
-            c.dt_bits = 0x7f7fffffu;
-            c.tiles_done = 0u;
-            int ev = 0;
-            if (errs || !(dmin > 0.f) || isnan(dmin)) {
-                c.status = kFailed;
-            } else if (!(c.t < c.t_end)) {
-                c.status = kDone;
-            } else if (c.max_steps >= 0 && c.step >= c.max_steps) {
-                c.events = kEvStepBudget;
-                c.status = kDone;
-            } else {
-                if (f < nf && c.t * c.T >= tf[f]) ev |= kEvFault;
-                if (c.save_nc >= 0.0 && c.t >= c.next_nc) ev |= kEvSnapshot;
-                if (c.save_ts >= 0.0 && c.t >= c.next_ts) {
-                    if (s.ngauges > 0 && !(ev & kEvFault)) {
-                        // the loop's gauge event on the device: same time test
-                        // and interval update as the host's
-                        s_sample = (int)(c.gauge_count % kGaugeRing);
-                        s.gauge_ring_t[s_sample] = c.t * c.T;
-                        c.next_ts += c.save_ts;
-                        c.gauge_count += 1;
-                    } else {
-                        ev |= kEvSeries;
-                    }
-                }
-                if (ev) {
-                    c.events = ev;
-                    c.status = kPaused;
-                }
-            }
-            cp->t = c.t;
-            cp->dt = c.dt;
-            cp->step = c.step;
-            cp->parity = c.parity;
-            cp->jumping = c.jumping;
-            cp->dt_bits = c.dt_bits;
-            cp->tiles_done = c.tiles_done;
-            cp->events = c.events;
-            cp->status = c.status;
-            cp->next_ts = c.next_ts;
-            cp->gauge_count = c.gauge_count;
+            s_sample = advance_scenario(c, s, __uint_as_float(c.dt_bits), c.errors);
+            if (s_sample >= 0) s.gauge_ring_t[s_sample] = c.t * c.T;
+            store_advanced(cp, c);
             s_parity = c.parity;
         }
     }

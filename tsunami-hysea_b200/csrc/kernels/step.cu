@@ -23,10 +23,10 @@
 // Phase 0 (the general kernel's arithmetic, one unit per CTA) computes the
 // initial dt.
 //
-// Row marching (general kernel): a unit is 4 column strips side by side, each
+// Row marching (general kernel, step_parts.cuh): a unit is 4 column strips side by side, each
 // in row groups (a tiling: 1, 2 or 8), and each (strip, row group) is a task
 // of one warp, claimed independently of the others; each lane owns one
-// column and the warp marches down its rows keeping a five-row window of its
+// column and the warp marches down its rows keeping a four-row window of its
 // column in registers.  The y edge below the current
 // row needs nothing but that window; x edges take their left/right
 // neighbours from warp shuffles.  The 32 lanes cover 28 output columns plus
@@ -41,328 +41,13 @@
 // Reference: src/GPU/Timestep.cu:11-120 (launch sequence),
 // src/GPU/Arista_kernel.cu (edge fluxes), src/GPU/Volumen_kernel.cu (cell
 // updates), src/GPU/Reduccion_kernel.cu (dt min).
-#include "device.cuh"
-#include "kernels.h"
+#include "step_parts.cuh"
 
 #include <algorithm>
 #include <type_traits>
 #include <cfloat>
 
 namespace thy {
-
-constexpr int STRIPS = kStepThreads / 32;   // column strips of a tile
-constexpr int OUTW = 28;              // output columns per strip
-constexpr int TY = kTileY;            // output rows per tile
-static_assert(kTileX == STRIPS * OUTW, "tile width = strips x 28 columns");
-static_assert(STRIPS == 4, "deep and general kernels: 4 column-strip warps per row group");
-
-// one cell of a lane's column: depth, surface elevation, still-water depth, discharges
-struct Cell {
-    float h, e, D, qx, qy;
-};
-
-// Column of a loaded cell: periodic wrap or clamp (src/GPU/Arista_kernel.cu:6-21).
-// Halo lanes beyond the grid load a valid column (modulo / clamp); only the
-// columns the reference would read are used by an edge.
-__device__ __forceinline__ int map_col(int gx, int nx, int periodic)
-{
-    if (gx >= 0 && gx < nx) return gx;
-    if (periodic) {
-        const int m = gx % nx;
-        return m < 0 ? m + nx : m;
-    }
-    return gx < 0 ? 0 : nx - 1;
-}
-
-__device__ __forceinline__ int clamp_row(int gy, int ny) { return gy < 0 ? 0 : (gy >= ny ? ny - 1 : gy); }
-
-__device__ __forceinline__ Cell load_cell(const float *__restrict__ eta, const float *__restrict__ dep,
-                                          const float *__restrict__ qx, const float *__restrict__ qy, size_t idx)
-{
-    Cell c;
-    c.e = __ldg(eta + idx);
-    c.D = __ldg(dep + idx);
-    c.qx = __ldg(qx + idx);
-    c.qy = __ldg(qy + idx);
-    c.h = c.e + c.D;
-    return c;
-}
-
-// raw loads of a row that is still in flight (prefetch two rows ahead); in
-// phase 1 also the cell's max-height / arrival-time / initial-surface values
-struct RawCell {
-    float e, D, qx, qy;
-    float em, ar, ei;
-};
-
-template <bool DIAG>
-__device__ __forceinline__ RawCell load_raw(const ScenarioDev &s, const float *__restrict__ eta,
-                                            const float *__restrict__ qx, const float *__restrict__ qy, size_t idx,
-                                            bool diag)
-{
-    RawCell r;
-    r.e = __ldg(eta + idx);
-    r.D = __ldg(s.dep + idx);
-    r.qx = __ldg(qx + idx);
-    r.qy = __ldg(qy + idx);
-    r.em = r.ar = r.ei = 0.f;
-    if (DIAG && diag) {
-        r.em = s.eta_max[idx];
-        r.ar = s.arr[idx];
-        r.ei = __ldg(s.eta_ini + idx);
-    }
-    return r;
-}
-
-// Max-height / arrival-time update of one cell from the state the step starts
-// from (src/GPU/Metrics.cu:23-77).
-__device__ __forceinline__ void diagnostics(const ScenarioDev &s, const RawCell &r, size_t idx, float t_sec)
-{
-    const float h = r.e + r.D;
-    if (r.e > r.em && h > s.eps_h) s.eta_max[idx] = r.e;
-    if (r.ar < 0.f && fabsf(r.e - r.ei) > s.dif_at) s.arr[idx] = t_sec;
-}
-
-__device__ __forceinline__ Cell finish(const RawCell &r)
-{
-    Cell c;
-    c.e = r.e;
-    c.D = r.D;
-    c.qx = r.qx;
-    c.qy = r.qy;
-    c.h = r.e + r.D;
-    return c;
-}
-
-__device__ __forceinline__ float shup(float v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-__device__ __forceinline__ float shdn(float v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
-
-// Wave-speed term of one edge for the initial dt (src/GPU/Arista_kernel.cu:1237-1280);
-// x edges carry len/cos in e.len.
-__device__ __forceinline__ float initial_speed(Edge &e, const ScenarioDev &s)
-{
-    if (e.front) {
-        swapf(e.h0, e.h1);
-        swapf(e.u0, e.u1);
-    }
-    const float w0 = e.u0 * e.normal, w1 = e.u1 * e.normal;
-    const float h0 = e.h0, h1 = e.h1, hij = 0.5f * (h0 + h1);
-    const float u0n = inv_depth(h0, s.eps_h) * w0, u1n = inv_depth(h1, s.eps_h) * w1;
-    const float s0 = sqrt_ap(h0), s1 = sqrt_ap(h1);
-    const float uij = (s0 * u0n + s1 * u1n) / (s0 + s1 + kEps);
-    float maxa = fabsf(uij) + sqrt_ap(hij);
-    if (maxa < s.eps_h) maxa += s.eps_h;
-    return e.len * maxa;
-}
-
-// Edge between rows gy-1 (a) and gy (b) of this lane's column, stencil rows
-// gy-2 .. gy+1 = (m, a, b, p).  "u" is qy (normal), "v" qx (tangential).
-// ka, kb: row metrics {cos, ilcos, area, dlon} of rows clamp(gy-1) and
-// clamp(gy); dlon: the edge row's length (rowpack[gy].w).
-__device__ __forceinline__ void gather_y(Edge &e, const ScenarioDev &s, const Cell &m, const Cell &a, const Cell &b,
-                                         const Cell &p, int gy, const float4 &ka, const float4 &kb, float dlon)
-{
-    e.h0m = m.h; e.h0 = a.h; e.h1 = b.h; e.h1p = p.h;
-    e.e0m = m.e; e.e0 = a.e; e.e1 = b.e; e.e1p = p.e;
-    e.D0 = a.D; e.D1 = b.D;
-    e.u0m = m.qy; e.u0 = a.qy; e.u1 = b.qy; e.u1p = p.qy;
-    e.v0m = m.qx; e.v0 = a.qx; e.v1 = b.qx; e.v1p = p.qx;
-    e.area0 = ka.z; e.cos0 = ka.x;
-    e.area1 = kb.z; e.cos1 = kb.x;
-    e.len = dlon;
-    e.normal = 1.f;
-    e.front = false;
-    if (gy == 0) {
-        e.u0 *= s.b_up;
-        e.normal = -1.f;
-        e.front = true;
-    }
-    if (gy == s.ny) e.u1 *= s.b_low;
-    e.no_lim = (gy < 2) || (gy > s.ny - 2);
-}
-
-// contributions of an edge to the cell on its low side (lo) and high side (hi):
-// {mass or qx, qy, lambda}
-struct Contrib {
-    float a, b, lam;
-};
-
-template <int PHASE>
-__device__ __forceinline__ void y_edge(const ScenarioDev &s, const Cell &m, const Cell &a, const Cell &b, const Cell &p,
-                                       int gy, float dt, Contrib &lo, Contrib &hi, const float4 &ka, const float4 &kb,
-                                       float dlon)
-{
-    Edge e;
-    gather_y(e, s, m, a, b, p, gy, ka, kb, dlon);
-    const bool ghost_lo = (gy == 0);
-    if (PHASE == 1) {
-        const float F = mass_flux<true>(e, s, dt);
-        lo = {-F / e.cos0, 0.f, 0.f};
-        // top ghost: the boundary cell is the low side of the mirrored edge
-        hi = ghost_lo ? Contrib{-F / e.cos0, 0.f, 0.f} : Contrib{F / e.cos1, 0.f, 0.f};
-    } else if (PHASE == 2) {
-        MomFlux f = momentum_flux_y(e, s, dt);
-        if (!f.active) { f.m_x = f.m_y = f.p_x = f.p_y = f.lam = 0.f; }
-        lo = {-f.m_x, -f.m_y, f.lam};
-        hi = ghost_lo ? lo : Contrib{-f.p_x, -f.p_y, f.lam};
-    } else {
-        const float lam = initial_speed(e, s);
-        lo = {0.f, 0.f, lam};
-        hi = lo;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Work units and their classes.  A unit is a half tile (kTileX x kHalfRows
-// cells; tile column tx starts at grid column x_org + tx kTileX, so tile 0
-// and the last tile may hold fewer columns); work-list entry w (scenario,
-// tile) holds units 2w (upper half) and 2w+1 (lower half).  Phase 1 records each unit's depth summary (UnitSum);
-// from the unit's own cells and the border strips and corners of its eight
-// neighbours - exactly its two-cell stencil ring -
-//   deep:  every cell of unit and ring deeper than hpos, and the unit at
-//          least two cells from the boundaries and outside the sponge
-//          layers - every edge is a pure 2s edge and no cell is dried,
-//          damped or relaxed;
-//   dry:   every cell of unit and ring dry (depth 0) at three consecutive
-//          classifications - then both state buffers hold the scheme's
-//          fixed point (eta = -dep, q = 0), which a step would write again,
-//          so the unit is skipped;
-//   general: the rest.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ int units_y(const ScenarioDev &s) { return (s.ny + kHalfRows - 1) / kHalfRows; }
-
-// The geometric tests imply 1 <= tx <= tiles_x - 2 and 1 <= uy <= units_y - 2.
-// *hmin: the smallest depth over the unit and its two-cell ring (when deep).
-__device__ __forceinline__ bool unit_deep(const ScenarioDev &s, const UnitSum *__restrict__ sum, int tx, int uy,
-                                          float *hmin)
-{
-    if (!s.tmap) return false;
-    const int x0 = s.x_org + tx * kTileX, yb = uy * kHalfRows;
-    if (x0 < max(2, s.sp_left) || x0 + kTileX > s.nx - max(2, s.sp_right)) return false;
-    if (yb < max(2, s.sp_up) || yb + kHalfRows > s.ny - max(2, s.sp_low)) return false;
-    const int W = s.tiles_x;
-    const UnitSum *c = sum + (size_t)uy * W + tx;
-    const float hp = s.hpos;
-    // all nine loads first and no short-circuit, so that they are in flight
-    // together (a NaN, an unknown summary, fails its test as before)
-    const float v0 = c->all.x, v1 = c[-1].R.x, v2 = c[1].L.x, v3 = c[-W].B.x, v4 = c[W].T.x;
-    const float v5 = c[-W - 1].BR.x, v6 = c[-W + 1].BL.x, v7 = c[W - 1].TR.x, v8 = c[W + 1].TL.x;
-    *hmin = fminf(fminf(fminf(v0, v1), fminf(v2, v3)), fminf(fminf(v4, v5), fminf(fminf(v6, v7), v8)));
-    return (v0 > hp) & (v1 > hp) & (v2 > hp) & (v3 > hp) & (v4 > hp) & (v5 > hp) & (v6 > hp) & (v7 > hp) & (v8 > hp);
-}
-
-// Deep-list entries: the unit code (2 x work-list index + half) and, in bit
-// kJumpPlain, whether every surface jump of the unit's edges in the state
-// the list was made for is the plain difference of the elevations (its unit
-// and ring deeper than unit_gmax, with a margin for the FP32 rounding of the
-// test itself).
-constexpr int kJumpPlain = 30;
-__device__ __forceinline__ int unit_code(int entry) { return entry & ((1 << kJumpPlain) - 1); }
-__device__ __forceinline__ bool jump_plain(int entry) { return (entry >> kJumpPlain) & 1; }
-
-// Outside the grid counts as dry (ghost cells copy the boundary cell), except
-// across a periodic x boundary, where the wrapped unit counts.
-__device__ __forceinline__ bool unit_dry(const ScenarioDev &s, const UnitSum *__restrict__ sum, int tx, int uy)
-{
-    const int ny_u = units_y(s), nx_u = s.tiles_x;
-    bool dry = true;
-    // every neighbour's load issued without waiting for the previous test
-#pragma unroll
-    for (int dy = -1; dy <= 1; dy++) {
-        const int y = uy + dy;
-        if (y < 0 || y >= ny_u) continue;
-#pragma unroll
-        for (int dx = -1; dx <= 1; dx++) {
-            int x = tx + dx;
-            if (x < 0 || x >= nx_u) {
-                if (!s.periodic) continue;
-                x = (x + nx_u) % nx_u;
-            }
-            const UnitSum &u = sum[(size_t)y * nx_u + x];
-            // the part of neighbour (dx, dy) inside the ring
-            const float2 v = (dx == 0 && dy == 0) ? u.all
-                           : (dy == 0) ? (dx < 0 ? u.R : u.L)
-                           : (dx == 0) ? (dy < 0 ? u.B : u.T)
-                           : (dy < 0) ? (dx < 0 ? u.BR : u.BL)
-                                      : (dx < 0 ? u.TR : u.TL);
-            dry &= (v.y <= 0.f);
-        }
-    }
-    return dry;
-}
-
-// Per-lane depth accumulators of a unit: every row, the unit's first two
-// rows and its last two rows.
-struct DepthAcc {
-    float amin, amax, tmin, tmax, bmin, bmax;
-    __device__ __forceinline__ void init()
-    {
-        amin = tmin = bmin = FLT_MAX;
-        amax = tmax = bmax = -FLT_MAX;
-    }
-    __device__ __forceinline__ void add(float h, bool top, bool bot)
-    {
-        amin = fminf(amin, h);
-        amax = fmaxf(amax, h);
-        if (top) { tmin = fminf(tmin, h); tmax = fmaxf(tmax, h); }
-        if (bot) { bmin = fminf(bmin, h); bmax = fmaxf(bmax, h); }
-    }
-};
-
-// {min, max} over the lanes of a warp that are members
-__device__ __forceinline__ float2 warp_minmax(float mn, float mx, bool member)
-{
-    if (!member) {
-        mn = FLT_MAX;
-        mx = -FLT_MAX;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    return make_float2(mn, mx);
-}
-
-// The nine {min, max} of one warp for the unit summary: lanes in the unit's
-// first two / last two columns (is_l / is_r); every field of a warp without
-// such cells is the empty value.  Written to slot[0..8] in UnitSum order.
-__device__ __forceinline__ void warp_unit_summary(const DepthAcc &a, bool cell, bool is_l, bool is_r, float2 *slot)
-{
-    // rows / columns a warp holds no cell of are skipped (warp-uniform tests)
-    const float2 none = make_float2(FLT_MAX, -FLT_MAX);
-    const bool has_t = __any_sync(0xffffffffu, cell && a.tmin != FLT_MAX);
-    const bool has_b = __any_sync(0xffffffffu, cell && a.bmin != FLT_MAX);
-    const bool has_l = __any_sync(0xffffffffu, is_l), has_r = __any_sync(0xffffffffu, is_r);
-    const float2 all = warp_minmax(a.amin, a.amax, cell);
-    const float2 top = has_t ? warp_minmax(a.tmin, a.tmax, cell) : none;
-    const float2 bot = has_b ? warp_minmax(a.bmin, a.bmax, cell) : none;
-    const float2 L = has_l ? warp_minmax(a.amin, a.amax, is_l) : none;
-    const float2 R = has_r ? warp_minmax(a.amin, a.amax, is_r) : none;
-    const float2 TL = (has_l && has_t) ? warp_minmax(a.tmin, a.tmax, is_l) : none;
-    const float2 TR = (has_r && has_t) ? warp_minmax(a.tmin, a.tmax, is_r) : none;
-    const float2 BL = (has_l && has_b) ? warp_minmax(a.bmin, a.bmax, is_l) : none;
-    const float2 BR = (has_r && has_b) ? warp_minmax(a.bmin, a.bmax, is_r) : none;
-    if ((threadIdx.x & 31) == 0) {
-        slot[0] = all; slot[1] = L; slot[2] = R; slot[3] = top; slot[4] = bot;
-        slot[5] = TL; slot[6] = TR; slot[7] = BL; slot[8] = BR;
-    }
-}
-
-// Combines the per-warp slots (nw warps, 9 float2 each, UnitSum order) into
-// the unit summary: thread t < 18 reduces float t (a field's min or max).
-__device__ __forceinline__ void store_unit_summary(UnitSum *dst, const float2 *slots, int nw)
-{
-    static_assert(sizeof(UnitSum) == 18 * sizeof(float), "UnitSum is 9 float2");
-    const int t = threadIdx.x;
-    if (t < 18) {
-        const float *v = reinterpret_cast<const float *>(slots) + t;
-        float r = v[0];
-        for (int w = 1; w < nw; w++) r = (t & 1) ? fmaxf(r, v[18 * w]) : fminf(r, v[18 * w]);
-        reinterpret_cast<float *>(dst)[t] = r;
-    }
-}
-
-constexpr int kDryAge = 3;   // classifications a unit must stay dry before it is skipped
 
 // ---------------------------------------------------------------------------
 // TMA staging: one elected thread issues 2D tensor copies of a half tile's
@@ -397,20 +82,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity)
     return ok != 0;
 }
 
-__device__ __forceinline__ unsigned long long global_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// Waits for the phase with this parity to complete; false when it has not
-// after kWaitNs of global time or 2^28 polls, whichever comes first (each
-// try_wait may suspend the thread for a while), so that no wait is endless.
-// A staging copy lands within microseconds; the limit is seconds so that a
-// context that is time-sliced or pre-empted on a shared GPU does not take a
-// healthy copy for a lost one.
-constexpr unsigned long long kWaitNs = 4000000000ull;
 // try_wait that may suspend the thread for up to hint_ns while the phase is
 // incomplete (it resumes as soon as the phase completes), so that waiting
 // warps do not take issue slots from the warps that compute
@@ -427,6 +98,8 @@ __device__ __forceinline__ bool mbar_try_wait_hint(uint64_t *bar, uint32_t parit
     return ok != 0;
 }
 constexpr uint32_t kSuspendNs = 1000000;   // at most 1 ms per try
+// Waits for the phase with this parity to complete; false when it has not
+// after kWaitNs or 2^28 tries.
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity)
 {
     if (mbar_try_wait(bar, parity)) return true;
@@ -495,16 +168,6 @@ __host__ __device__ constexpr size_t deep_stage_bytes(int phase)
 {
     return deep_raw_rows_offset(phase) + (kRawRowBytes + 127) / 128 * 128;   // 128-byte aligned
 }
-struct DeepRow {
-    float4 m;      // cos, ilcos, area, dlon (edge row)
-    float icos;    // 1/cos, correctly rounded
-    // phase 2, for the unit's dt: dt / area, 1 / (2 cfl area), the x edges'
-    // XRowK::kdes, and the YRowK of the y edge above the row (y0: len, cmid,
-    // cdiff, c10; y1: c01, li0, kdes0, kdes1)
-    float dtA, kcfl, kdx;
-    float4 y0, y1;
-};
-static_assert(sizeof(DeepRow) == 64, "row metrics: four float4");
 __host__ __device__ constexpr size_t deep_misc_offset(int phase) { return 2 * deep_stage_bytes(phase); }
 static size_t deep_smem_bytes(int phase, int ng)
 {
@@ -625,41 +288,6 @@ __global__ void __launch_bounds__(kClassifyThreads) classify_kernel(const Scenar
     }
 }
 
-// ---------------------------------------------------------------------------
-// Deep phase 2 in pairs: a lane steps two adjacent columns, and the 2s
-// momentum fluxes, y edges and updates of the pair run in packed FP32x2
-// arithmetic (two lanes of FP32 per instruction, explicit round-to-nearest,
-// so no compiler contraction changes a result between code copies).  The
-// formulas are those of momentum_2s_x / momentum_2s_y.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-__device__ __forceinline__ float2 bc2(float a) { return make_float2(a, a); }
-__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
-__device__ __forceinline__ float2 sel2(bool px, bool py, float2 a, float2 b)
-{
-    return make_float2(px ? a.x : b.x, py ? a.y : b.y);
-}
-// Square roots of a pair (sqrt_ap per component, with its zero test: written
-// as a packed x * rsqrt(x) without it, the 16-warp deep phase 2 no longer
-// rounded like the other tilings), and 1/h and sqrt(h) of a cell pair from one
-// reciprocal square root per cell (deep cells: h > hpos >= 0)
-__device__ __forceinline__ float2 sqrt2(float2 h) { return make_float2(sqrt_ap(h.x), sqrt_ap(h.y)); }
-struct Depth2 {
-    float2 rh, sh;
-};
-__device__ __forceinline__ Depth2 depth2(float2 h)
-{
-    const float2 rs = make_float2(rsqrt_ap(h.x), rsqrt_ap(h.y));
-    return Depth2{mul2(rs, rs), make_float2(h.x == 0.f ? 0.f : __fmul_rn(h.x, rs.x), h.y == 0.f ? 0.f : __fmul_rn(h.y, rs.y))};
-}
-
-// two cells of a staged row (columns i, i + 1; i even)
-struct Cell2 {
-    float2 h, e, D, qx, qy;
-};
 __device__ __forceinline__ Cell2 staged_cell2(const float *st, int i)
 {
     Cell2 c;
@@ -669,119 +297,6 @@ __device__ __forceinline__ Cell2 staged_cell2(const float *st, int i)
     c.qy = *reinterpret_cast<const float2 *>(st + 3 * SPLANE + i);
     c.h = add2(c.e, c.D);
     return c;
-}
-
-struct MomFlux2 {
-    float2 m_x, m_y, p_x, p_y, lam;
-};
-// an edge's fluxes into one of its cells, as momentum_2s_* returns them (the
-// cell's update subtracts dt/area times their sum), and its wave-speed term
-struct Contrib2 {
-    float2 a, b, lam;
-};
-
-// momentum_2s_x for two edges at once
-__device__ __forceinline__ void momentum_2s_x2(MomFlux2 &r, float2 h0, float2 h1, float2 rh0, float2 rh1, float2 s0,
-                                               float2 s1, float2 u0, float2 u1, float2 v0, float2 v1, float2 jump,
-                                               const XRowK &k)
-{
-    const float2 hij = mul2(bc2(0.5f), add2(h0, h1));
-    const float2 u0n = mul2(u0, rh0), u1n = mul2(u1, rh1);
-    const float2 num = fma2(s0, u0n, mul2(s1, u1n));
-    const float2 den = add2(add2(s0, s1), bc2(kEps));
-    const float2 uijn = make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
-    const float2 maxa = add2(make_float2(fabsf(uijn.x), fabsf(uijn.y)), sqrt2(hij));
-    const bool nx_ = uijn.x < 0.f, ny_ = uijn.y < 0.f;
-    const float2 un = sel2(nx_, ny_, u1n, u0n), uu = sel2(nx_, ny_, u1, u0), vv = sel2(nx_, ny_, v1, v0);
-    const float2 il = bc2(k.ilcos);
-    const float2 mx0 = mul2(mul2(un, uu), il);
-    const float2 mx = fma2(mul2(hij, jump), il, mx0);
-    const float2 my = mul2(mul2(un, vv), il);
-    const float2 des = mul2(mul2(bc2(k.kdes), mul2(maxa, maxa)), sub2(u1, u0));
-    r.m_x = sub2(mx, des);
-    r.m_y = my;
-    r.p_x = sub2(des, mx0);
-    r.p_y = neg2(my);
-    r.lam = mul2(il, maxa);
-}
-
-// momentum_2s_y for two edges at once (one row pair: the constants are shared)
-__device__ __forceinline__ void momentum_2s_y2(MomFlux2 &r, float2 h0, float2 h1, float2 rh0, float2 rh1, float2 s0,
-                                               float2 s1, float2 u0, float2 u1, float2 v0, float2 v1, float2 jump,
-                                               const YRowK &k)
-{
-    const float2 hij = mul2(bc2(0.5f), add2(h0, h1));
-    const float2 u0n = mul2(u0, rh0), u1n = mul2(u1, rh1);
-    const float2 num = fma2(s0, u0n, mul2(s1, u1n));
-    const float2 den = add2(add2(s0, s1), bc2(kEps));
-    const float2 uijn = make_float2(__fdividef(num.x, den.x), __fdividef(num.y, den.y));
-    const float2 maxa = add2(make_float2(fabsf(uijn.x), fabsf(uijn.y)), sqrt2(hij));
-    const float2 deta = fma2(neg2(mul2(uijn, uijn)), bc2(k.cdiff), mul2(bc2(k.cmid), jump));
-    const bool nx_ = uijn.x < 0.f, ny_ = uijn.y < 0.f;
-    const float2 un = sel2(nx_, ny_, u1n, u0n), uu = sel2(nx_, ny_, u1, u0), vv = sel2(nx_, ny_, v1, v0);
-    const float2 len = bc2(k.len);
-    const float2 fym0 = mul2(mul2(un, uu), len);
-    // upwind from below: fyp = -fym0, fym = fym0 cos1/cos0; from above: fyp = -fym0 cos0/cos1, fym = fym0
-    const float2 fyp = mul2(neg2(fym0), sel2(nx_, ny_, bc2(1.f), bc2(k.c01)));
-    const float2 fym = fma2(mul2(hij, deta), bc2(k.li0), mul2(fym0, sel2(nx_, ny_, bc2(k.c10), bc2(1.f))));
-    const float2 fxm = mul2(mul2(un, vv), len);
-    const float2 m2 = mul2(mul2(maxa, maxa), fma2(u1, bc2(k.cos1), neg2(mul2(u0, bc2(k.cos0)))));
-    r.m_x = fxm;
-    r.m_y = fma2(bc2(-k.kdes0), m2, fym);
-    r.p_x = neg2(fxm);
-    r.p_y = fma2(bc2(k.kdes1), m2, fyp);
-    r.lam = mul2(len, maxa);
-}
-
-// y edge between rows gy-1 (a, row metrics ra) and gy (b, rb) of a deep tile;
-// phase 2 also takes 1/h and sqrt(h) of both cells, and the edge's constants
-// from rb
-template <int PHASE>
-__device__ __forceinline__ void y_edge_deep(const ScenarioDev &s, const Cell &a, const Cell &b, float rha, float sha,
-                                            float rhb, float shb, const DeepRow &ra, const DeepRow &rb, float dt,
-                                            Contrib &lo, Contrib &hi)
-{
-    const float cos0 = ra.m.x, cos1 = rb.m.x;
-    if (PHASE == 1) {
-        const float F = mass_2s_y(a.qy, rb.m.w, cos0, cos1, a.h, b.h, dt, ra.m.z, rb.m.z);
-        lo = {-F * ra.icos, 0.f, 0.f};
-        hi = {F * rb.icos, 0.f, 0.f};
-    } else {
-        YRowK k;
-        k.len = rb.y0.x; k.cmid = rb.y0.y; k.cdiff = rb.y0.z; k.c10 = rb.y0.w;
-        k.c01 = rb.y1.x; k.li0 = rb.y1.y; k.kdes0 = rb.y1.z; k.kdes1 = rb.y1.w;
-        k.cos0 = cos0; k.cos1 = cos1;
-        MomFlux f;
-        momentum_2s_y(f, a.h, b.h, rha, rhb, sha, shb, a.qy, b.qy, a.qx, b.qx, surface_jump(a.e, b.e, a.D, b.D), k);
-        lo = {-f.m_x, -f.m_y, f.lam};
-        hi = {-f.p_x, -f.p_y, f.lam};
-    }
-}
-
-// surface jumps of two edges (e0 -> e1); PLAIN: the unit's depths exceed its
-// depth steps, so each is the plain difference (the same value)
-template <bool PLAIN>
-__device__ __forceinline__ float2 jump2(float2 e0, float2 e1, float2 D0, float2 D1)
-{
-    if (PLAIN) return sub2(e1, e0);
-    return make_float2(surface_jump(e0.x, e1.x, D0.x, D1.x), surface_jump(e0.y, e1.y, D0.y, D1.y));
-}
-
-// y edge of phase 2 between rows a (metrics ra) and b (rb) for two columns
-template <bool PLAIN>
-__device__ __forceinline__ void y_edge_deep2(const Cell2 &a, const Cell2 &b, float2 rha, float2 sha, float2 rhb,
-                                             float2 shb, const DeepRow &ra, const DeepRow &rb, Contrib2 &lo,
-                                             Contrib2 &hi)
-{
-    YRowK k;
-    k.len = rb.y0.x; k.cmid = rb.y0.y; k.cdiff = rb.y0.z; k.c10 = rb.y0.w;
-    k.c01 = rb.y1.x; k.li0 = rb.y1.y; k.kdes0 = rb.y1.z; k.kdes1 = rb.y1.w;
-    k.cos0 = ra.m.x; k.cos1 = rb.m.x;
-    const float2 jump = jump2<PLAIN>(a.e, b.e, a.D, b.D);
-    MomFlux2 f;
-    momentum_2s_y2(f, a.h, b.h, rha, rhb, sha, shb, a.qy, b.qy, a.qx, b.qx, jump, k);
-    lo = {f.m_x, f.m_y, f.lam};
-    hi = {f.p_x, f.p_y, f.lam};
 }
 
 // A deep work unit: unit code u = 2 * (work-list index) + half.
@@ -942,7 +457,6 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                 }
             }
         } else if (d.run) {
-            const ScenarioDev &s = *d.s;
             ScenarioCtl *ctl = d.ctl;
             const int x0 = d.x0, yb = d.yb;
             const float dt = d.dt;
@@ -986,30 +500,18 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                 const int gx = x0 - 4 + sc;                             // grid column
                 const bool has_cell = (lane >= 2) && (lane <= 29);
                 const int dcol = strip * 28 - 2 + lane;                 // diagnostics column (cells only)
-                float local_min = FLT_MAX;    // phase 1: depth minimum
-                float local_max = -FLT_MAX;   // phase 1: depth maximum; phase 2: max of lam / (2 cfl area)
+                float local_min = FLT_MAX, local_max = -FLT_MAX;   // depths
                 bool bad = false;
                 int i = r_first * kStageW + sc;
                 Cell c = staged_cell(stage, i);
-                float rh_c = 0.f, sh_c = 0.f;
-                if (PHASE == 2) {
-                    rh_c = rcp_depth(c.h);
-                    sh_c = sqrt_ap(c.h);
-                }
                 DeepRow rc = row(r_first);
-                Contrib top;
+                float top;   // share of the y edge above the row in its cell
                 {
                     const Cell a = staged_cell(stage, i - kStageW);
-                    float rh_a = 0.f, sh_a = 0.f;
-                    if (PHASE == 2) {
-                        rh_a = rcp_depth(a.h);
-                        sh_a = sqrt_ap(a.h);
-                    }
-                    Contrib dummy;
-                    y_edge_deep<PHASE>(s, a, c, rh_a, sh_a, rh_c, sh_c, row(r_first - 1), rc, dt, dummy, top);
+                    const DeepRow ra = row(r_first - 1);
+                    top = mul(mass_2s_y(a.qy, rc.m.w, ra.m.x, rc.m.x, a.h, c.h, dt, ra.m.z, rc.m.z), rc.icos);
                 }
                 float *out0 = d.out0;
-                float *out1 = d.out1;
                 int off = (yb + r_first - 1) * pitch + gx;
                 // running sum of the cells' new values: non-finite iff one of them is
                 float fin = 0.f;
@@ -1017,80 +519,37 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                     const DeepRow rn = row(r_first + k + 1);
                     const Cell n = staged_cell(stage, i + kStageW);
                     const float area = rc.m.z;
-                    float rh_n = 0.f, sh_n = 0.f;
-                    if (PHASE == 2) {
-                        rh_n = rcp_depth(n.h);
-                        sh_n = sqrt_ap(n.h);
-                    }
-                    // y edge below this row
-                    Contrib below, next_top;
-                    y_edge_deep<PHASE>(s, c, n, rh_c, sh_c, rh_n, sh_n, rc, rn, dt, below, next_top);
-                    // x edge left of this lane's cell
-                    Contrib xl, xr;
-                    if (PHASE == 1) {
-                        const float F = mass_2s_x(stage[2 * SPLANE + i - 1], rc.m.y, stage[i - 1] + stage[SPLANE + i - 1],
-                                                  c.h, dt, area, area);
-                        xl = {-F, 0.f, 0.f};
-                        xr = {F, 0.f, 0.f};
-                    } else {
-                        const float e0 = stage[i - 1], D0 = stage[SPLANE + i - 1];
-                        MomFlux f;
-                        momentum_2s_x(f, e0 + D0, c.h, shup(rh_c, 1), rh_c, shup(sh_c, 1), sh_c, stage[2 * SPLANE + i - 1],
-                                      c.qx, stage[3 * SPLANE + i - 1], c.qy, surface_jump(e0, c.e, D0, c.D),
-                                      XRowK{rc.m.y, rc.kdx});
-                        xl = {-f.m_x, -f.m_y, f.lam};
-                        xr = {-f.p_x, -f.p_y, f.lam};
-                    }
+                    // y edge below this row, x edge left of this lane's cell
+                    const float Fb = mass_2s_y(c.qy, rn.m.w, rc.m.x, rn.m.x, c.h, n.h, dt, rc.m.z, rn.m.z);
+                    const float F = mass_2s_x(stage[2 * SPLANE + i - 1], rc.m.y, stage[i - 1] + stage[SPLANE + i - 1], c.h,
+                                              dt, area, area);
                     // the right edge of this cell is the left edge of lane+1
-                    Contrib xrr;
-                    xrr.a = shdn(xl.a, 1);
-                    if (PHASE == 2) {
-                        xrr.b = shdn(xl.b, 1);
-                        xrr.lam = shdn(xl.lam, 1);
-                    }
-                    if (PHASE == 1 && has_cell) {
+                    const float Fr = shdn(F, 1);
+                    if (has_cell) {
                         // diagnostics of the state the step starts from (src/GPU/Metrics.cu:23-77)
                         const float *dg = stage + 4 * SPLANE + (r_first - 1 + k) * kTileX + dcol;
                         const float em = dg[0], ar = dg[DPLANE], ei = dg[2 * DPLANE];
                         if (c.e > em && c.h > d.eps_h) d.eta_max[off] = c.e;
                         if (ar < 0.f && fabsf(c.e - ei) > d.dif_at) d.arr[off] = t_sec;
-                        // mass update (src/GPU/Volumen_kernel.cu:111-157)
-                        const float acc = ((xr.a + xrr.a) + top.a) + below.a;
-                        float eta = c.e + rc.dtA * acc;
-                        if (!(eta + c.D > 0.f)) eta = -c.D;
+                        const float eta = deep_eta(c, F, Fr, top, Fb, rc.icos, rc.dtA);
                         fin += eta;
                         out0[off] = eta;
                         local_min = fminf(local_min, eta + c.D);
                         local_max = fmaxf(local_max, eta + c.D);
-                    } else if (PHASE == 2 && has_cell) {
-                        // momentum update; no sponge, filter or friction in a deep
-                        // tile.  The cell's dt bound 2 cfl area / lam (1e30 for
-                        // lam < eps) is taken as the unit's largest lam / (2 cfl
-                        // area), inverted once per unit.
-                        const float lam = ((xr.lam + xrr.lam) + top.lam) + below.lam;
-                        local_max = fmaxf(local_max, (lam < kEps) ? 0.f : lam * rc.kcfl);
-                        const float val = rc.dtA;
-                        const float qx = c.qx + val * (((xr.a + xrr.a) + top.a) + below.a);
-                        const float qy = c.qy + val * (((xr.b + xrr.b) + top.b) + below.b);
-                        fin += qx + qy;
-                        out0[off] = qx;
-                        out1[off] = qy;
                     }
-                    top = next_top;
+                    top = mul(Fb, rn.icos);
                     rc = rn;
                     c = n;
-                    rh_c = rh_n;
-                    sh_c = sh_n;
                 }
                 if (!isfinite(fin)) bad = true;
                 if (bad) atomicOr(&ctl->errors, 1u);
                 for (int o = 16; o > 0; o >>= 1) {
-                    if (PHASE == 1) local_min = fminf(local_min, __shfl_xor_sync(0xffffffffu, local_min, o));
+                    local_min = fminf(local_min, __shfl_xor_sync(0xffffffffu, local_min, o));
                     local_max = fmaxf(local_max, __shfl_xor_sync(0xffffffffu, local_max, o));
                 }
                 if (lane == 0) {
-                    red[warp] = (PHASE == 1) ? local_min : local_max;
-                    if (PHASE == 1) red[NW + warp] = local_max;
+                    red[warp] = local_min;
+                    red[NW + warp] = local_max;
                 }
               } else {
                 // phase 2 in pairs: two column strips of 56 cells; lane l
@@ -1232,258 +691,6 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
     }
 }
 
-// General kernel: units that are not deep water (boundaries, sponge layers,
-// coasts, wet/dry fronts).  A unit's work is split into tasks of one warp
-// each: column strip `strip` (28 output columns and a two-column halo on
-// each side) and row group `group` (kHalfRows / NG rows).  general_part runs
-// one task: it marches the group's rows and returns the lane's dt bound
-// (phases 0 / 2), depth summary (phase 1) and error flag; cell: the lane
-// holds one of the strip's output cells, gx_out its grid column.
-template <int PHASE, int NG>
-__device__ __forceinline__ void general_part(const ScenarioDev &s, const ScenarioCtl *ctl, int tx, int uy, int strip,
-                                             int group, float &local_min, DepthAcc &hacc, bool &bad, bool &cell,
-                                             int &gx_out)
-{
-    constexpr int GROWS = kHalfRows / NG;
-    static_assert(kHalfRows % NG == 0, "row groups of equal height");
-    const int lane = threadIdx.x & 31;
-    const int nx = s.nx, ny = s.ny;
-    const int uy0 = uy * kHalfRows;
-    const int unit_end = min(uy0 + kHalfRows, ny);
-    // this warp: column strip `strip`, rows y0 .. y_end-1 of the unit
-    const int x0 = s.x_org + tx * kTileX + strip * OUTW, y0 = uy0 + group * GROWS;
-    const int p = ctl->parity;
-    const float dt = (float)ctl->dt;
-    const float t_sec = (float)(ctl->t * ctl->T);
-    const int gx = x0 - 2 + lane;
-    const int col = map_col(gx, nx, s.periodic);
-    const bool has_edge = (lane >= 2) && (lane <= 30) && (gx >= 0) && (gx <= nx);
-    const bool has_cell = (lane >= 2) && (lane <= 29) && (gx >= 0) && (gx < nx);
-    const int y_end = min(y0 + GROWS, unit_end);
-    const float *eta_in = (PHASE == 2) ? s.eta[p ^ 1] : s.eta[p];
-    const float *qx_in = s.qx[p], *qy_in = s.qy[p];
-    const size_t pitch = (size_t)s.pitch;
-    const bool x_ghost_lo = !s.periodic && gx == 0, x_ghost_hi = !s.periodic && gx == nx;
-    const bool x_nolim = (gx < 2) || (gx > nx - 2);
-    const bool sponge = (s.sp_left | s.sp_right | s.sp_up | s.sp_low) != 0;
-    local_min = FLT_MAX;
-    hacc.init();
-    bad = false;
-    gx_out = gx;
-    cell = has_cell && x0 < nx && x0 + OUTW > 0;
-
-    if (x0 < nx && x0 + OUTW > 0 && y0 < y_end) {
-        constexpr bool DIAG = (PHASE == 1);
-        Cell c0 = load_cell(eta_in, s.dep, qx_in, qy_in, clamp_row(y0 - 2, ny) * pitch + col);
-        Cell c1 = load_cell(eta_in, s.dep, qx_in, qy_in, clamp_row(y0 - 1, ny) * pitch + col);
-        Cell c2, c3, c4;
-        {
-            // rows y0 .. y0+2 with their diagnostics (rows below the grid are clamped and skipped)
-            const RawCell r0 = load_raw<DIAG>(s, eta_in, qx_in, qy_in, clamp_row(y0, ny) * pitch + col, has_cell);
-            const RawCell r1 = load_raw<DIAG>(s, eta_in, qx_in, qy_in, clamp_row(y0 + 1, ny) * pitch + col,
-                                              has_cell && y0 + 1 < y_end);
-            const RawCell r2 = load_raw<DIAG>(s, eta_in, qx_in, qy_in, clamp_row(y0 + 2, ny) * pitch + col,
-                                              has_cell && y0 + 2 < y_end);
-            if (DIAG && has_cell) {
-                diagnostics(s, r0, (size_t)y0 * pitch + col, t_sec);
-                if (y0 + 1 < y_end) diagnostics(s, r1, (size_t)(y0 + 1) * pitch + col, t_sec);
-                if (y0 + 2 < y_end) diagnostics(s, r2, (size_t)(y0 + 2) * pitch + col, t_sec);
-            }
-            c2 = finish(r0);
-            c3 = finish(r1);
-            c4 = finish(r2);
-        }
-        RawCell n1 = load_raw<DIAG>(s, eta_in, qx_in, qy_in, clamp_row(y0 + 3, ny) * pitch + col,
-                                    has_cell && y0 + 3 < y_end);
-        // y edge at the top of the first row (stencil rows y0-2 .. y0+1)
-        // row metrics {cos, ilcos, area, dlon} (rowpack), loaded a row
-        // ahead: kc of row yo, kn of row yo+1 (entry ny: dlon only)
-        const float4 *__restrict__ rp = s.rowpack;
-        float4 kc = __ldg(rp + y0);
-        float4 kn = __ldg(rp + y0 + 1);
-        Contrib top, dummy;
-        y_edge<PHASE>(s, c0, c1, c2, c3, y0, dt, dummy, top, __ldg(rp + clamp_row(y0 - 1, ny)), kc, kc.w);
-
-        for (int yo = y0; yo < y_end; yo++) {
-            const float4 knn = __ldg(rp + min(yo + 2, ny));
-            // rows yo+3 (loaded an iteration ago) and yo+4 (now) are in flight
-            const RawCell n2 = load_raw<DIAG>(s, eta_in, qx_in, qy_in, clamp_row(yo + 4, ny) * pitch + col,
-                                              has_cell && yo + 4 < y_end);
-            const size_t idx = (size_t)yo * pitch + col;
-            // ---- y edge below this row (between yo and yo+1) ----
-            Contrib below, next_top;
-            y_edge<PHASE>(s, c1, c2, c3, c4, yo + 1, dt, below, next_top, kc, (yo + 1 < ny) ? kn : kc, kn.w);
-
-            // ---- x edge left of this lane's cell (row yo) ----
-            Edge e;
-            e.h0m = shup(c2.h, 2);
-            e.e0m = shup(c2.e, 2);
-            e.h0 = shup(c2.h, 1);
-            e.u0 = shup(c2.qx, 1);
-            e.h1 = c2.h;
-            e.u1 = c2.qx;
-            if (PHASE != 0) {
-                e.e0 = shup(c2.e, 1);
-                e.D0 = shup(c2.D, 1);
-                e.h1p = shdn(c2.h, 1);
-                e.e1p = shdn(c2.e, 1);
-                e.e1 = c2.e;
-                e.D1 = c2.D;
-            }
-            if (PHASE == 2) {
-                // the tangential discharge only enters the momentum flux
-                e.v0m = shup(c2.qy, 2);
-                e.v0 = shup(c2.qy, 1);
-                e.v1p = shdn(c2.qy, 1);
-                e.v1 = c2.qy;
-            } else {
-                e.v0m = e.v0 = e.v1p = e.v1 = 0.f;
-            }
-            e.u0m = e.u1p = 0.f;
-            const float area = kc.z;
-            e.area0 = e.area1 = area;
-            e.cos0 = e.cos1 = kc.x;
-            e.len = kc.y;
-            e.normal = 1.f;
-            e.front = false;
-            if (x_ghost_lo) {
-                e.u0 *= s.b_left;
-                e.normal = -1.f;
-                e.front = true;
-            }
-            if (x_ghost_hi) e.u1 *= s.b_right;
-            e.no_lim = x_nolim;
-            Contrib xl = {0.f, 0.f, 0.f}, xr = {0.f, 0.f, 0.f};
-            if (has_edge) {
-                if (PHASE == 1) {
-                    const float F = mass_flux<false>(e, s, dt);
-                    xl = {-F, 0.f, 0.f};
-                    xr = x_ghost_lo ? Contrib{-F, 0.f, 0.f} : Contrib{F, 0.f, 0.f};
-                } else if (PHASE == 2) {
-                    MomFlux f = momentum_flux_x(e, s, dt);
-                    if (!f.active) { f.m_x = f.m_y = f.p_x = f.p_y = f.lam = 0.f; }
-                    xl = {-f.m_x, -f.m_y, f.lam};
-                    xr = x_ghost_lo ? xl : Contrib{-f.p_x, -f.p_y, f.lam};
-                } else {
-                    const float lam = initial_speed(e, s);
-                    xl = {0.f, 0.f, lam};
-                    xr = xl;
-                }
-            }
-            // the right edge of this cell is the left edge of lane+1
-            Contrib xrr;
-            xrr.a = shdn(xl.a, 1);
-            if (PHASE == 2) xrr.b = shdn(xl.b, 1);
-            if (PHASE != 1) xrr.lam = shdn(xl.lam, 1);
-
-            // ---- cell (gx, yo) ----
-            if (has_cell) {
-                if (PHASE == 0) {
-                    const float lam = ((xr.lam + xrr.lam) + top.lam) + below.lam;
-                    const float step = (lam < kEps) ? 1e30f : __fdividef(2.f * s.cfl * area, lam);
-                    local_min = fminf(local_min, step);
-                } else if (PHASE == 1) {
-                    // mass update (src/GPU/Volumen_kernel.cu:111-157); the
-                    // diagnostics run when a row's loads complete
-                    const float acc = ((xr.a + xrr.a) + top.a) + below.a;
-                    const float D = c2.D;
-                    float eta = c2.e + __fdividef(dt, area) * acc;
-                    if (!(eta + D > 0.f)) eta = -D;
-                    if (sponge && ((gx < s.sp_left) || (gx >= nx - s.sp_right) || (yo < s.sp_up) ||
-                                   (yo >= ny - s.sp_low))) {
-                        const float dx = __ldg(s.row.dlon + yo), dy = __ldg(s.row.dlat + yo);
-                        float dl = (s.sp_left - gx - 0.5f) * dx, dr = (gx - (nx - 1 - s.sp_right) - 0.5f) * dx;
-                        float du = (s.sp_up - yo - 0.5f) * dy, dd = (yo - (ny - 1 - s.sp_low) - 0.5f) * dy;
-                        if (dl <= 0.f) dl = 1e30f;
-                        if (dr <= 0.f) dr = 1e30f;
-                        if (du <= 0.f) du = 1e30f;
-                        if (dd <= 0.f) dd = 1e30f;
-                        float dist, ls;
-                        if ((dl <= dr) && (dl <= du) && (dl <= dd)) { dist = dl; ls = dx * s.sp_left; }
-                        else if ((dr <= dl) && (dr <= du) && (dr <= dd)) { dist = dr; ls = dx * s.sp_right; }
-                        else if ((du <= dl) && (du <= dr) && (du <= dd)) { dist = du; ls = dy * s.sp_up; }
-                        else { dist = dd; ls = dy * s.sp_low; }
-                        const float rr = dist / ls, co = 0.9f * rr * rr;
-                        // relax h towards max(D + sea level, 0), expressed on eta
-                        const float eta_rest = (D + s.sea > 0.f) ? s.sea : -D;
-                        eta -= co * (eta - eta_rest);
-                        if (!(eta + D >= 0.f)) eta = -D;
-                    }
-                    if (!isfinite(eta)) bad = true;
-                    s.eta[p ^ 1][idx] = eta;
-                    hacc.add(eta + D, yo - uy0 < 2, unit_end - yo <= 2);
-                } else {
-                    // momentum update (src/GPU/Volumen_kernel.cu:175-219)
-                    const float lam = ((xr.lam + xrr.lam) + top.lam) + below.lam;
-                    const float step = (lam < kEps) ? 1e30f : __fdividef(2.f * s.cfl * area, lam);
-                    local_min = fminf(local_min, step);
-                    const float val = __fdividef(dt, area);
-                    const float qx_old = c2.qx, qy_old = c2.qy;
-                    float qx = qx_old + val * (((xr.a + xrr.a) + top.a) + below.a);
-                    float qy = qy_old + val * (((xr.b + xrr.b) + top.b) + below.b);
-                    const float h = c2.h;
-                    if (sponge) {
-                        const float dx = __ldg(s.row.dlon + yo), dy = __ldg(s.row.dlat + yo);
-                        if (gx < s.sp_left) {
-                            const float rr = ((s.sp_left - gx - 0.5f) * dx) / (dx * s.sp_left);
-                            qx -= 0.9f * rr * rr * qx;
-                        }
-                        if (gx >= nx - s.sp_right) {
-                            const float rr = ((gx - (nx - 1 - s.sp_right) - 0.5f) * dx) / (dx * s.sp_right);
-                            qx -= 0.9f * rr * rr * qx;
-                        }
-                        if (yo < s.sp_up) {
-                            const float rr = ((s.sp_up - yo - 0.5f) * dy) / (dy * s.sp_up);
-                            qy -= 0.9f * rr * rr * qy;
-                        }
-                        if (yo >= ny - s.sp_low) {
-                            const float rr = ((yo - (ny - 1 - s.sp_low) - 0.5f) * dy) / (dy * s.sp_low);
-                            qy -= 0.9f * rr * rr * qy;
-                        }
-                    }
-                    if (h <= s.hpos) {
-                        // damping of almost-dry cells and velocity cap (filtroEstado)
-                        const float f = h / s.eps_h;
-                        const float damp = __expf(-dt * (1.f / (pow4f(f) + kEps)));
-                        qx *= damp;
-                        qy *= damp;
-                        const float fac = inv_depth(h, s.eps_h);
-                        if (s.vmax > 0.f) {
-                            float ux = fac * qx, uy = fac * qy;
-                            const float uu = sqrt_ap(ux * ux + uy * uy);
-                            if (uu > s.vmax) { ux *= s.vmax / uu; uy *= s.vmax / uu; }
-                            qx = ux * h;
-                            qy = uy * h;
-                        }
-                        // semi-implicit Manning friction with the pre-update speed (disImplicita)
-                        const float u1x = fac * qx, u1y = fac * qy;
-                        const float u1 = sqrt_ap(qx_old * qx_old + qy_old * qy_old) * fac;
-                        if (h > 0.f) {
-                            const float c1 = dt * s.mf0 * fabsf(u1) / (exp2f(log2f(h) * (4.f / 3.f)) + kEps);
-                            const float fr = h / (1.f + c1);
-                            qx = fr * u1x;
-                            qy = fr * u1y;
-                        }
-                    }
-                    if (!isfinite(qx) || !isfinite(qy)) bad = true;
-                    s.qx[p ^ 1][idx] = qx;
-                    s.qy[p ^ 1][idx] = qy;
-                }
-            }
-            top = next_top;
-            kc = kn;
-            kn = knn;
-            c0 = c1;
-            c1 = c2;
-            c2 = c3;
-            c3 = c4;
-            if (DIAG && has_cell && yo + 3 < y_end) diagnostics(s, n1, idx + 3 * pitch, t_sec);
-            c4 = finish(n1);
-            n1 = n2;
-        }
-    }
-}
-
 // Phase 0 (the initial dt) over every unit of the work list, one unit per CTA
 // iteration, 4 x NG warps; the last unit of a scenario stores its dt.
 template <int NG>
@@ -1503,12 +710,10 @@ __global__ void __launch_bounds__(128 * NG) initial_dt_kernel(const ScenarioDev 
         const int ty = item.y / s.tiles_x, tx = item.y - ty * s.tiles_x;
         const int uy = 2 * ty + (u & 1);
         if (uy * kHalfRows >= s.ny) continue;   // a unit below the grid (CTA-uniform)
+        constexpr int GROWS = kHalfRows / NG;
+        const int y0 = uy * kHalfRows + group * GROWS;
         float local_min;
-        DepthAcc hacc;
-        bool bad, cell;
-        int gx;
-        general_part<0, NG>(s, ctl, tx, uy, strip, group, local_min, hacc, bad, cell, gx);
-        if (bad) atomicOr(&ctl->errors, 1u);
+        initial_rows(s, ctl->parity, tx, uy, strip, y0, min(y0 + GROWS, min(uy * kHalfRows + kHalfRows, s.ny)), local_min);
         for (int o = 16; o > 0; o >>= 1) local_min = fminf(local_min, __shfl_xor_sync(0xffffffffu, local_min, o));
         if (lane == 0) red[warp] = local_min;
         __syncthreads();
@@ -1527,41 +732,6 @@ __global__ void __launch_bounds__(128 * NG) initial_dt_kernel(const ScenarioDev 
             }
         }
         __syncthreads();   // red[] is reused by the next unit
-    }
-}
-
-// Folds one warp's share of a unit's depth summary (nine {min, max}, UnitSum
-// order; a field the warp holds no cell of is left alone) into the unit's
-// summary with integer atomics on the float bits: depths are >= 0, where the
-// bit patterns order as the values do (a -0 counts as +0), and min and max are
-// exact in any order, so the summary does not depend on which warp came
-// first.  The classification resets the summaries of the general units it
-// lists to the empty value (FLT_MAX, -FLT_MAX) before this phase runs.
-__device__ __forceinline__ void fold_unit_summary(const DepthAcc &a, bool cell, bool is_l, bool is_r, UnitSum *dst)
-{
-    const float2 none = make_float2(FLT_MAX, -FLT_MAX);
-    const bool has_t = __any_sync(0xffffffffu, cell && a.tmin != FLT_MAX);
-    const bool has_b = __any_sync(0xffffffffu, cell && a.bmin != FLT_MAX);
-    const bool has_l = __any_sync(0xffffffffu, is_l), has_r = __any_sync(0xffffffffu, is_r);
-    float2 f[9];
-    f[0] = warp_minmax(a.amin, a.amax, cell);
-    f[1] = has_l ? warp_minmax(a.amin, a.amax, is_l) : none;
-    f[2] = has_r ? warp_minmax(a.amin, a.amax, is_r) : none;
-    f[3] = has_t ? warp_minmax(a.tmin, a.tmax, cell) : none;
-    f[4] = has_b ? warp_minmax(a.bmin, a.bmax, cell) : none;
-    f[5] = (has_l && has_t) ? warp_minmax(a.tmin, a.tmax, is_l) : none;
-    f[6] = (has_r && has_t) ? warp_minmax(a.tmin, a.tmax, is_r) : none;
-    f[7] = (has_l && has_b) ? warp_minmax(a.bmin, a.bmax, is_l) : none;
-    f[8] = (has_r && has_b) ? warp_minmax(a.bmin, a.bmax, is_r) : none;
-    if ((threadIdx.x & 31) == 0) {
-        int *d = reinterpret_cast<int *>(dst);
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            if (f[k].x == FLT_MAX) continue;   // no cell of this field in the task
-            const int lo = __float_as_int(f[k].x), hi = __float_as_int(f[k].y);
-            atomicMin(d + 2 * k, lo == (int)0x80000000 ? 0 : lo);
-            atomicMax(d + 2 * k + 1, hi == (int)0x80000000 ? 0 : hi);
-        }
     }
 }
 
@@ -1607,8 +777,7 @@ __global__ void __launch_bounds__(kGeneralThreads, 4) general_kernel(const Scena
                                   &s.usum[ctl->parity ^ 1][(size_t)uy * s.tiles_x + tx]);
             } else {
                 // the minimum is exact in any order
-                for (int o = 16; o > 0; o >>= 1)
-                    local_min = fminf(local_min, __shfl_xor_sync(0xffffffffu, local_min, o));
+                local_min = warp_min_bound(local_min);
                 if (lane == 0) atomicMin(&ctl->dt_bits, __float_as_uint(local_min));
             }
         }
