@@ -1,0 +1,83 @@
+"""Chunks of steps that stay resident on the device (kernels/resident.cu)
+against the launched kernels: the same code of every cell, so bitwise the same
+fields, samples, step counts and unit counts, at sizes around the edges of
+strips (28 columns), tiles (112), units (16 rows) and of the task splits, up to
+the largest resident work."""
+import numpy as np
+import pytest
+
+import thysea
+from thysea import synth
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("max_height", "arrival", "deformed_bathy", "eta", "ux", "uy")
+
+
+def _problem(nx, ny, kind, sim_time):
+    rng = np.random.default_rng(nx * 10007 + ny)
+    lon, lat = synth.lonlat_grid(nx, ny, lat_centre=12.0)
+    z = synth.shelf_bathymetry(nx, ny, rng) if kind != "shallow" else (
+        -15.0 + 20.0 * synth.gaussian_random_field(nx, ny, 4.0, rng)).astype(np.float32)
+    p = synth.Problem(name="resident", lon=lon, lat=lat, z=z, sim_time=sim_time)
+    if kind in ("file", "shallow"):
+        p.eta_init = synth.gaussian_random_field(nx, ny, 5.0, rng).astype(np.float32)
+    else:
+        c = synth.random_fault(lon, lat, z, rng)
+        p.faults = [c]
+        if kind == "late":
+            p.faults = [c, synth.random_fault(lon, lat, z, rng, time=0.5 * sim_time)]
+    p.borders = {"file": (-1.0, -1.0, -1.0, -1.0), "periodic": (1.0, -1.0, 2.0, 2.0)}.get(kind, (1.0, 1.0, 1.0, 1.0))
+    if kind == "late":
+        p.points = np.stack([lon[rng.integers(0, nx, 5)], lat[rng.integers(0, ny, 5)]], axis=1)
+        p.series_time, p.save_time = sim_time / 20.0, sim_time / 3.0
+    return p
+
+
+def _run(prep):
+    r = thysea.run(prep)
+    return {k: r[k].copy() for k in FIELDS}, r
+
+
+@pytest.mark.parametrize("nx,ny,kind,sim_time", [
+    (2, 2, "file", 30.0), (3, 17, "file", 60.0), (28, 16, "shallow", 120.0), (29, 33, "shallow", 200.0),
+    (112, 48, "periodic", 300.0), (113, 95, "late", 400.0), (229, 160, "late", 400.0), (336, 337, "open", 400.0),
+    (500, 411, "shallow", 400.0), (641, 512, "periodic", 500.0), (1024, 700, "late", 300.0), (1700, 1790, "open", 120.0),
+])
+def test_resident_chunks_match_the_launched_kernels(gpu, nx, ny, kind, sim_time):
+    prep = thysea.Prepared(_problem(nx, ny, kind, sim_time))
+    thysea.force_tiling((0, 0, 0))   # a forced tiling names the launched kernels
+    try:
+        ref, r0 = _run(prep)
+    finally:
+        thysea.force_tiling(None)
+    got, r = _run(prep)
+    assert r["kernel_launches"] < r["iterations"] < r0["kernel_launches"]   # one launch a chunk against six a step
+    for k in ("iterations", "final_time", "deep_tiles", "dry_tiles", "nseries", "nsnaps"):
+        assert r[k] == r0[k], k
+    for k in FIELDS:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k
+    for part in ("snapshots", "series"):
+        for k in r0[part]:
+            assert np.array_equal(r[part][k], r0[part][k], equal_nan=True), (part, k)
+
+
+def test_resident_batch_matches_alone(gpu):
+    """several scenarios in one resident chunk, each with its own dt, end and
+    gauges-free events, against their launched runs"""
+    probs = [_problem(nx, ny, kind, t) for nx, ny, kind, t in
+             ((120, 100, "open", 300.0), (257, 130, "periodic", 500.0), (64, 64, "shallow", 100.0), (300, 222, "file", 350.0))]
+    thysea.force_tiling((0, 0, 0))
+    try:
+        alone = [_run(thysea.Prepared(p)) for p in probs]
+    finally:
+        thysea.force_tiling(None)
+    srv = thysea.Server(hbm_budget_bytes=2 << 30, max_scenarios=8)
+    ids = [srv.submit(p) for p in probs]
+    srv.drain()
+    srv.close()
+    for rid, (ref, r) in zip(ids, alone):
+        assert srv.results[rid]["status"] == 0
+        assert srv.results[rid]["stats"]["steps"] == r["iterations"]
+        for k in FIELDS:
+            assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k

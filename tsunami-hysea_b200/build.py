@@ -28,6 +28,7 @@ INCLUDES = ["-I" + os.path.join(ROOT, "include"), "-I" + os.path.join(CSRC, "ncl
 
 CUDA_SOURCES = [
     "kernels/step.cu",
+    "kernels/resident.cu",
     "kernels/init_extract.cu",
     "kernels/okada.cu",
     "runtime/engine.cu",
@@ -43,7 +44,7 @@ C_SOURCES = ["nclite/nclite.c"]
 EXPORTS = os.path.join(CSRC, "exports.map")
 # FP32 stepping kernels: approximate division / sqrt / exp (<= 2 ulp); the FP64
 # Okada and set-up kernels keep IEEE arithmetic
-FAST_MATH = {"kernels/step.cu"}
+FAST_MATH = {"kernels/step.cu", "kernels/resident.cu"}
 
 
 def _obj(src: str) -> str:

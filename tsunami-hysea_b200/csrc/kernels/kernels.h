@@ -98,6 +98,33 @@ void launch_initial_dt(const StepLaunch &L, cudaStream_t st);
 // lists for the current states of the work list's scenarios (from the host,
 // before a chunk: after the work list or a state changed)
 void launch_lists_current(const StepLaunch &L, cudaStream_t st);
+// resident.cu: a chunk of steps in one cooperative launch, one CTA per SM, for
+// work whose steps are bound by the latency of their launches
+constexpr int kResidentSlots = 64;      // scenarios of such a chunk at most
+// Barrier words, zero before the first launch (the kernel leaves the ones of
+// its next launch zero): arrivals in the upper half; in the lower half of
+// phase 2's the scenario's dt bound, as the largest of 0x7f7fffff - its bits.
+struct ResidentSync {
+    struct alignas(128) Word {
+        unsigned long long v, pad[15];
+    };
+    Word start, phase1[3], phase2[3];   // by step modulo 3, counted on from launch to launch
+    int next;                           // the next launch's first step, modulo 3
+    int counts[3];                      // units by class at the start of the chunk
+    unsigned int dt_bits[3][kResidentSlots];   // several scenarios: their smallest dt bounds
+};
+struct ResidentLaunch {
+    const ScenarioDev *tab;    // the stepped scenarios (nslots of them)
+    const int2 *units;         // their work units: (index into tab, unit)
+    int *order;                // scratch, 3 x cap: the units by class
+    ResidentSync *sync;
+    int nslots, nunits, cap, steps;
+    int rows_general, rows_deep;   // rows of a task: 1, 2, 4 or 8
+};
+int resident_warps(int sms);             // warps of a launch
+int resident_tasks_capacity(int warps);  // tasks they can hold
+cudaError_t configure_resident_kernel();
+cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st);
 // init_extract.cu: the step controller of every slot (launch 5 of a step)
 void launch_controller(const StepLaunch &L, cudaStream_t st);
 // init_extract.cu: per-unit depth steps (ScenarioDev::unit_gmax), after the

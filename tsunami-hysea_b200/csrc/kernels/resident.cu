@@ -1,0 +1,658 @@
+// A chunk of time steps in one cooperative launch, for work that does not
+// fill the GPU.
+//
+// What bounds such work is latency, not throughput: as separate launches
+// (step.cu) a step is a chain of six kernels and a memset, each of which reads
+// its lists, work items, descriptors and control words one after the other
+// before its first cell.  Here one CTA per SM stays on the device for the whole
+// chunk with the scenarios' descriptors in shared memory, and a step is
+//     phase 1 | grid barrier | classes, phase 2 | grid barrier, control
+// A task is a column strip of a unit and a few of its rows.  The tasks are dealt
+// to the CTAs once per chunk, general units first (they cost most), and a CTA's
+// warps claim them from shared memory.  The classes that the classification
+// launch would list are evaluated in place, one thread per task of the CTA, so
+// that a step has no list to build; a unit that changes class during the chunk is
+// stepped by the same tasks, each step by the class it has.  Every CTA advances
+// the control blocks for itself from the barrier's dt minimum, which saves a hop
+// through a controlling CTA.
+//
+// What bounds it now: the chain of a task's edges (about 3.8 us a row of WAF
+// edges in both phases on an otherwise idle SM), two barriers of 1.3 us, and the
+// spread of the tasks' costs over the SMs.  us a step, launched -> resident:
+// 96 x 80 28 -> 14, 512^2 48 -> 24, 1024^2 70 -> 44, 1600^2 95 -> 78.
+//
+// Arithmetic, classes, depth summaries, dry counts and the control are those
+// of the launches in step.cu; results are bitwise the same.
+//
+// Reference: src/GPU/Timestep.cu:11-120 (the launches of a step),
+// src/GPU/ShallowWater.cu:396-450 (the loop around it).
+#include "step_parts.cuh"
+
+#include <algorithm>
+
+namespace thy {
+
+namespace {
+
+constexpr int kResWarps = 16, kResThreads = 32 * kResWarps;
+constexpr int kMaxDeepRows = 8;     // rows of a deep task at most
+constexpr int kTaskRows = kMaxDeepRows + 2;
+constexpr int kDealStep = 61;       // odd: units of one column of a grid alternate in the lists
+
+enum : int { kClsGeneral = 0, kClsDeep = 1, kClsDry = 2, kClsPlain = 4 };   // kClsPlain: a flag of deep units
+
+// the step state of a scenario
+struct alignas(16) StepState {
+    float dt, t_sec;
+    int parity, status;
+};
+
+// a task of one warp: unit (tx, uy) of scenario `slot`, its sub-task and the rows of one
+struct Task {
+    short slot, tx, uy;
+    unsigned char sub, rows;
+};
+
+struct Shared {
+    ScenarioDev *tab;      // nslots
+    ScenarioCtl *ctl;      // nslots: every CTA advances its own copy
+    StepState *state;      // nslots
+    unsigned *dt_bits;     // nslots: the block's smallest dt bound of the step
+    Task *tasks;           // kResThreads: this CTA's tasks, one thread evaluates the class of each
+    unsigned char *cls;    // kResThreads
+    DeepRow *rows;         // kResWarps x kTaskRows
+};
+
+constexpr size_t kTasksBytes = sizeof(Task) * kResThreads;
+constexpr size_t kClsBytes = kResThreads;
+constexpr size_t kRowsBytes = sizeof(DeepRow) * kResWarps * kTaskRows;
+__host__ __device__ constexpr size_t up16(size_t b) { return (b + 15) / 16 * 16; }
+__host__ __device__ inline size_t shared_bytes(int nslots)
+{
+    return kRowsBytes + kTasksBytes + up16(kClsBytes) + nslots * (up16(sizeof(ScenarioDev)) + up16(sizeof(ScenarioCtl)) +
+                                                                   sizeof(StepState)) + up16(nslots * sizeof(unsigned));
+}
+__device__ __forceinline__ Shared shared_layout(unsigned char *m, int nslots)
+{
+    Shared h;
+    h.rows = reinterpret_cast<DeepRow *>(m);
+    m += kRowsBytes;
+    h.tasks = reinterpret_cast<Task *>(m);
+    m += kTasksBytes;
+    h.cls = m;
+    m += up16(kClsBytes);
+    h.state = reinterpret_cast<StepState *>(m);
+    m += nslots * sizeof(StepState);
+    h.dt_bits = reinterpret_cast<unsigned *>(m);
+    m += up16(nslots * sizeof(unsigned));
+    h.tab = reinterpret_cast<ScenarioDev *>(m);
+    m += up16(nslots * sizeof(ScenarioDev));
+    h.ctl = reinterpret_cast<ScenarioCtl *>(m);
+    return h;
+}
+
+// ---------------------------------------------------------------------------
+// Grid barriers: one thread per CTA adds to a counter and polls it.  Arrivals
+// release, waits acquire (which also drops the SM's L1 lines, so that plain
+// loads after a barrier see what other SMs wrote before it).  Measured on 148
+// CTAs: 1.27 us a barrier; a tag per CTA that every CTA polls 6.0 us, a
+// gathering CTA that answers with one word 2.9 us.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
+{
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+// arrives at w and waits for n arrivals: the word then, or 0 after kWaitNs of
+// global time (or 2^28 polls), so that no wait is endless
+__device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word &w, unsigned n)
+{
+    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&w.v), "l"(1ull << 32) : "memory");
+    unsigned long long v = ld_acquire(&w.v);
+    if ((unsigned)(v >> 32) == n) return v;
+    const unsigned long long t0 = global_ns();
+    for (int i = 0; i < (1 << 28); i++) {
+        v = ld_acquire(&w.v);
+        if ((unsigned)(v >> 32) == n) return v;
+        if ((i & 63) == 63 && global_ns() - t0 > kWaitNs) break;
+    }
+    return 0ull;
+}
+
+// ---------------------------------------------------------------------------
+// Deep units.  The formulas and roundings are those of the deep-water kernels
+// (step.cu), with the rows loaded straight from global memory: a task has a
+// few rows, and the state of this work stays in L2.
+// ---------------------------------------------------------------------------
+
+// phase 1: columns x0 .. x0+27, rows y0 .. y0+nrows-1; the warp's depth {min, max}
+__device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt, float t_sec, int x0, int y0, int nrows,
+                                          DeepRow *rows, float &mn, float &mx, bool &bad)
+{
+    const int lane = threadIdx.x & 31;
+    const size_t pitch = (size_t)s.pitch;
+    const int gx = x0 - 2 + lane;
+    const bool has_cell = (lane >= 2) && (lane <= 29);
+    const float *eta = s.eta[p], *qx = s.qx[p], *qy = s.qy[p];
+    float *out = s.eta[p ^ 1];
+    size_t off = (size_t)y0 * pitch + gx;
+    // row y0 - 1 + t of the window at rows[t]
+    if (lane < nrows + 2) {
+        DeepRow r;
+        r.m = __ldg(s.rowpack + y0 - 1 + lane);
+        r.icos = __frcp_rn(r.m.x);
+        r.dtA = __fdividef(dt, r.m.z);
+        rows[lane].m = r.m;
+        rows[lane].icos = r.icos;
+        rows[lane].dtA = r.dtA;
+    }
+    const Cell a = load_cell<true>(eta, s.dep, qx, qy, off - pitch);
+    Cell c = load_cell<true>(eta, s.dep, qx, qy, off);
+    Cell n = load_cell<true>(eta, s.dep, qx, qy, off + pitch);
+    float em = 0.f, ar = 0.f, ei = 0.f;
+    if (has_cell) {
+        em = s.eta_max[off];
+        ar = s.arr[off];
+        ei = s.eta_ini[off];
+    }
+    __syncwarp();
+    float4 mc = rows[1].m;
+    float icos_c = rows[1].icos, top;
+    {
+        const float4 ma = rows[0].m;
+        top = mul(mass_2s_y(a.qy, mc.w, ma.x, mc.x, a.h, c.h, dt, ma.z, mc.z), icos_c);
+    }
+    mn = FLT_MAX;
+    mx = -FLT_MAX;
+    for (int k = 0; k < nrows; k++, off += pitch) {
+        const float4 mr = rows[k + 2].m;
+        const float icos_n = rows[k + 2].icos;
+        // the row after the next one and the next row's diagnostics
+        Cell nn = n;
+        float em1 = 0.f, ar1 = 0.f, ei1 = 0.f;
+        if (k + 1 < nrows) {
+            nn = load_cell<true>(eta, s.dep, qx, qy, off + 2 * pitch);
+            if (has_cell) {
+                em1 = s.eta_max[off + pitch];
+                ar1 = s.arr[off + pitch];
+                ei1 = s.eta_ini[off + pitch];
+            }
+        }
+        const float Fb = mass_2s_y(c.qy, mr.w, mc.x, mr.x, c.h, n.h, dt, mc.z, mr.z);
+        const float F = mass_2s_x(shup(c.qx, 1), mc.y, shup(c.h, 1), c.h, dt, mc.z, mc.z);
+        const float Fr = shdn(F, 1);
+        if (has_cell) {
+            if (c.e > em && c.h > s.eps_h) s.eta_max[off] = c.e;
+            if (ar < 0.f && fabsf(c.e - ei) > s.dif_at) s.arr[off] = t_sec;
+            const float e = deep_eta(c, F, Fr, top, Fb, icos_c, rows[k + 1].dtA);
+            if (!isfinite(e)) bad = true;
+            out[off] = e;
+            mn = fminf(mn, e + c.D);
+            mx = fmaxf(mx, e + c.D);
+        }
+        top = mul(Fb, icos_n);
+        c = n;
+        n = nn;
+        mc = mr;
+        icos_c = icos_n;
+        em = em1;
+        ar = ar1;
+        ei = ei1;
+    }
+    const float2 v = warp_minmax(mn, mx, has_cell);
+    mn = v.x;
+    mx = v.y;
+    __syncwarp();   // rows is reused by the warp's next task
+}
+
+__device__ __forceinline__ Cell2 load_cell2(const float *eta, const float *dep, const float *qx, const float *qy, size_t off)
+{
+    Cell2 c;
+    c.e = *reinterpret_cast<const float2 *>(eta + off);
+    c.D = *reinterpret_cast<const float2 *>(dep + off);
+    c.qx = *reinterpret_cast<const float2 *>(qx + off);
+    c.qy = *reinterpret_cast<const float2 *>(qy + off);
+    c.h = add2(c.e, c.D);
+    return c;
+}
+
+// phase 2 in column pairs: columns x0 .. x0+55 (x0 even), rows y0 ..
+// y0+nrows-1; the warp's largest lam / (2 cfl area)
+template <bool PLAIN>
+__device__ __forceinline__ float momentum_rows(const ScenarioDev &s, int p, float dt, int x0, int y0, int nrows, DeepRow *rows,
+                                               bool &bad)
+{
+    const int lane = threadIdx.x & 31;
+    const size_t pitch = (size_t)s.pitch;
+    const bool out_lane = (lane >= 1) && (lane <= 28);
+    const float *eta = s.eta[p ^ 1], *qx_in = s.qx[p], *qy_in = s.qy[p];
+    float *qx_out = s.qx[p ^ 1], *qy_out = s.qy[p ^ 1];
+    size_t off = (size_t)y0 * pitch + x0 - 2 + 2 * min(lane, 29);
+    const Cell2 a = load_cell2(eta, s.dep, qx_in, qy_in, off - pitch);
+    Cell2 c = load_cell2(eta, s.dep, qx_in, qy_in, off);
+    Cell2 n = load_cell2(eta, s.dep, qx_in, qy_in, off + pitch);
+    if (lane < nrows + 2) {
+        DeepRow r;
+        r.m = __ldg(s.rowpack + y0 - 1 + lane);
+        const float4 ra = __ldg(s.rowpack + y0 - 2 + lane);   // the row above
+        r.icos = __frcp_rn(r.m.x);
+        r.dtA = __fdividef(dt, r.m.z);
+        r.kcfl = 1.f / (2.f * s.cfl * r.m.z);
+        r.kdx = make_xrow(r.m.y, r.m.z + r.m.z, dt, s.cvis).kdes;
+        const YRowK k = make_yrow(ra.x, r.m.x, __frcp_rn(ra.x), r.icos, r.m.w, ra.z + r.m.z, dt, s.cvis);
+        r.y0 = make_float4(k.len, k.cmid, k.cdiff, k.c10);
+        r.y1 = make_float4(k.c01, k.li0, k.kdes0, k.kdes1);
+        rows[lane] = r;
+    }
+    __syncwarp();
+    Depth2 fc = depth2(c.h);
+    DeepRow rc = rows[1];
+    Contrib2 top;
+    {
+        Contrib2 dummy;
+        const Depth2 fa = depth2(a.h);
+        y_edge_deep2<PLAIN>(a, c, fa.rh, fa.sh, fc.rh, fc.sh, rows[0], rc, dummy, top);
+    }
+    float local_max = 0.f;
+    for (int k = 0; k < nrows; k++, off += pitch) {
+        const DeepRow rn = rows[k + 2];
+        Cell2 nn = n;
+        if (k + 1 < nrows) nn = load_cell2(eta, s.dep, qx_in, qy_in, off + 2 * pitch);
+        const Depth2 fn = depth2(n.h);
+        Contrib2 below, next_top;
+        y_edge_deep2<PLAIN>(c, n, fc.rh, fc.sh, fn.rh, fn.sh, rc, rn, below, next_top);
+        const float le = shup(c.e.y, 1), lh = shup(c.h.y, 1);
+        const float lqx = shup(c.qx.y, 1), lqy = shup(c.qy.y, 1);
+        const float rhL = shup(fc.rh.y, 1), shL = shup(fc.sh.y, 1);
+        const float2 jump = PLAIN ? sub2(c.e, make_float2(le, c.e.x))
+                                  : jump2<false>(make_float2(le, c.e.x), c.e, make_float2(shup(c.D.y, 1), c.D.x), c.D);
+        MomFlux2 f;
+        momentum_2s_x2(f, make_float2(lh, c.h.x), c.h, make_float2(rhL, fc.rh.x), fc.rh, make_float2(shL, fc.sh.x), fc.sh,
+                       make_float2(lqx, c.qx.x), c.qx, make_float2(lqy, c.qy.x), c.qy, jump, XRowK{rc.m.y, rc.kdx});
+        const Contrib2 xr = {f.p_x, f.p_y, f.lam};
+        const Contrib2 xrr = {make_float2(f.m_x.y, shdn(f.m_x.x, 1)), make_float2(f.m_y.y, shdn(f.m_y.x, 1)),
+                              make_float2(f.lam.y, shdn(f.lam.x, 1))};
+        const float2 lam = add2(add2(add2(xr.lam, xrr.lam), top.lam), below.lam);
+        const float2 w = mul2(lam, bc2(rc.kcfl));
+        const float wm = fmaxf(lam.x < kEps ? 0.f : w.x, lam.y < kEps ? 0.f : w.y);
+        const float2 val = bc2(-rc.dtA);
+        const float2 qx = fma2(val, add2(add2(add2(xr.a, xrr.a), top.a), below.a), c.qx);
+        const float2 qy = fma2(val, add2(add2(add2(xr.b, xrr.b), top.b), below.b), c.qy);
+        if (out_lane) {
+            local_max = fmaxf(local_max, wm);
+            if (!isfinite(qx.x + qx.y + qy.x + qy.y)) bad = true;
+            *reinterpret_cast<float2 *>(qx_out + off) = qx;
+            *reinterpret_cast<float2 *>(qy_out + off) = qy;
+        }
+        top = next_top;
+        rc = rn;
+        c = n;
+        n = nn;
+        fc = fn;
+    }
+    local_max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(local_max)));   // (>= 0)
+    __syncwarp();   // rows is reused by the warp's next task
+    return local_max;
+}
+
+// Class of a unit for the state its summaries `sum` describe, as unit_deep and
+// unit_dry find it, from one round of nine loads; *age: its dry count
+// (advance: the classification of a step, which moves the count); gmax: the
+// unit's depth step.
+__device__ __forceinline__ int unit_class(const ScenarioDev &s, const UnitSum *sum, int tx, int uy, float gmax, bool advance,
+                                          int &age)
+{
+    const int W = s.tiles_x, ny_u = units_y(s);
+    const int x0 = s.x_org + tx * kTileX, yb = uy * kHalfRows;
+    const bool inside = s.tmap && x0 >= max(2, s.sp_left) && x0 + kTileX <= s.nx - max(2, s.sp_right) &&
+                        yb >= max(2, s.sp_up) && yb + kHalfRows <= s.ny - max(2, s.sp_low);
+    const bool l = tx > 0 || s.periodic, r = tx + 1 < W || s.periodic, t = uy > 0, b = uy + 1 < ny_u;
+    const UnitSum *c = sum + (size_t)uy * W + tx;
+    // neighbours: the wrapped unit across a periodic boundary; the unit itself
+    // where there is none (outside counts as dry, and the unit is not inside)
+    const int dl = !l ? 0 : tx > 0 ? -1 : W - 1, dr = !r ? 0 : tx + 1 < W ? 1 : 1 - W;
+    const int dt = t ? -W : 0, db = b ? W : 0;
+    const float2 v0 = c->all, v1 = c[dl].R, v2 = c[dr].L, v3 = c[dt].B, v4 = c[db].T;
+    const float2 v5 = c[dt + dl].BR, v6 = c[dt + dr].BL, v7 = c[db + dl].TR, v8 = c[db + dr].TL;
+    const float hp = s.hpos;
+    const bool deep = inside & (v0.x > hp) & (v1.x > hp) & (v2.x > hp) & (v3.x > hp) & (v4.x > hp) & (v5.x > hp) &
+                      (v6.x > hp) & (v7.x > hp) & (v8.x > hp);
+    const bool dry = (v0.y <= 0.f) & (!l | (v1.y <= 0.f)) & (!r | (v2.y <= 0.f)) & (!t | (v3.y <= 0.f)) &
+                     (!b | (v4.y <= 0.f)) & (!(t & l) | (v5.y <= 0.f)) & (!(t & r) | (v6.y <= 0.f)) &
+                     (!(b & l) | (v7.y <= 0.f)) & (!(b & r) | (v8.y <= 0.f));
+    if (advance) age = (!deep && dry) ? min(age + 1, 255) : 0;
+    if (age >= kDryAge) return kClsDry;
+    if (!deep) return kClsGeneral;
+    const float hmin = fminf(fminf(fminf(v0.x, v1.x), fminf(v2.x, v3.x)),
+                             fminf(fminf(v4.x, v5.x), fminf(fminf(v6.x, v7.x), v8.x)));
+    return kClsDeep | (hmin > 1.001f * gmax + 1e-6f ? kClsPlain : 0);
+}
+
+__device__ __forceinline__ void clear_summary(UnitSum *u)
+{
+    float2 *e = reinterpret_cast<float2 *>(u);
+#pragma unroll
+    for (int f = 0; f < 9; f++) e[f] = make_float2(FLT_MAX, -FLT_MAX);
+}
+
+__device__ __forceinline__ StepState step_state(const ScenarioCtl &c)
+{
+    return StepState{(float)c.dt, (float)(c.t * c.T), c.parity, c.status};
+}
+
+// the warp's next task of the CTA
+__device__ __forceinline__ int claim(int *next)
+{
+    int j = 0;
+    if ((threadIdx.x & 31) == 0) j = atomicAdd(next, 1);
+    return __shfl_sync(0xffffffffu, j, 0);
+}
+
+__global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const ResidentLaunch L)
+{
+    extern __shared__ __align__(16) unsigned char dsm[];
+    __shared__ bool s_ok;            // no wait has run out
+    __shared__ unsigned s_bad;       // one scenario: a value of this block is not finite
+    __shared__ unsigned s_min;       // one scenario: the step's smallest dt bound
+    __shared__ int s_next[2];        // the CTA's next task of phase 1 and 2
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int nblk = gridDim.x, NW = nblk * kResWarps;
+    const bool single = L.nslots == 1;
+    const Shared h = shared_layout(dsm, L.nslots);
+    ResidentSync *sync = L.sync;
+    Task *tasks = h.tasks;
+    unsigned char *cls = h.cls;
+    DeepRow *rows = h.rows + warp * kTaskRows;
+
+    // ---- the scenarios' descriptors and states ----
+    {
+        const int words = L.nslots * (int)(sizeof(ScenarioDev) / 4);
+        const unsigned *src = reinterpret_cast<const unsigned *>(L.tab);
+        unsigned *dst = reinterpret_cast<unsigned *>(h.tab);
+        for (int k = tid; k < words; k += kResThreads) dst[k] = __ldg(src + k);
+    }
+    if (tid == 0) {
+        s_ok = true;
+        s_bad = 0u;
+    }
+    __syncthreads();
+    for (int k = tid; k < L.nslots; k += kResThreads) {
+        h.ctl[k] = *h.tab[k].ctl;
+        h.state[k] = step_state(h.ctl[k]);
+        h.dt_bits[k] = 0x7f7fffffu;
+        if (blockIdx.x == 0) sync->dt_bits[0][k] = sync->dt_bits[1][k] = sync->dt_bits[2][k] = 0x7f7fffffu;
+    }
+    __syncthreads();
+
+    // ---- the units by class (as the classification before a chunk) ----
+    for (int base = (blockIdx.x * kResWarps + warp) * 32; base < L.nunits; base += NW * 32) {
+        const int u = base + lane;
+        int c = -1;
+        if (u < L.nunits) {
+            const int2 item = L.units[u];
+            const ScenarioDev &s = h.tab[item.x];
+            const int uy = item.y / s.tiles_x, tx = item.y - uy * s.tiles_x;
+            const int par = h.state[item.x].parity;
+            int age = s.dry_age[item.y];
+            c = unit_class(s, s.usum[par], tx, uy, 0.f, false, age) & 3;
+            // phase 1 folds its summary into the other parity's entry
+            if (c != kClsDry) clear_summary(&s.usum[par ^ 1][item.y]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            const unsigned m = __ballot_sync(0xffffffffu, c == k);
+            if (!m) continue;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&sync->counts[k], __popc(m));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (c == k) L.order[k * L.cap + at + __popc(m & ((1u << lane) - 1u))] = u;
+        }
+    }
+    int at = __ldcg(&sync->next);   // this launch's first barrier words
+    __syncthreads();
+    if (tid == 0 && !arrive_and_wait(sync->start, nblk)) s_ok = false;
+    __syncthreads();
+
+    // ---- this CTA's tasks, dealt in rounds: the general units' first, then the
+    // deep units', then the dry ones'; consecutive tasks are the same rows of
+    // different units and strips, and each round starts at another CTA, so that
+    // no CTA gets the boundary strips (the costly ones) of all its units.  Its
+    // warps claim them in this order. ----
+    int ntask, age = 0;
+    float gmax = 0.f;
+    int counted_deep = 0, counted_dry = 0;
+    {
+        const int ng = sync->counts[kClsGeneral], nd = sync->counts[kClsDeep], nz = sync->counts[kClsDry];
+        const int tg = STRIPS * (kHalfRows / L.rows_general), td = STRIPS * (kHalfRows / L.rows_deep);
+        const int total = ng * tg + nd * td + nz * tg;
+        // round k gives this CTA task k nblk + (blockIdx.x + kDealStep k) mod nblk
+        const auto dealt = [&](int k) { return k * nblk + (int)((blockIdx.x + (unsigned)kDealStep * k) % nblk); };
+        ntask = total / nblk;
+        ntask = min(kResThreads, ntask + (dealt(ntask) < total ? 1 : 0));
+        if (s_ok && tid < ntask) {
+            int i = dealt(tid), k, n = ng;
+            if (i < ng * tg) k = kClsGeneral;
+            else if ((i -= ng * tg) < nd * td) { k = kClsDeep; n = nd; }
+            else { i -= nd * td; k = kClsDry; n = nz; }
+            const int u = i % n, sub = i / n;
+            const int2 item = L.units[L.order[k * L.cap + u]];
+            const ScenarioDev &s = h.tab[item.x];
+            Task t;
+            t.slot = (short)item.x;
+            t.uy = (short)(item.y / s.tiles_x);
+            t.tx = (short)(item.y - t.uy * s.tiles_x);
+            t.sub = (unsigned char)((sub & ~3) | ((sub + u) & 3));
+            t.rows = (unsigned char)(k == kClsDeep ? L.rows_deep : L.rows_general);
+            tasks[tid] = t;
+            age = s.dry_age[item.y];
+            gmax = s.unit_gmax[item.y];
+            cls[tid] = (unsigned char)unit_class(s, s.usum[h.state[item.x].parity], t.tx, t.uy, gmax, false, age);
+        }
+        if (tid < 2) s_next[tid] = kResWarps;
+    }
+    __syncthreads();
+
+    for (int step = 0; step < L.steps && s_ok; step++) {
+        // ---- phase 1 ----
+        for (int j = warp; j < ntask; j = claim(&s_next[0])) {
+            const Task t = tasks[j];
+            const StepState q = h.state[t.slot];
+            const int c = cls[j];
+            if (q.status != kRunning || (c & 3) == kClsDry) continue;
+            const ScenarioDev &s = h.tab[t.slot];
+            const int uidx = t.uy * s.tiles_x + t.tx;
+            const int strip = t.sub & 3, y0 = t.uy * kHalfRows + (t.sub >> 2) * t.rows;
+            UnitSum *dst = &s.usum[q.parity ^ 1][uidx];
+            bool bad = false;
+            if (c & kClsDeep) {
+                float mn, mx;
+                mass_rows(s, q.parity, q.dt, q.t_sec, s.x_org + t.tx * kTileX + strip * OUTW, y0, t.rows, rows, mn, mx, bad);
+                // a deep unit reports its whole-unit {min, max} for its strips and
+                // corners too: lane f folds float f of the summary
+                if (lane < 18) {
+                    int *d = reinterpret_cast<int *>(dst) + lane;
+                    if (lane & 1) atomicMax(d, __float_as_int(mx));
+                    else atomicMin(d, __float_as_int(mn));
+                }
+            } else {
+                float local_min;
+                DepthAcc hacc;
+                bool cell;
+                int gx;
+                general_rows<1, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0,
+                                      min(y0 + t.rows, min(t.uy * kHalfRows + kHalfRows, s.ny)), local_min, hacc, bad, cell, gx);
+                const int tx0 = s.x_org + t.tx * kTileX, ux0 = max(tx0, 0), ux1 = min(tx0 + kTileX, s.nx);
+                fold_unit_summary(hacc, cell, cell && gx < ux0 + 2, cell && gx >= ux1 - 2, dst);
+            }
+            if (bad) {
+                atomicOr(&s.ctl->errors, 1u);
+                s_bad = 1u;
+            }
+        }
+        __syncthreads();
+        if (tid == 0) {
+            s_next[0] = kResWarps;
+            if (!arrive_and_wait(sync->phase1[at], nblk)) s_ok = false;
+        }
+        __syncthreads();
+        if (!s_ok) break;
+
+        // ---- classes for the state phase 1 produced (for phase 2 of this
+        // step and phase 1 of the next), one thread per task ----
+        if (tid < ntask) {
+            const Task t = tasks[tid];
+            const StepState q = h.state[t.slot];
+            if (q.status == kRunning) {
+                const ScenarioDev &s = h.tab[t.slot];
+                const int c = unit_class(s, s.usum[q.parity ^ 1], t.tx, t.uy, gmax, true, age);
+                cls[tid] = (unsigned char)c;
+                if (t.sub == 0) {
+                    // the next phase 1 folds this unit's summary into the entry
+                    // that the last classification read
+                    if (c != kClsDry) clear_summary(&s.usum[q.parity][t.uy * s.tiles_x + t.tx]);
+                    counted_deep += (c & kClsDeep) ? 1 : 0;
+                    counted_dry += c == kClsDry ? 1 : 0;
+                }
+            }
+        }
+        __syncthreads();
+
+        // ---- phase 2 ----
+        for (int j = warp; j < ntask; j = claim(&s_next[1])) {
+            const Task t = tasks[j];
+            const StepState q = h.state[t.slot];
+            const int c = cls[j];
+            if (q.status != kRunning || (c & 3) == kClsDry) continue;
+            const ScenarioDev &s = h.tab[t.slot];
+            bool bad = false;
+            float bound;
+            if (c & kClsDeep) {
+                // two pair strips; row groups of half the rows of phase 1 (a
+                // single row is not halved: half the sub-tasks step it)
+                const int half = max(t.rows >> 1, 1), g = t.sub >> 1;
+                if (g * half >= kHalfRows) continue;
+                const int x0 = s.x_org + t.tx * kTileX + (t.sub & 1) * 2 * OUTW, y0 = t.uy * kHalfRows + g * half;
+                const float m = (c & kClsPlain) ? momentum_rows<true>(s, q.parity, q.dt, x0, y0, half, rows, bad)
+                                                : momentum_rows<false>(s, q.parity, q.dt, x0, y0, half, rows, bad);
+                // (the reciprocal is monotone, so the smallest over the tasks is
+                // that of the unit's largest lam / (2 cfl area))
+                bound = (m > 0.f) ? 1.f / m : 1e30f;
+            } else {
+                const int strip = t.sub & 3, y0 = t.uy * kHalfRows + (t.sub >> 2) * t.rows;
+                DepthAcc hacc;
+                bool cell;
+                int gx;
+                general_rows<2, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0,
+                                      min(y0 + t.rows, min(t.uy * kHalfRows + kHalfRows, s.ny)), bound, hacc, bad, cell, gx);
+                bound = warp_min_bound(bound);
+            }
+            if (lane == 0) atomicMin(&h.dt_bits[t.slot], __float_as_uint(bound));
+            if (bad) {
+                atomicOr(&s.ctl->errors, 1u);
+                s_bad = 1u;
+            }
+        }
+        __syncthreads();
+        // one scenario: the block's bound goes into the barrier word (0, no valid
+        // dt, for a value that is not finite); several: into a word each
+        unsigned *gmin = sync->dt_bits[at];
+        if (!single) {
+            for (int k = tid; k < L.nslots; k += kResThreads)
+                if (h.dt_bits[k] != 0x7f7fffffu) {
+                    atomicMin(gmin + k, h.dt_bits[k]);
+                    h.dt_bits[k] = 0x7f7fffffu;
+                }
+            __syncthreads();
+        }
+        if (tid == 0) {
+            s_next[1] = kResWarps;
+            ResidentSync::Word &w = sync->phase2[at];
+            if (single) {
+                const unsigned key = 0x7f7fffffu - (s_bad ? 0u : min(h.dt_bits[0], 0x7f7fffffu));
+                if (key) atomicMax(reinterpret_cast<unsigned *>(&w.v), key);
+                h.dt_bits[0] = 0x7f7fffffu;
+            }
+            const unsigned long long v = arrive_and_wait(w, nblk);
+            if (!v) s_ok = false;
+            s_min = 0x7f7fffffu - (unsigned)v;
+        }
+        __syncthreads();
+        if (!s_ok) break;
+
+        // ---- the step's control, by every CTA for itself: a thread per
+        // scenario (the gauge samples by CTA 0) ----
+        const int clear = at == 0 ? 2 : at - 1;   // the words every CTA is done with
+        for (int k = tid; k < L.nslots; k += kResThreads) {
+            ScenarioCtl &c = h.ctl[k];
+            if (c.status != kRunning) continue;
+            const ScenarioDev &s = h.tab[k];
+            const unsigned bits = single ? s_min : __ldcg(gmin + k);
+            const unsigned errs = single ? 0u : __ldcg(&s.ctl->errors);
+            const int sample = advance_scenario(c, s, __uint_as_float(bits), errs);
+            h.state[k] = step_state(c);
+            if (blockIdx.x == 0) {
+                sync->dt_bits[clear][k] = 0x7f7fffffu;
+                if (sample >= 0) {
+                    s.gauge_ring_t[sample] = c.t * c.T;
+                    float *dst = s.gauge_ring + (size_t)sample * 4 * s.ngauges;
+                    for (int g = 0; g < s.ngauges; g++)
+                        gauge_values(s, c.parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
+                }
+            }
+        }
+        at = at == 2 ? 0 : at + 1;
+        if (blockIdx.x == 0 && tid == kResThreads - 1) {
+            sync->phase1[clear].v = sync->phase2[clear].v = sync->start.v = 0ull;
+            sync->counts[0] = sync->counts[1] = sync->counts[2] = 0;
+            sync->next = at;
+        }
+        __syncthreads();
+        // nothing left to step: every scenario of the chunk is paused or done
+        bool any = false;
+        for (int k = lane; k < L.nslots; k += 32) any |= h.state[k].status == kRunning;
+        if (!__any_sync(0xffffffffu, any)) break;
+    }
+
+    // ---- the end of the chunk: counts and control blocks back ----
+    if (s_ok && tid < ntask) {
+        const Task t = tasks[tid];
+        if (t.sub == 0) {
+            const ScenarioDev &s = h.tab[t.slot];
+            s.dry_age[t.uy * s.tiles_x + t.tx] = (unsigned char)age;
+            if (counted_deep) atomicAdd(&s.ctl->units_deep, (unsigned long long)counted_deep);
+            if (counted_dry) atomicAdd(&s.ctl->units_dry, (unsigned long long)counted_dry);
+        }
+    }
+    if (blockIdx.x != 0) return;
+    for (int k = tid; k < L.nslots; k += kResThreads) {
+        ScenarioCtl *c = h.tab[k].ctl;
+        if (s_ok) {
+            store_advanced(c, h.ctl[k]);
+        } else if (c->status == kRunning) {
+            // a barrier's wait ran out: the host reports it
+            atomicOr(&c->errors, 2u);
+            c->status = kFailed;
+        }
+    }
+}
+
+}  // namespace
+
+int resident_warps(int sms) { return sms * kResWarps; }
+int resident_tasks_capacity(int warps) { return warps * 32; }
+
+cudaError_t configure_resident_kernel()
+{
+    return cudaFuncSetAttribute(resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)shared_bytes(kResidentSlots));
+}
+
+cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st)
+{
+    void *args[] = {const_cast<ResidentLaunch *>(&L)};
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(resident_kernel), dim3(sms), dim3(kResThreads), args,
+                                       shared_bytes(L.nslots), st);
+}
+
+}  // namespace thy

@@ -9,7 +9,8 @@
 // synchronisation per chunk instead of one blocking copy per step.  When an
 // event is due (fault time, snapshot time, gauge time) the controller pauses
 // the scenario; later launches of the chunk do nothing for it, and the host
-// performs the event exactly at that step before resuming.
+// performs the event exactly at that step before resuming.  Work that does not
+// fill the GPU takes its chunks as one resident launch each (resident.cu).
 #include "engine.h"
 #include "tuner.h"
 
@@ -55,6 +56,7 @@ int ensure_device()
     THY_CK(cudaSetDevice(g_device));
     if (!g_configured[g_device]) {
         THY_CK(configure_step_kernels());
+        THY_CK(configure_resident_kernel());
         THY_CK(preload_output_kernels());
         THY_CK(preload_okada_kernels());
         // device buffers come from the stream-ordered default pool; freed
@@ -802,6 +804,10 @@ Batch::~Batch()
     if (d_nwork0) cudaFreeAsync(d_nwork0, st);
     if (d_lists) cudaFreeAsync(d_lists, st);
     if (d_claims) cudaFreeAsync(d_claims, st);
+    if (d_rtab) cudaFreeAsync(d_rtab, st);
+    if (d_runits) cudaFreeAsync(d_runits, st);
+    if (d_rorder) cudaFreeAsync(d_rorder, st);
+    if (d_rsync) cudaFreeAsync(d_rsync, st);
     if (d_ctl) cudaFreeAsync(d_ctl, st);
     pinned_free(h_ctl);
     if (ev0) cudaEventDestroy(ev0);
@@ -931,6 +937,11 @@ int Batch::init(int cap, int max_work, cudaStream_t stream)
     THY_CK(cudaMemsetAsync(d_lists, 0, 2 * sizeof(int), st));
     THY_CK(cudaMallocAsync(&d_claims, 4 * sizeof(int), st));
     THY_CK(cudaMemsetAsync(d_claims, 0, 4 * sizeof(int), st));
+    THY_CK(cudaMallocAsync(&d_rtab, kResidentSlots * sizeof(ScenarioDev), st));
+    THY_CK(cudaMallocAsync(&d_runits, kResidentUnits * sizeof(int2), st));
+    THY_CK(cudaMallocAsync(&d_rorder, 3 * kResidentUnits * sizeof(int), st));
+    THY_CK(cudaMallocAsync(&d_rsync, sizeof(ResidentSync), st));
+    THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
     THY_CK(cudaEventCreate(&ev0));
     THY_CK(cudaEventCreate(&ev1));
     THY_CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
@@ -975,11 +986,15 @@ int Batch::update(const std::vector<char> *selected)
 {
     std::vector<ScenarioDev> table(capacity);
     std::vector<int2> work;
+    std::vector<ScenarioDev> rtab;
+    long long runits = 0;
     for (int i = 0; i < capacity; i++) {
         if (!members[i]) continue;
         table[i] = members[i]->desc;
         if (selected && !(*selected)[i]) continue;
         for (int t = 0; t < members[i]->desc.ntiles; t++) work.push_back(make_int2(i, t));
+        rtab.push_back(members[i]->desc);
+        runits += members[i]->units();
     }
     if ((int)work.size() > work_capacity) {
         // the captured graph holds the list pointers: grow, then recapture
@@ -997,8 +1012,23 @@ int Batch::update(const std::vector<char> *selected)
     THY_CK(cudaMemcpyAsync(d_table, table.data(), capacity * sizeof(ScenarioDev), cudaMemcpyHostToDevice, st));
     if (nwork) THY_CK(cudaMemcpyAsync(d_work, work.data(), nwork * sizeof(int2), cudaMemcpyHostToDevice, st));
     THY_CK(cudaMemcpyAsync(d_nwork, &nwork, sizeof(int), cudaMemcpyHostToDevice, st));
+    // the same work for resident chunks, where it is small enough
+    const bool fits = !rtab.empty() && rtab.size() <= kResidentSlots && runits <= kResidentUnits;
+    res_slots = fits ? (int)rtab.size() : 0;
+    res_units = fits ? (int)runits : 0;
+    std::vector<int2> units;
+    if (fits) {
+        for (int i = 0; i < res_slots; i++) {
+            const ScenarioDev &d = rtab[i];
+            const int n = d.tiles_x * ((d.ny + kHalfRows - 1) / kHalfRows);
+            for (int u = 0; u < n; u++) units.push_back(make_int2(i, u));
+        }
+        THY_CK(cudaMemcpyAsync(d_rtab, rtab.data(), res_slots * sizeof(ScenarioDev), cudaMemcpyHostToDevice, st));
+        THY_CK(cudaMemcpyAsync(d_runits, units.data(), res_units * sizeof(int2), cudaMemcpyHostToDevice, st));
+    }
     THY_CK(cudaStreamSynchronize(st));
-    return reset_lists();
+    reset_lists();
+    return THY_OK;
 }
 
 void Batch::drop_graphs()
@@ -1089,6 +1119,7 @@ int Batch::rebuild()
     // the work now attached), a full chunk and one step, so that no capture
     // falls into the time loop of a run whose work needs no tuning
     bool sampling = false, known = false;
+    if (resident()) return THY_OK;
     if ((rc = use_tiling(tuner_pick(tune_key(&known), &sampling)))) return rc;
     for (const auto &g : graphs)
         if (g.tiling == tiling && g.len == 1) return THY_OK;
@@ -1118,10 +1149,63 @@ StepLaunch Batch::params() const
     return L;
 }
 
-int Batch::reset_lists()
+int Batch::fresh_lists()
 {
+    if (!lists_stale) return THY_OK;
     launch_lists_current(params(), st);
     THY_CK(cudaGetLastError());
+    lists_stale = false;
+    return THY_OK;
+}
+
+// Resident chunks step work of up to kResidentUnits units; a forced or default
+// tiling (THY_TILING, THY_TUNE=0, thy_tiling_force) names the launched kernels,
+// and the staging-copy test hook has nothing to withhold in a resident chunk.
+bool Batch::resident() const
+{
+    if (res_units == 0 || !tuner_free()) return false;
+    for (auto *m : members)
+        if (m && (m->hctl.inject & 1)) return false;
+    return true;
+}
+
+// Rows of the tasks of a resident chunk: the fewest general rows (1, 2, 4, 8)
+// that leave a warp at most five tasks, and twice as many deep rows.  Short tasks
+// shorten a step's chain while warps are idle; each evaluates one y edge row more
+// than it has rows, which costs more once every warp has several.  (us per step,
+// 148 SMs, general rows 1 / 2 / 4 / 8: 56 units 16.3 / 19.5 / 27.0 / 42.6; 192
+// units 24.7 / 23.9 / 31.5 / 46.5; 231 units 35.1 / 29.8 / 30.7 / 45.2; 704 units
+// 55.2 / 47.2 / 44.1 / 50.4.)  Work the tuner searches takes its variants of the
+// general kernel and of deep phase 2 as half and double the rows.
+static void resident_rows(int units, int warps, const Tiling &t, int *general, int *deep)
+{
+    int r = 1;
+    while (r < 8 && units * (64 / r) > 5 * warps) r *= 2;
+    const auto variant = [](int rows, int v) { return std::min(8, std::max(1, v == 1 ? 2 * rows : v == 2 ? rows / 2 : rows)); };
+    *general = variant(r, t.general);
+    *deep = variant(std::min(8, 2 * r), t.deep2);
+    // (a CTA holds one task a thread)
+    while (units * (64 / std::min(*general, *deep)) > resident_tasks_capacity(warps)) {
+        *general = std::min(8, 2 * *general);
+        *deep = std::min(8, 2 * *deep);
+    }
+}
+
+int Batch::run_resident(int len, const Tiling &rows)
+{
+    const int sms = device_sm_count();
+    ResidentLaunch R;
+    R.tab = d_rtab;
+    R.units = d_runits;
+    R.order = d_rorder;
+    R.sync = d_rsync;
+    R.nslots = res_slots;
+    R.nunits = res_units;
+    R.cap = kResidentUnits;
+    R.steps = len;
+    resident_rows(res_units, resident_warps(sms), rows, &R.rows_general, &R.rows_deep);
+    THY_CK(launch_resident(R, sms, st));
+    lists_stale = true;
     return THY_OK;
 }
 
@@ -1145,12 +1229,19 @@ int Batch::run_chunk(bool timed, int len)
     bool sampling = false, known = false;
     if (len <= 0 || len > chunk) len = chunk;
     const TuneKey key = tune_key(&known);
-    if ((rc = use_tiling(tuner_pick(key, &sampling)))) return rc;
+    const Tiling pick = tuner_pick(key, &sampling);
+    const bool res = resident();
+    if (res) {
+        tiling = pick;
+        gexec = nullptr;
+    } else if ((rc = use_tiling(pick)) || (rc = fresh_lists())) {
+        return rc;
+    }
     // a full chunk is one graph launch; a shorter one launches the 1-step
     // graph `len` times (two captures per tiling in all)
     cudaGraphExec_t exec = gexec;
     int repeat = 1;
-    if (len != chunk) {
+    if (!res && len != chunk) {
         exec = nullptr;
         for (auto &g : graphs)
             if (g.tiling == tiling && g.len == 1) exec = g.exec;
@@ -1175,7 +1266,11 @@ int Batch::run_chunk(bool timed, int len)
             running++;
         }
     if (timed) THY_CK(cudaEventRecord(ev0, st));
-    for (int i = 0; i < repeat; i++) THY_CK(cudaGraphLaunch(exec, st));
+    if (res) {
+        if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling()))) return rc;
+    } else {
+        for (int i = 0; i < repeat; i++) THY_CK(cudaGraphLaunch(exec, st));
+    }
     if (timed) THY_CK(cudaEventRecord(ev1, st));
     THY_CK(cudaMemcpyAsync(h_ctl, d_ctl, capacity * sizeof(ScenarioCtl), cudaMemcpyDeviceToHost, st));
     THY_CK(cudaStreamSynchronize(st));
@@ -1184,7 +1279,7 @@ int Batch::run_chunk(bool timed, int len)
         THY_CK(cudaEventElapsedTime(&ms, ev0, ev1));
         device_ms += ms;
     }
-    launches += (long long)kLaunchesPerStep * len;
+    launches += res ? 1 : (long long)kLaunchesPerStep * len;
     chunks_run++;
     bool full = running > 0 && len == chunk;
     double stepped = 0;   // deep + general units stepped in the chunk
@@ -1195,6 +1290,8 @@ int Batch::run_chunk(bool timed, int len)
         if (b0[i].step < 0) continue;
         const long long k = m->hctl.step - b0[i].step;
         if (m->hctl.status == kFailed || k != chunk) full = false;
+        // (a resident chunk that gave up a barrier leaves its words behind)
+        if (res && (m->hctl.errors & 2u)) THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
         if (k > 0) {
             const double deep = (double)(m->hctl.units_deep - b0[i].deep);
             const double dry = (double)(m->hctl.units_dry - b0[i].dry);
@@ -1403,7 +1500,7 @@ extern "C" int thy_run(const thy_problem *p, const thy_outputs *o, thy_stats *st
                 const auto te = std::chrono::steady_clock::now();
                 bool changed = false;
                 if ((rc = handle_events_ex(s, o, st, &changed))) goto out;
-                if (changed && (rc = b.reset_lists())) goto out;
+                if (changed) b.reset_lists();
                 event_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - te).count();
             }
             s.hctl.status = kRunning;
@@ -1488,12 +1585,13 @@ extern "C" int thy_session_open(const thy_problem *p, thy_session **out)
     q.max_steps = 0;
     if ((rc = S->b.init(1, (p->nx / kTileX + 2) * (p->ny / kTileY + 2), S->st)) || (rc = S->b.attach(&S->s)) ||
         (rc = S->s.setup(&q, S->st)) || (rc = S->b.rebuild()) || (rc = initial_dt(S->b)) ||
-        (rc = S->s.apply_due_faults(S->st)) || (rc = S->b.reset_lists())) {
+        (rc = S->s.apply_due_faults(S->st))) {
         cudaStream_t st = S->st;
         delete S;
         cudaStreamDestroy(st);
         return rc;
     }
+    S->b.reset_lists();
     *out = S;
     return THY_OK;
 }
@@ -1538,7 +1636,7 @@ extern "C" int thy_session_profile_launches(thy_session *S, long long steps, dou
     s.hctl.max_steps = s.hctl.step + steps;
     s.hctl.status = kRunning;
     s.hctl.events = 0;
-    if ((rc = s.upload_ctl(S->st))) return rc;
+    if ((rc = s.upload_ctl(S->st)) || (rc = b.fresh_lists())) return rc;
     std::vector<cudaEvent_t> ev((NL + 1) * steps);
     for (auto &e : ev) THY_CK(cudaEventCreate(&e));
     for (long long k = 0; k < steps; k++) {

@@ -110,6 +110,14 @@ struct Batch {
     int *d_nwork0 = nullptr;
     int *d_lists = nullptr;            // deep / general lists of the current step (StepLaunch::lists)
     int *d_claims = nullptr;           // StepLaunch::claims
+    // resident chunks (kernels/resident.cu), for work of up to kResidentUnits
+    // units: the stepped members' descriptors and units, packed; scratch
+    ScenarioDev *d_rtab = nullptr;
+    int2 *d_runits = nullptr;
+    int *d_rorder = nullptr;
+    ResidentSync *d_rsync = nullptr;
+    int res_slots = 0, res_units = 0;  // of the current work list (0: too much work)
+    bool lists_stale = false;          // d_lists not made for the current states (made when a step is launched)
     ScenarioCtl *d_ctl = nullptr;      // slots
     ScenarioCtl *h_ctl = nullptr;      // pinned mirror
     int capacity = 0;
@@ -146,7 +154,7 @@ struct Batch {
     int attach(DevScenario *s);      // gives s a control slot
     int detach(DevScenario *s);
     // upload the member table and the work list (of the members with
-    // selected[slot] != 0, all of them without a selection) and classify
+    // selected[slot] != 0, all of them without a selection)
     int update(const std::vector<char> *selected = nullptr);
     // (re)capture the `len`-step graph of `tiling` for the current capacity
     // (len 0: the full chunk, which becomes gexec)
@@ -156,7 +164,8 @@ struct Batch {
     int rebuild();                    // update(), and capture() when there is no graph yet
     int initial_dt_of(DevScenario *s);   // initial dt of one member (phase 0 over its units only)
     // `len` steps (0 or more than `chunk`: the full chunk, one graph launch;
-    // fewer: the 1-step graph launched len times) + control download
+    // fewer: the 1-step graph launched len times; one launch for a resident
+    // chunk) + control download
     // (synchronous); the tiling is the autotuner's pick, and a full timed
     // chunk is one of its samples
     int run_chunk(bool timed, int len = 0);
@@ -171,8 +180,17 @@ struct Batch {
     // *known: each of them has been measured
     TuneKey tune_key(bool *known = nullptr, bool all_members = false) const;
     StepLaunch params() const;
-    int reset_lists();               // classify again: after the host changed a member's state
+    void reset_lists() { lists_stale = true; }   // classify again: after the host changed a member's state
+    int fresh_lists();               // the classification, if it is due (before a launch of the stepping kernels)
+    bool resident() const;           // the next chunk is one resident launch
+    int run_resident(int len, const Tiling &rows);
 };
+
+// Largest work of a resident chunk, in units (us a step resident / launched: 704
+// units 44 / 70, 1600 units 78 / 95, 2034 units 99 / 103, 2560 units 126 / 113:
+// the launched kernels stage the deep units, which pays once every SM has enough
+// of them to hide the launches).
+constexpr int kResidentUnits = 2048;
 
 // Single-scenario batches of thy_run, kept per device between runs with
 // their buffers, stream and captured graphs, so that a run of a grid size the

@@ -317,11 +317,10 @@ extern "C" int thy_server_progress(thy_server *S, int *active)
     if (S->members_changed || sel != S->selected) {
         // table + the work list of the stepped scenarios, classified for their current states
         if ((rc = S->b.update(&sel))) return rc;
-        if (!S->b.gexec && (rc = S->b.capture())) return rc;   // the list outgrew its capacity
         S->members_changed = false;
         S->selected = sel;
     } else if (state_changed) {
-        if ((rc = S->b.reset_lists())) return rc;
+        S->b.reset_lists();
     }
     if (any_running) {
         // no longer than the steps the first stepped scenario has left

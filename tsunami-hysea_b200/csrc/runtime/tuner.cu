@@ -233,6 +233,16 @@ void tuner_force(const Tiling *t)
     if (t) s.force = *t;
 }
 
+bool tuner_free()
+{
+    State &s = state();
+    std::lock_guard<std::mutex> g(s.mu);
+    read_env(s);
+    return !s.forced && !s.off;
+}
+
+bool tuner_searches(const TuneKey &k) { return tuner_free() && !small_work(k); }
+
 void tuner_clear()
 {
     State &s = state();

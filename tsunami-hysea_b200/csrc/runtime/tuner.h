@@ -13,7 +13,9 @@
 //
 // Steps of at most 512 work units are not tuned: they run the tiling with
 // the most row groups in the phase-2 kernels (deep 1 default, deep 2 and
-// general variant 2).
+// general variant 2).  Chunks that stay resident on the device (resident.cu)
+// take the variants of deep phase 2 and of the general kernel as the rows of
+// their tasks (Batch::run_resident), small ones a fixed choice.
 //
 // Environment: THY_TILING="d1,d2,g" forces a tiling (variant indices);
 // THY_TUNE=0 keeps the default tiling; THY_TUNE_CACHE=<file> keeps decided
@@ -41,6 +43,8 @@ Tiling tuner_pick(const TuneKey &k, bool *sampling);
 void tuner_sample(const TuneKey &k, const Tiling &t, double ms_per_unit_step);
 bool tuner_decided(const TuneKey &k, Tiling *best);
 void tuner_force(const Tiling *t);                   // nullptr: tune again
+bool tuner_free();                                   // no tiling forced, tuning not off
+bool tuner_searches(const TuneKey &k);               // ... and this work is searched, not small
 void tuner_clear();                                  // forget every key (not the cache file)
 
 }  // namespace thy
