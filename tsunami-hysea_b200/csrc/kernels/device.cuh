@@ -74,7 +74,7 @@ struct ScenarioCtl {
 // Gauge samples taken on the device between two reads by the host: at most
 // one per step, and the host reads them after every chunk of at most
 // kGaugeRing steps.
-constexpr int kGaugeRing = 32;
+constexpr int kGaugeRing = 64;
 
 // Opaque 128-byte TMA tensor map (CUtensorMap), 64-byte aligned in device memory.
 struct alignas(64) TmaMap {

@@ -1109,7 +1109,9 @@ long long Batch::steps_to_event(const DevScenario &s)
     return std::max(1ll, n);
 }
 
-int Batch::chunk_for(long long steps) const { return (int)std::max(1ll, std::min<long long>(steps, chunk)); }
+int Batch::max_chunk() const { return resident() && !tuner_searches(tune_key()) ? kResidentChunk : chunk; }
+
+int Batch::chunk_for(long long steps) const { return (int)std::max(1ll, std::min<long long>(steps, max_chunk())); }
 
 int Batch::rebuild()
 {
@@ -1227,7 +1229,7 @@ int Batch::run_chunk(bool timed, int len)
 {
     int rc;
     bool sampling = false, known = false;
-    if (len <= 0 || len > chunk) len = chunk;
+    if (len <= 0 || len > max_chunk()) len = chunk;
     const TuneKey key = tune_key(&known);
     const Tiling pick = tuner_pick(key, &sampling);
     const bool res = resident();

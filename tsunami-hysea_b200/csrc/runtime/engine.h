@@ -172,8 +172,11 @@ struct Batch {
     // steps a member can take before its next event or its end, estimated
     // from its current dt (at least 1)
     static long long steps_to_event(const DevScenario &s);
-    // the chunk length for `steps` steps: at most `chunk`, at least 1
+    // the chunk length for `steps` steps: at least 1, at most `chunk`, or
+    // kResidentChunk where the chunk is one resident launch and not a sample of
+    // the tuner's
     int chunk_for(long long steps) const;
+    int max_chunk() const;
     // the autotuner's key of the next chunk: this device, the deep and
     // general units per step estimated from each stepping member's last
     // chunk (members with status running; every member when all_members);
@@ -191,6 +194,11 @@ struct Batch {
 // the launched kernels stage the deep units, which pays once every SM has enough
 // of them to hide the launches).
 constexpr int kResidentUnits = 2048;
+// Longest resident chunk.  Between chunks the GPU waits for the host (the
+// control blocks' copy, a launch: about 40 us, as long as one or two steps of this
+// work); the steps between them are kept by the gauge ring.
+constexpr int kResidentChunk = 64;
+static_assert(kResidentChunk <= kGaugeRing, "at most one gauge sample a step");
 
 // Single-scenario batches of thy_run, kept per device between runs with
 // their buffers, stream and captured graphs, so that a run of a grid size the
