@@ -110,13 +110,13 @@ struct ResidentSync {
     };
     Word start, phase1[3], phase2[3];   // by step modulo 3, counted on from launch to launch
     int next;                           // the next launch's first step, modulo 3
-    int counts[3];                      // units by class at the start of the chunk
+    int counts[4];                      // units per list at the start of the chunk
     unsigned int dt_bits[3][kResidentSlots];   // several scenarios: their smallest dt bounds
 };
 struct ResidentLaunch {
     const ScenarioDev *tab;    // the stepped scenarios (nslots of them)
     const int2 *units;         // their work units: (index into tab, unit)
-    int *order;                // scratch, 3 x cap: the units by class
+    int *order;                // scratch, 4 x cap: the units by class
     ResidentSync *sync;
     int nslots, nunits, cap, steps;
     int rows_general, rows_deep;   // rows of a task: 1, 2, 4 or 8

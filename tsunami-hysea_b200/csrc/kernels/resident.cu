@@ -8,7 +8,8 @@
 // chunk with the scenarios' descriptors in shared memory, and a step is
 //     phase 1 | grid barrier | classes, phase 2 | grid barrier, control
 // A task is a column strip of a unit and a few of its rows.  The tasks are dealt
-// to the CTAs once per chunk, general units first (they cost most), and a CTA's
+// to the CTAs once per chunk, by falling cost (shallow general units, the other
+// general ones, deep units), and a CTA's
 // warps claim them from shared memory.  The classes that the classification
 // launch would list are evaluated in place, one thread per task of the CTA, so
 // that a step has no list to build; a unit that changes class during the chunk is
@@ -19,8 +20,10 @@
 // What bounds it now: the chain of a task's edges (about 3.8 us a row of WAF
 // edges in both phases on an otherwise idle SM), two barriers of 1.3 us, and the
 // spread of the tasks' costs over the SMs.  us a step, launched -> resident:
-// 96 x 80 28 -> 14, 512^2 48 -> 24, 1024^2 70 -> 44, 1600^2 95 -> 78.
-//
+// 96 x 80 28 -> 14, 512^2 48 -> 24, 1024^2 70 -> 40, 1600^2 94 -> 70, 2048^2
+// 113 -> 104.  Deep rows go in column pairs in both phases: packed arithmetic
+// and half the loads and stores of one column a lane (phase 1 with one column a
+// lane: 1024^2 44.5, 2048^2 126).
 // Arithmetic, classes, depth summaries, dry counts and the control are those
 // of the launches in step.cu; results are bitwise the same.
 //
@@ -39,7 +42,9 @@ constexpr int kMaxDeepRows = 8;     // rows of a deep task at most
 constexpr int kTaskRows = kMaxDeepRows + 2;
 constexpr int kDealStep = 61;       // odd: units of one column of a grid alternate in the lists
 
-enum : int { kClsGeneral = 0, kClsDeep = 1, kClsDry = 2, kClsPlain = 4 };   // kClsPlain: a flag of deep units
+// classes of a unit; kClsPlain: a flag of deep units; kClsShallow: a flag of
+// general units with water no deeper than hpos (their edges take the costly path)
+enum : int { kClsGeneral = 0, kClsDeep = 1, kClsDry = 2, kClsPlain = 4, kClsShallow = 8 };
 
 // the step state of a scenario
 struct alignas(16) StepState {
@@ -47,11 +52,26 @@ struct alignas(16) StepState {
     int parity, status;
 };
 
-// a task of one warp: unit (tx, uy) of scenario `slot`, its sub-task and the rows of one
+// A task of one warp: unit (tx, uy) of scenario `slot`, its sub-task and the rows
+// of one.  Sub-tasks are (strip of 28 columns) + 4 (row group), or, of the units
+// that were deep when the tasks were dealt (kPairTask in rows), (strip of 56
+// columns) + 2 (row group).  A unit whose class has changed is covered by the
+// same sub-tasks: a deep unit by strips of 56 and half the rows, a general one by
+// both strips of 28 in turn.
+constexpr int kPairTask = 0x80;
 struct Task {
     short slot, tx, uy;
     unsigned char sub, rows;
+    __device__ __forceinline__ bool pair() const { return (rows & kPairTask) != 0; }
+    __device__ __forceinline__ int nrows() const { return rows & (kPairTask - 1); }
 };
+// the deep rows of a task: first row in the unit and rows (0: covered by others)
+__device__ __forceinline__ int2 deep_rows(const Task &t)
+{
+    if (t.pair()) return make_int2((t.sub >> 1) * t.nrows(), t.nrows());
+    const int half = max(t.nrows() >> 1, 1), y = (t.sub >> 1) * half;   // (a single row is not halved)
+    return make_int2(y, y < kHalfRows ? half : 0);
+}
 
 struct Shared {
     ScenarioDev *tab;      // nslots
@@ -126,99 +146,101 @@ __device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word
 // few rows, and the state of this work stays in L2.
 // ---------------------------------------------------------------------------
 
-// phase 1: columns x0 .. x0+27, rows y0 .. y0+nrows-1; the warp's depth {min, max}
+// the loads of a row of column pairs that is still in flight
+struct Raw2 {
+    float2 e, D, qx, qy;
+};
+__device__ __forceinline__ Raw2 load_raw2(const float *eta, const float *dep, const float *qx, const float *qy, size_t off)
+{
+    Raw2 c;
+    c.e = *reinterpret_cast<const float2 *>(eta + off);
+    c.D = *reinterpret_cast<const float2 *>(dep + off);
+    c.qx = *reinterpret_cast<const float2 *>(qx + off);
+    c.qy = *reinterpret_cast<const float2 *>(qy + off);
+    return c;
+}
+__device__ __forceinline__ Cell2 cell2(const Raw2 &r)
+{
+    return Cell2{add2(r.e, r.D), r.e, r.D, r.qx, r.qy};
+}
+
+// Column pairs: lane l holds columns x0 - 2 + 2l and the next one (x0 even) of a
+// strip of 56 columns; lanes 1..28 are cells, lanes 0 and 29 the halo, lanes 30
+// and 31 repeat lane 29.
+
+// phase 1: columns x0 .. x0+55, rows y0 .. y0+nrows-1; the warp's depth {min, max}
 __device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt, float t_sec, int x0, int y0, int nrows,
                                           DeepRow *rows, float &mn, float &mx, bool &bad)
 {
     const int lane = threadIdx.x & 31;
     const size_t pitch = (size_t)s.pitch;
-    const int gx = x0 - 2 + lane;
-    const bool has_cell = (lane >= 2) && (lane <= 29);
+    const bool out_lane = (lane >= 1) && (lane <= 28);
     const float *eta = s.eta[p], *qx = s.qx[p], *qy = s.qy[p];
     float *out = s.eta[p ^ 1];
-    size_t off = (size_t)y0 * pitch + gx;
+    size_t off = (size_t)y0 * pitch + x0 - 2 + 2 * min(lane, 29);
+    const Raw2 ra = load_raw2(eta, s.dep, qx, qy, off - pitch), rc = load_raw2(eta, s.dep, qx, qy, off);
+    Raw2 rn = load_raw2(eta, s.dep, qx, qy, off + pitch);
     // row y0 - 1 + t of the window at rows[t]
     if (lane < nrows + 2) {
-        DeepRow r;
-        r.m = __ldg(s.rowpack + y0 - 1 + lane);
-        r.icos = __frcp_rn(r.m.x);
-        r.dtA = __fdividef(dt, r.m.z);
-        rows[lane].m = r.m;
-        rows[lane].icos = r.icos;
-        rows[lane].dtA = r.dtA;
-    }
-    const Cell a = load_cell<true>(eta, s.dep, qx, qy, off - pitch);
-    Cell c = load_cell<true>(eta, s.dep, qx, qy, off);
-    Cell n = load_cell<true>(eta, s.dep, qx, qy, off + pitch);
-    float em = 0.f, ar = 0.f, ei = 0.f;
-    if (has_cell) {
-        em = s.eta_max[off];
-        ar = s.arr[off];
-        ei = s.eta_ini[off];
+        const float4 m = __ldg(s.rowpack + y0 - 1 + lane);
+        rows[lane].m = m;
+        rows[lane].icos = __frcp_rn(m.x);
+        rows[lane].dtA = __fdividef(dt, m.z);
     }
     __syncwarp();
-    float4 mc = rows[1].m;
-    float icos_c = rows[1].icos, top;
-    {
-        const float4 ma = rows[0].m;
-        top = mul(mass_2s_y(a.qy, mc.w, ma.x, mc.x, a.h, c.h, dt, ma.z, mc.z), icos_c);
-    }
+    Cell2 c = cell2(rc);
+    float2 top = mul2(mass_y2(cell2(ra), c, rows[0].m, rows[1].m, dt), bc2(rows[1].icos));
     mn = FLT_MAX;
     mx = -FLT_MAX;
+    float2 fin = make_float2(0.f, 0.f);   // running sum: non-finite iff a new value is
+#pragma unroll 1
     for (int k = 0; k < nrows; k++, off += pitch) {
-        const float4 mr = rows[k + 2].m;
-        const float icos_n = rows[k + 2].icos;
-        // the row after the next one and the next row's diagnostics
-        Cell nn = n;
-        float em1 = 0.f, ar1 = 0.f, ei1 = 0.f;
-        if (k + 1 < nrows) {
-            nn = load_cell<true>(eta, s.dep, qx, qy, off + 2 * pitch);
-            if (has_cell) {
-                em1 = s.eta_max[off + pitch];
-                ar1 = s.arr[off + pitch];
-                ei1 = s.eta_ini[off + pitch];
-            }
+        // the row after the next one; this row's diagnostics
+        Raw2 rnn = rn;
+        if (k + 1 < nrows) rnn = load_raw2(eta, s.dep, qx, qy, off + 2 * pitch);
+        float2 em, ar, ei;
+        if (out_lane) {
+            em = *reinterpret_cast<const float2 *>(s.eta_max + off);
+            ar = *reinterpret_cast<const float2 *>(s.arr + off);
+            ei = *reinterpret_cast<const float2 *>(s.eta_ini + off);
         }
-        const float Fb = mass_2s_y(c.qy, mr.w, mc.x, mr.x, c.h, n.h, dt, mc.z, mr.z);
-        const float F = mass_2s_x(shup(c.qx, 1), mc.y, shup(c.h, 1), c.h, dt, mc.z, mc.z);
-        const float Fr = shdn(F, 1);
-        if (has_cell) {
-            if (c.e > em && c.h > s.eps_h) s.eta_max[off] = c.e;
-            if (ar < 0.f && fabsf(c.e - ei) > s.dif_at) s.arr[off] = t_sec;
-            const float e = deep_eta(c, F, Fr, top, Fb, icos_c, rows[k + 1].dtA);
-            if (!isfinite(e)) bad = true;
-            out[off] = e;
-            mn = fminf(mn, e + c.D);
-            mx = fmaxf(mx, e + c.D);
+        const Cell2 n = cell2(rn);
+        const float4 mk = rows[k + 1].m;
+        // mass fluxes below the row, left of and between the lane's columns
+        const float2 Fb = mass_y2(c, n, mk, rows[k + 2].m, dt);
+        const float2 lq = make_float2(shup(c.qx.y, 1), c.qx.x), lh = make_float2(shup(c.h.y, 1), c.h.x);
+        const float2 F = limit2(mul2(lq, bc2(mk.y)), lh, c.h, 1.f, 1.f, mk.z, mk.z, dt, mk.z);
+        const float2 Fr = make_float2(F.y, shdn(F.x, 1));
+        // mass update (src/GPU/Volumen_kernel.cu:111-157)
+        const float2 acc = fma2(neg2(Fb), bc2(rows[k + 1].icos), add2(sub2(F, Fr), top));
+        top = mul2(Fb, bc2(rows[k + 2].icos));
+        float2 e = fma2(bc2(rows[k + 1].dtA), acc, c.e);
+        float2 h = add2(e, c.D);
+        e = sel2(h.x > 0.f, h.y > 0.f, e, neg2(c.D));
+        if (out_lane) {
+            h = add2(e, c.D);
+            fin = add2(fin, e);
+            *reinterpret_cast<float2 *>(out + off) = e;
+            mn = fminf(mn, fminf(h.x, h.y));
+            mx = fmaxf(mx, fmaxf(h.x, h.y));
+            // diagnostics of the state the step starts from (src/GPU/Metrics.cu:23-77)
+            if (c.e.x > em.x && c.h.x > s.eps_h) s.eta_max[off] = c.e.x;
+            if (c.e.y > em.y && c.h.y > s.eps_h) s.eta_max[off + 1] = c.e.y;
+            if (ar.x < 0.f && fabsf(c.e.x - ei.x) > s.dif_at) s.arr[off] = t_sec;
+            if (ar.y < 0.f && fabsf(c.e.y - ei.y) > s.dif_at) s.arr[off + 1] = t_sec;
         }
-        top = mul(Fb, icos_n);
         c = n;
-        n = nn;
-        mc = mr;
-        icos_c = icos_n;
-        em = em1;
-        ar = ar1;
-        ei = ei1;
+        rn = rnn;
     }
-    const float2 v = warp_minmax(mn, mx, has_cell);
+    bad = !isfinite(fin.x) || !isfinite(fin.y);
+    const float2 v = warp_minmax(mn, mx, out_lane);
     mn = v.x;
     mx = v.y;
     __syncwarp();   // rows is reused by the warp's next task
 }
 
-__device__ __forceinline__ Cell2 load_cell2(const float *eta, const float *dep, const float *qx, const float *qy, size_t off)
-{
-    Cell2 c;
-    c.e = *reinterpret_cast<const float2 *>(eta + off);
-    c.D = *reinterpret_cast<const float2 *>(dep + off);
-    c.qx = *reinterpret_cast<const float2 *>(qx + off);
-    c.qy = *reinterpret_cast<const float2 *>(qy + off);
-    c.h = add2(c.e, c.D);
-    return c;
-}
-
-// phase 2 in column pairs: columns x0 .. x0+55 (x0 even), rows y0 ..
-// y0+nrows-1; the warp's largest lam / (2 cfl area)
+// phase 2: columns x0 .. x0+55, rows y0 .. y0+nrows-1; the warp's largest lam /
+// (2 cfl area)
 template <bool PLAIN>
 __device__ __forceinline__ float momentum_rows(const ScenarioDev &s, int p, float dt, int x0, int y0, int nrows, DeepRow *rows,
                                                bool &bad)
@@ -229,68 +251,45 @@ __device__ __forceinline__ float momentum_rows(const ScenarioDev &s, int p, floa
     const float *eta = s.eta[p ^ 1], *qx_in = s.qx[p], *qy_in = s.qy[p];
     float *qx_out = s.qx[p ^ 1], *qy_out = s.qy[p ^ 1];
     size_t off = (size_t)y0 * pitch + x0 - 2 + 2 * min(lane, 29);
-    const Cell2 a = load_cell2(eta, s.dep, qx_in, qy_in, off - pitch);
-    Cell2 c = load_cell2(eta, s.dep, qx_in, qy_in, off);
-    Cell2 n = load_cell2(eta, s.dep, qx_in, qy_in, off + pitch);
-    if (lane < nrows + 2) {
-        DeepRow r;
-        r.m = __ldg(s.rowpack + y0 - 1 + lane);
-        const float4 ra = __ldg(s.rowpack + y0 - 2 + lane);   // the row above
-        r.icos = __frcp_rn(r.m.x);
-        r.dtA = __fdividef(dt, r.m.z);
-        r.kcfl = 1.f / (2.f * s.cfl * r.m.z);
-        r.kdx = make_xrow(r.m.y, r.m.z + r.m.z, dt, s.cvis).kdes;
-        const YRowK k = make_yrow(ra.x, r.m.x, __frcp_rn(ra.x), r.icos, r.m.w, ra.z + r.m.z, dt, s.cvis);
-        r.y0 = make_float4(k.len, k.cmid, k.cdiff, k.c10);
-        r.y1 = make_float4(k.c01, k.li0, k.kdes0, k.kdes1);
-        rows[lane] = r;
-    }
+    const Raw2 ra = load_raw2(eta, s.dep, qx_in, qy_in, off - pitch), rc = load_raw2(eta, s.dep, qx_in, qy_in, off);
+    Raw2 rn = load_raw2(eta, s.dep, qx_in, qy_in, off + pitch);
+    if (lane < nrows + 2)
+        rows[lane] = deep_row(__ldg(s.rowpack + y0 - 1 + lane), __ldg(s.rowpack + y0 - 2 + lane), dt, s.cfl, s.cvis);
     __syncwarp();
+    Cell2 c = cell2(rc);
     Depth2 fc = depth2(c.h);
-    DeepRow rc = rows[1];
     Contrib2 top;
     {
         Contrib2 dummy;
+        const Cell2 a = cell2(ra);
         const Depth2 fa = depth2(a.h);
-        y_edge_deep2<PLAIN>(a, c, fa.rh, fa.sh, fc.rh, fc.sh, rows[0], rc, dummy, top);
+        y_edge_deep2<PLAIN>(a, c, fa.rh, fa.sh, fc.rh, fc.sh, rows[0], rows[1], dummy, top);
     }
     float local_max = 0.f;
+    float2 fin = make_float2(0.f, 0.f);   // running sum: non-finite iff a new value is
+#pragma unroll 1
     for (int k = 0; k < nrows; k++, off += pitch) {
-        const DeepRow rn = rows[k + 2];
-        Cell2 nn = n;
-        if (k + 1 < nrows) nn = load_cell2(eta, s.dep, qx_in, qy_in, off + 2 * pitch);
+        Raw2 rnn = rn;
+        if (k + 1 < nrows) rnn = load_raw2(eta, s.dep, qx_in, qy_in, off + 2 * pitch);
+        const Cell2 n = cell2(rn);
         const Depth2 fn = depth2(n.h);
         Contrib2 below, next_top;
-        y_edge_deep2<PLAIN>(c, n, fc.rh, fc.sh, fn.rh, fn.sh, rc, rn, below, next_top);
-        const float le = shup(c.e.y, 1), lh = shup(c.h.y, 1);
-        const float lqx = shup(c.qx.y, 1), lqy = shup(c.qy.y, 1);
-        const float rhL = shup(fc.rh.y, 1), shL = shup(fc.sh.y, 1);
-        const float2 jump = PLAIN ? sub2(c.e, make_float2(le, c.e.x))
-                                  : jump2<false>(make_float2(le, c.e.x), c.e, make_float2(shup(c.D.y, 1), c.D.x), c.D);
-        MomFlux2 f;
-        momentum_2s_x2(f, make_float2(lh, c.h.x), c.h, make_float2(rhL, fc.rh.x), fc.rh, make_float2(shL, fc.sh.x), fc.sh,
-                       make_float2(lqx, c.qx.x), c.qx, make_float2(lqy, c.qy.x), c.qy, jump, XRowK{rc.m.y, rc.kdx});
-        const Contrib2 xr = {f.p_x, f.p_y, f.lam};
-        const Contrib2 xrr = {make_float2(f.m_x.y, shdn(f.m_x.x, 1)), make_float2(f.m_y.y, shdn(f.m_y.x, 1)),
-                              make_float2(f.lam.y, shdn(f.lam.x, 1))};
-        const float2 lam = add2(add2(add2(xr.lam, xrr.lam), top.lam), below.lam);
-        const float2 w = mul2(lam, bc2(rc.kcfl));
-        const float wm = fmaxf(lam.x < kEps ? 0.f : w.x, lam.y < kEps ? 0.f : w.y);
-        const float2 val = bc2(-rc.dtA);
-        const float2 qx = fma2(val, add2(add2(add2(xr.a, xrr.a), top.a), below.a), c.qx);
-        const float2 qy = fma2(val, add2(add2(add2(xr.b, xrr.b), top.b), below.b), c.qy);
+        y_edge_deep2<PLAIN>(c, n, fc.rh, fc.sh, fn.rh, fn.sh, rows[k + 1], rows[k + 2], below, next_top);
+        float2 qx, qy;
+        float wm;
+        pair_update<PLAIN>(c, fc, rows[k + 1], top, below, qx, qy, wm);
         if (out_lane) {
             local_max = fmaxf(local_max, wm);
-            if (!isfinite(qx.x + qx.y + qy.x + qy.y)) bad = true;
+            fin = add2(fin, add2(qx, qy));
             *reinterpret_cast<float2 *>(qx_out + off) = qx;
             *reinterpret_cast<float2 *>(qy_out + off) = qy;
         }
         top = next_top;
-        rc = rn;
         c = n;
-        n = nn;
+        rn = rnn;
         fc = fn;
     }
+    bad = !isfinite(fin.x) || !isfinite(fin.y);
     local_max = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(local_max)));   // (>= 0)
     __syncwarp();   // rows is reused by the warp's next task
     return local_max;
@@ -323,7 +322,7 @@ __device__ __forceinline__ int unit_class(const ScenarioDev &s, const UnitSum *s
                      (!(b & l) | (v7.y <= 0.f)) & (!(b & r) | (v8.y <= 0.f));
     if (advance) age = (!deep && dry) ? min(age + 1, 255) : 0;
     if (age >= kDryAge) return kClsDry;
-    if (!deep) return kClsGeneral;
+    if (!deep) return kClsGeneral | (v0.x > hp ? 0 : kClsShallow);
     const float hmin = fminf(fminf(fminf(v0.x, v1.x), fminf(v2.x, v3.x)),
                              fminf(fminf(v4.x, v5.x), fminf(fminf(v6.x, v7.x), v8.x)));
     return kClsDeep | (hmin > 1.001f * gmax + 1e-6f ? kClsPlain : 0);
@@ -395,12 +394,13 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             const int uy = item.y / s.tiles_x, tx = item.y - uy * s.tiles_x;
             const int par = h.state[item.x].parity;
             int age = s.dry_age[item.y];
-            c = unit_class(s, s.usum[par], tx, uy, 0.f, false, age) & 3;
+            c = unit_class(s, s.usum[par], tx, uy, 0.f, false, age);
             // phase 1 folds its summary into the other parity's entry
             if (c != kClsDry) clear_summary(&s.usum[par ^ 1][item.y]);
+            c = (c & kClsShallow) ? 0 : 1 + (c & 3);   // the list
         }
 #pragma unroll
-        for (int k = 0; k < 3; k++) {
+        for (int k = 0; k < 4; k++) {
             const unsigned m = __ballot_sync(0xffffffffu, c == k);
             if (!m) continue;
             int at = 0;
@@ -414,36 +414,40 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     if (tid == 0 && !arrive_and_wait(sync->start, nblk)) s_ok = false;
     __syncthreads();
 
-    // ---- this CTA's tasks, dealt in rounds: the general units' first, then the
-    // deep units', then the dry ones'; consecutive tasks are the same rows of
-    // different units and strips, and each round starts at another CTA, so that
-    // no CTA gets the boundary strips (the costly ones) of all its units.  Its
-    // warps claim them in this order. ----
+    // ---- this CTA's tasks, dealt in rounds: the shallow general units' first,
+    // then the other general units', the deep units' and the dry ones' (by falling
+    // cost); consecutive tasks are the same rows of different units and strips, and
+    // each round starts at another CTA, so that no CTA gets the boundary strips of
+    // all its units.  Its warps claim them in this order. ----
     int ntask, age = 0;
     float gmax = 0.f;
     int counted_deep = 0, counted_dry = 0;
     {
-        const int ng = sync->counts[kClsGeneral], nd = sync->counts[kClsDeep], nz = sync->counts[kClsDry];
-        const int tg = STRIPS * (kHalfRows / L.rows_general), td = STRIPS * (kHalfRows / L.rows_deep);
-        const int total = ng * tg + nd * td + nz * tg;
+        int n[4], per[4], total = 0;
+        for (int k = 0; k < 4; k++) {
+            n[k] = sync->counts[k];
+            per[k] = k == 2 ? 2 * (kHalfRows / L.rows_deep) : STRIPS * (kHalfRows / L.rows_general);
+            total += n[k] * per[k];
+        }
         // round k gives this CTA task k nblk + (blockIdx.x + kDealStep k) mod nblk
         const auto dealt = [&](int k) { return k * nblk + (int)((blockIdx.x + (unsigned)kDealStep * k) % nblk); };
         ntask = total / nblk;
         ntask = min(kResThreads, ntask + (dealt(ntask) < total ? 1 : 0));
         if (s_ok && tid < ntask) {
-            int i = dealt(tid), k, n = ng;
-            if (i < ng * tg) k = kClsGeneral;
-            else if ((i -= ng * tg) < nd * td) { k = kClsDeep; n = nd; }
-            else { i -= nd * td; k = kClsDry; n = nz; }
-            const int u = i % n, sub = i / n;
+            int i = dealt(tid), k = 0;
+            while (i >= n[k] * per[k]) {
+                i -= n[k] * per[k];
+                k++;
+            }
+            const int u = i % n[k], sub = i / n[k];
             const int2 item = L.units[L.order[k * L.cap + u]];
             const ScenarioDev &s = h.tab[item.x];
             Task t;
             t.slot = (short)item.x;
             t.uy = (short)(item.y / s.tiles_x);
             t.tx = (short)(item.y - t.uy * s.tiles_x);
-            t.sub = (unsigned char)((sub & ~3) | ((sub + u) & 3));
-            t.rows = (unsigned char)(k == kClsDeep ? L.rows_deep : L.rows_general);
+            t.sub = (unsigned char)(k == 2 ? sub : (sub & ~3) | ((sub + u) & 3));
+            t.rows = (unsigned char)(k == 2 ? L.rows_deep | kPairTask : L.rows_general);
             tasks[tid] = t;
             age = s.dry_age[item.y];
             gmax = s.unit_gmax[item.y];
@@ -461,13 +465,14 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             const int c = cls[j];
             if (q.status != kRunning || (c & 3) == kClsDry) continue;
             const ScenarioDev &s = h.tab[t.slot];
-            const int uidx = t.uy * s.tiles_x + t.tx;
-            const int strip = t.sub & 3, y0 = t.uy * kHalfRows + (t.sub >> 2) * t.rows;
-            UnitSum *dst = &s.usum[q.parity ^ 1][uidx];
+            UnitSum *dst = &s.usum[q.parity ^ 1][t.uy * s.tiles_x + t.tx];
             bool bad = false;
             if (c & kClsDeep) {
+                const int2 y = deep_rows(t);
+                if (!y.y) continue;
                 float mn, mx;
-                mass_rows(s, q.parity, q.dt, q.t_sec, s.x_org + t.tx * kTileX + strip * OUTW, y0, t.rows, rows, mn, mx, bad);
+                mass_rows(s, q.parity, q.dt, q.t_sec, s.x_org + t.tx * kTileX + (t.sub & 1) * 2 * OUTW,
+                          t.uy * kHalfRows + y.x, y.y, rows, mn, mx, bad);
                 // a deep unit reports its whole-unit {min, max} for its strips and
                 // corners too: lane f folds float f of the summary
                 if (lane < 18) {
@@ -476,14 +481,21 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                     else atomicMin(d, __float_as_int(mn));
                 }
             } else {
-                float local_min;
-                DepthAcc hacc;
-                bool cell;
-                int gx;
-                general_rows<1, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0,
-                                      min(y0 + t.rows, min(t.uy * kHalfRows + kHalfRows, s.ny)), local_min, hacc, bad, cell, gx);
+                const int y0 = t.uy * kHalfRows + (t.pair() ? t.sub >> 1 : t.sub >> 2) * t.nrows();
+                const int y1 = min(y0 + t.nrows(), min(t.uy * kHalfRows + kHalfRows, s.ny));
                 const int tx0 = s.x_org + t.tx * kTileX, ux0 = max(tx0, 0), ux1 = min(tx0 + kTileX, s.nx);
-                fold_unit_summary(hacc, cell, cell && gx < ux0 + 2, cell && gx >= ux1 - 2, dst);
+                int strip = t.pair() ? 2 * (t.sub & 1) : t.sub & 3;
+                const int last = t.pair() ? strip + 1 : strip;
+#pragma unroll 1
+                for (; strip <= last; strip++) {
+                    float local_min;
+                    DepthAcc hacc;
+                    bool cell, b;
+                    int gx;
+                    general_rows<1, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0, y1, local_min, hacc, b, cell, gx);
+                    bad |= b;
+                    fold_unit_summary(hacc, cell, cell && gx < ux0 + 2, cell && gx >= ux1 - 2, dst);
+                }
             }
             if (bad) {
                 atomicOr(&s.ctl->errors, 1u);
@@ -528,24 +540,30 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             bool bad = false;
             float bound;
             if (c & kClsDeep) {
-                // two pair strips; row groups of half the rows of phase 1 (a
-                // single row is not halved: half the sub-tasks step it)
-                const int half = max(t.rows >> 1, 1), g = t.sub >> 1;
-                if (g * half >= kHalfRows) continue;
-                const int x0 = s.x_org + t.tx * kTileX + (t.sub & 1) * 2 * OUTW, y0 = t.uy * kHalfRows + g * half;
-                const float m = (c & kClsPlain) ? momentum_rows<true>(s, q.parity, q.dt, x0, y0, half, rows, bad)
-                                                : momentum_rows<false>(s, q.parity, q.dt, x0, y0, half, rows, bad);
+                const int2 y = deep_rows(t);
+                if (!y.y) continue;
+                const int x0 = s.x_org + t.tx * kTileX + (t.sub & 1) * 2 * OUTW, y0 = t.uy * kHalfRows + y.x;
+                const float m = (c & kClsPlain) ? momentum_rows<true>(s, q.parity, q.dt, x0, y0, y.y, rows, bad)
+                                                : momentum_rows<false>(s, q.parity, q.dt, x0, y0, y.y, rows, bad);
                 // (the reciprocal is monotone, so the smallest over the tasks is
                 // that of the unit's largest lam / (2 cfl area))
                 bound = (m > 0.f) ? 1.f / m : 1e30f;
             } else {
-                const int strip = t.sub & 3, y0 = t.uy * kHalfRows + (t.sub >> 2) * t.rows;
-                DepthAcc hacc;
-                bool cell;
-                int gx;
-                general_rows<2, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0,
-                                      min(y0 + t.rows, min(t.uy * kHalfRows + kHalfRows, s.ny)), bound, hacc, bad, cell, gx);
-                bound = warp_min_bound(bound);
+                const int y0 = t.uy * kHalfRows + (t.pair() ? t.sub >> 1 : t.sub >> 2) * t.nrows();
+                const int y1 = min(y0 + t.nrows(), min(t.uy * kHalfRows + kHalfRows, s.ny));
+                int strip = t.pair() ? 2 * (t.sub & 1) : t.sub & 3;
+                const int last = t.pair() ? strip + 1 : strip;
+                bound = FLT_MAX;
+#pragma unroll 1
+                for (; strip <= last; strip++) {
+                    float local_min;
+                    DepthAcc hacc;
+                    bool cell, b;
+                    int gx;
+                    general_rows<2, true>(s, q.parity, q.dt, q.t_sec, t.tx, t.uy, strip, y0, y1, local_min, hacc, b, cell, gx);
+                    bad |= b;
+                    bound = fminf(bound, warp_min_bound(local_min));
+                }
             }
             if (lane == 0) atomicMin(&h.dt_bits[t.slot], __float_as_uint(bound));
             if (bad) {
@@ -604,7 +622,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
         at = at == 2 ? 0 : at + 1;
         if (blockIdx.x == 0 && tid == kResThreads - 1) {
             sync->phase1[clear].v = sync->phase2[clear].v = sync->start.v = 0ull;
-            sync->counts[0] = sync->counts[1] = sync->counts[2] = 0;
+            sync->counts[0] = sync->counts[1] = sync->counts[2] = sync->counts[3] = 0;
             sync->next = at;
         }
         __syncthreads();

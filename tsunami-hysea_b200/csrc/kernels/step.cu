@@ -466,17 +466,7 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                 // row constants of the window with the unit's dt folded in, from
                 // the staged row metrics (row t of the window at t + 1; staged
                 // row t is grid row yb - 1 + t)
-                DeepRow r;
-                r.m = raw[threadIdx.x + 1];
-                const float4 a = raw[threadIdx.x];   // the row above
-                r.icos = __frcp_rn(r.m.x);
-                r.dtA = __fdividef(dt, r.m.z);
-                r.kcfl = 1.f / (2.f * d.cfl * r.m.z);
-                r.kdx = make_xrow(r.m.y, r.m.z + r.m.z, dt, d.cvis).kdes;
-                const YRowK k = make_yrow(a.x, r.m.x, __frcp_rn(a.x), r.icos, r.m.w, a.z + r.m.z, dt, d.cvis);
-                r.y0 = make_float4(k.len, k.cmid, k.cdiff, k.c10);
-                r.y1 = make_float4(k.c01, k.li0, k.kdes0, k.kdes1);
-                rows[threadIdx.x] = r;
+                rows[threadIdx.x] = deep_row(raw[threadIdx.x + 1], raw[threadIdx.x], dt, d.cfl, d.cvis);
             }
             if (PHASE == 1 && threadIdx.x < kStageRows) {
                 // phase 1 row constants from the staged row metrics: 1/cos for
@@ -597,37 +587,11 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                         // y edges below this row
                         Contrib2 below, next_top;
                         y_edge_deep2<PLAIN>(c, n, rh_c, sh_c, rh_n, sh_n, rc, rn, below, next_top);
-                        // x edges left of column sc0 (its left neighbour, with its 1/h
-                        // and sqrt h, is lane l-1's second column) and between sc0 and
-                        // sc0 + 1 (lane 0 is halo: its left edge is not used)
-                        const float le = shup(c.e.y, 1), lh = shup(c.h.y, 1);
-                        const float lqx = shup(c.qx.y, 1), lqy = shup(c.qy.y, 1);
-                        const float rhL = shup(rh_c.y, 1), shL = shup(sh_c.y, 1);
-                        // (the left depth D only for the wet/dry tests of the jump)
-                        const float2 jump = PLAIN ? sub2(c.e, make_float2(le, c.e.x))
-                                                  : jump2<false>(make_float2(le, c.e.x), c.e,
-                                                                 make_float2(shup(c.D.y, 1), c.D.x), c.D);
-                        MomFlux2 f;
-                        momentum_2s_x2(f, make_float2(lh, c.h.x), c.h, make_float2(rhL, rh_c.x), rh_c,
-                                       make_float2(shL, sh_c.x), sh_c, make_float2(lqx, c.qx.x), c.qx,
-                                       make_float2(lqy, c.qy.x), c.qy, jump, XRowK{rc.m.y, rc.kdx});
-                        // column sc0: right cell of the left edge, left cell of the
-                        // middle edge; column sc0 + 1: right cell of the middle edge,
-                        // left cell of lane l+1's left edge
-                        const Contrib2 xr = {f.p_x, f.p_y, f.lam};
-                        const Contrib2 xrr = {make_float2(f.m_x.y, shdn(f.m_x.x, 1)),
-                                              make_float2(f.m_y.y, shdn(f.m_y.x, 1)),
-                                              make_float2(f.lam.y, shdn(f.lam.x, 1))};
-                        // momentum update; the dt bound as in the scalar path
-                        const float2 lam = add2(add2(add2(xr.lam, xrr.lam), top.lam), below.lam);
-                        const float2 w = mul2(lam, bc2(rc.kcfl));
-                        const float wm = fmaxf(lam.x < kEps ? 0.f : w.x, lam.y < kEps ? 0.f : w.y);
+                        // x edges and update
+                        float2 qx, qy;
+                        float wm;
+                        pair_update<PLAIN>(c, Depth2{rh_c, sh_c}, rc, top, below, qx, qy, wm);
                         if (out_lane) local_max = fmaxf(local_max, wm);
-                        // q - dtA * (sum of the fluxes), bitwise the sum of the
-                        // negated fluxes times dtA (negation is exact)
-                        const float2 val = bc2(-rc.dtA);
-                        const float2 qx = fma2(val, add2(add2(add2(xr.a, xrr.a), top.a), below.a), c.qx);
-                        const float2 qy = fma2(val, add2(add2(add2(xr.b, xrr.b), top.b), below.b), c.qy);
                         if (out_lane) {
                             fin = add2(fin, add2(qx, qy));
                             *reinterpret_cast<float2 *>(out0 + off) = qx;

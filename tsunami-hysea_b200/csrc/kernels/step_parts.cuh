@@ -396,6 +396,76 @@ __device__ __forceinline__ void y_edge_deep2(const Cell2 &a, const Cell2 &b, flo
     hi = {f.p_x, f.p_y, f.lam};
 }
 
+// Phase 2 of a row of pairs in a deep unit: the x edges left of each lane's
+// first column (its left neighbour, with its 1/h and sqrt h, is lane-1's second
+// column) and between its two columns, and the momentum update with the shares
+// top and below of the y edges.  Lane 0 is halo: its left edge is not used.
+// w: the pair's largest lam / (2 cfl area) (0 for lam < eps).
+template <bool PLAIN>
+__device__ __forceinline__ void pair_update(const Cell2 &c, const Depth2 &f, const DeepRow &rc, const Contrib2 &top,
+                                            const Contrib2 &below, float2 &qx, float2 &qy, float &w)
+{
+    const float le = shup(c.e.y, 1), lh = shup(c.h.y, 1);
+    const float lqx = shup(c.qx.y, 1), lqy = shup(c.qy.y, 1);
+    const float rhL = shup(f.rh.y, 1), shL = shup(f.sh.y, 1);
+    // (the left depth D only for the wet/dry tests of the jump)
+    const float2 jump = PLAIN ? sub2(c.e, make_float2(le, c.e.x))
+                              : jump2<false>(make_float2(le, c.e.x), c.e, make_float2(shup(c.D.y, 1), c.D.x), c.D);
+    MomFlux2 m;
+    momentum_2s_x2(m, make_float2(lh, c.h.x), c.h, make_float2(rhL, f.rh.x), f.rh, make_float2(shL, f.sh.x), f.sh,
+                   make_float2(lqx, c.qx.x), c.qx, make_float2(lqy, c.qy.x), c.qy, jump, XRowK{rc.m.y, rc.kdx});
+    // first column: right cell of the left edge, left cell of the middle edge;
+    // second column: right cell of the middle edge, left cell of lane+1's left edge
+    const Contrib2 xr = {m.p_x, m.p_y, m.lam};
+    const Contrib2 xrr = {make_float2(m.m_x.y, shdn(m.m_x.x, 1)), make_float2(m.m_y.y, shdn(m.m_y.x, 1)),
+                          make_float2(m.lam.y, shdn(m.lam.x, 1))};
+    const float2 lam = add2(add2(add2(xr.lam, xrr.lam), top.lam), below.lam);
+    const float2 k = mul2(lam, bc2(rc.kcfl));
+    w = fmaxf(lam.x < kEps ? 0.f : k.x, lam.y < kEps ? 0.f : k.y);
+    // q - dtA * (sum of the fluxes), bitwise the sum of the negated fluxes times
+    // dtA (negation is exact)
+    const float2 val = bc2(-rc.dtA);
+    qx = fma2(val, add2(add2(add2(xr.a, xrr.a), top.a), below.a), c.qx);
+    qy = fma2(val, add2(add2(add2(xr.b, xrr.b), top.b), below.b), c.qy);
+}
+
+// row constants of a deep unit's window: m the row's metrics, above those of the
+// row above it, dt folded in
+__device__ __forceinline__ DeepRow deep_row(const float4 &m, const float4 &above, float dt, float cfl, float cvis)
+{
+    DeepRow r;
+    r.m = m;
+    r.icos = __frcp_rn(m.x);
+    r.dtA = __fdividef(dt, m.z);
+    r.kcfl = 1.f / (2.f * cfl * m.z);
+    r.kdx = make_xrow(m.y, m.z + m.z, dt, cvis).kdes;
+    const YRowK k = make_yrow(above.x, m.x, __frcp_rn(above.x), r.icos, m.w, above.z + m.z, dt, cvis);
+    r.y0 = make_float4(k.len, k.cmid, k.cdiff, k.c10);
+    r.y1 = make_float4(k.c01, k.li0, k.kdes0, k.kdes1);
+    return r;
+}
+
+// Mass fluxes of two deep edges: len q [cos], outflow-limited (mass_2s_x / _y).
+// The limit is tested in pairs with a margin (0.24 of the smaller depth instead
+// of 0.25 of the upwind one; km: the smaller cos area of the two sides), the
+// exact test and the limit themselves run only where an edge may be limited.
+__device__ __forceinline__ float2 limit2(float2 F, float2 h0, float2 h1, float c0, float c1, float a0, float a1, float dt,
+                                         float km)
+{
+    const float2 lhs = mul2(bc2(dt), add2(make_float2(fabsf(F.x), fabsf(F.y)), bc2(kEps)));
+    const float2 cap = mul2(bc2(0.24f * km), make_float2(fminf(h0.x, h1.x), fminf(h0.y, h1.y)));
+    if (__any_sync(0xffffffffu, !(lhs.x <= cap.x) || !(lhs.y <= cap.y))) {
+        F.x = limit_outflow(F.x, h0.x, h1.x, c0, c1, dt, a0, a1);
+        F.y = limit_outflow(F.y, h0.y, h1.y, c0, c1, dt, a0, a1);
+    }
+    return F;
+}
+__device__ __forceinline__ float2 mass_y2(const Cell2 &a, const Cell2 &b, const float4 &ka, const float4 &kb, float dt)
+{
+    const float2 F = mul2(mul2(bc2(kb.w), a.qy), bc2(ka.x));
+    return limit2(F, a.h, b.h, ka.x, kb.x, ka.z, kb.z, dt, fminf(ka.x, kb.x) * fminf(ka.z, kb.z));
+}
+
 // General units: those that are not deep water (boundaries, sponge layers,
 // coasts, wet/dry fronts).  A unit's work is split into tasks of one warp
 // each: column strip `strip` (28 output columns and a two-column halo on

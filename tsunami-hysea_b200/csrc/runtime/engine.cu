@@ -939,7 +939,7 @@ int Batch::init(int cap, int max_work, cudaStream_t stream)
     THY_CK(cudaMemsetAsync(d_claims, 0, 4 * sizeof(int), st));
     THY_CK(cudaMallocAsync(&d_rtab, kResidentSlots * sizeof(ScenarioDev), st));
     THY_CK(cudaMallocAsync(&d_runits, kResidentUnits * sizeof(int2), st));
-    THY_CK(cudaMallocAsync(&d_rorder, 3 * kResidentUnits * sizeof(int), st));
+    THY_CK(cudaMallocAsync(&d_rorder, 4 * kResidentUnits * sizeof(int), st));
     THY_CK(cudaMallocAsync(&d_rsync, sizeof(ResidentSync), st));
     THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
     THY_CK(cudaEventCreate(&ev0));
@@ -1171,18 +1171,20 @@ bool Batch::resident() const
     return true;
 }
 
-// Rows of the tasks of a resident chunk: the fewest general rows (1, 2, 4, 8)
-// that leave a warp at most five tasks, and twice as many deep rows.  Short tasks
-// shorten a step's chain while warps are idle; each evaluates one y edge row more
-// than it has rows, which costs more once every warp has several.  (us per step,
-// 148 SMs, general rows 1 / 2 / 4 / 8: 56 units 16.3 / 19.5 / 27.0 / 42.6; 192
-// units 24.7 / 23.9 / 31.5 / 46.5; 231 units 35.1 / 29.8 / 30.7 / 45.2; 704 units
-// 55.2 / 47.2 / 44.1 / 50.4.)  Work the tuner searches takes its variants of the
-// general kernel and of deep phase 2 as half and double the rows.
+// Rows of the tasks of a resident chunk: r = 1, 2, 4 or 8 general rows, the
+// first with at most 3 r^2 / 64 units a warp, and twice as many deep rows.  Short
+// tasks shorten a step's chain while warps are idle; each evaluates one y edge
+// row more than it has rows, which costs more once every warp has several.  (us
+// per step, 2368 warps, r = 1 / 2 / 4 / 8: 88 units 19.7 / 21.3 / 28.8 / 46.1; 108
+// units 21.8 / 22.6 / 29.7 / 47.0; 240 units 30.4 / 26.3 / 31.8 / 49.1; 456 units
+// 42.0 / 34.9 / 35.6 / 51.1; 640 units 52.2 / 42.8 / 40.7 / 54.2; 984 units 72.5 /
+// 56.9 / 51.5 / 58.6; 1500 units r = 4 / 8 69.3 / 71.8; 1921 units 84.9 / 82.8.)
+// Work the tuner searches takes its variants of the general kernel and of deep
+// phase 2 as half and double the rows.
 static void resident_rows(int units, int warps, const Tiling &t, int *general, int *deep)
 {
     int r = 1;
-    while (r < 8 && units * (64 / r) > 5 * warps) r *= 2;
+    while (r < 8 && units * 64 > 3 * r * r * warps) r *= 2;
     const auto variant = [](int rows, int v) { return std::min(8, std::max(1, v == 1 ? 2 * rows : v == 2 ? rows / 2 : rows)); };
     *general = variant(r, t.general);
     *deep = variant(std::min(8, 2 * r), t.deep2);

@@ -189,11 +189,11 @@ struct Batch {
     int run_resident(int len, const Tiling &rows);
 };
 
-// Largest work of a resident chunk, in units (us a step resident / launched: 704
-// units 44 / 70, 1600 units 78 / 95, 2034 units 99 / 103, 2560 units 126 / 113:
-// the launched kernels stage the deep units, which pays once every SM has enough
-// of them to hide the launches).
-constexpr int kResidentUnits = 2048;
+// Largest work of a resident chunk, in units (us a step resident / launched: 640
+// units 40 / 70, 1500 units 70 / 94, 1921 units 83 / 101, 2432 units 104 / 113,
+// 2825 units 118 / 120, 5076 units 210 / 182: the launched kernels stage the deep
+// units, which pays once every SM has enough of them to hide the launches).
+constexpr int kResidentUnits = 2816;
 // Longest resident chunk.  Between chunks the GPU waits for the host (the
 // control blocks' copy, a launch: about 40 us, as long as one or two steps of this
 // work); the steps between them are kept by the gauge ring.
