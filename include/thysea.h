@@ -190,8 +190,8 @@ int thy_run_netcdf(const thy_problem *p, const char *problem_name, const char *p
  * lat0 + j*dlat; H is the depth scale; crop_flag / crop_value as in
  * thy_problem.  Computes U_Z in FP64, crops, then H -= U_Z/H_scale and
  * eta_initial += U_Z/H_scale.  Runs on the caller's current device and
- * `stream` (a cudaStream_t, NULL = default stream); allocates its nx*ny
- * doubles of scratch with cudaMalloc and returns after the stream is idle. */
+ * `stream` (a cudaStream_t, NULL = default stream) and returns after the stream
+ * is idle.  Relative cropping evaluates the deformation twice. */
 int thy_apply_okada(int nx, int ny, double lon0, double dlon, double lat0, double dlat, const double *fault,
                     double H, int crop_flag, double crop_value, void *d_state1, double *d_eta_initial, void *stream);
 

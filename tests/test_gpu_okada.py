@@ -52,3 +52,17 @@ def test_apply_okada_matches_oracle(k, crop):
     assert np.abs(out[:, 1] - (state[:, 1] - U)).max() < 1e-12
     assert np.abs(eta - U).max() < 1e-12
     assert np.abs(U).max() > 1e-4                          # a real deformation
+
+
+# sizes at the edges of a block's cells (128 to 512 of a row, one to four a
+# thread), with relative cropping as two evaluations
+@pytest.mark.parametrize("nx,ny", [(2, 2), (127, 3), (129, 70), (300, 640), (512, 900), (1027, 517)])
+@pytest.mark.parametrize("crop", [(0, 0.0), (1, 5e-3)])
+def test_apply_okada_sizes(nx, ny, crop):
+    # the fault's centre on a station, along a column of stations: corners over
+    # the axes take the general formula
+    fault = [0.0, 9.0 + (nx // 2) / 60.0, 3.5 + (ny // 2) / 60.0, 10.0, 60.0, 30.0, 0.0, 40.0, 70.0, 4.0]
+    out, eta, state, U = okada_case(fault, *crop, nx=nx, ny=ny)
+    assert np.array_equal(out[:, 0], state[:, 0])
+    assert np.abs(out[:, 1] - (state[:, 1] - U)).max() < 1e-12
+    assert np.abs(eta - U).max() < 1e-12

@@ -150,6 +150,11 @@ void launch_okada(const ScenarioDev *s_host, double *def, double lon0, double dl
 void launch_absmax(const double *def, long long n, unsigned int *max_bits, cudaStream_t st);
 void launch_apply_deformation(const ScenarioDev *s_host, const double *def, int crop_flag, double crop_value,
                               const unsigned int *max_bits, cudaStream_t st);
+// the whole stage on the reference's device state; crop_flag 1 uses max_bits (one
+// word) and, if given, def (nx*ny doubles), otherwise both may be null
+void launch_okada_reference(int nx, int ny, int sms, double lon0, double dlon, double lat0, double dlat, const OkadaFault &f,
+                            double Hs, int crop_flag, double crop_value, double *state, double *eta_initial,
+                            unsigned int *max_bits, double *def, cudaStream_t st);
 
 // extract.cu: dimensional output fields (src/GPU/netcdf_kernel.cu)
 enum Field { kFieldEta = 0, kFieldUx = 1, kFieldUy = 2, kFieldMaxHeight = 3, kFieldArrival = 4, kFieldDeformed = 5 };

@@ -10,6 +10,28 @@
 // relative / absolute cropping and the update bathymetry -= U_Z,
 // eta_initial += U_Z (src/GPU/Deformacion.cu:13-53,118-143); the water depth
 // h is unchanged, so the surface rises by U_Z.
+//
+// What bounds it: FP64 instructions.  A cell takes 4 corners of the dislocation
+// with 2 logarithms and 2 arc tangents each in the closed form.  For the
+// reference's double state (thy_apply_okada) the corners' sum is evaluated as
+// one logarithm of each kind (of the ratio of the corners' arguments), one atan2
+// (of the product of the corners' complex numbers, with its turns counted) and
+// one division for all the fractions; the sines of the fault's angles come from
+// the host and those of a row are shared by a thread's cells.  2048^2 cells on a
+// B200: 3041 -> 967 instructions a cell (1227 -> 468 of them FP64), 550 -> 167 us;
+// the FP64 pipe is busy 65 % of that.  The kernel that computes the deformation
+// applies it; relative cropping, which needs the largest one first, computes it
+// twice where the caller brings no scratch, which is less than an allocation costs
+// (0.4 to 1.3 ms).  Calls of thy_apply_okada, 2048^2: 1.9 -> 0.21 ms, with
+// relative cropping 0.37 ms; 256^2 0.67 -> 0.06 ms.  Error against extended
+// precision over 4 million random points as before (rms 5e-14 to 3e-13 of the
+// slip).
+// Scenarios keep the corners' own closed form: their fields are single precision,
+// and the arrival time is a threshold on them, so that last bits of the double
+// which round the other way move it in a few cells.
+#include <algorithm>
+#include <cmath>
+
 #include "device.cuh"
 #include "kernels.h"
 
@@ -36,7 +58,7 @@ __device__ void gauss_krueger(double lat, double lon, double lat0, double lon0, 
 // u_z at the surface; x along strike, y across (km), d centroid depth (km),
 // fault length L and width W (km) centred on the reference point, U1
 // strike-slip and U2 dip-slip (m).  mu/(lambda+mu) = 1/2 (alpha = 2/3).
-__device__ double okada_uz(double x, double y, double d, double dip_deg, double L, double W, double U1, double U2)
+__device__ double okada_closed(double x, double y, double d, double dip_deg, double L, double W, double U1, double U2)
 {
     const double two_pi = 6.283185307179586, eps = 1e-6, k = 0.5;
     double sd = sin(dip_deg * (two_pi / 360.0)), cd = cos(dip_deg * (two_pi / 360.0));
@@ -105,7 +127,7 @@ __global__ void okada_kernel(int nx, int ny, double *__restrict__ def, double lo
     const double ss = sin(rad * f.strike), cs = cos(rad * f.strike);
     double xp, yp;
     gauss_krueger(lat, lon, f.lat_c, f.lon_c, xp, yp);
-    const double uz = okada_uz(xp * ss + yp * cs, -xp * cs + yp * ss, f.depth_c, f.dip, f.length, f.width,
+    const double uz = okada_closed(xp * ss + yp * cs, -xp * cs + yp * ss, f.depth_c, f.dip, f.length, f.width,
                                f.slip * cos(rad * f.rake), f.slip * sin(rad * f.rake));
     def[(size_t)y * nx + x] = uz / Hs;
 }
@@ -173,6 +195,231 @@ void launch_apply_deformation(const ScenarioDev *s_host, const double *def, int 
 {
     dim3 grid((s_host->nx + 255) / 256, s_host->ny);
     apply_deformation_kernel<<<grid, 256, 0, st>>>(*s_host, def, crop_flag, crop_value, max_bits);
+}
+
+// ---- the reference's double state ----
+namespace {
+
+// what the cells of a fault share
+struct OkadaConst {
+    double lon0, dlon, lat0, dlat;     // the lattice
+    double lon_c, lat_c, d;            // reference point, its depth (km)
+    double ss, cs, sd, cd, kcd;        // sine and cosine of strike and dip, k / cd
+    double hl, hw, u1, u2;             // half length and width (km), slips over -2 pi (m)
+    double inv_scale;                  // 1 / depth scale
+    OkadaFault f;                      // for the points left to okada_closed
+};
+
+// The projection with a row's shares of it taken once.
+struct OkadaRow {
+    double lat, a, b, e;
+};
+
+constexpr double kDeg = 0.017453292371619689;
+
+__device__ inline OkadaRow okada_row(const OkadaConst &c, int y)
+{
+    OkadaRow r;
+    r.lat = c.lat0 + y * c.dlat;
+    double s, co;
+    sincos(r.lat * kDeg, &s, &co);
+    const double v2 = co * 0.0067397251 * co + 1.0;
+    r.a = v2 * 0.5 * s * co * kDeg;
+    r.b = co * (6378.16 / 57.29578);
+    r.e = cos(r.lat * kDeg * 2.0) / 19696.838434850401;
+    return r;
+}
+
+__device__ inline void gauss_krueger(const OkadaConst &c, const OkadaRow &r, int x, double &px, double &py)
+{
+    const double dl = c.lon0 + x * c.dlon - c.lon_c, dl2 = dl * dl;
+    const double ph1 = r.lat + r.a * dl2;
+    const double s1 = sin(ph1 * kDeg), s2 = sin((ph1 + c.lat_c) * 0.5 * kDeg);
+    const double im = rsqrt(1.0 - s2 * 0.0066946053 * s2), in = rsqrt(1.0 - s1 * 0.0066946053 * s1);
+    py = (ph1 - c.lat_c) * (6335.4607362597517 / 57.29578) * (im * (im * im));
+    px = dl * r.b * in * (dl2 * r.e + 1.0);
+}
+
+// (re, im) *= (w, s), w > 0: the argument grows by less than a quarter turn
+// either way; turns counts its passes of the negative real axis
+__device__ inline void turn(double &re, double &im, int &turns, double w, double s)
+{
+    const double r = re * w - im * s, i = re * s + im * w;
+    turns += (im >= 0.0 && s > 0.0 && i < 0.0) ? 1 : 0;
+    turns -= (im < 0.0 && s < 0.0 && i >= 0.0) ? 1 : 0;
+    re = r;
+    im = i;
+}
+
+// The same for the other points: no corner coordinate, q or cd vanishes.  The
+// corners' sum with its logarithms, arc tangents and divisions taken together.
+__device__ inline double okada_uz(const OkadaConst &c, double x, double y)
+{
+    const double eps = 1e-6;
+    const double xi[2] = {x + c.hl, x - c.hl};
+    const double p = y * c.cd + c.d * c.sd, q = y * c.sd - c.d * c.cd;
+    const double et[2] = {p + c.hw, p - c.hw};
+    const double qq = q * q, aq = fabs(q), qc = q * c.cd;
+    bool regular = aq >= eps && c.cd != 0.0;
+    double n4[4], n5[4], D[4], S[4], A[4];   // by corner: kk * 2 + j
+    double re = 1.0, im = 0.0;
+    int turns = 0;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const double X = xi[j], X2q = X * X + qq, Xs = sqrt(X2q), aX = fabs(X) * fabs(c.cd);
+        const bool neg = (X < 0.0) != (c.cd < 0.0);
+        regular = regular && fabs(X) >= eps;
+#pragma unroll
+        for (int kk = 0; kk < 2; kk++) {
+            const int k = 2 * kk + j;
+            const double E = et[kk], R = sqrt(X2q + E * E);
+            const double dt = E * c.sd - qc, a = R + E, b = R + X, t = R + dt;
+            // (a corner that the general formula takes apart)
+            regular = regular && a >= eps && b >= eps && t > 0.0 && fabs(E) >= eps;
+            A[k] = a;
+            S[k] = t;
+            D[k] = R * a * b;
+            n4[k] = b * (dt + c.sd * R);
+            n5[k] = a * dt;
+            // theta = atan(X E / (q R)) and the arc tangent of I5, each as the
+            // argument of a number with a positive real part; the corner's sign
+            // and the minus of I5 are conjugations
+            const double g = R + Xs;
+            const double w1 = aq * R, v1 = X * E, w2 = aX * g, v2 = E * (Xs + qc) + Xs * g * c.sd;
+            const bool minus = j + kk == 1;
+            const double s1 = ((q < 0.0) != minus) ? -v1 : v1, s2 = (neg != minus) ? v2 : -v2;
+            turn(re, im, turns, w1, s1);
+            turn(re, im, turns, w2, s2);
+        }
+    }
+    // one division for the corners' fractions and the two ratios
+    const double D01 = D[0] * D[1], D23 = D[2] * D[3], da = A[1] * A[2], ds = S[1] * S[2];
+    const double dd = D01 * D23, dr = da * ds;
+    const double inv = 1.0 / (dd * dr), id = inv * dr, ir = inv * dd;
+    const double i01 = id * D23, i23 = id * D01;
+    const double w0 = i01 * D[1], w1 = i01 * D[0], w2 = i23 * D[3], w3 = i23 * D[2];
+    const double f4 = n4[0] * w0 - n4[1] * w1 - n4[2] * w2 + n4[3] * w3;
+    const double f5 = n5[0] * w0 - n5[1] * w1 - n5[2] * w2 + n5[3] * w3;
+    const double ls = log(S[0] * S[3] * (ir * da)), la = log(A[0] * A[3] * (ir * ds));
+    const double angle = atan2(im, re) + 6.283185307179586 * turns;
+    const double uz = c.u1 * (q * f4 + c.sd * c.kcd * (ls - c.sd * la)) + c.u2 * (q * f5 + c.sd * angle);
+    if (regular && fabs(uz) <= 1e300) return uz;
+    const double two_pi = 6.283185307179586;
+    return okada_closed(x, y, c.d, c.f.dip, c.f.length, c.f.width, -c.u1 * two_pi, -c.u2 * two_pi);
+}
+
+OkadaConst okada_const(double lon0, double dlon, double lat0, double dlat, const OkadaFault &f, double Hs)
+{
+    const double rad = M_PI / 180.0, two_pi = 6.283185307179586, k = 0.5;   // k = mu / (lambda + mu)
+    OkadaConst c;
+    c.lon0 = lon0;
+    c.dlon = dlon;
+    c.lat0 = lat0;
+    c.dlat = dlat;
+    c.lon_c = f.lon_c;
+    c.lat_c = f.lat_c;
+    c.d = f.depth_c;
+    c.ss = std::sin(rad * f.strike);
+    c.cs = std::cos(rad * f.strike);
+    c.sd = std::sin(f.dip * (two_pi / 360.0));
+    c.cd = std::cos(f.dip * (two_pi / 360.0));
+    if (std::fabs(c.cd) < 1e-6) c.cd = 0.0;   // (vertical: the general formula)
+    c.kcd = k / c.cd;
+    c.hl = 0.5 * f.length;
+    c.hw = 0.5 * f.width;
+    c.u1 = f.slip * std::cos(rad * f.rake) / -two_pi;
+    c.u2 = f.slip * std::sin(rad * f.rake) / -two_pi;
+    c.inv_scale = 1.0 / Hs;
+    c.f = f;
+    return c;
+}
+
+// the reference's device state, double2 (h, H) per cell
+struct ReferenceState {
+    double *state, *eta_initial;
+    __device__ __forceinline__ void operator()(size_t i, double U) const
+    {
+        state[2 * i + 1] -= U;
+        if (eta_initial) eta_initial[i] += U;
+    }
+};
+
+// the cropping of U_Z (src/GPU/Deformacion.cu:13-36)
+struct OkadaCrop {
+    int flag;
+    double value;
+    const unsigned int *max_bits;   // flag 1: the largest (float)|U_Z|, as float bits
+    __device__ __forceinline__ double limit() const
+    {
+        return flag == 1 ? value * (double)__uint_as_float(*max_bits) : flag == 2 ? value : 0.0;
+    }
+    static __device__ __forceinline__ double apply(double U, double limit) { return fabs(U) < limit ? 0.0 : U; }
+};
+
+constexpr int kOkadaThreads = 128;
+
+// A block takes `per` x kOkadaThreads cells of a row.  max_bits given: only the
+// largest (float)|U_Z| (non-negative floats order as unsigned) and, with def
+// given, U_Z itself; else U_Z is applied.  One kernel for all of them: a cell's
+// U_Z is the same bits in each.
+__global__ void __launch_bounds__(kOkadaThreads, 5) okada_reference_kernel(int nx, int segs, int per, OkadaConst c, ReferenceState out,
+                                                                           OkadaCrop crop, unsigned int *max_bits,
+                                                                           double *__restrict__ def)
+{
+    const int y = blockIdx.x / segs, x0 = (blockIdx.x - y * segs) * per * kOkadaThreads + threadIdx.x;
+    const OkadaRow row = okada_row(c, y);
+    const double limit = max_bits ? 0.0 : crop.limit();
+    float m = 0.f;
+#pragma unroll 1
+    for (int k = 0, x = x0; k < per && x < nx; k++, x += kOkadaThreads) {
+        double px, py;
+        gauss_krueger(c, row, x, px, py);
+        const double U = okada_uz(c, px * c.ss + py * c.cs, -px * c.cs + py * c.ss) * c.inv_scale;
+        const size_t i = (size_t)y * nx + x;
+        if (max_bits) {
+            m = fmaxf(m, (float)fabs(U));
+            if (def) def[i] = U;
+        } else {
+            out(i, OkadaCrop::apply(U, limit));
+        }
+    }
+    if (max_bits) {
+        const unsigned int v = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
+        if ((threadIdx.x & 31) == 0 && v > *(volatile unsigned int *)max_bits) atomicMax(max_bits, v);
+    }
+}
+
+// applies the U_Z of a scratch field
+__global__ void apply_reference_kernel(size_t n, const double *__restrict__ def, ReferenceState out, OkadaCrop crop)
+{
+    const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (i < n) out(i, OkadaCrop::apply(def[i], crop.limit()));
+}
+
+}  // namespace
+
+void launch_okada_reference(int nx, int ny, int sms, double lon0, double dlon, double lat0, double dlat, const OkadaFault &f,
+                            double Hs, int crop_flag, double crop_value, double *state, double *eta_initial,
+                            unsigned int *max_bits, double *def, cudaStream_t st)
+{
+    const OkadaConst c = okada_const(lon0, dlon, lat0, dlat, f, Hs);
+    const ReferenceState out{state, eta_initial};
+    const OkadaCrop crop{crop_flag, crop_value, max_bits};
+    // up to 4 cells a thread, which share the row's sines, as long as every SM has
+    // its 5 blocks
+    const long long n = (long long)nx * ny;
+    const int per = (int)std::min(4ll, std::max(1ll, n / ((long long)sms * 5 * kOkadaThreads)));
+    const int segs = (nx + per * kOkadaThreads - 1) / (per * kOkadaThreads);
+    const unsigned blocks = (unsigned)segs * (unsigned)ny;
+    if (crop_flag == 1) {
+        cudaMemsetAsync(max_bits, 0, sizeof(unsigned int), st);
+        okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, segs, per, c, out, crop, max_bits, def);
+        if (def) {
+            apply_reference_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((size_t)n, def, out, crop);
+            return;
+        }
+    }
+    okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, segs, per, c, out, crop, nullptr, nullptr);
 }
 
 cudaError_t preload_okada_kernels()

@@ -4,11 +4,13 @@
 // deformation of one fault, optional relative / absolute cropping, then
 // H -= U_Z and eta_initial += U_Z (src/GPU/Deformacion.cu:38-53).
 //
-// Two entry points run the same kernels and differ only in where the
-// scratch (the nx*ny deformation field and one word for the cropping
-// maximum) lives: thy_apply_okada takes it from cudaMalloc for the call;
-// thy_apply_okada_noalloc uses the fixed-size device arrays below, for
-// callers that must not allocate device memory at all.
+// Two entry points run the same kernels.  Neither allocates device memory,
+// except that more than 64 overlapping calls of thy_apply_okada with relative
+// cropping on a device take a word each from cudaMalloc.  Relative cropping needs
+// the largest deformation before any is applied: thy_apply_okada evaluates the
+// deformation twice (any grid size), thy_apply_okada_noalloc keeps it in the
+// fixed-size device array below (and only enqueues its work).
+#include <atomic>
 #include <mutex>
 
 #include <cuda.h>
@@ -18,7 +20,7 @@
 namespace thy {
 
 // Scratch of thy_apply_okada_noalloc.  File-scope device arrays: every GPU
-// that loads the library holds them (8 MiB + 4 bytes) until the process
+// that loads the library holds them (8 MiB) until the process
 // exits, and every call shares them.
 static __device__ __align__(256) double g_okada_scratch[THY_OKADA_NOALLOC_MAX_CELLS];
 static __device__ __align__(256) unsigned int g_okada_scratch_max;
@@ -53,47 +55,58 @@ CtxGetCurrentFn ctx_get_current_fn()
 }
 }  // namespace
 
-__global__ void okada_kernel(int nx, int ny, double *__restrict__ def, double lon0, double dlon, double lat0,
-                             double dlat, OkadaFault f, double Hs);
-__global__ void absmax_kernel(const double *__restrict__ def, long long n, unsigned int *max_bits);
+namespace {
+// Cropping maxima of thy_apply_okada calls in progress: a call holds a word of its
+// device from its start until its stream is idle.
+constexpr int kMaxWords = 64;
+__device__ unsigned int g_okada_max[kMaxWords];
+std::atomic<unsigned long long> g_words_held[64];
 
-__global__ void apply_deformation_reference_layout(long long n, double2 *__restrict__ state,
-                                                   double *__restrict__ eta_initial, const double *__restrict__ def,
-                                                   int crop_flag, double crop_value,
-                                                   const unsigned int *__restrict__ max_bits)
-{
-    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double U = def[i];
-    if (crop_flag == 1) {
-        if (fabs(U) < crop_value * (double)__uint_as_float(*max_bits)) U = 0.0;
-    } else if (crop_flag == 2) {
-        if (fabs(U) < crop_value) U = 0.0;
+class MaxWord {
+public:
+    ~MaxWord()
+    {
+        if (bit_) g_words_held[dev_].fetch_and(~bit_);
+        else if (word_) cudaFree(word_);
     }
-    state[i].y -= U;
-    if (eta_initial) eta_initial[i] += U;
-}
+    cudaError_t claim(int dev)
+    {
+        if (dev < 64) {
+            unsigned long long held = g_words_held[dev].load();
+            while (~held) {
+                const unsigned long long bit = ~held & (held + 1);   // the lowest free one
+                if (!g_words_held[dev].compare_exchange_weak(held, held | bit)) continue;
+                dev_ = dev;
+                bit_ = bit;
+                void *p = nullptr;
+                const cudaError_t e = cudaGetSymbolAddress(&p, g_okada_max);
+                if (e == cudaSuccess) word_ = (unsigned int *)p + __builtin_ctzll(bit);
+                return e;
+            }
+        }
+        return cudaMalloc(&word_, sizeof(unsigned int));
+    }
+    unsigned int *get() const { return word_; }
 
-// Enqueues the Okada stage on `st` with caller-provided scratch: def holds
-// def_cells doubles (at least nx*ny, else THY_ERR_TOO_LARGE before any
-// work), max_bits one word.
-int enqueue_okada_reference_layout(int nx, int ny, double lon0, double dlon, double lat0, double dlat,
-                                   const double *fault, double H, int crop_flag, double crop_value, double2 *state,
-                                   double *eta_initial, double *def, size_t def_cells, unsigned int *max_bits,
-                                   cudaStream_t st)
+private:
+    int dev_ = 0;
+    unsigned long long bit_ = 0;
+    unsigned int *word_ = nullptr;
+};
+
+int enqueue(int nx, int ny, double lon0, double dlon, double lat0, double dlat, const double *fault, double H, int crop_flag,
+            double crop_value, void *state, double *eta_initial, unsigned int *max_bits, double *def, cudaStream_t st)
 {
-    const long long n = (long long)nx * ny;
-    if (n > (long long)def_cells) return THY_ERR_TOO_LARGE;
-    OkadaFault f{fault[1], fault[2], fault[3], fault[4], fault[5], fault[6], fault[7], fault[8], fault[9]};
-    dim3 block(32, 4), grid((nx + 31) / 32, (ny + 3) / 4);
-    okada_kernel<<<grid, block, 0, st>>>(nx, ny, def, lon0, dlon, lat0, dlat, f, H);
-    THY_CK(cudaMemsetAsync(max_bits, 0, sizeof(unsigned int), st));
-    if (crop_flag == 1) absmax_kernel<<<296, 256, 0, st>>>(def, n, max_bits);
-    apply_deformation_reference_layout<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(n, state, eta_initial, def,
-                                                                                  crop_flag, crop_value, max_bits);
+    int dev = 0, sms = 0;
+    THY_CK(cudaGetDevice(&dev));
+    THY_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const OkadaFault f{fault[1], fault[2], fault[3], fault[4], fault[5], fault[6], fault[7], fault[8], fault[9]};
+    launch_okada_reference(nx, ny, sms, lon0, dlon, lat0, dlat, f, H, crop_flag, crop_value, (double *)state, eta_initial, max_bits,
+                           def, st);
     THY_CK(cudaGetLastError());
     return THY_OK;
 }
+}  // namespace
 
 int check_okada_args(int nx, int ny, const double *fault, int crop_flag, const void *state)
 {
@@ -117,26 +130,21 @@ extern "C" int thy_apply_okada(int nx, int ny, double lon0, double dlon, double 
     int rc = check_okada_args(nx, ny, fault, crop_flag, d_state1);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    double *def = nullptr;
-    unsigned int *mx = nullptr;
-    const size_t n = (size_t)nx * ny;
-    THY_CK(cudaMalloc(&def, n * sizeof(double)));
-    if (cudaMalloc(&mx, sizeof(unsigned int)) != cudaSuccess) {
-        cudaFree(def);
-        return THY_ERR_GPU_MEMORY;
+    MaxWord word;
+    if (crop_flag == 1) {
+        int dev = 0;
+        THY_CK(cudaGetDevice(&dev));
+        THY_CK(word.claim(dev));
     }
-    rc = enqueue_okada_reference_layout(nx, ny, lon0, dlon, lat0, dlat, fault, H, crop_flag, crop_value,
-                                        (double2 *)d_state1, d_eta_initial, def, n, mx, st);
+    rc = enqueue(nx, ny, lon0, dlon, lat0, dlat, fault, H, crop_flag, crop_value, d_state1, d_eta_initial, word.get(), nullptr, st);
     cudaError_t e = cudaStreamSynchronize(st);
-    cudaFree(def);
-    cudaFree(mx);
     if (rc) return rc;
     THY_CK(e);
     return THY_OK;
 }
 
-// Same computation with the library's fixed device scratch instead of a
-// cudaMalloc: for callers that cannot allocate device memory (a caching or
+// Same computation with the library's fixed device scratch and without waiting
+// for the work: for callers that cannot allocate device memory (a caching or
 // budgeted allocator owns the GPU, or an allocation's implicit device-wide
 // synchronisation is not acceptable).  Up to THY_OKADA_NOALLOC_MAX_CELLS
 // cells; larger grids return THY_ERR_TOO_LARGE before any work.  The first
@@ -181,7 +189,6 @@ extern "C" int thy_apply_okada_noalloc(int nx, int ny, double lon0, double dlon,
         def = a.def;
         mx = a.max;
     }
-    return enqueue_okada_reference_layout(nx, ny, lon0, dlon, lat0, dlat, fault, H, crop_flag, crop_value,
-                                          (double2 *)d_state1, d_eta_initial, def, THY_OKADA_NOALLOC_MAX_CELLS, mx,
-                                          (cudaStream_t)stream);
+    return enqueue(nx, ny, lon0, dlon, lat0, dlat, fault, H, crop_flag, crop_value, d_state1, d_eta_initial, mx, def,
+                   (cudaStream_t)stream);
 }
