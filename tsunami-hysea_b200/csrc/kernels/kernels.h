@@ -56,18 +56,19 @@ struct Tiling {
     bool operator==(const Tiling &o) const { return deep1 == o.deep1 && deep2 == o.deep2 && general == o.general; }
     bool operator!=(const Tiling &o) const { return !(*this == o); }
 };
-// compute warps per CTA = 4 x deep_ng: deep phase 1 {3, 2, 4} (4 column strips
-// x that many row groups), deep phase 2 {2, 1, 4} (2 column strips of column
-// pairs x twice that many row groups); general {2, 1, 8} row groups (one warp
-// task per strip and row group; 8 groups of 2 rows for short chains)
+// compute warps per CTA = 4 x deep_ng {1, 2, 4}: 2 column strips of column pairs x
+// twice that many row groups; general {2, 1, 8} row groups (one warp task per strip
+// and row group; 8 groups of 2 rows for short chains).  (4096^2, us a launch: deep
+// phase 1 95 / 98 / 107, deep phase 2 86 / 98 / 146, general 48 / 51 / 59.)
 __host__ __device__ constexpr int deep_ng(int phase, int v)
 {
-    return phase == 1 ? (v == 0 ? 3 : v == 1 ? 2 : 4) : (v == 0 ? 2 : v == 1 ? 1 : 4);
+    (void)phase;
+    return v == 0 ? 1 : v == 1 ? 2 : 4;
 }
-// resident CTAs per SM the deep kernels are compiled for: phase 1 is held to
-// two by its staging buffers; phase 2 (its lanes hold two columns) two, three
-// or one as its registers allow
-__host__ __device__ constexpr int deep_minb(int phase, int v) { return phase == 1 ? 2 : (v == 0 ? 2 : v == 1 ? 3 : 1); }
+// resident CTAs per SM the deep kernels are compiled for: phase 1 is held to two
+// by its staging buffers (one of the largest variant, by its registers), phase 2
+// to three, two or one
+__host__ __device__ constexpr int deep_minb(int phase, int v) { return v == 0 ? (phase == 1 ? 2 : 3) : v == 1 ? 2 : 1; }
 __host__ __device__ constexpr int general_ng(int v) { return v == 0 ? 2 : v == 1 ? 1 : 8; }
 
 // step.cu

@@ -205,20 +205,9 @@ __device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt,
             ei = *reinterpret_cast<const float2 *>(s.eta_ini + off);
         }
         const Cell2 n = cell2(rn);
-        const float4 mk = rows[k + 1].m;
-        // mass fluxes below the row, left of and between the lane's columns
-        const float2 Fb = mass_y2(c, n, mk, rows[k + 2].m, dt);
-        const float2 lq = make_float2(shup(c.qx.y, 1), c.qx.x), lh = make_float2(shup(c.h.y, 1), c.h.x);
-        const float2 F = limit2(mul2(lq, bc2(mk.y)), lh, c.h, 1.f, 1.f, mk.z, mk.z, dt, mk.z);
-        const float2 Fr = make_float2(F.y, shdn(F.x, 1));
-        // mass update (src/GPU/Volumen_kernel.cu:111-157)
-        const float2 acc = fma2(neg2(Fb), bc2(rows[k + 1].icos), add2(sub2(F, Fr), top));
-        top = mul2(Fb, bc2(rows[k + 2].icos));
-        float2 e = fma2(bc2(rows[k + 1].dtA), acc, c.e);
-        float2 h = add2(e, c.D);
-        e = sel2(h.x > 0.f, h.y > 0.f, e, neg2(c.D));
+        const float2 e = mass_pair(c, n, rows[k + 1], rows[k + 2], dt, top);
         if (out_lane) {
-            h = add2(e, c.D);
+            const float2 h = add2(e, c.D);
             fin = add2(fin, e);
             *reinterpret_cast<float2 *>(out + off) = e;
             mn = fminf(mn, fminf(h.x, h.y));

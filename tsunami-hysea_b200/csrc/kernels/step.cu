@@ -153,7 +153,7 @@ static_assert((SPLANE * 4) % 128 == 0 && (DPLANE * 4) % 128 == 0, "staged planes
 // and descriptor, one slot per buffer parity) and the error flag, the staged
 // row metrics of the current unit and the reduction scratch (one set per
 // buffer parity).
-constexpr size_t kNextBytes = 16 + 2 * 112;   // s_next[2], s_err, pad, s_unit[2]
+constexpr size_t kNextBytes = 16 + 3 * 112;   // s_next[2], s_err, pad, s_unit[3]
 // A staging buffer also receives the unit's packed row metrics, rows
 // yb-2 .. yb+16 (a deep unit lies at least two rows inside the grid), copied
 // with the planes so that they arrive one unit ahead too; each phase derives
@@ -172,18 +172,6 @@ __host__ __device__ constexpr size_t deep_misc_offset(int phase) { return 2 * de
 static size_t deep_smem_bytes(int phase, int ng)
 {
     return deep_misc_offset(phase) + 16 + kNextBytes + kStageRows * sizeof(DeepRow) + 2 * 2 * 4 * ng * sizeof(float);
-}
-
-// one cell of a staged row (shared memory; the depth is formed here)
-__device__ __forceinline__ Cell staged_cell(const float *st, int i)
-{
-    Cell c;
-    c.e = st[i];
-    c.D = st[SPLANE + i];
-    c.qx = st[2 * SPLANE + i];
-    c.qy = st[3 * SPLANE + i];
-    c.h = c.e + c.D;
-    return c;
 }
 
 // Work lists of a step (device memory, cap entries each): lists[0] = deep
@@ -309,14 +297,15 @@ struct DeepUnit {
     float *out0, *out1;       // phase 1: eta at the new parity; phase 2: qx, qy at the new parity
     float *eta_max, *arr;     // phase 1 diagnostics
     const float4 *rowpack;    // phase 2 row metrics
-    int uidx, x0, yb, p;      // uidx: the unit's index in the scenario's unit grid
+    UnitSum *sum;             // phase 1: the unit's summary at the new parity
+    int x0, yb, p;
     int pitch;
     float dt, t_sec, eps_h, dif_at, cfl, cvis;
     bool run;
     bool drop;                // test hook: issue no copy for it (its wait runs out)
     bool plain;               // phase 2: every surface jump of the unit is the plain difference
 };
-static_assert(2 * sizeof(DeepUnit) + 16 <= kNextBytes, "claimed units' slots in shared memory");
+static_assert(3 * sizeof(DeepUnit) + 16 <= kNextBytes, "claimed units' slots in shared memory");
 
 template <int PHASE>
 __device__ __forceinline__ DeepUnit deep_unit(const ScenarioDev *__restrict__ scen, const int2 *__restrict__ work,
@@ -330,7 +319,6 @@ __device__ __forceinline__ DeepUnit deep_unit(const ScenarioDev *__restrict__ sc
     d.s = &scen[item.x];
     const int ty = item.y / d.s->tiles_x, tx = item.y - ty * d.s->tiles_x;
     const int uy = 2 * ty + (u & 1);
-    d.uidx = uy * d.s->tiles_x + tx;
     d.x0 = d.s->x_org + tx * kTileX;
     d.yb = uy * kHalfRows;
     const ScenarioDev &s = *d.s;
@@ -346,6 +334,7 @@ __device__ __forceinline__ DeepUnit deep_unit(const ScenarioDev *__restrict__ sc
     d.dif_at = s.dif_at;
     d.cfl = s.cfl;
     d.cvis = s.cvis;
+    d.sum = &s.usum[d.p ^ 1][uy * s.tiles_x + tx];
     d.out0 = (PHASE == 1) ? s.eta[d.p ^ 1] : s.qx[d.p ^ 1];
     d.out1 = s.qy[d.p ^ 1];
     d.eta_max = s.eta_max;
@@ -386,9 +375,14 @@ __device__ __forceinline__ void deep_issue(const DeepUnit &d, float *stage, uint
 // one above and one below, columns x0-4 .. x0+115 of eta, dep, qx, qy, and in
 // phase 1 the diagnostics of its own cells and the row metrics - is staged by
 // TMA, the next unit's copy in flight while the current one is computed.
-// Compute warp w marches its row group (w >> 2) of column strip w & 3 (28
-// output columns, lanes 2..29) with a two-row window; one more warp is the
-// producer.
+// Compute warp w marches its row group (w >> 1) of column strip w & 1 (56 output
+// columns, two a lane) with a two-row window; one more warp is the producer.
+//
+// What bounds it (4096^2, 8074 units): phase 1 memory, 476 MB in 92 us, 80 % of
+// the measured copy rate (one column a lane: 99 us; a third of its instructions
+// went with the pairs); phase 2 issue, 57 M warp instructions at 0.64 a scheduler
+// and cycle in 86 us (89 with the next unit's descriptor read only when its buffer
+// was free).
 template <int PHASE, int NG, int MINB>
 __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const ScenarioDev *__restrict__ scen,
                                                                 const int2 *__restrict__ work,
@@ -403,14 +397,11 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
     uint64_t *bars = reinterpret_cast<uint64_t *>(misc);
     int *s_next = reinterpret_cast<int *>(misc + 16);          // [parity]: the unit after the current one
     int &s_err = *reinterpret_cast<int *>(misc + 24);          // a copy did not land in time
-    DeepUnit *s_unit = reinterpret_cast<DeepUnit *>(misc + 32);   // [parity]: its descriptor
+    DeepUnit *s_unit = reinterpret_cast<DeepUnit *>(misc + 32);   // descriptors, unit k of the CTA in slot k % 3
     DeepRow *rows = reinterpret_cast<DeepRow *>(misc + 16 + kNextBytes);
     float *red0 = reinterpret_cast<float *>(rows + kStageRows);   // [parity][2 NW]: per warp dt, or depth min and max
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool producer = warp == NW;
-    const int strip = warp & 3, group = warp >> 2;
-    // a compute warp's rows of the unit: kHalfRows * group / NG .. kHalfRows * (group + 1) / NG - 1
-    const int row0 = kHalfRows * group / NG, nrows = kHalfRows * (group + 1) / NG - row0;
     const int nunits = lists[0];
     if (blockIdx.x >= nunits) return;
     // TMA destinations must be 128-byte aligned: a misaligned buffer is
@@ -429,32 +420,59 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
     __syncthreads();
     uint32_t phase_bits = 0;     // bit b: parity of the next completion of bars[b]
     const TmaMap *acq = nullptr; // maps acquired by this CTA (producer)
-    DeepUnit d = deep_unit<PHASE>(scen, work, lists, blockIdx.x);
-    if (threadIdx.x == PT && d.run && !d.drop) deep_issue<PHASE>(d, reinterpret_cast<float *>(dsm), &bars[0], acq);
-    int buf = 0;
     // The first two waves take units blockIdx.x and blockIdx.x + gridDim.x;
     // after that each CTA claims its units from the counter (2 gridDim.x,
     // 2 gridDim.x + 1, ...), so a CTA that started late, or whose units took
-    // longer, takes fewer.  A producer warp claims the units, reads their
-    // descriptors, issues their copies one unit ahead and reduces each unit's
-    // results, while the compute warps step the current unit; they meet once
-    // per unit, and the producer publishes the next unit there.
-    int pending = blockIdx.x + gridDim.x;   // producer: the unit after the next one
+    // longer, takes fewer.  A producer warp issues the copies of the next unit,
+    // reduces the previous unit's results, and claims the unit after the next one
+    // and reads its descriptor (a chain of five loads, done by the time its buffer
+    // is free), while the compute warps step the current unit; they meet once per
+    // unit, and the producer publishes the next unit there.
+    DeepUnit d = deep_unit<PHASE>(scen, work, lists, blockIdx.x);
+    int next = blockIdx.x + gridDim.x, slot = 1;   // producer: the next unit; its descriptor's slot
+    if (threadIdx.x == PT) {
+        if (d.run && !d.drop) deep_issue<PHASE>(d, reinterpret_cast<float *>(dsm), &bars[0], acq);
+        if (next < nunits) s_unit[1] = deep_unit<PHASE>(scen, work, lists, next);
+    }
+    // a unit's results from its warps' (thread PT)
+    auto reduce = [&](const DeepUnit &q, const float *red) {
+        float m = red[0];
+        for (int k = 1; k < NW; k++) m = (PHASE == 1) ? fminf(m, red[k]) : fmaxf(m, red[k]);
+        if (PHASE == 1) {
+            // a deep unit reports its whole-unit {min, max} for its strips
+            // and corners too: conservative for a neighbour's deep test,
+            // and a wet unit fails a neighbour's dry test either way
+            float mx = red[NW];
+            for (int k = 1; k < NW; k++) mx = fmaxf(mx, red[NW + k]);
+            const float2 v = make_float2(m, mx);
+            *q.sum = UnitSum{v, v, v, v, v, v, v, v, v};
+        } else {
+            // the unit's dt bound from its largest lam / (2 cfl area), inverted
+            // once per unit so that it does not depend on the warps' rows
+            m = (m > 0.f) ? 1.f / m : 1e30f;
+            atomicMin(&q.ctl->dt_bits, __float_as_uint(m));
+            atomicAdd(&q.ctl->units_deep, 1ull);
+        }
+    };
+    DeepUnit prev;   // thread PT: the previous unit
+    prev.run = false;
+    int buf = 0;
     for (int u = blockIdx.x; u < nunits; buf ^= 1) {
         float *red = red0 + buf * 2 * NW;
         if (producer) {
             // the next unit's copy goes to the other buffer, free since the
             // compute warps passed the end of the previous unit
             if (lane == 0) {
-                const int un = pending;
-                s_next[buf ^ 1] = un;
-                if (un < nunits) {
-                    const DeepUnit dn = deep_unit<PHASE>(scen, work, lists, un);
-                    s_unit[buf ^ 1] = dn;
+                s_next[buf ^ 1] = next;
+                if (next < nunits) {
+                    const DeepUnit &dn = s_unit[slot];
                     if (dn.run && !dn.drop)
                         deep_issue<PHASE>(dn, reinterpret_cast<float *>(dsm + (buf ^ 1) * SB), &bars[buf ^ 1], acq);
-                    pending = 2 * (int)gridDim.x + atomicAdd(claim, 1);
+                    next = 2 * (int)gridDim.x + atomicAdd(claim, 1);
+                    // (three slots: the compute warps may still be reading the current unit's)
+                    if (next < nunits) s_unit[slot == 2 ? 0 : slot + 1] = deep_unit<PHASE>(scen, work, lists, next);
                 }
+                if (prev.run) reduce(prev, red0 + (buf ^ 1) * 2 * NW);
             }
         } else if (d.run) {
             ScenarioCtl *ctl = d.ctl;
@@ -480,77 +498,55 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
             // the compute warps only: the row constants are written, every copy checked
             asm volatile("bar.sync 1, %0;" ::"r"(PT) : "memory");
             if (!s_err) {
+              // in pairs: two column strips of 56 cells; lane l steps staged
+              // columns sc0 and sc0 + 1 (lanes 1..28 are cells, lanes 0 and 29 the
+              // halo, lanes 30 and 31 repeat lane 29)
+              constexpr int NG2 = 2 * NG, nrows = kHalfRows / NG2;   // row groups, rows per warp
+              static_assert(kHalfRows % NG2 == 0, "row groups of equal height");
+              const int strip2 = warp & 1, prow0 = nrows * (warp >> 1);
+              const int sc0 = strip2 * 56 + 2 + 2 * min(lane, 29);
+              const bool out_lane = (lane >= 1) && (lane <= 28);
               if constexpr (PHASE == 1) {
-                auto row = [&](int t) { return rows[t]; };
                 const float *stage = reinterpret_cast<const float *>(dsm + buf * SB);
                 const float t_sec = d.t_sec;
-                const int pitch = d.pitch;
-                const int r_first = row0 + 1;                           // staged row of this warp's first output row
-                const int sc = strip * 28 + 2 + lane;                   // staged column of this lane
-                const int gx = x0 - 4 + sc;                             // grid column
-                const bool has_cell = (lane >= 2) && (lane <= 29);
-                const int dcol = strip * 28 - 2 + lane;                 // diagnostics column (cells only)
                 float local_min = FLT_MAX, local_max = -FLT_MAX;   // depths
-                bool bad = false;
-                int i = r_first * kStageW + sc;
-                Cell c = staged_cell(stage, i);
-                DeepRow rc = row(r_first);
-                float top;   // share of the y edge above the row in its cell
-                {
-                    const Cell a = staged_cell(stage, i - kStageW);
-                    const DeepRow ra = row(r_first - 1);
-                    top = mul(mass_2s_y(a.qy, rc.m.w, ra.m.x, rc.m.x, a.h, c.h, dt, ra.m.z, rc.m.z), rc.icos);
-                }
-                float *out0 = d.out0;
-                int off = (yb + r_first - 1) * pitch + gx;
-                // running sum of the cells' new values: non-finite iff one of them is
-                float fin = 0.f;
-                for (int k = 0; k < nrows; k++, i += kStageW, off += pitch) {
-                    const DeepRow rn = row(r_first + k + 1);
-                    const Cell n = staged_cell(stage, i + kStageW);
-                    const float area = rc.m.z;
-                    // y edge below this row, x edge left of this lane's cell
-                    const float Fb = mass_2s_y(c.qy, rn.m.w, rc.m.x, rn.m.x, c.h, n.h, dt, rc.m.z, rn.m.z);
-                    const float F = mass_2s_x(stage[2 * SPLANE + i - 1], rc.m.y, stage[i - 1] + stage[SPLANE + i - 1], c.h,
-                                              dt, area, area);
-                    // the right edge of this cell is the left edge of lane+1
-                    const float Fr = shdn(F, 1);
-                    if (has_cell) {
+                int i = prow0 * kStageW + sc0;                     // staged cells of the row above
+                const float *dg = stage + 4 * SPLANE + prow0 * kTileX + strip2 * 56 + 2 * (lane - 1);   // (of output lanes)
+                int off = (yb + prow0) * d.pitch + x0 - 4 + sc0;
+                Cell2 a = staged_cell2(stage, i), c = staged_cell2(stage, i + kStageW);
+                float2 top = mul2(mass_y2(a, c, rows[prow0].m, rows[prow0 + 1].m, dt), bc2(rows[prow0 + 1].icos));
+                float2 fin = make_float2(0.f, 0.f);   // running sum: non-finite iff a new value is
+#pragma unroll 1
+                for (int k = prow0 + 1; k <= prow0 + nrows; k++, off += d.pitch, dg += kTileX) {
+                    i += kStageW;
+                    const Cell2 n = staged_cell2(stage, i + kStageW);
+                    const float2 e = mass_pair(c, n, rows[k], rows[k + 1], dt, top);
+                    if (out_lane) {
                         // diagnostics of the state the step starts from (src/GPU/Metrics.cu:23-77)
-                        const float *dg = stage + 4 * SPLANE + (r_first - 1 + k) * kTileX + dcol;
-                        const float em = dg[0], ar = dg[DPLANE], ei = dg[2 * DPLANE];
-                        if (c.e > em && c.h > d.eps_h) d.eta_max[off] = c.e;
-                        if (ar < 0.f && fabsf(c.e - ei) > d.dif_at) d.arr[off] = t_sec;
-                        const float eta = deep_eta(c, F, Fr, top, Fb, rc.icos, rc.dtA);
-                        fin += eta;
-                        out0[off] = eta;
-                        local_min = fminf(local_min, eta + c.D);
-                        local_max = fmaxf(local_max, eta + c.D);
+                        const float2 em = *reinterpret_cast<const float2 *>(dg);
+                        const float2 ar = *reinterpret_cast<const float2 *>(dg + DPLANE);
+                        const float2 ei = *reinterpret_cast<const float2 *>(dg + 2 * DPLANE);
+                        if (c.e.x > em.x && c.h.x > d.eps_h) d.eta_max[off] = c.e.x;
+                        if (c.e.y > em.y && c.h.y > d.eps_h) d.eta_max[off + 1] = c.e.y;
+                        if (ar.x < 0.f && fabsf(c.e.x - ei.x) > d.dif_at) d.arr[off] = t_sec;
+                        if (ar.y < 0.f && fabsf(c.e.y - ei.y) > d.dif_at) d.arr[off + 1] = t_sec;
+                        const float2 h = add2(e, c.D);
+                        fin = add2(fin, e);
+                        *reinterpret_cast<float2 *>(d.out0 + off) = e;
+                        local_min = fminf(local_min, fminf(h.x, h.y));
+                        local_max = fmaxf(local_max, fmaxf(h.x, h.y));
                     }
-                    top = mul(Fb, rn.icos);
-                    rc = rn;
                     c = n;
                 }
-                if (!isfinite(fin)) bad = true;
-                if (bad) atomicOr(&ctl->errors, 1u);
-                for (int o = 16; o > 0; o >>= 1) {
-                    local_min = fminf(local_min, __shfl_xor_sync(0xffffffffu, local_min, o));
-                    local_max = fmaxf(local_max, __shfl_xor_sync(0xffffffffu, local_max, o));
-                }
+                if (!isfinite(fin.x) || !isfinite(fin.y)) atomicOr(&ctl->errors, 1u);
+                const float2 mm = warp_minmax(local_min, local_max, out_lane);
+                local_min = mm.x;
+                local_max = mm.y;
                 if (lane == 0) {
                     red[warp] = local_min;
                     red[NW + warp] = local_max;
                 }
               } else {
-                // phase 2 in pairs: two column strips of 56 cells; lane l
-                // steps staged columns sc0 and sc0 + 1 (lanes 1..28 are cells,
-                // lanes 0 and 29 the halo, lanes 30 and 31 repeat lane 29)
-                constexpr int NG2 = 2 * NG, PROWS = kHalfRows / NG2;   // row groups, rows per warp
-                static_assert(kHalfRows % NG2 == 0, "phase-2 row groups of equal height");
-                const int strip2 = warp & 1, group2 = warp >> 1;
-                const int prow0 = PROWS * group2;
-                const int sc0 = strip2 * 56 + 2 + 2 * min(lane, 29);
-                const bool out_lane = (lane >= 1) && (lane <= 28);
                 float local_max = -FLT_MAX;                        // max of lam / (2 cfl area)
                 float2 fin = make_float2(0.f, 0.f);   // running sum: non-finite iff a new value is
                 // the row loop in two copies: surface jumps with their wet/dry
@@ -579,7 +575,7 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
                     // rather than copied (every operation here is explicitly
                     // rounded: the copies compute alike)
     #pragma unroll 2
-                    for (int k = 0; k < PROWS; k++, i += kStageW, off += pitch) {
+                    for (int k = 0; k < nrows; k++, i += kStageW, off += pitch) {
                         const DeepRow rn = rows[r_first + k + 1];
                         const Cell2 n = staged_cell2(stage, i + kStageW);
                         const Depth2 fn = depth2(n.h);
@@ -622,37 +618,17 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
             if (threadIdx.x == PT) {
                 atomicOr(&d.s->ctl->errors, 2u);
                 if (!d.drop) mbar_wait_bounded(&bars[buf], ((phase_bits >> buf) & 1u) ^ 1u);
-                if (s_next[buf ^ 1] < nunits && s_unit[buf ^ 1].run && !s_unit[buf ^ 1].drop)
+                if (s_next[buf ^ 1] < nunits && s_unit[slot].run && !s_unit[slot].drop)
                     mbar_wait_bounded(&bars[buf ^ 1], (phase_bits >> (buf ^ 1)) & 1u);
             }
             return;
         }
-        const int un = s_next[buf ^ 1];
-        const DeepUnit dn = s_unit[buf ^ 1];   // valid when un < nunits
-        if (d.run && threadIdx.x == PT) {
-            const ScenarioDev &s = *d.s;
-            ScenarioCtl *ctl = d.ctl;
-            float m = red[0];
-            for (int k = 1; k < NW; k++) m = (PHASE == 1) ? fminf(m, red[k]) : fmaxf(m, red[k]);
-            // phase 2: the unit's dt bound from its largest lam / (2 cfl area),
-            // inverted once per unit so that it does not depend on the warps' rows
-            if (PHASE == 2) m = (m > 0.f) ? 1.f / m : 1e30f;
-            if (PHASE == 1) {
-                // a deep unit reports its whole-unit {min, max} for its strips
-                // and corners too: conservative for a neighbour's deep test,
-                // and a wet unit fails a neighbour's dry test either way
-                float mx = red[NW];
-                for (int k = 1; k < NW; k++) mx = fmaxf(mx, red[NW + k]);
-                const float2 v = make_float2(m, mx);
-                s.usum[d.p ^ 1][d.uidx] = UnitSum{v, v, v, v, v, v, v, v, v};
-            } else {
-                atomicMin(&ctl->dt_bits, __float_as_uint(m));
-                atomicAdd(&ctl->units_deep, 1ull);
-            }
-        }
-        u = un;
-        d = dn;
+        if (threadIdx.x == PT) prev = d;
+        u = s_next[buf ^ 1];
+        d = s_unit[slot];   // valid when u < nunits
+        slot = slot == 2 ? 0 : slot + 1;
     }
+    if (threadIdx.x == PT && prev.run) reduce(prev, red0 + (buf ^ 1) * 2 * NW);
 }
 
 // Phase 0 (the initial dt) over every unit of the work list, one unit per CTA

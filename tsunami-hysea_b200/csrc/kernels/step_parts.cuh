@@ -360,16 +360,6 @@ __device__ __forceinline__ void momentum_2s_y2(MomFlux2 &r, float2 h0, float2 h1
     r.lam = mul2(len, maxa);
 }
 
-// mass update of a deep cell (src/GPU/Volumen_kernel.cu:111-157): F and Fr, the
-// mass fluxes of its left and right edges, top the share of the edge above it,
-// Fb the flux of the edge below it
-__device__ __forceinline__ float deep_eta(const Cell &c, float F, float Fr, float top, float Fb, float icos, float dtA)
-{
-    const float acc = fma_(-Fb, icos, add(sub(F, Fr), top));
-    const float eta = fma_(dtA, acc, c.e);
-    return (add(eta, c.D) > 0.f) ? eta : -c.D;
-}
-
 // surface jumps of two edges (e0 -> e1); PLAIN: the unit's depths exceed its
 // depth steps, so each is the plain difference (the same value)
 template <bool PLAIN>
@@ -464,6 +454,25 @@ __device__ __forceinline__ float2 mass_y2(const Cell2 &a, const Cell2 &b, const 
 {
     const float2 F = mul2(mul2(bc2(kb.w), a.qy), bc2(ka.x));
     return limit2(F, a.h, b.h, ka.x, kb.x, ka.z, kb.z, dt, fminf(ka.x, kb.x) * fminf(ka.z, kb.z));
+}
+
+// Phase 1 of a pair: its new surface elevations (src/GPU/Volumen_kernel.cu:111-157).
+// c and n: its row and the row below with their metrics (1/cos in icos, dt/area in
+// dtA); top: the share of the edge above, then of the edge below in its cells
+__device__ __forceinline__ float2 mass_pair(const Cell2 &c, const Cell2 &n, const DeepRow &rc, const DeepRow &rn, float dt,
+                                            float2 &top)
+{
+    const float4 m = rc.m;
+    // mass fluxes below the row, left of and between the lane's columns
+    const float2 Fb = mass_y2(c, n, m, rn.m, dt);
+    const float2 lq = make_float2(shup(c.qx.y, 1), c.qx.x), lh = make_float2(shup(c.h.y, 1), c.h.x);
+    const float2 F = limit2(mul2(lq, bc2(m.y)), lh, c.h, 1.f, 1.f, m.z, m.z, dt, m.z);
+    const float2 Fr = make_float2(F.y, shdn(F.x, 1));
+    const float2 acc = fma2(neg2(Fb), bc2(rc.icos), add2(sub2(F, Fr), top));
+    top = mul2(Fb, bc2(rn.icos));
+    const float2 e = fma2(bc2(rc.dtA), acc, c.e);
+    const float2 h = add2(e, c.D);
+    return sel2(h.x > 0.f, h.y > 0.f, e, neg2(c.D));
 }
 
 // General units: those that are not deep water (boundaries, sponge layers,

@@ -1066,9 +1066,15 @@ int Batch::capture(int len)
         }
     if (len == chunk) gexec = nullptr;
     // Each phase's general and deep-water kernels step disjoint tiles and
-    // share only atomically updated scenario fields, so they are two
-    // branches of the graph: the deep tiles fill the SMs the general
-    // kernel's last wave leaves idle.
+    // share only atomically updated scenario fields, so they are two branches of
+    // the graph.  The branch that goes on from the node before the fork starts
+    // first.  In phase 1 that is the deep kernel: memory-bound, it leaves registers
+    // for two CTAs an SM of the general kernel, which run in its shade.  In phase 2
+    // both are bound by issue, nothing is gained side by side, and the general
+    // kernel first lets the deep one fill the SMs that its last wave leaves idle.
+    // (us a step, 4096^2 / 5400 x 1801 belt: general first in both phases 266 / 193,
+    // this order 255 / 187; with time stamps in the kernels 271 / 198, deep first in
+    // both phases 268 / 198, this order 262 / 193.)
     const StepLaunch L = params();
     cudaGraph_t g;
     cudaGraphExec_t exec = nullptr;
@@ -1077,8 +1083,8 @@ int Batch::capture(int len)
         for (int ph = 0; ph < 2; ph++) {
             THY_CK(cudaEventRecord(ev_fork, st));
             THY_CK(cudaStreamWaitEvent(st_side, ev_fork, 0));
-            launch_step_kernel(3 * ph + 1, L, st);        // general
-            launch_step_kernel(3 * ph, L, st_side);       // deep
+            launch_step_kernel(ph == 0 ? 0 : 4, L, st);
+            launch_step_kernel(ph == 0 ? 1 : 3, L, st_side);
             THY_CK(cudaEventRecord(ev_join, st_side));
             THY_CK(cudaStreamWaitEvent(st, ev_join, 0));
             if (ph == 0) launch_step_kernel(2, L, st);   // classification for phase 2 and the next phase 1
