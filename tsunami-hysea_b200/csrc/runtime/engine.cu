@@ -176,7 +176,18 @@ DevScenario::~DevScenario()
     if (rowpack) cudaFreeAsync(rowpack, ast);
 }
 
+// Enqueues the set-up on `st` and returns without waiting for it (the host
+// tables it copies from are kept): a queue's scenarios are set up while the GPU
+// works on the ones before.  The problem's arrays are read until the stream has
+// passed it; after an error nothing of it is in flight.
 int DevScenario::setup(const thy_problem *p, cudaStream_t st)
+{
+    const int rc = enqueue_setup(p, st);
+    if (rc) cudaStreamSynchronize(st);
+    return rc;
+}
+
+int DevScenario::enqueue_setup(const thy_problem *p, cudaStream_t st)
 {
     if (!p || p->nx < 2 || p->ny < 2 || !p->h || !p->Hs || !p->area_cos || !p->dlon || !p->dlat || !p->lon || !p->lat)
         return THY_ERR_INVALID;
@@ -216,10 +227,9 @@ int DevScenario::setup(const thy_problem *p, cudaStream_t st)
         THY_CK(cudaMallocAsync(&def, n * sizeof(double), st));
         THY_CK(cudaMallocAsync(&maxbits, sizeof(unsigned int), st));
         THY_CK(cudaMallocAsync(&fault_times_d, nf * sizeof(double), st));
-        std::vector<double> tf(nf);
-        for (int i = 0; i < nf; i++) tf[i] = faults[10 * i];
-        THY_CK(cudaMemcpyAsync(fault_times_d, tf.data(), nf * sizeof(double), cudaMemcpyHostToDevice, st));
-        THY_CK(cudaStreamSynchronize(st));
+        h_tf.resize(nf);
+        for (int i = 0; i < nf; i++) h_tf[i] = faults[10 * i];
+        THY_CK(cudaMemcpyAsync(fault_times_d, h_tf.data(), nf * sizeof(double), cudaMemcpyHostToDevice, st));
     }
     if (!cells.empty()) {
         // gauge cells, the ring of device samples and the extremes of eta
@@ -231,16 +241,17 @@ int DevScenario::setup(const thy_problem *p, cudaStream_t st)
         THY_CK(cudaMallocAsync(&d_gring_t, kGaugeRing * sizeof(double), st));
         THY_CK(cudaMallocAsync(&d_gminmax, np * sizeof(float2), st));
         THY_CK(cudaMemcpyAsync(d_cells, cells.data(), np * sizeof(int), cudaMemcpyHostToDevice, st));
-        std::vector<float2> mm(np);
+        std::vector<float2> &mm = h_mm;
+        mm.resize(np);
         for (size_t i = 0; i < np; i++) mm[i] = cells[i] < 0 ? make_float2(-9999.0f, -9999.0f) : make_float2(1e30f, -1e30f);
         THY_CK(cudaMemcpyAsync(d_gminmax, mm.data(), np * sizeof(float2), cudaMemcpyHostToDevice, st));
-        THY_CK(cudaStreamSynchronize(st));
     }
     gauges_read = 0;
 
     // per-row metric terms: computed in FP64, stored once as FP32
     {
-        std::vector<float> r((size_t)(5 * ny + 1));
+        std::vector<float> &r = h_rows;
+        r.resize((size_t)(5 * ny + 1));
         float *cosr = r.data(), *ilc = cosr + ny, *ar = ilc + ny, *dlo = ar + ny, *dla = dlo + ny + 1;
         for (int y = 0; y < ny; y++) {
             const double area = p->area_cos[2 * y], c = p->area_cos[2 * y + 1];
@@ -250,7 +261,8 @@ int DevScenario::setup(const thy_problem *p, cudaStream_t st)
             dla[y] = (float)p->dlat[y];
         }
         for (int y = 0; y <= ny; y++) dlo[y] = (float)p->dlon[y];
-        std::vector<float4> pk((size_t)ny + 1);
+        std::vector<float4> &pk = h_pk;
+        pk.resize((size_t)ny + 1);
         for (int y = 0; y <= ny; y++) {
             const bool cell = y < ny;
             pk[y] = make_float4(cell ? cosr[y] : 1.f, cell ? ilc[y] : 0.f, cell ? ar[y] : 1.f, dlo[y]);
@@ -258,7 +270,6 @@ int DevScenario::setup(const thy_problem *p, cudaStream_t st)
         THY_CK(cudaMallocAsync(&rowpack, pk.size() * sizeof(float4), st));
         THY_CK(cudaMemcpyAsync(rows, r.data(), r.size() * sizeof(float), cudaMemcpyHostToDevice, st));
         THY_CK(cudaMemcpyAsync(rowpack, pk.data(), pk.size() * sizeof(float4), cudaMemcpyHostToDevice, st));
-        THY_CK(cudaStreamSynchronize(st));
         desc.rowpack = rowpack;
         desc.row.cosphi = rows;
         desc.row.ilcos = rows + ny;
@@ -332,7 +343,6 @@ int DevScenario::setup(const thy_problem *p, cudaStream_t st)
         launch_init_state(&desc, nullptr, tmp, tmp + n, hasq ? tmp + 2 * n : nullptr, hasq ? tmp + 3 * n : nullptr, Hmin, st);
         THY_CK(cudaGetLastError());
         THY_CK(invalidate_tile_minima(st));
-        THY_CK(cudaStreamSynchronize(st));
         cudaFreeAsync(tmp, st);
     }
 
@@ -394,7 +404,8 @@ int DevScenario::encode_tensor_maps(cudaStream_t st)
         set_last_cuda_error(cudaErrorSymbolNotFound, "cuTensorMapEncodeTiled entry point", __FILE__, __LINE__);
         return THY_ERR_CUDA;
     }
-    CUtensorMap h[kNumMaps];
+    h_maps.resize(kNumMaps);
+    CUtensorMap *h = reinterpret_cast<CUtensorMap *>(h_maps.data());
     float *base[kNumMaps] = {desc.eta[0], desc.eta[1], desc.qx[0], desc.qx[1], desc.qy[0], desc.qy[1],
                              desc.dep, desc.eta_max, desc.arr, desc.eta_ini};
     for (int k = 0; k < kNumMaps; k++) {
@@ -416,7 +427,6 @@ int DevScenario::encode_tensor_maps(cudaStream_t st)
     }
     THY_CK(cudaMallocAsync(&tmaps, kNumMaps * sizeof(TmaMap), st));
     THY_CK(cudaMemcpyAsync(tmaps, h, kNumMaps * sizeof(TmaMap), cudaMemcpyHostToDevice, st));
-    THY_CK(cudaStreamSynchronize(st));
     desc.tmap = tmaps;
     return THY_OK;
 }
@@ -467,13 +477,14 @@ int DevScenario::apply_due_faults(cudaStream_t st)
     return THY_OK;
 }
 
+// Enqueues the extraction of a field and its copy (the caller waits for it).
+// (consecutive fields share d_out in stream order)
 int DevScenario::extract(int field, float *host_out, cudaStream_t st)
 {
     const size_t n = (size_t)nx * ny;
     launch_extract(&desc, field, hctl.parity, d_out, Hs, Qs, Hmin, st);
     THY_CK(cudaGetLastError());
     THY_CK(cudaMemcpyAsync(host_out, d_out, n * sizeof(float), cudaMemcpyDeviceToHost, st));
-    THY_CK(cudaStreamSynchronize(st));
     return THY_OK;
 }
 
@@ -765,12 +776,15 @@ int DevScenario::finish(const thy_outputs *o, cudaStream_t st)
     // every snapshot and gauge sample is delivered before the final fields
     if (pipe && (rc = pipe->drain())) return rc;
     if (!o) return THY_OK;
-    if (o->max_height && (rc = extract(kFieldMaxHeight, o->max_height, st))) return rc;
-    if (o->arrival && (rc = extract(kFieldArrival, o->arrival, st))) return rc;
-    if (o->deformed_bathy && (rc = extract(kFieldDeformed, o->deformed_bathy, st))) return rc;
-    if (o->eta && (rc = extract(kFieldEta, o->eta, st))) return rc;
-    if (o->ux && (rc = extract(kFieldUx, o->ux, st))) return rc;
-    if (o->uy && (rc = extract(kFieldUy, o->uy, st))) return rc;
+    const std::pair<int, float *> wanted[] = {{kFieldMaxHeight, o->max_height}, {kFieldArrival, o->arrival},
+                                              {kFieldDeformed, o->deformed_bathy}, {kFieldEta, o->eta},
+                                              {kFieldUx, o->ux}, {kFieldUy, o->uy}};
+    rc = THY_OK;
+    for (const auto &w : wanted)
+        if (w.second && !rc) rc = extract(w.first, w.second, st);
+    const cudaError_t done = cudaStreamSynchronize(st);   // (after an error too: the arrays are the caller's)
+    if (rc) return rc;
+    THY_CK(done);
     const int np = (int)cells.size();
     if (np > 0 && (o->series_min || o->series_max || o->series_bathy)) {
         std::vector<float> g(4 * (size_t)np);
@@ -1361,20 +1375,20 @@ static int initial_dt(Batch &b)
     return THY_OK;
 }
 
-// Initial dt of one member that joins a running batch: phase 0 over its own
-// units (a work list of its tiles), the other members untouched.
-int Batch::initial_dt_of(DevScenario *s)
+// Initial dt of members that join a running batch: phase 0 over their own
+// units (a work list of their tiles), the other members untouched.
+int Batch::initial_dt_of(const std::vector<DevScenario *> &joining)
 {
-    int slot = -1;
-    for (int i = 0; i < capacity; i++)
-        if (members[i] == s) slot = i;
-    if (slot < 0) return THY_ERR_INVALID;
-    std::vector<int2> w(s->desc.ntiles);
-    for (int t = 0; t < s->desc.ntiles; t++) w[t] = make_int2(slot, t);
+    std::vector<int2> w;
+    int rc;
+    for (int i = 0; i < capacity; i++) {
+        DevScenario *s = members[i];
+        if (!s || std::find(joining.begin(), joining.end(), s) == joining.end()) continue;
+        for (int t = 0; t < s->desc.ntiles; t++) w.push_back(make_int2(i, t));
+        if ((rc = s->upload_ctl(st))) return rc;
+    }
     const int n = (int)w.size();
     if (n > work_capacity) return THY_ERR_INVALID;
-    int rc;
-    if ((rc = s->upload_ctl(st))) return rc;
     THY_CK(cudaMemcpyAsync(d_work0, w.data(), n * sizeof(int2), cudaMemcpyHostToDevice, st));
     THY_CK(cudaMemcpyAsync(d_nwork0, &n, sizeof(int), cudaMemcpyHostToDevice, st));
     StepLaunch L = params();
@@ -1382,10 +1396,14 @@ int Batch::initial_dt_of(DevScenario *s)
     L.nwork = d_nwork0;
     launch_initial_dt(L, st);
     THY_CK(cudaGetLastError());
-    THY_CK(cudaMemcpyAsync(&h_ctl[slot], d_ctl + slot, sizeof(ScenarioCtl), cudaMemcpyDeviceToHost, st));
+    THY_CK(cudaMemcpyAsync(h_ctl, d_ctl, capacity * sizeof(ScenarioCtl), cudaMemcpyDeviceToHost, st));
     THY_CK(cudaStreamSynchronize(st));
-    s->hctl = h_ctl[slot];
-    truncate_initial_dt(s);
+    for (int i = 0; i < capacity; i++) {
+        DevScenario *s = members[i];
+        if (!s || std::find(joining.begin(), joining.end(), s) == joining.end()) continue;
+        s->hctl = h_ctl[i];
+        truncate_initial_dt(s);
+    }
     return THY_OK;
 }
 

@@ -80,17 +80,24 @@ struct DevScenario {
     double mix_deep = 0, mix_dry = 0;
     bool mix_known = false;
     std::unique_ptr<OutputPipe> pipe;   // created at the first snapshot / gauge sample
+    // what the set-up's copies read
+    std::vector<double> h_tf;
+    std::vector<float2> h_mm;
+    std::vector<float> h_rows;
+    std::vector<float4> h_pk;
+    std::vector<TmaMap> h_maps;
 
     long long units() const { return (long long)desc.tiles_x * ((ny + kHalfRows - 1) / kHalfRows); }   // work units
     DevScenario();
     ~DevScenario();
-    int setup(const thy_problem *p, cudaStream_t st);   // allocate, upload, initial dt
+    int setup(const thy_problem *p, cudaStream_t st);   // allocate, upload (enqueued)
+    int enqueue_setup(const thy_problem *p, cudaStream_t st);
     int upload_ctl(cudaStream_t st);
     int download_ctl(cudaStream_t st);                   // async into hctl (pinned by the batch)
     int apply_due_faults(cudaStream_t st);               // faults with time <= t (the loop's first action)
     cudaError_t invalidate_tile_minima(cudaStream_t st);
     int encode_tensor_maps(cudaStream_t st);
-    int extract(int field, float *host_out, cudaStream_t st);
+    int extract(int field, float *host_out, cudaStream_t st);   // enqueued
     int open_outputs(const thy_outputs *o, cudaStream_t st);
     int snapshot(const thy_outputs *o, cudaStream_t st);
     int sample_gauges(const thy_outputs *o, cudaStream_t st);
@@ -162,7 +169,7 @@ struct Batch {
     int use_tiling(const Tiling &t);  // switch graphs (capturing the tiling's graph if it has none)
     void drop_graphs();
     int rebuild();                    // update(), and capture() when there is no graph yet
-    int initial_dt_of(DevScenario *s);   // initial dt of one member (phase 0 over its units only)
+    int initial_dt_of(const std::vector<DevScenario *> &joining);   // initial dt of some members (phase 0 over their units only)
     // `len` steps (0 or more than `chunk`: the full chunk, one graph launch;
     // fewer: the 1-step graph launched len times; one launch for a resident
     // chunk) + control download

@@ -106,11 +106,15 @@ static void complete(thy_server *S, int slot, int status)
 // of them into an empty server, one a round otherwise (the set-up of each -
 // uploads, table, initial dt - holds the stepping thread, so a queue that
 // built up behind a large request joins one request a chunk, the first one
-// stepping as soon as it is set up).
+// stepping as soon as it is set up).  The set-ups are enqueued one after the
+// other; the table, the work list and the initial dt follow for all of them, with
+// one wait each.  (A queue of 24 requests of 256^2, with the outputs' waits
+// taken out too: 36.7 -> 33.7 ms.)
 static int admit(thy_server *S)
 {
     bool resident = false;
     for (auto *a : S->slots) resident |= a != nullptr;
+    std::vector<int> joining;
     for (int n = 0; !S->queue.empty() && !(resident && n >= 1); n++) {
         Request &r = S->queue.front();
         if (S->in_use + r.bytes > S->budget && S->in_use > 0) break;   // wait for memory (an empty server admits anyway)
@@ -129,15 +133,25 @@ static int admit(thy_server *S)
         int rc = S->b.attach(a->s.get());
         if (rc == THY_OK) rc = a->s->setup(a->r.p, S->st);
         a->s->desc.ctl = a->s->ctl;
-        if (rc == THY_OK) rc = S->b.update();
-        if (rc == THY_OK) rc = S->b.initial_dt_of(a->s.get());
         if (rc != THY_OK) {
             cudaGetLastError();
             complete(S, slot, rc);
             continue;
         }
-        S->members_changed = true;
+        joining.push_back(slot);
     }
+    if (joining.empty()) return THY_OK;
+    std::vector<DevScenario *> who;
+    for (int slot : joining) who.push_back(S->slots[slot]->s.get());
+    int rc = S->b.update();
+    if (rc == THY_OK) rc = S->b.initial_dt_of(who);
+    if (rc != THY_OK) {
+        cudaGetLastError();
+        cudaStreamSynchronize(S->st);   // nothing reads the requests' problems any more
+        for (int slot : joining) complete(S, slot, rc);
+        return THY_OK;
+    }
+    S->members_changed = true;
     return THY_OK;
 }
 

@@ -171,13 +171,27 @@ def run(problem, max_steps: int = -1, snapshots: bool = True, series: bool = Tru
     pts = {k: np.empty(npts, np.float32) for k in ("series_min", "series_max", "series_bathy")}
     snaps = {"time": [], "eta": [], "ux": [], "uy": []}
     ser = {"time": [], "eta": [], "ux": [], "uy": []}
+    # the snapshots' stacks, filled as they arrive (pages of snapshots that do
+    # not come are never touched); of more than a GiB each, arrays stacked at the
+    # end
+    stack = {}
+    if snapshots and pc.save_nc > 0.0:
+        slots = pc.t_end / pc.save_nc + 2.0
+        if slots * ny * nx * 4 <= 1 << 30:
+            stack = {k: np.empty((int(slots), ny, nx), np.float32) for k in ("eta", "ux", "uy")}
 
     def on_snap(user, idx, t, e, u, v):
         n = nx * ny
+        at = len(snaps["time"])
         snaps["time"].append(t)
-        snaps["eta"].append(np.ctypeslib.as_array(e, (n,)).reshape(ny, nx).copy())
-        snaps["ux"].append(np.ctypeslib.as_array(u, (n,)).reshape(ny, nx).copy())
-        snaps["uy"].append(np.ctypeslib.as_array(v, (n,)).reshape(ny, nx).copy())
+        for k, src in (("eta", e), ("ux", u), ("uy", v)):
+            field = np.ctypeslib.as_array(src, (n,)).reshape(ny, nx)
+            if stack and at < len(stack[k]):
+                stack[k][at] = field
+                field = stack[k][at]
+            else:
+                field = field.copy()
+            snaps[k].append(field)
 
     def on_ser(user, idx, t, e, u, v):
         n = pc.npoints
@@ -197,7 +211,9 @@ def run(problem, max_steps: int = -1, snapshots: bool = True, series: bool = Tru
     st = _ffi.Stats()
     _check(L.thy_run(prep.view, ctypes.byref(o), ctypes.byref(st)), "thy_run")
     res: Dict = dict(fields)
-    res["snapshots"] = {k: (np.asarray(v) if v else np.empty((0,))) for k, v in snaps.items()}
+    taken = len(snaps["time"])
+    res["snapshots"] = {k: (stack[k][:taken] if k in stack and taken <= len(stack[k]) else np.asarray(v))
+                        if v else np.empty((0,)) for k, v in snaps.items()}
     res["series"] = {k: (np.asarray(v) if v else np.empty((0,))) for k, v in ser.items()}
     res["series"].update(min=pts["series_min"][:pc.npoints], max=pts["series_max"][:pc.npoints],
                          bathy=pts["series_bathy"][:pc.npoints])
@@ -214,7 +230,7 @@ def run(problem, max_steps: int = -1, snapshots: bool = True, series: bool = Tru
 
 # Warp tilings of the stepping kernels (thy_tiling): row groups per work unit
 # of each variant index, per kernel.  Results never depend on the tiling.
-TILING_GROUPS = {"deep1": (3, 2, 4), "deep2": (4, 2, 8), "general": (2, 1, 8)}
+TILING_GROUPS = {"deep1": (2, 4, 8), "deep2": (2, 4, 8), "general": (2, 1, 8)}
 
 
 def force_tiling(tiling=None):
