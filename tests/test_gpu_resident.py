@@ -81,3 +81,36 @@ def test_resident_batch_matches_alone(gpu):
         assert srv.results[rid]["stats"]["steps"] == r["iterations"]
         for k in FIELDS:
             assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("ngauges", [1, 33, 700])
+@pytest.mark.parametrize("launched", [False, True])
+def test_gauge_samples_on_the_device(gpu, launched, ngauges):
+    """samples taken at a step's end by a resident chunk's first CTA and by the
+    last CTA of a launched step, a thread a gauge, also with more gauges than
+    threads: the eta of a snapshot of the same step at the gauge's cell (each one
+    rounding of the same product, hence two units of the last place)"""
+    nx, ny = 180, 150
+    p = _problem(nx, ny, "open", 300.0)
+    rng = np.random.default_rng(ngauges)
+    ix, iy = rng.integers(0, nx, ngauges), rng.integers(0, ny, ngauges)
+    p.points = np.stack([p.lon[ix], p.lat[iy]], axis=1)
+    p.series_time = p.save_time = 25.0
+    prep = thysea.Prepared(p)
+    thysea.force_tiling((0, 0, 0) if launched else None)
+    try:
+        r = thysea.run(prep)
+    finally:
+        thysea.force_tiling(None)
+    s, f = r["series"], r["snapshots"]
+    assert r["nseries"] == r["nsnaps"] > 5
+    assert np.array_equal(s["time"], f["time"])
+    # (points of one cell are one gauge)
+    cells = np.ctypeslib.as_array(prep.c.point_cell, (prep.npoints,))
+    assert set(cells) == set(iy * nx + ix)
+    for k in range(r["nseries"]):
+        at = f["eta"][k].reshape(-1)[cells]
+        wet = np.abs(at) < 1e3
+        assert wet.any()
+        np.testing.assert_allclose(np.asarray(s["eta"][k])[wet], at[wet], rtol=2.4e-7, atol=0)
+    assert np.abs(np.asarray(s["eta"])).max() > 1e-3

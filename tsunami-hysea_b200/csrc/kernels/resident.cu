@@ -344,6 +344,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     __shared__ unsigned s_bad;       // one scenario: a value of this block is not finite
     __shared__ unsigned s_min;       // one scenario: the step's smallest dt bound
     __shared__ int s_next[2];        // the CTA's next task of phase 1 and 2
+    __shared__ int s_sample[kResidentSlots];   // CTA 0: the step's gauge samples (ring slots)
+    __shared__ bool s_sampled;       // some
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nblk = gridDim.x, NW = nblk * kResWarps;
     const bool single = L.nslots == 1;
@@ -363,12 +365,14 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     if (tid == 0) {
         s_ok = true;
         s_bad = 0u;
+        s_sampled = false;
     }
     __syncthreads();
     for (int k = tid; k < L.nslots; k += kResThreads) {
         h.ctl[k] = *h.tab[k].ctl;
         h.state[k] = step_state(h.ctl[k]);
         h.dt_bits[k] = 0x7f7fffffu;
+        s_sample[k] = -1;
         if (blockIdx.x == 0) sync->dt_bits[0][k] = sync->dt_bits[1][k] = sync->dt_bits[2][k] = 0x7f7fffffu;
     }
     __syncthreads();
@@ -600,11 +604,10 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             h.state[k] = step_state(c);
             if (blockIdx.x == 0) {
                 sync->dt_bits[clear][k] = 0x7f7fffffu;
+                s_sample[k] = sample;
                 if (sample >= 0) {
                     s.gauge_ring_t[sample] = c.t * c.T;
-                    float *dst = s.gauge_ring + (size_t)sample * 4 * s.ngauges;
-                    for (int g = 0; g < s.ngauges; g++)
-                        gauge_values(s, c.parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
+                    s_sampled = true;
                 }
             }
         }
@@ -615,6 +618,20 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             sync->next = at;
         }
         __syncthreads();
+        if (s_sampled) {
+            for (int k = 0; k < L.nslots; k++) {
+                const int sample = s_sample[k];
+                if (sample < 0) continue;
+                const ScenarioDev &s = h.tab[k];
+                float *dst = s.gauge_ring + (size_t)sample * 4 * s.ngauges;
+                for (int g = tid; g < s.ngauges; g += kResThreads)
+                    gauge_values(s, h.state[k].parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
+            }
+            __syncthreads();
+            if (tid < kResidentSlots) s_sample[tid] = -1;
+            if (tid == 0) s_sampled = false;
+            __syncthreads();
+        }
         // nothing left to step: every scenario of the chunk is paused or done
         bool any = false;
         for (int k = lane; k < L.nslots; k += 32) any |= h.state[k].status == kRunning;
