@@ -81,19 +81,23 @@ struct StepLaunch {
     const int *nwork;          // its length (device)
     int *lists;                // deep / general lists of the step: 2 counts + 2 x cap indices
     int *claims;               // units claimed beyond the first wave by deep phase 1 / 2 and the general
-                               // kernel of phase 1 / 2 (zeroed by classification)
+                               // kernel of phase 1 / 2 (zeroed by classification); CTAs that have read the
+                               // lists' lengths in phase 1, CTAs that have finished phase 2
     int cap;                   // list capacity (>= work-list length)
     int grid;                  // general kernel grid
     int deep_grid[2];          // persistent deep kernel grids, phase 1 and 2
     int classify_grid;
     int nslots;
     Tiling tiling;
+    bool control;              // phase 2's last CTA runs the step controller (launch 5 is left out)
 };
 
 // The kLaunchesPerStep launches of a time step, in order: 0 deep phase 1,
 // 1 general phase 1, 2 work-list classification, 3 deep phase 2, 4 general
-// phase 2, 5 step controller.  Launches 0/1 and 3/4 may run concurrently.
+// phase 2, 5 step controller.  Launches 0/1 and 3/4 may run concurrently; 0 and 1,
+// and 3 and 4, are always launched both.
 constexpr int kLaunchesPerStep = 6;
+constexpr int kClaims = 6;   // words of StepLaunch::claims
 void launch_step_kernel(int k, const StepLaunch &L, cudaStream_t st);
 void launch_initial_dt(const StepLaunch &L, cudaStream_t st);
 // lists for the current states of the work list's scenarios (from the host,

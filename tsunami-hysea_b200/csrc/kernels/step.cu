@@ -190,7 +190,7 @@ __device__ __forceinline__ const int *general_items(const int *lists, int cap) {
 // current parity for every scenario, dry counts unchanged; a state the host
 // changed has unknown (NaN) summaries, so its units are general.  Units below
 // the grid (the lower half of a last tile row of <= 16 rows) are not listed.
-// The counts are zeroed before the launch.
+// The counts are zero before the launch (lists_read, or the host).
 constexpr int kClassifyThreads = 128, kClassifyWarps = kClassifyThreads / 32;
 __global__ void __launch_bounds__(kClassifyThreads) classify_kernel(const ScenarioDev *__restrict__ scen,
                                                                    const int2 *__restrict__ work,
@@ -370,6 +370,73 @@ __device__ __forceinline__ void deep_issue(const DeepUnit &d, float *stage, uint
     }
 }
 
+// What the CTAs of a phase's two launches do together: phase 1's zero the lists'
+// lengths for the classification once all have read them, and the last one to
+// finish phase 2 runs the step controller: two nodes less in a step's chain (us a
+// step, 4096^2 255 -> 253, 5400 x 1801 belt 187 -> 184.5, 2048^2 112.5 -> 110.5).
+constexpr int kStepMaxThreads = 128 * 4 + 32;   // of a deep or general CTA
+struct StepEnds {
+    int *count;   // CTAs so far; left zero
+    int ctas;     // of both launches
+    int nslots;   // phase 2: scenario slots to control, 0: the controller is a launch of its own
+};
+
+// Every thread of the CTA calls it after its read of the lengths.
+__device__ __forceinline__ void lists_read(int *lists, const StepEnds &e)
+{
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(e.count, 1) == e.ctas - 1) {
+            lists[0] = lists[1] = 0;
+            *e.count = 0;
+        }
+    }
+}
+
+// the step controller of every slot (controller_kernel), by one CTA
+__device__ __noinline__ void control_slots(const ScenarioDev *scen, int nslots, int *s_sample)
+{
+    for (int base = 0; base < nslots; base += blockDim.x) {
+        const int k = base + threadIdx.x;
+        int sample = -1;
+        if (k < nslots && scen[k].ctl && scen[k].ctl->status == kRunning) {
+            const ScenarioDev &s = scen[k];
+            ScenarioCtl c = *s.ctl;
+            // (what phase 2 changes, not from this SM's cache)
+            sample = advance_scenario(c, s, __uint_as_float(__ldcg(&s.ctl->dt_bits)), __ldcg(&s.ctl->errors));
+            if (sample >= 0) s.gauge_ring_t[sample] = c.t * c.T;
+            store_advanced(s.ctl, c);
+        }
+        s_sample[threadIdx.x] = sample;
+        if (!__syncthreads_or(sample >= 0)) continue;
+        for (int j = 0; j < (int)blockDim.x && base + j < nslots; j++) {
+            if (s_sample[j] < 0) continue;
+            const ScenarioDev &s = scen[base + j];
+            const int parity = *(volatile const int *)&s.ctl->parity;
+            float *dst = s.gauge_ring + (size_t)s_sample[j] * 4 * s.ngauges;
+            for (int g = threadIdx.x; g < s.ngauges; g += blockDim.x)
+                gauge_values(s, parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
+        }
+        __syncthreads();   // s_sample is reused by the next round
+    }
+}
+
+__device__ __forceinline__ void phase2_done(const ScenarioDev *scen, const StepEnds &e)
+{
+    if (e.nslots == 0) return;
+    __shared__ int s_last, s_sample[kStepMaxThreads];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        s_last = atomicAdd(e.count, 1) == e.ctas - 1;
+        if (s_last) *e.count = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) control_slots(scen, e.nslots, s_sample);
+}
+
 // Phase 1 / 2 of the deep tiles, persistent, over the units of the deep list
 // (two per tile: its upper and lower half).  A unit's window - its rows plus
 // one above and one below, columns x0-4 .. x0+115 of eta, dep, qx, qy, and in
@@ -383,10 +450,9 @@ __device__ __forceinline__ void deep_issue(const DeepUnit &d, float *stage, uint
 // went with the pairs); phase 2 issue, 57 M warp instructions at 0.64 a scheduler
 // and cycle in 86 us (89 with the next unit's descriptor read only when its buffer
 // was free).
-template <int PHASE, int NG, int MINB>
-__global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const ScenarioDev *__restrict__ scen,
-                                                                const int2 *__restrict__ work,
-                                                                const int *__restrict__ lists, int *__restrict__ claim)
+template <int PHASE, int NG>
+__device__ __forceinline__ void deep_units(const ScenarioDev *__restrict__ scen, const int2 *__restrict__ work, int *lists,
+                                           int *claim, const StepEnds &ends)
 {
     extern __shared__ __align__(1024) unsigned char dsm[];
     constexpr size_t SB = deep_stage_bytes(PHASE);
@@ -403,6 +469,7 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool producer = warp == NW;
     const int nunits = lists[0];
+    if (PHASE == 1) lists_read(lists, ends);
     if (blockIdx.x >= nunits) return;
     // TMA destinations must be 128-byte aligned: a misaligned buffer is
     // reported on every scenario of the CTA's units and nothing is copied
@@ -631,6 +698,15 @@ __global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const Scenari
     if (threadIdx.x == PT && prev.run) reduce(prev, red0 + (buf ^ 1) * 2 * NW);
 }
 
+template <int PHASE, int NG, int MINB>
+__global__ void __launch_bounds__(128 * NG + 32, MINB) deep_kernel(const ScenarioDev *__restrict__ scen,
+                                                                const int2 *__restrict__ work, int *lists, int *claim,
+                                                                const StepEnds ends)
+{
+    deep_units<PHASE, NG>(scen, work, lists, claim, ends);
+    if (PHASE == 2) phase2_done(scen, ends);
+}
+
 // Phase 0 (the initial dt) over every unit of the work list, one unit per CTA
 // iteration, 4 x NG warps; the last unit of a scenario stores its dt.
 template <int NG>
@@ -685,13 +761,14 @@ constexpr int kGeneralThreads = 128;
 template <int PHASE, int NG>
 __global__ void __launch_bounds__(kGeneralThreads, 4) general_kernel(const ScenarioDev *__restrict__ scen,
                                                                     const int2 *__restrict__ work,
-                                                                    const int *__restrict__ lists, int cap,
-                                                                    int *__restrict__ claim)
+                                                                    int *lists, int cap, int *claim,
+                                                                    const StepEnds ends)
 {
     constexpr int TASKS = STRIPS * NG;   // tasks per unit
     constexpr int WPB = kGeneralThreads / 32;
     const int lane = threadIdx.x & 31;
     const int ntasks = lists[1] * TASKS;
+    if (PHASE == 1) lists_read(lists, ends);
     const int first_wave = (int)gridDim.x * WPB;
     int t = blockIdx.x * WPB + (threadIdx.x >> 5);
     while (t < ntasks) {
@@ -725,6 +802,13 @@ __global__ void __launch_bounds__(kGeneralThreads, 4) general_kernel(const Scena
         if (lane == 0) next = first_wave + atomicAdd(claim, 1);
         t = __shfl_sync(0xffffffffu, next, 0);
     }
+    if (PHASE == 2) phase2_done(scen, ends);
+}
+
+template <int PHASE>
+static StepEnds step_ends(const StepLaunch &L)
+{
+    return StepEnds{L.claims + 3 + PHASE, L.deep_grid[PHASE - 1] + L.grid, PHASE == 2 && L.control ? L.nslots : 0};
 }
 
 // One launch of deep phase PHASE / the general kernel in variant V.
@@ -734,7 +818,7 @@ static void launch_deep(const StepLaunch &L, cudaStream_t st)
     constexpr int NG = deep_ng(PHASE, V);
     deep_kernel<PHASE, NG, deep_minb(PHASE, V)>
         <<<L.deep_grid[PHASE - 1], 128 * NG + 32, deep_smem_bytes(PHASE, NG), st>>>(L.scen, L.work, L.lists,
-                                                                            L.claims + (PHASE - 1));
+                                                                            L.claims + (PHASE - 1), step_ends<PHASE>(L));
 }
 template <int PHASE>
 static void launch_deep_any(const StepLaunch &L, cudaStream_t st)
@@ -749,7 +833,7 @@ template <int PHASE, int V>
 static void launch_general_v(const StepLaunch &L, cudaStream_t st)
 {
     general_kernel<PHASE, general_ng(V)><<<L.grid, kGeneralThreads, 0, st>>>(L.scen, L.work, L.lists, L.cap,
-                                                                            L.claims + 2 + (PHASE - 1));
+                                                                            L.claims + 2 + (PHASE - 1), step_ends<PHASE>(L));
 }
 template <int PHASE>
 static void launch_general(const StepLaunch &L, cudaStream_t st)
@@ -767,7 +851,6 @@ void launch_step_kernel(int k, const StepLaunch &L, cudaStream_t st)
     case 0: launch_deep_any<1>(L, st); break;
     case 1: launch_general<1>(L, st); break;
     case 2:
-        cudaMemsetAsync(L.lists, 0, 2 * sizeof(int), st);
         classify_kernel<<<L.classify_grid, kClassifyThreads, 0, st>>>(L.scen, L.work, L.nwork, L.lists, L.cap, 0, L.claims);
         break;
     case 3: launch_deep_any<2>(L, st); break;

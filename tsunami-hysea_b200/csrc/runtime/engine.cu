@@ -949,8 +949,8 @@ int Batch::init(int cap, int max_work, cudaStream_t stream)
     THY_CK(cudaMallocAsync(&d_nwork0, sizeof(int), st));
     THY_CK(cudaMallocAsync(&d_lists, (2 + 4 * (size_t)std::max(max_work, 1)) * sizeof(int), st));
     THY_CK(cudaMemsetAsync(d_lists, 0, 2 * sizeof(int), st));
-    THY_CK(cudaMallocAsync(&d_claims, 4 * sizeof(int), st));
-    THY_CK(cudaMemsetAsync(d_claims, 0, 4 * sizeof(int), st));
+    THY_CK(cudaMallocAsync(&d_claims, kClaims * sizeof(int), st));
+    THY_CK(cudaMemsetAsync(d_claims, 0, kClaims * sizeof(int), st));
     THY_CK(cudaMallocAsync(&d_rtab, kResidentSlots * sizeof(ScenarioDev), st));
     THY_CK(cudaMallocAsync(&d_runits, kResidentUnits * sizeof(int2), st));
     THY_CK(cudaMallocAsync(&d_rorder, 4 * kResidentUnits * sizeof(int), st));
@@ -1089,7 +1089,8 @@ int Batch::capture(int len)
     // (us a step, 4096^2 / 5400 x 1801 belt: general first in both phases 266 / 193,
     // this order 255 / 187; with time stamps in the kernels 271 / 198, deep first in
     // both phases 268 / 198, this order 262 / 193.)
-    const StepLaunch L = params();
+    StepLaunch L = params();
+    L.control = true;
     cudaGraph_t g;
     cudaGraphExec_t exec = nullptr;
     THY_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
@@ -1103,7 +1104,6 @@ int Batch::capture(int len)
             THY_CK(cudaStreamWaitEvent(st, ev_join, 0));
             if (ph == 0) launch_step_kernel(2, L, st);   // classification for phase 2 and the next phase 1
         }
-        launch_step_kernel(5, L, st);                     // controller
     }
     THY_CK(cudaStreamEndCapture(st, &g));
     cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
@@ -1168,6 +1168,7 @@ StepLaunch Batch::params() const
     L.deep_grid[1] = std::max(1, std::min(2 * work_capacity, sms * std::max(1, deep_blocks_per_sm(2, tiling.deep2))));
     L.classify_grid = std::max(1, std::min((2 * work_capacity + 127) / 128, 8 * device_sm_count()));
     L.nslots = capacity;
+    L.control = false;
     return L;
 }
 
@@ -1303,7 +1304,7 @@ int Batch::run_chunk(bool timed, int len)
         THY_CK(cudaEventElapsedTime(&ms, ev0, ev1));
         device_ms += ms;
     }
-    launches += res ? 1 : (long long)kLaunchesPerStep * len;
+    launches += res ? 1 : (long long)(kLaunchesPerStep - 1) * len;   // (the controller is part of phase 2)
     chunks_run++;
     bool full = running > 0 && len == chunk;
     double stepped = 0;   // deep + general units stepped in the chunk
