@@ -141,7 +141,7 @@ typedef struct thy_stats {
     thy_tiling tiling;        /* the warp tiling of the loop's last chunk */
     long long tune_samples;   /* chunks of the loop timed for the autotuner */
     double release_seconds;   /* release of the device buffers, graphs and streams after the outputs */
-    long long chunks;         /* graph launches of the time loop */
+    long long chunks;         /* chunks of the time loop: steps between two waits of the host */
     long long graph_captures; /* step graphs captured (per tiling and chunk length) */
     double capture_seconds;   /* host time spent capturing and instantiating them */
     double event_seconds;     /* host time spent on the loop's events (faults, snapshots, gauges) */
@@ -280,7 +280,7 @@ typedef struct thy_server_opts {
 } thy_server_opts;
 typedef struct thy_server_stats {
     long long submitted, admitted, completed, failed, cancelled, rejected;
-    long long chunks;             /* graph launches */
+    long long chunks;             /* chunks of steps, as in thy_stats */
     int queued, running;
     long long hbm_in_use, hbm_budget;
     double device_ms;             /* device time of the chunks */

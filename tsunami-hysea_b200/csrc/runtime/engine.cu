@@ -1129,7 +1129,12 @@ long long Batch::steps_to_event(const DevScenario &s)
     return std::max(1ll, n);
 }
 
-int Batch::max_chunk() const { return resident() && !tuner_searches(tune_key()) ? kResidentChunk : chunk; }
+int Batch::max_chunk() const
+{
+    const TuneKey key = tune_key();
+    Tiling best;
+    return tuner_searches(key) && !tuner_decided(key, &best) ? chunk : kMaxChunk;
+}
 
 int Batch::chunk_for(long long steps) const { return (int)std::max(1ll, std::min<long long>(steps, max_chunk())); }
 
@@ -1262,19 +1267,16 @@ int Batch::run_chunk(bool timed, int len)
     } else if ((rc = use_tiling(pick)) || (rc = fresh_lists())) {
         return rc;
     }
-    // a full chunk is one graph launch; a shorter one launches the 1-step
-    // graph `len` times (two captures per tiling in all)
-    cudaGraphExec_t exec = gexec;
-    int repeat = 1;
-    if (!res && len != chunk) {
-        exec = nullptr;
+    // every `chunk` steps are one graph launch, each step of the rest one of
+    // the 1-step graph (two captures per tiling in all)
+    cudaGraphExec_t one = nullptr;
+    if (!res && len % chunk) {
         for (auto &g : graphs)
-            if (g.tiling == tiling && g.len == 1) exec = g.exec;
-        if (!exec) {
+            if (g.tiling == tiling && g.len == 1) one = g.exec;
+        if (!one) {
             if ((rc = capture(1))) return rc;
-            exec = graphs.back().exec;
+            one = graphs.back().exec;
         }
-        repeat = len;
     }
     // a sample needs a chunk in which every running member steps `chunk`
     // times (no member reaches its end or an event before the chunk's last
@@ -1294,7 +1296,8 @@ int Batch::run_chunk(bool timed, int len)
     if (res) {
         if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling()))) return rc;
     } else {
-        for (int i = 0; i < repeat; i++) THY_CK(cudaGraphLaunch(exec, st));
+        for (int i = 0; i < len / chunk; i++) THY_CK(cudaGraphLaunch(gexec, st));
+        for (int i = 0; i < len % chunk; i++) THY_CK(cudaGraphLaunch(one, st));
     }
     if (timed) THY_CK(cudaEventRecord(ev1, st));
     THY_CK(cudaMemcpyAsync(h_ctl, d_ctl, capacity * sizeof(ScenarioCtl), cudaMemcpyDeviceToHost, st));

@@ -150,7 +150,7 @@ struct Batch {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double device_ms = 0;
     long long launches = 0;
-    long long chunks_run = 0;          // graph launches
+    long long chunks_run = 0;
     long long captures = 0;            // graphs captured
     double capture_s = 0;              // host time spent capturing and instantiating them
     bool owns_stream = false;          // st was created for the batch (pooled batches of thy_run)
@@ -170,18 +170,16 @@ struct Batch {
     void drop_graphs();
     int rebuild();                    // update(), and capture() when there is no graph yet
     int initial_dt_of(const std::vector<DevScenario *> &joining);   // initial dt of some members (phase 0 over their units only)
-    // `len` steps (0 or more than `chunk`: the full chunk, one graph launch;
-    // fewer: the 1-step graph launched len times; one launch for a resident
-    // chunk) + control download
-    // (synchronous); the tiling is the autotuner's pick, and a full timed
-    // chunk is one of its samples
+    // `len` steps (0 or more than max_chunk(): `chunk`; one launch for a resident
+    // chunk, else a graph launch per `chunk` steps and one of the 1-step graph for
+    // each of the rest) + control download (synchronous); the tiling is the
+    // autotuner's pick, and a timed chunk of `chunk` steps is one of its samples
     int run_chunk(bool timed, int len = 0);
     // steps a member can take before its next event or its end, estimated
     // from its current dt (at least 1)
     static long long steps_to_event(const DevScenario &s);
-    // the chunk length for `steps` steps: at least 1, at most `chunk`, or
-    // kResidentChunk where the chunk is one resident launch and not a sample of
-    // the tuner's
+    // the chunk length for `steps` steps: at least 1, at most `chunk` for a sample
+    // of the tuner's, else kMaxChunk
     int chunk_for(long long steps) const;
     int max_chunk() const;
     // the autotuner's key of the next chunk: this device, the deep and
@@ -201,11 +199,14 @@ struct Batch {
 // 2825 units 118 / 120, 5076 units 210 / 182: the launched kernels stage the deep
 // units, which pays once every SM has enough of them to hide the launches).
 constexpr int kResidentUnits = 2816;
-// Longest resident chunk.  Between chunks the GPU waits for the host (the
-// control blocks' copy, a launch: about 40 us, as long as one or two steps of this
-// work); the steps between them are kept by the gauge ring.
-constexpr int kResidentChunk = 64;
-static_assert(kResidentChunk <= kGaugeRing, "at most one gauge sample a step");
+// Longest chunk that is no sample of the autotuner.  Between chunks the GPU waits
+// for the host (the control blocks' copy, a launch: about 40 us before a resident
+// chunk, more with a graph launch); the gauge ring keeps the samples of the steps
+// between.  A queue's launched chunks stay at `chunk` steps, after which it
+// admits and retires.  (Loop less device time of runs whose chunks after tuning have
+// 16 / 64 steps: 1024^2, 443 steps, 0.88 / 0.44 ms; 2048^2, 986 steps, 2.0 / 1.1 ms.)
+constexpr int kMaxChunk = 64;
+static_assert(kMaxChunk <= kGaugeRing, "at most one gauge sample a step");
 
 // Single-scenario batches of thy_run, kept per device between runs with
 // their buffers, stream and captured graphs, so that a run of a grid size the

@@ -340,7 +340,7 @@ extern "C" int thy_server_progress(thy_server *S, int *active)
         // no longer than the steps the first stepped scenario has left
         // before an event or its end, so that it is handled (and a finished
         // one retired, its slot and memory free) without idle launches
-        long long horizon = S->b.max_chunk();
+        long long horizon = S->b.resident() ? S->b.max_chunk() : S->b.chunk;
         for (int i = 0; i < cap; i++)
             if (S->slots[i] && sel[i]) horizon = std::min(horizon, Batch::steps_to_event(*S->slots[i]->s));
         if ((rc = S->b.run_chunk(true, S->b.chunk_for(horizon)))) return rc;
