@@ -164,6 +164,21 @@ __device__ __forceinline__ Cell2 cell2(const Raw2 &r)
     return Cell2{add2(r.e, r.D), r.e, r.D, r.qx, r.qy};
 }
 
+// the diagnostics of a cell pair
+struct Diag2 {
+    float2 em, ar, ei;
+};
+__device__ __forceinline__ Diag2 load_diag2(const ScenarioDev &s, size_t off, bool cell)
+{
+    Diag2 d{};
+    if (cell) {
+        d.em = *reinterpret_cast<const float2 *>(s.eta_max + off);
+        d.ar = *reinterpret_cast<const float2 *>(s.arr + off);
+        d.ei = *reinterpret_cast<const float2 *>(s.eta_ini + off);
+    }
+    return d;
+}
+
 // Column pairs: lane l holds columns x0 - 2 + 2l and the next one (x0 even) of a
 // strip of 56 columns; lanes 1..28 are cells, lanes 0 and 29 the halo, lanes 30
 // and 31 repeat lane 29.
@@ -180,6 +195,7 @@ __device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt,
     size_t off = (size_t)y0 * pitch + x0 - 2 + 2 * min(lane, 29);
     const Raw2 ra = load_raw2(eta, s.dep, qx, qy, off - pitch), rc = load_raw2(eta, s.dep, qx, qy, off);
     Raw2 rn = load_raw2(eta, s.dep, qx, qy, off + pitch);
+    Diag2 dg = load_diag2(s, off, out_lane);
     // row y0 - 1 + t of the window at rows[t]
     if (lane < nrows + 2) {
         const float4 m = __ldg(s.rowpack + y0 - 1 + lane);
@@ -195,15 +211,11 @@ __device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt,
     float2 fin = make_float2(0.f, 0.f);   // running sum: non-finite iff a new value is
 #pragma unroll 1
     for (int k = 0; k < nrows; k++, off += pitch) {
-        // the row after the next one; this row's diagnostics
+        // the row after the next one; the next row's diagnostics
         Raw2 rnn = rn;
         if (k + 1 < nrows) rnn = load_raw2(eta, s.dep, qx, qy, off + 2 * pitch);
-        float2 em, ar, ei;
-        if (out_lane) {
-            em = *reinterpret_cast<const float2 *>(s.eta_max + off);
-            ar = *reinterpret_cast<const float2 *>(s.arr + off);
-            ei = *reinterpret_cast<const float2 *>(s.eta_ini + off);
-        }
+        Diag2 dn = dg;
+        if (k + 1 < nrows) dn = load_diag2(s, off + pitch, out_lane);
         const Cell2 n = cell2(rn);
         const float2 e = mass_pair(c, n, rows[k + 1], rows[k + 2], dt, top);
         if (out_lane) {
@@ -213,13 +225,14 @@ __device__ __forceinline__ void mass_rows(const ScenarioDev &s, int p, float dt,
             mn = fminf(mn, fminf(h.x, h.y));
             mx = fmaxf(mx, fmaxf(h.x, h.y));
             // diagnostics of the state the step starts from (src/GPU/Metrics.cu:23-77)
-            if (c.e.x > em.x && c.h.x > s.eps_h) s.eta_max[off] = c.e.x;
-            if (c.e.y > em.y && c.h.y > s.eps_h) s.eta_max[off + 1] = c.e.y;
-            if (ar.x < 0.f && fabsf(c.e.x - ei.x) > s.dif_at) s.arr[off] = t_sec;
-            if (ar.y < 0.f && fabsf(c.e.y - ei.y) > s.dif_at) s.arr[off + 1] = t_sec;
+            if (c.e.x > dg.em.x && c.h.x > s.eps_h) s.eta_max[off] = c.e.x;
+            if (c.e.y > dg.em.y && c.h.y > s.eps_h) s.eta_max[off + 1] = c.e.y;
+            if (dg.ar.x < 0.f && fabsf(c.e.x - dg.ei.x) > s.dif_at) s.arr[off] = t_sec;
+            if (dg.ar.y < 0.f && fabsf(c.e.y - dg.ei.y) > s.dif_at) s.arr[off + 1] = t_sec;
         }
         c = n;
         rn = rnn;
+        dg = dn;
     }
     bad = !isfinite(fin.x) || !isfinite(fin.y);
     const float2 v = warp_minmax(mn, mx, out_lane);
