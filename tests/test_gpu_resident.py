@@ -114,3 +114,18 @@ def test_gauge_samples_on_the_device(gpu, launched, ngauges):
         assert wet.any()
         np.testing.assert_allclose(np.asarray(s["eta"][k])[wet], at[wet], rtol=2.4e-7, atol=0)
     assert np.abs(np.asarray(s["eta"])).max() > 1e-3
+
+
+def test_largest_resident_work(gpu):
+    """close to the largest work of a resident chunk (25 x 148 units)"""
+    prep = thysea.Prepared(_problem(2640, 2360, "open", 60.0))
+    thysea.force_tiling((0, 0, 0))
+    try:
+        ref, r0 = _run(prep)
+    finally:
+        thysea.force_tiling(None)
+    got, r = _run(prep)
+    assert r["kernel_launches"] < r["iterations"] < r0["kernel_launches"]
+    assert r["iterations"] == r0["iterations"] and r["deep_tiles"] == r0["deep_tiles"]
+    for k in FIELDS:
+        assert np.array_equal(got[k], ref[k], equal_nan=True), k

@@ -19,11 +19,14 @@
 //
 // What bounds it now: the chain of a task's edges (about 3.8 us a row of WAF
 // edges in both phases on an otherwise idle SM), two barriers of 1.3 us, and the
-// spread of the tasks' costs over the SMs.  us a step, launched -> resident:
-// 96 x 80 28 -> 14, 512^2 48 -> 24, 1024^2 70 -> 40, 1600^2 94 -> 70, 2048^2
-// 113 -> 104.  Deep rows go in column pairs in both phases: packed arithmetic
-// and half the loads and stores of one column a lane (phase 1 with one column a
-// lane: 1024^2 44.5, 2048^2 126).
+// spread of the tasks' costs over the SMs; from 1024^2 on also the loads of the
+// deep rows, which are issued a row ahead (a second row ahead: 1 % slower).  us a
+// step, launched -> resident: 96 x 80 28 -> 14, 512^2 48 -> 23, 1024^2 70 -> 38,
+// 1600^2 94 -> 64, 2048^2 111 -> 95.  Deep rows go in column pairs in both phases:
+// packed arithmetic and half the loads and stores of one column a lane (phase 1
+// with one column a lane: 1024^2 44.5, 2048^2 126; with a row's diagnostics loaded
+// in the iteration that uses them: 40, 103).
+//
 // Arithmetic, classes, depth summaries, dry counts and the control are those
 // of the launches in step.cu; results are bitwise the same.
 //

@@ -195,10 +195,11 @@ struct Batch {
 };
 
 // Largest work of a resident chunk, in units (us a step resident / launched: 640
-// units 40 / 70, 1500 units 70 / 94, 1921 units 83 / 101, 2432 units 104 / 113,
-// 2825 units 118 / 120, 5076 units 210 / 182: the launched kernels stage the deep
-// units, which pays once every SM has enough of them to hide the launches).
-constexpr int kResidentUnits = 2816;
+// units 38 / 70, 1500 units 64 / 94, 2560 units 95 / 111, 3168 units 120 / 127,
+// 3768 units 135 / 136, 4394 units 153 / 147, 5264 units 197 / 172: the launched
+// kernels stage the deep units, which pays once every SM has enough of them to
+// hide the launches).
+constexpr int kResidentUnits = 3712;
 // Longest chunk that is no sample of the autotuner.  Between chunks the GPU waits
 // for the host (the control blocks' copy, a launch: about 40 us before a resident
 // chunk, more with a graph launch); the gauge ring keeps the samples of the steps
