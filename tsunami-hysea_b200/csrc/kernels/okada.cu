@@ -18,14 +18,16 @@
 // (of the product of the corners' complex numbers, with its turns counted) and
 // one division for all the fractions; the sines of the fault's angles come from
 // the host and those of a row are shared by a thread's cells.  2048^2 cells on a
-// B200: 3041 -> 967 instructions a cell (1227 -> 468 of them FP64), 550 -> 167 us;
+// B200: 3041 -> 1134 instructions a cell (1227 -> 549 of them FP64), 550 -> 192 us;
 // the FP64 pipe is busy 65 % of that.  The kernel that computes the deformation
 // applies it; relative cropping, which needs the largest one first, computes it
 // twice where the caller brings no scratch, which is less than an allocation costs
-// (0.4 to 1.3 ms).  Calls of thy_apply_okada, 2048^2: 1.9 -> 0.21 ms, with
-// relative cropping 0.37 ms; 256^2 0.67 -> 0.06 ms.  Error against extended
-// precision over 4 million random points as before (rms 5e-14 to 3e-13 of the
-// slip).
+// (0.4 to 1.3 ms).  Calls of thy_apply_okada, 2048^2: 1.9 -> 0.24 ms, with
+// relative cropping 0.42 ms; 256^2 0.67 -> 0.06 ms.  R + E, R + X and R + dt, which
+// cancel beside a fault's lines, are formed as quotients (22 instructions a corner,
+// 0.03 ms a pass): the error against extended precision over 4 million points of
+// random faults is 1e-16 to 1e-15 of the slip (rms), 5e-14 to 3e-13 corner by
+// corner.
 // Scenarios keep the corners' own closed form: their fields are single precision,
 // and the arrival time is a threshold on them, so that last bits of the double
 // which round the other way move it in a few cells.
@@ -261,7 +263,7 @@ __device__ inline double okada_uz(const OkadaConst &c, double x, double y)
     const double et[2] = {p + c.hw, p - c.hw};
     const double qq = q * q, aq = fabs(q), qc = q * c.cd;
     bool regular = aq >= eps && c.cd != 0.0;
-    double n4[4], n5[4], D[4], S[4], A[4];   // by corner: kk * 2 + j
+    double n4[4], n5[4], D[4], S[4], A[4], Ss[4], As[4];   // by corner: kk * 2 + j
     double re = 1.0, im = 0.0;
     int turns = 0;
 #pragma unroll
@@ -273,14 +275,20 @@ __device__ inline double okada_uz(const OkadaConst &c, double x, double y)
         for (int kk = 0; kk < 2; kk++) {
             const int k = 2 * kk + j;
             const double E = et[kk], R = sqrt(X2q + E * E);
-            const double dt = E * c.sd - qc, a = R + E, b = R + X, t = R + dt;
+            const double dt = E * c.sd - qc, o = E * c.cd + q * c.sd;
+            // R + E, R + X and R + dt as quotients p / s without cancellation
+            const double ap = E < 0.0 ? X2q : R + E, as = E < 0.0 ? R - E : 1.0;
+            const double bp = X < 0.0 ? E * E + qq : R + X, bs = X < 0.0 ? R - X : 1.0;
+            const double tp = dt < 0.0 ? X * X + o * o : R + dt, ts = dt < 0.0 ? R - dt : 1.0;
             // (a corner that the general formula takes apart)
-            regular = regular && a >= eps && b >= eps && t > 0.0 && fabs(E) >= eps;
-            A[k] = a;
-            S[k] = t;
-            D[k] = R * a * b;
-            n4[k] = b * (dt + c.sd * R);
-            n5[k] = a * dt;
+            regular = regular && ap >= eps * as && bp >= eps * bs && tp > 0.0 && fabs(E) >= eps;
+            A[k] = ap;
+            As[k] = as;
+            S[k] = tp;
+            Ss[k] = ts;
+            D[k] = R * ap * bp;
+            n4[k] = bp * (c.sd * ap - qc * as);
+            n5[k] = ap * bs * dt;
             // theta = atan(X E / (q R)) and the arc tangent of I5, each as the
             // argument of a number with a positive real part; the corner's sign
             // and the minus of I5 are conjugations
@@ -293,14 +301,15 @@ __device__ inline double okada_uz(const OkadaConst &c, double x, double y)
         }
     }
     // one division for the corners' fractions and the two ratios
-    const double D01 = D[0] * D[1], D23 = D[2] * D[3], da = A[1] * A[2], ds = S[1] * S[2];
+    const double D01 = D[0] * D[1], D23 = D[2] * D[3], da = A[1] * A[2] * (As[0] * As[3]),
+                 ds = S[1] * S[2] * (Ss[0] * Ss[3]);
     const double dd = D01 * D23, dr = da * ds;
     const double inv = 1.0 / (dd * dr), id = inv * dr, ir = inv * dd;
     const double i01 = id * D23, i23 = id * D01;
     const double w0 = i01 * D[1], w1 = i01 * D[0], w2 = i23 * D[3], w3 = i23 * D[2];
     const double f4 = n4[0] * w0 - n4[1] * w1 - n4[2] * w2 + n4[3] * w3;
     const double f5 = n5[0] * w0 - n5[1] * w1 - n5[2] * w2 + n5[3] * w3;
-    const double ls = log(S[0] * S[3] * (ir * da)), la = log(A[0] * A[3] * (ir * ds));
+    const double ls = log(S[0] * S[3] * (Ss[1] * Ss[2]) * (ir * da)), la = log(A[0] * A[3] * (As[1] * As[2]) * (ir * ds));
     const double angle = atan2(im, re) + 6.283185307179586 * turns;
     const double uz = c.u1 * (q * f4 + c.sd * c.kcd * (ls - c.sd * la)) + c.u2 * (q * f5 + c.sd * angle);
     if (regular && fabs(uz) <= 1e300) return uz;
