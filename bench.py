@@ -7,9 +7,9 @@ Workload: one 4096 x 4096 scenario, Gaussian-random-field
 bathymetry with a shelf and ~10 % dry cells, four contiguous Okada
 subfaults, 3600 s simulated; seeded synthetic inputs (no dataset exists).
 
-A "step" is one time step of the whole grid (16.8 M cell-updates: the six
-stepping launches - deep-water and general kernels of each phase, the
-work-unit classification and the step controller).  `value` = cell-updates/s over K steps with the state
+A "step" is one time step of the whole grid (16.8 M cell-updates: the five
+stepping launches - deep-water and general kernels of each phase, the last of
+which runs the step controller, and the work-unit classification).  `value` = cell-updates/s over K steps with the state
 resident in HBM, timed with CUDA events on the stepping stream (the 268 MB
 state exceeds the 126 MB L2, so no flush is needed between steps).
 `e2e` = the same metric through the public C ABI (thy_run) on host

@@ -2,7 +2,7 @@
 // fill the GPU.
 //
 // What bounds such work is latency, not throughput: as separate launches
-// (step.cu) a step is a chain of six kernels and a memset, each of which reads
+// (step.cu) a step is a chain of kernels, each of which reads
 // its lists, work items, descriptors and control words one after the other
 // before its first cell.  Here one CTA per SM stays on the device for the whole
 // chunk with the scenarios' descriptors in shared memory, and a step is

@@ -1,6 +1,7 @@
 // Time-step kernels of the B200 stepper.
 //
-// One time step = six launches over a work list of (scenario, tile) items:
+// One launched time step (work too large for resident.cu) = five launches over a
+// work list of (scenario, tile) items:
 //   phase 1  mass fluxes -> new surface elevation, fused with the
 //            max-height / arrival-time diagnostics of the state the step
 //            starts from (src/GPU/Metrics.cu:23-77) and with the depth
@@ -11,7 +12,7 @@
 //            sponge, shallow-water filter, Manning friction, local CFL dt,
 //            one atomicMin per deep unit or general warp task (deep and
 //            general kernels, concurrent);
-//   control  one block per scenario: time, next dt, events, gauges.
+//   control  (the last CTA of phase 2) time, next dt, events, gauges.
 // Phases 1 and 2 are each a deep-water kernel and a general kernel.  A tile
 // is deep when every cell within two cells of it is deeper than hpos and it
 // is at least two cells from the boundaries and outside the sponge layers:
@@ -23,8 +24,8 @@
 // Phase 0 (the general kernel's arithmetic, one unit per CTA) computes the
 // initial dt.
 //
-// Row marching (general kernel, step_parts.cuh): a unit is 4 column strips side by side, each
-// in row groups (a tiling: 1, 2 or 8), and each (strip, row group) is a task
+// Row marching (general kernel, step_parts.cuh): a unit is 4 column strips side by
+// side, each in row groups (a tiling: 1, 2 or 8), and each (strip, row group) is a task
 // of one warp, claimed independently of the others; each lane owns one
 // column and the warp marches down its rows keeping a four-row window of its
 // column in registers.  The y edge below the current

@@ -106,8 +106,8 @@ struct DevScenario {
 };
 
 // A set of scenarios stepped together: one work list over all their tiles,
-// one CUDA graph of `chunk` steps (kLaunchesPerStep launches per step) per
-// warp tiling the autotuner has run it with (tuner.h).
+// resident launches of the work that is small enough, and one CUDA graph of `chunk`
+// steps per warp tiling the autotuner has run it with (tuner.h).
 struct Batch {
     std::vector<DevScenario *> members;
     ScenarioDev *d_table = nullptr;
