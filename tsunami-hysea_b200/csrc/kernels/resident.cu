@@ -146,7 +146,7 @@ __device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word
 // ---------------------------------------------------------------------------
 // Deep units.  The formulas and roundings are those of the deep-water kernels
 // (step.cu), with the rows loaded straight from global memory: a task has a
-// few rows, and the state of this work stays in L2.
+// few rows, and the state of most of this work (up to about 1700^2) stays in L2.
 // ---------------------------------------------------------------------------
 
 // the loads of a row of column pairs that is still in flight
