@@ -129,3 +129,39 @@ def test_largest_resident_work(gpu):
     assert r["iterations"] == r0["iterations"] and r["deep_tiles"] == r0["deep_tiles"]
     for k in FIELDS:
         assert np.array_equal(got[k], ref[k], equal_nan=True), k
+
+
+def _spike(nx, ny):
+    """a finite initial state whose fluxes overflow in the first step"""
+    p = _problem(nx, ny, "file", 300.0)
+    p.eta_init[ny // 2, nx // 3] = 1e30
+    return p
+
+
+def test_scenarios_that_fail_in_a_resident_batch(gpu):
+    """values that are not finite end their scenario in the same step for every
+    CTA: a chunk whose last running scenarios fail ends, the others of a chunk
+    finish as alone, and the batch's next chunks find the barriers in order"""
+    goods = [_problem(256, 240, "open", 900.0), _problem(230, 256, "file", 900.0)]
+    alone = [_run(thysea.Prepared(p)) for p in goods]
+    spikes = [_spike(96, 80), _spike(113, 64), _spike(200, 190)]
+    srv = thysea.Server(hbm_budget_bytes=2 << 30, max_scenarios=8)
+    bad = [srv.submit(p) for p in spikes]   # no other scenario in these chunks
+    srv.drain()
+    before = srv.stats()["chunks"]
+    bad += [srv.submit(p) for p in spikes[:1]]
+    ids = [srv.submit(p) for p in goods]
+    bad += [srv.submit(p) for p in spikes[1:]]
+    srv.drain()
+    chunks = srv.stats()["chunks"] - before
+    srv.close()
+    for rid in bad:
+        assert srv.results[rid]["status"] == thysea.THY_ERR_NONFINITE
+        assert srv.results[rid]["stats"]["steps"] == 1
+    for rid, (ref, r) in zip(ids, alone):
+        assert srv.results[rid]["status"] == 0
+        assert srv.results[rid]["stats"]["steps"] == r["iterations"]
+        for k in FIELDS:
+            assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k
+    # (launched chunks of a queue are 16 steps long)
+    assert chunks < max(r["iterations"] for _, r in alone) / 16

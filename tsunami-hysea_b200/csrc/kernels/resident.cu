@@ -345,6 +345,16 @@ __device__ __forceinline__ StepState step_state(const ScenarioCtl &c)
     return StepState{(float)c.dt, (float)(c.t * c.T), c.parity, c.status};
 }
 
+// A value of the scenario is not finite: besides the error bit for the host, no
+// valid dt (0) among the block's bounds.  What ends the scenario is that bound, which
+// reaches every CTA through the step's barrier; the error bit would reach a CTA that
+// reads it late together with the next step's, and the CTAs would part.
+__device__ __forceinline__ void fail(const ScenarioDev &s, unsigned *dt_bits)
+{
+    atomicOr(&s.ctl->errors, 1u);
+    atomicMin(dt_bits, 0u);
+}
+
 // the warp's next task of the CTA
 __device__ __forceinline__ int claim(int *next)
 {
@@ -357,7 +367,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ bool s_ok;            // no wait has run out
-    __shared__ unsigned s_bad;       // one scenario: a value of this block is not finite
     __shared__ unsigned s_min;       // one scenario: the step's smallest dt bound
     __shared__ int s_next[2];        // the CTA's next task of phase 1 and 2
     __shared__ int s_sample[kResidentSlots];   // CTA 0: the step's gauge samples (ring slots)
@@ -380,7 +389,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
     if (tid == 0) {
         s_ok = true;
-        s_bad = 0u;
         s_sampled = false;
     }
     __syncthreads();
@@ -506,10 +514,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                     fold_unit_summary(hacc, cell, cell && gx < ux0 + 2, cell && gx >= ux1 - 2, dst);
                 }
             }
-            if (bad) {
-                atomicOr(&s.ctl->errors, 1u);
-                s_bad = 1u;
-            }
+            if (bad) fail(s, &h.dt_bits[t.slot]);
         }
         __syncthreads();
         if (tid == 0) {
@@ -575,14 +580,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                 }
             }
             if (lane == 0) atomicMin(&h.dt_bits[t.slot], __float_as_uint(bound));
-            if (bad) {
-                atomicOr(&s.ctl->errors, 1u);
-                s_bad = 1u;
-            }
+            if (bad) fail(s, &h.dt_bits[t.slot]);
         }
         __syncthreads();
-        // one scenario: the block's bound goes into the barrier word (0, no valid
-        // dt, for a value that is not finite); several: into a word each
+        // one scenario: the block's bound goes into the barrier word; several: into
+        // a word each
         unsigned *gmin = sync->dt_bits[at];
         if (!single) {
             for (int k = tid; k < L.nslots; k += kResThreads)
@@ -596,7 +598,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             s_next[1] = kResWarps;
             ResidentSync::Word &w = sync->phase2[at];
             if (single) {
-                const unsigned key = 0x7f7fffffu - (s_bad ? 0u : min(h.dt_bits[0], 0x7f7fffffu));
+                const unsigned key = 0x7f7fffffu - min(h.dt_bits[0], 0x7f7fffffu);
                 if (key) atomicMax(reinterpret_cast<unsigned *>(&w.v), key);
                 h.dt_bits[0] = 0x7f7fffffu;
             }
@@ -615,8 +617,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             if (c.status != kRunning) continue;
             const ScenarioDev &s = h.tab[k];
             const unsigned bits = single ? s_min : __ldcg(gmin + k);
-            const unsigned errs = single ? 0u : __ldcg(&s.ctl->errors);
-            const int sample = advance_scenario(c, s, __uint_as_float(bits), errs);
+            const int sample = advance_scenario(c, s, __uint_as_float(bits), 0u);
             h.state[k] = step_state(c);
             if (blockIdx.x == 0) {
                 sync->dt_bits[clear][k] = 0x7f7fffffu;
