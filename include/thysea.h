@@ -43,7 +43,7 @@ extern "C" {
 #define THY_ERR_BUDGET 7       /* a scenario does not fit the server's HBM budget */
 #define THY_ERR_CANCELLED 8    /* a served request was cancelled */
 #define THY_ERR_TOO_LARGE 9    /* grid larger than an allocation-free entry point's fixed scratch */
-#define THY_ERR_TIMEOUT 10     /* a bounded wait on the device ran out (a staging copy did not land) */
+#define THY_ERR_TIMEOUT 10     /* a bounded wait on the device ran out: a staging copy or a block of a resident chunk did not arrive */
 
 /* ------------------------------------------------------------------------
  * Raw problem: the contents of the problem .txt file and of its GRD and
@@ -241,8 +241,11 @@ void thy_session_close(thy_session *s);
 /* Test hook for failure detection: with `what` = 1 the deep-water kernels
    issue none of this session's staging copies, so their bounded waits
    (four seconds of global time) run out, the step stops and thy_session_steps
-   returns THY_ERR_TIMEOUT with the device context still usable; 0 turns it
-   off.  Nothing faults, traps or hangs. */
+   returns THY_ERR_TIMEOUT with the device context still usable; with 2 one
+   block of its resident chunks stays away from the barriers between the steps'
+   phases, and the other blocks' waits (0.2 s) run out the same way; 0 turns it
+   off (after 2 the session can step on: the chunk has advanced nothing).
+   Nothing faults, traps or hangs. */
 int thy_session_inject(thy_session *s, int what);
 
 /* Autotuner of the warp tilings.  Every full chunk of a run (of any entry

@@ -165,3 +165,33 @@ def test_scenarios_that_fail_in_a_resident_batch(gpu):
             assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k
     # (launched chunks of a queue are 16 steps long)
     assert chunks < max(r["iterations"] for _, r in alone) / 16
+
+
+def test_barrier_timeout_is_reported_and_the_chunk_can_be_stepped_again(gpu):
+    """one block that stays away from a resident chunk's barriers: the others'
+    waits run out, the steps fail with THY_ERR_TIMEOUT, and the next chunk starts
+    on cleared barrier words from the state of the last good one"""
+    prep = thysea.Prepared(_problem(641, 512, "open", 3600.0))
+    ref = thysea.Session(prep)
+    ref.steps(16)
+    ref.steps(48)
+    want = ref.fetch()
+    s = thysea.Session(prep)
+    _, k = s.steps(16)
+    before, t = s.launches(), s.time()
+    assert k == 16 and before < 16   # resident
+    s.inject(2)
+    for _ in range(2):
+        with pytest.raises(thysea.ThyError) as e:
+            s.steps(16)
+        assert e.value.code == thysea.THY_ERR_TIMEOUT
+        assert s.time() == t
+    s.inject(0)
+    _, k = s.steps(48)
+    assert k == 48
+    assert s.time() == ref.time() and s.tiles() == ref.tiles()
+    got = s.fetch()
+    for key in want:
+        assert np.array_equal(got[key], want[key], equal_nan=True), key
+    s.close()
+    ref.close()

@@ -71,6 +71,12 @@ __host__ __device__ constexpr int deep_ng(int phase, int v)
 __host__ __device__ constexpr int deep_minb(int phase, int v) { return v == 0 ? (phase == 1 ? 2 : 3) : v == 1 ? 2 : 1; }
 __host__ __device__ constexpr int general_ng(int v) { return v == 0 ? 2 : v == 1 ? 1 : 8; }
 
+// Limit of every wait on the device (global time; each also has a limit of
+// polls): what is waited for takes microseconds; the limit is seconds so that a
+// context that is time-sliced or pre-empted on a shared GPU does not take a
+// healthy copy or barrier for a lost one.
+constexpr unsigned long long kWaitNs = 4000000000ull;
+
 // step.cu
 cudaError_t configure_step_kernels();
 int step_blocks_per_sm(int general_variant);
@@ -106,8 +112,8 @@ void launch_lists_current(const StepLaunch &L, cudaStream_t st);
 // resident.cu: a chunk of steps in one cooperative launch, one CTA per SM, for
 // work whose steps are bound by the latency of their launches
 constexpr int kResidentSlots = 64;      // scenarios of such a chunk at most
-// Barrier words, zero before the first launch (the kernel leaves the ones of
-// its next launch zero): arrivals in the upper half; in the lower half of
+// Barrier words, zero before the first launch and after one that gave up a wait
+// (else the kernel leaves the ones of its next launch zero): arrivals in the upper half; in the lower half of
 // phase 2's the scenario's dt bound, as the largest of 0x7f7fffff - its bits.
 struct ResidentSync {
     struct alignas(128) Word {
@@ -125,6 +131,8 @@ struct ResidentLaunch {
     ResidentSync *sync;
     int nslots, nunits, cap, steps;
     int rows_general, rows_deep;   // rows of a task: 1, 2, 4 or 8
+    unsigned long long wait_ns;    // limit of a barrier's wait
+    bool drop;                     // test hook: a CTA stays away from the steps' barriers
 };
 int resident_warps(int sms);             // warps of a launch
 int resident_tasks_capacity(int warps);  // tasks they can hold

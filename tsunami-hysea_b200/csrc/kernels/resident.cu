@@ -127,9 +127,9 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-// arrives at w and waits for n arrivals: the word then, or 0 after kWaitNs of
+// arrives at w and waits for n arrivals: the word then, or 0 after wait_ns of
 // global time (or 2^28 polls), so that no wait is endless
-__device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word &w, unsigned n)
+__device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word &w, unsigned n, unsigned long long wait_ns)
 {
     asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&w.v), "l"(1ull << 32) : "memory");
     unsigned long long v = ld_acquire(&w.v);
@@ -138,7 +138,7 @@ __device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word
     for (int i = 0; i < (1 << 28); i++) {
         v = ld_acquire(&w.v);
         if ((unsigned)(v >> 32) == n) return v;
-        if ((i & 63) == 63 && global_ns() - t0 > kWaitNs) break;
+        if ((i & 63) == 63 && global_ns() - t0 > wait_ns) break;
     }
     return 0ull;
 }
@@ -374,6 +374,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nblk = gridDim.x, NW = nblk * kResWarps;
     const bool single = L.nslots == 1;
+    const bool absent = L.drop && blockIdx.x == nblk - 1;   // test hook: this CTA takes part in no barrier of the steps
     const Shared h = shared_layout(dsm, L.nslots);
     ResidentSync *sync = L.sync;
     Task *tasks = h.tasks;
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
     int at = __ldcg(&sync->next);   // this launch's first barrier words
     __syncthreads();
-    if (tid == 0 && !arrive_and_wait(sync->start, nblk)) s_ok = false;
+    if (tid == 0 && !arrive_and_wait(sync->start, nblk, L.wait_ns)) s_ok = false;
     __syncthreads();
 
     // ---- this CTA's tasks, dealt in rounds: the shallow general units' first,
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
     __syncthreads();
 
-    for (int step = 0; step < L.steps && s_ok; step++) {
+    for (int step = 0; step < L.steps && s_ok && !absent; step++) {
         // ---- phase 1 ----
         for (int j = warp; j < ntask; j = claim(&s_next[0])) {
             const Task t = tasks[j];
@@ -519,7 +520,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
         __syncthreads();
         if (tid == 0) {
             s_next[0] = kResWarps;
-            if (!arrive_and_wait(sync->phase1[at], nblk)) s_ok = false;
+            if (!arrive_and_wait(sync->phase1[at], nblk, L.wait_ns)) s_ok = false;
         }
         __syncthreads();
         if (!s_ok) break;
@@ -602,7 +603,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                 if (key) atomicMax(reinterpret_cast<unsigned *>(&w.v), key);
                 h.dt_bits[0] = 0x7f7fffffu;
             }
-            const unsigned long long v = arrive_and_wait(w, nblk);
+            const unsigned long long v = arrive_and_wait(w, nblk, L.wait_ns);
             if (!v) s_ok = false;
             s_min = 0x7f7fffffu - (unsigned)v;
         }
@@ -656,7 +657,8 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
 
     // ---- the end of the chunk: counts and control blocks back ----
-    if (s_ok && tid < ntask) {
+    const bool whole = s_ok && !absent;
+    if (whole && tid < ntask) {
         const Task t = tasks[tid];
         if (t.sub == 0) {
             const ScenarioDev &s = h.tab[t.slot];
@@ -665,16 +667,15 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             if (counted_dry) atomicAdd(&s.ctl->units_dry, (unsigned long long)counted_dry);
         }
     }
-    if (blockIdx.x != 0) return;
+    // A CTA whose wait ran out has stepped less than the others and kept its counts:
+    // whichever it is, it reports every scenario that it has not seen end, and the
+    // host fails those and clears the barrier words.
     for (int k = tid; k < L.nslots; k += kResThreads) {
         ScenarioCtl *c = h.tab[k].ctl;
-        if (s_ok) {
-            store_advanced(c, h.ctl[k]);
-        } else if (c->status == kRunning) {
-            // a barrier's wait ran out: the host reports it
-            atomicOr(&c->errors, 2u);
-            c->status = kFailed;
-        }
+        const int status = h.state[k].status;
+        const bool ended = status == kDone || status == kFailed;
+        if (!whole && !ended) atomicOr(&c->errors, 2u);
+        if (blockIdx.x == 0 && (whole || ended)) store_advanced(c, h.ctl[k]);
     }
 }
 

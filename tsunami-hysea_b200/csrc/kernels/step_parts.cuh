@@ -245,12 +245,6 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// Limit of every wait on the device (global time; each also has a limit of
-// polls): what is waited for takes microseconds; the limit is seconds so that a
-// context that is time-sliced or pre-empted on a shared GPU does not take a
-// healthy copy or barrier for a lost one.
-constexpr unsigned long long kWaitNs = 4000000000ull;
-
 struct DeepRow {
     float4 m;      // cos, ilcos, area, dlon (edge row)
     float icos;    // 1/cos, correctly rounded

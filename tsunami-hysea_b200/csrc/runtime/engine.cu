@@ -1234,6 +1234,9 @@ int Batch::run_resident(int len, const Tiling &rows)
     R.cap = kResidentUnits;
     R.steps = len;
     resident_rows(res_units, resident_warps(sms), rows, &R.rows_general, &R.rows_deep);
+    R.drop = false;
+    for (auto *m : members) R.drop |= m && (m->hctl.inject & 2);
+    R.wait_ns = R.drop ? kWaitNs / 20 : kWaitNs;
     THY_CK(launch_resident(R, sms, st));
     lists_stale = true;
     return THY_OK;
@@ -1317,9 +1320,13 @@ int Batch::run_chunk(bool timed, int len)
         m->hctl = h_ctl[i];
         if (b0[i].step < 0) continue;
         const long long k = m->hctl.step - b0[i].step;
+        if (res && (m->hctl.errors & 2u)) {
+            // some CTA gave up a barrier: the scenario has not been stepped by all
+            // of them, and the barrier words are left as they were
+            m->hctl.status = kFailed;
+            THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
+        }
         if (m->hctl.status == kFailed || k != chunk) full = false;
-        // (a resident chunk that gave up a barrier leaves its words behind)
-        if (res && (m->hctl.errors & 2u)) THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
         if (k > 0) {
             const double deep = (double)(m->hctl.units_deep - b0[i].deep);
             const double dry = (double)(m->hctl.units_dry - b0[i].dry);
@@ -1450,7 +1457,7 @@ extern "C" const char *thy_strerror(int code)
     case THY_ERR_CUDA: return last_error_text()[0] ? last_error_text() : "CUDA error";
     case THY_ERR_NO_DEVICE: return "there is no CUDA device";
     case THY_ERR_NONFINITE: return "the state or the time step became non-finite";
-    case THY_ERR_TIMEOUT: return "a bounded wait on the device ran out (a staging copy did not land)";
+    case THY_ERR_TIMEOUT: return "a bounded wait on the device ran out (a staging copy or a block of a resident chunk did not arrive)";
     case THY_ERR_BUDGET: return "scenario does not fit the HBM budget";
     case THY_ERR_CANCELLED: return "request cancelled";
     case THY_ERR_TOO_LARGE: return "grid exceeds the allocation-free entry point's maximum of 1048576 cells";
@@ -1733,7 +1740,9 @@ extern "C" double thy_session_time(const thy_session *S) { return S ? S->s.hctl.
 
 extern "C" int thy_session_inject(thy_session *S, int what)
 {
-    if (!S || what < 0 || what > 1) return THY_ERR_INVALID;
+    if (!S || what < 0 || what > 2) return THY_ERR_INVALID;
+    // (a resident chunk that was given up has advanced nothing: it can be stepped again)
+    if (S->s.hctl.inject == 2) S->s.hctl.errors &= ~2u;
     S->s.hctl.inject = what;
     return S->s.upload_ctl(S->st);
 }

@@ -288,8 +288,9 @@ class Session:
 
     def inject(self, what: int):
         """Test hook (thy_session_inject): 1 = the deep-water kernels issue
-        none of this session's staging copies, so their bounded waits run out
-        and the next steps fail with THY_ERR_TIMEOUT; 0 = off."""
+        none of this session's staging copies, 2 = a block of its resident
+        chunks stays away from the barriers, so that bounded waits run out and
+        the next steps fail with THY_ERR_TIMEOUT; 0 = off."""
         _check(_ffi.lib().thy_session_inject(self._h, what), "thy_session_inject")
 
     def tuned(self):
