@@ -113,16 +113,16 @@ void launch_lists_current(const StepLaunch &L, cudaStream_t st);
 // work whose steps are bound by the latency of their launches
 constexpr int kResidentSlots = 64;      // scenarios of such a chunk at most
 // Barrier words, zero before the first launch and after one that gave up a wait
-// (else the kernel leaves the ones of its next launch zero): arrivals in the upper half; in the lower half of
-// phase 2's the scenario's dt bound, as the largest of 0x7f7fffff - its bits.
+// (else the kernel leaves the ones of its next launch zero), and the scenarios'
+// smallest dt bounds of a step (float bits).
 struct ResidentSync {
     struct alignas(128) Word {
-        unsigned long long v, pad[15];
+        unsigned arrived, pad[31];
     };
     Word start, phase1[3], phase2[3];   // by step modulo 3, counted on from launch to launch
+    unsigned int dt_bits[3][kResidentSlots];
     int next;                           // the next launch's first step, modulo 3
     int counts[4];                      // units per list at the start of the chunk
-    unsigned int dt_bits[3][kResidentSlots];   // several scenarios: their smallest dt bounds
 };
 struct ResidentLaunch {
     const ScenarioDev *tab;    // the stepped scenarios (nslots of them)

@@ -119,28 +119,32 @@ __device__ __forceinline__ Shared shared_layout(unsigned char *m, int nslots)
 // release, waits acquire (which also drops the SM's L1 lines, so that plain
 // loads after a barrier see what other SMs wrote before it).  Measured on 148
 // CTAs: 1.27 us a barrier; a tag per CTA that every CTA polls 6.0 us, a
-// gathering CTA that answers with one word 2.9 us.
+// gathering CTA that answers with one word 2.9 us.  The dt bounds lie in words of
+// their own, read after the wait: one more load than a bound in the counter's word
+// (0.15 to 0.35 us a step), but accesses of two sizes to one word have no defined
+// order in the PTX memory model.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p)
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
 {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
-// arrives at w and waits for n arrivals: the word then, or 0 after wait_ns of
-// global time (or 2^28 polls), so that no wait is endless
-__device__ __forceinline__ unsigned long long arrive_and_wait(ResidentSync::Word &w, unsigned n, unsigned long long wait_ns)
+// arrives at w and waits for n arrivals; false after wait_ns of global time (or
+// 2^28 polls), so that no wait is endless
+__device__ __forceinline__ bool arrive_and_wait(ResidentSync::Word &w, unsigned n, unsigned long long wait_ns)
 {
-    asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(&w.v), "l"(1ull << 32) : "memory");
-    unsigned long long v = ld_acquire(&w.v);
-    if ((unsigned)(v >> 32) == n) return v;
-    const unsigned long long t0 = global_ns();
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&w.arrived) : "memory");
+    unsigned long long t0 = 0;
     for (int i = 0; i < (1 << 28); i++) {
-        v = ld_acquire(&w.v);
-        if ((unsigned)(v >> 32) == n) return v;
-        if ((i & 63) == 63 && global_ns() - t0 > wait_ns) break;
+        if (ld_acquire(&w.arrived) == n) return true;
+        if ((i & 63) == 63) {
+            const unsigned long long now = global_ns();
+            if (!t0) t0 = now;
+            else if (now - t0 > wait_ns) break;
+        }
     }
-    return 0ull;
+    return false;
 }
 
 // ---------------------------------------------------------------------------
@@ -367,13 +371,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 {
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ bool s_ok;            // no wait has run out
-    __shared__ unsigned s_min;       // one scenario: the step's smallest dt bound
     __shared__ int s_next[2];        // the CTA's next task of phase 1 and 2
     __shared__ int s_sample[kResidentSlots];   // CTA 0: the step's gauge samples (ring slots)
-    __shared__ bool s_sampled;       // some
+    __shared__ bool s_sampled, s_any;          // some; some scenario still runs
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int nblk = gridDim.x, NW = nblk * kResWarps;
-    const bool single = L.nslots == 1;
     const bool absent = L.drop && blockIdx.x == nblk - 1;   // test hook: this CTA takes part in no barrier of the steps
     const Shared h = shared_layout(dsm, L.nslots);
     ResidentSync *sync = L.sync;
@@ -390,7 +392,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
     if (tid == 0) {
         s_ok = true;
-        s_sampled = false;
     }
     __syncthreads();
     for (int k = tid; k < L.nslots; k += kResThreads) {
@@ -584,58 +585,54 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             if (bad) fail(s, &h.dt_bits[t.slot]);
         }
         __syncthreads();
-        // one scenario: the block's bound goes into the barrier word; several: into
-        // a word each
+        // the block's bounds into the step's words
         unsigned *gmin = sync->dt_bits[at];
-        if (!single) {
-            for (int k = tid; k < L.nslots; k += kResThreads)
-                if (h.dt_bits[k] != 0x7f7fffffu) {
-                    atomicMin(gmin + k, h.dt_bits[k]);
-                    h.dt_bits[k] = 0x7f7fffffu;
-                }
-            __syncthreads();
-        }
-        if (tid == 0) {
-            s_next[1] = kResWarps;
-            ResidentSync::Word &w = sync->phase2[at];
-            if (single) {
-                const unsigned key = 0x7f7fffffu - min(h.dt_bits[0], 0x7f7fffffu);
-                if (key) atomicMax(reinterpret_cast<unsigned *>(&w.v), key);
-                h.dt_bits[0] = 0x7f7fffffu;
+        for (int k = tid; k < L.nslots; k += kResThreads)
+            if (h.dt_bits[k] != 0x7f7fffffu) {
+                atomicMin(gmin + k, h.dt_bits[k]);
+                h.dt_bits[k] = 0x7f7fffffu;
             }
-            const unsigned long long v = arrive_and_wait(w, nblk, L.wait_ns);
-            if (!v) s_ok = false;
-            s_min = 0x7f7fffffu - (unsigned)v;
-        }
-        __syncthreads();
-        if (!s_ok) break;
+        if (L.nslots > 1) __syncthreads();   // (one scenario: the arriving thread's own)
 
-        // ---- the step's control, by every CTA for itself: a thread per
+        // ---- the step's control, by every CTA for itself: warp 0, a lane per
         // scenario (the gauge samples by CTA 0) ----
-        const int clear = at == 0 ? 2 : at - 1;   // the words every CTA is done with
-        for (int k = tid; k < L.nslots; k += kResThreads) {
-            ScenarioCtl &c = h.ctl[k];
-            if (c.status != kRunning) continue;
-            const ScenarioDev &s = h.tab[k];
-            const unsigned bits = single ? s_min : __ldcg(gmin + k);
-            const int sample = advance_scenario(c, s, __uint_as_float(bits), 0u);
-            h.state[k] = step_state(c);
-            if (blockIdx.x == 0) {
-                sync->dt_bits[clear][k] = 0x7f7fffffu;
-                s_sample[k] = sample;
-                if (sample >= 0) {
-                    s.gauge_ring_t[sample] = c.t * c.T;
-                    s_sampled = true;
+        if (warp == 0) {
+            bool go = lane != 0 || arrive_and_wait(sync->phase2[at], nblk, L.wait_ns);
+            go = __all_sync(0xffffffffu, go);
+            __syncwarp();   // (the bounds are read after lane 0's wait)
+            const int clear = at == 0 ? 2 : at - 1;   // the words every CTA is done with
+            bool any = false, sampled = false;
+            for (int k = lane; go && k < L.nslots; k += 32) {
+                ScenarioCtl &c = h.ctl[k];
+                if (c.status != kRunning) continue;
+                const ScenarioDev &s = h.tab[k];
+                const int sample = advance_scenario(c, s, __uint_as_float(__ldcg(gmin + k)), 0u);
+                h.state[k] = step_state(c);
+                any |= c.status == kRunning;
+                if (blockIdx.x == 0) {
+                    sync->dt_bits[clear][k] = 0x7f7fffffu;
+                    s_sample[k] = sample;
+                    if (sample >= 0) s.gauge_ring_t[sample] = c.t * c.T;
+                    sampled |= sample >= 0;
+                }
+            }
+            any = __any_sync(0xffffffffu, any);
+            sampled = __any_sync(0xffffffffu, sampled);
+            if (lane == 0) {
+                s_next[1] = kResWarps;
+                s_ok = go;
+                s_any = any;
+                s_sampled = sampled;
+                if (blockIdx.x == 0 && go) {
+                    sync->phase1[clear].arrived = sync->phase2[clear].arrived = sync->start.arrived = 0u;
+                    sync->counts[0] = sync->counts[1] = sync->counts[2] = sync->counts[3] = 0;
+                    sync->next = at == 2 ? 0 : at + 1;
                 }
             }
         }
         at = at == 2 ? 0 : at + 1;
-        if (blockIdx.x == 0 && tid == kResThreads - 1) {
-            sync->phase1[clear].v = sync->phase2[clear].v = sync->start.v = 0ull;
-            sync->counts[0] = sync->counts[1] = sync->counts[2] = sync->counts[3] = 0;
-            sync->next = at;
-        }
         __syncthreads();
+        if (!s_ok) break;
         if (s_sampled) {
             for (int k = 0; k < L.nslots; k++) {
                 const int sample = s_sample[k];
@@ -647,13 +644,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             }
             __syncthreads();
             if (tid < kResidentSlots) s_sample[tid] = -1;
-            if (tid == 0) s_sampled = false;
             __syncthreads();
         }
-        // nothing left to step: every scenario of the chunk is paused or done
-        bool any = false;
-        for (int k = lane; k < L.nslots; k += 32) any |= h.state[k].status == kRunning;
-        if (!__any_sync(0xffffffffu, any)) break;
+        if (!s_any) break;   // nothing left to step: every scenario of the chunk is paused or done
     }
 
     // ---- the end of the chunk: counts and control blocks back ----
