@@ -1,6 +1,7 @@
 // Launch wrappers of the device kernels (host-callable, no CUDA types beyond
 // cudaStream_t / int2 in the signatures).
 #pragma once
+#include <algorithm>
 #include <cstddef>
 #include <cuda_runtime.h>
 
@@ -134,8 +135,41 @@ struct ResidentLaunch {
     unsigned long long wait_ns;    // limit of a barrier's wait
     bool drop;                     // test hook: a CTA stays away from the steps' barriers
 };
-int resident_warps(int sms);             // warps of a launch
-int resident_tasks_capacity(int warps);  // tasks they can hold
+constexpr int kResidentWarps = 16;       // warps of a CTA
+constexpr int resident_warps(int sms) { return sms * kResidentWarps; }           // of a launch
+constexpr int resident_tasks_capacity(int warps) { return warps * 32; }          // tasks they can hold
+// Largest work of a resident chunk, in units (us a step resident / launched: 640
+// units 38 / 70, 1500 units 64 / 94, 2560 units 95 / 111, 3168 units 120 / 127,
+// 3768 units 135 / 136, 4394 units 153 / 147, 5264 units 197 / 172: the launched
+// kernels stage the deep units, which pays once every SM has enough of them to
+// hide the launches).  Measured on 148 SMs; a device with fewer has as much less of
+// a resident chunk's tasks and registers.
+constexpr int kResidentUnits = 3712;
+constexpr int resident_units(int sms) { return sms < 148 ? kResidentUnits * sms / 148 : kResidentUnits; }
+static_assert(resident_units(1) * 8 <= resident_tasks_capacity(resident_warps(1)), "in rows of 8: 8 tasks a unit");
+// Rows of the tasks of a resident chunk: r = 1, 2, 4 or 8 general rows, the
+// first with at most 3 r^2 / 64 units a warp, and twice as many deep rows.  Short
+// tasks shorten a step's chain while warps are idle; each evaluates one y edge
+// row more than it has rows, which costs more once every warp has several.  (us
+// per step, 2368 warps, r = 1 / 2 / 4 / 8: 88 units 19.7 / 21.3 / 28.8 / 46.1; 108
+// units 21.8 / 22.6 / 29.7 / 47.0; 240 units 30.4 / 26.3 / 31.8 / 49.1; 456 units
+// 42.0 / 34.9 / 35.6 / 51.1; 640 units 52.2 / 42.8 / 40.7 / 54.2; 984 units 72.5 /
+// 56.9 / 51.5 / 58.6; 1500 units r = 4 / 8 69.3 / 71.8; 1921 units 84.9 / 82.8.)
+// Work the tuner searches takes its variants of the general kernel and of deep
+// phase 2 as half and double the rows.
+inline void resident_rows(int units, int warps, const Tiling &t, int *general, int *deep)
+{
+    int r = 1;
+    while (r < 8 && units * 64 > 3 * r * r * warps) r *= 2;
+    const auto variant = [](int rows, int v) { return std::min(8, std::max(1, v == 1 ? 2 * rows : v == 2 ? rows / 2 : rows)); };
+    *general = variant(r, t.general);
+    *deep = variant(std::min(8, 2 * r), t.deep2);
+    // (a CTA holds one task a thread; resident_units() fit in rows of 8)
+    while (std::min(*general, *deep) < 8 && units * (64 / std::min(*general, *deep)) > resident_tasks_capacity(warps)) {
+        *general = std::min(8, 2 * *general);
+        *deep = std::min(8, 2 * *deep);
+    }
+}
 cudaError_t configure_resident_kernel();
 cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st);
 // init_extract.cu: the step controller of every slot (launch 5 of a step)

@@ -40,7 +40,7 @@ namespace thy {
 
 namespace {
 
-constexpr int kResWarps = 16, kResThreads = 32 * kResWarps;
+constexpr int kResWarps = kResidentWarps, kResThreads = 32 * kResWarps;
 constexpr int kMaxDeepRows = 8;     // rows of a deep task at most
 constexpr int kTaskRows = kMaxDeepRows + 2;
 constexpr int kDealStep = 61;       // odd: units of one column of a grid alternate in the lists
@@ -673,9 +673,6 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 }
 
 }  // namespace
-
-int resident_warps(int sms) { return sms * kResWarps; }
-int resident_tasks_capacity(int warps) { return warps * 32; }
 
 cudaError_t configure_resident_kernel()
 {

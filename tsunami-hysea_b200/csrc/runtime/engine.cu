@@ -1027,7 +1027,7 @@ int Batch::update(const std::vector<char> *selected)
     if (nwork) THY_CK(cudaMemcpyAsync(d_work, work.data(), nwork * sizeof(int2), cudaMemcpyHostToDevice, st));
     THY_CK(cudaMemcpyAsync(d_nwork, &nwork, sizeof(int), cudaMemcpyHostToDevice, st));
     // the same work for resident chunks, where it is small enough
-    const bool fits = !rtab.empty() && rtab.size() <= kResidentSlots && runits <= kResidentUnits;
+    const bool fits = !rtab.empty() && rtab.size() <= kResidentSlots && runits <= resident_units(device_sm_count());
     res_slots = fits ? (int)rtab.size() : 0;
     res_units = fits ? (int)runits : 0;
     std::vector<int2> units;
@@ -1186,7 +1186,7 @@ int Batch::fresh_lists()
     return THY_OK;
 }
 
-// Resident chunks step work of up to kResidentUnits units; a forced or default
+// Resident chunks step work of up to resident_units() units; a forced or default
 // tiling (THY_TILING, THY_TUNE=0, thy_tiling_force) names the launched kernels,
 // and the staging-copy test hook has nothing to withhold in a resident chunk.
 bool Batch::resident() const
@@ -1195,30 +1195,6 @@ bool Batch::resident() const
     for (auto *m : members)
         if (m && (m->hctl.inject & 1)) return false;
     return true;
-}
-
-// Rows of the tasks of a resident chunk: r = 1, 2, 4 or 8 general rows, the
-// first with at most 3 r^2 / 64 units a warp, and twice as many deep rows.  Short
-// tasks shorten a step's chain while warps are idle; each evaluates one y edge
-// row more than it has rows, which costs more once every warp has several.  (us
-// per step, 2368 warps, r = 1 / 2 / 4 / 8: 88 units 19.7 / 21.3 / 28.8 / 46.1; 108
-// units 21.8 / 22.6 / 29.7 / 47.0; 240 units 30.4 / 26.3 / 31.8 / 49.1; 456 units
-// 42.0 / 34.9 / 35.6 / 51.1; 640 units 52.2 / 42.8 / 40.7 / 54.2; 984 units 72.5 /
-// 56.9 / 51.5 / 58.6; 1500 units r = 4 / 8 69.3 / 71.8; 1921 units 84.9 / 82.8.)
-// Work the tuner searches takes its variants of the general kernel and of deep
-// phase 2 as half and double the rows.
-static void resident_rows(int units, int warps, const Tiling &t, int *general, int *deep)
-{
-    int r = 1;
-    while (r < 8 && units * 64 > 3 * r * r * warps) r *= 2;
-    const auto variant = [](int rows, int v) { return std::min(8, std::max(1, v == 1 ? 2 * rows : v == 2 ? rows / 2 : rows)); };
-    *general = variant(r, t.general);
-    *deep = variant(std::min(8, 2 * r), t.deep2);
-    // (a CTA holds one task a thread)
-    while (units * (64 / std::min(*general, *deep)) > resident_tasks_capacity(warps)) {
-        *general = std::min(8, 2 * *general);
-        *deep = std::min(8, 2 * *deep);
-    }
 }
 
 int Batch::run_resident(int len, const Tiling &rows)

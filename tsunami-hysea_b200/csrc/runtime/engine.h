@@ -194,12 +194,6 @@ struct Batch {
     int run_resident(int len, const Tiling &rows);
 };
 
-// Largest work of a resident chunk, in units (us a step resident / launched: 640
-// units 38 / 70, 1500 units 64 / 94, 2560 units 95 / 111, 3168 units 120 / 127,
-// 3768 units 135 / 136, 4394 units 153 / 147, 5264 units 197 / 172: the launched
-// kernels stage the deep units, which pays once every SM has enough of them to
-// hide the launches).
-constexpr int kResidentUnits = 3712;
 // Longest chunk that is no sample of the autotuner.  Between chunks the GPU waits
 // for the host (the control blocks' copy, a launch: about 40 us before a resident
 // chunk, more with a graph launch); the gauge ring keeps the samples of the steps
