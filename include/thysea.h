@@ -244,7 +244,9 @@ void thy_session_close(thy_session *s);
    returns THY_ERR_TIMEOUT with the device context still usable; with 2 one
    block of its resident chunks stays away from the barriers between the steps'
    phases, and the other blocks' waits (0.2 s) run out the same way; 0 turns it
-   off (after 2 the session can step on: the chunk has advanced nothing).
+   off (after 2 the session can step on: the chunk has advanced nothing).  With 4
+   the launch of its next resident chunk counts as refused by the driver, and the
+   session is stepped by separate launches from then on.
    Nothing faults, traps or hangs. */
 int thy_session_inject(thy_session *s, int what);
 

@@ -195,3 +195,25 @@ def test_barrier_timeout_is_reported_and_the_chunk_can_be_stepped_again(gpu):
         assert np.array_equal(got[key], want[key], equal_nan=True), key
     s.close()
     ref.close()
+
+
+def test_refused_resident_launch_takes_the_launched_kernels(gpu):
+    """a resident launch that the driver refuses (a partition of the GPU): the
+    chunk is stepped by separate launches, with the same results"""
+    prep = thysea.Prepared(_problem(500, 411, "open", 3600.0))
+    ref, s = thysea.Session(prep), thysea.Session(prep)
+    ref.steps(16)
+    ref.steps(40)
+    s.steps(16)
+    assert s.launches() < 16
+    s.inject(4)
+    n = s.launches()
+    _, k = s.steps(40)
+    assert k == 40 and s.launches() - n == 5 * 40   # five launches a step
+    assert ref.launches() < 16
+    assert s.time() == ref.time() and s.tiles() == ref.tiles()
+    got, want = s.fetch(), ref.fetch()
+    for key in want:
+        assert np.array_equal(got[key], want[key], equal_nan=True), key
+    s.close()
+    ref.close()

@@ -170,7 +170,7 @@ inline void resident_rows(int units, int warps, const Tiling &t, int *general, i
         *deep = std::min(8, 2 * *deep);
     }
 }
-cudaError_t configure_resident_kernel();
+cudaError_t configure_resident_kernel(int device, bool *usable);   // usable: the device takes such launches
 cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st);
 // init_extract.cu: the step controller of every slot (launch 5 of a step)
 void launch_controller(const StepLaunch &L, cudaStream_t st);

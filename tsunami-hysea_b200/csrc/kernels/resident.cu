@@ -674,10 +674,21 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 
 }  // namespace
 
-cudaError_t configure_resident_kernel()
+cudaError_t configure_resident_kernel(int device, bool *usable)
 {
-    return cudaFuncSetAttribute(resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)shared_bytes(kResidentSlots));
+    *usable = false;
+    int coop = 0, smem = 0, ctas = 0;
+    cudaError_t e;
+    if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device)) ||
+        (e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)))
+        return e;
+    const size_t need = shared_bytes(kResidentSlots);
+    if (!coop || need > (size_t)smem) return cudaSuccess;
+    if ((e = cudaFuncSetAttribute(resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need)) ||
+        (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, resident_kernel, kResThreads, need)))
+        return e;
+    *usable = ctas > 0;
+    return cudaSuccess;
 }
 
 cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st)

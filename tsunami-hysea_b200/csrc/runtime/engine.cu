@@ -35,6 +35,7 @@ namespace {
 thread_local char g_err[512] = "";
 int g_device = 0;
 bool g_configured[64] = {};
+bool g_resident[64] = {};   // the device takes resident chunks
 int g_sms[64] = {};
 }  // namespace
 
@@ -56,7 +57,7 @@ int ensure_device()
     THY_CK(cudaSetDevice(g_device));
     if (!g_configured[g_device]) {
         THY_CK(configure_step_kernels());
-        THY_CK(configure_resident_kernel());
+        THY_CK(configure_resident_kernel(g_device, &g_resident[g_device]));
         THY_CK(preload_output_kernels());
         THY_CK(preload_okada_kernels());
         // device buffers come from the stream-ordered default pool; freed
@@ -1186,12 +1187,13 @@ int Batch::fresh_lists()
     return THY_OK;
 }
 
-// Resident chunks step work of up to resident_units() units; a forced or default
-// tiling (THY_TILING, THY_TUNE=0, thy_tiling_force) names the launched kernels,
-// and the staging-copy test hook has nothing to withhold in a resident chunk.
+// Resident chunks step work of up to resident_units() units, where the device takes
+// their launches; a forced or default tiling (THY_TILING, THY_TUNE=0,
+// thy_tiling_force) names the launched kernels, and the staging-copy test hook has
+// nothing to withhold in a resident chunk.
 bool Batch::resident() const
 {
-    if (res_units == 0 || !tuner_free()) return false;
+    if (res_units == 0 || res_refused || !g_resident[device] || !tuner_free()) return false;
     for (auto *m : members)
         if (m && (m->hctl.inject & 1)) return false;
     return true;
@@ -1211,9 +1213,21 @@ int Batch::run_resident(int len, const Tiling &rows)
     R.steps = len;
     resident_rows(res_units, resident_warps(sms), rows, &R.rows_general, &R.rows_deep);
     R.drop = false;
-    for (auto *m : members) R.drop |= m && (m->hctl.inject & 2);
+    bool refuse = false;   // (test hook)
+    for (auto *m : members) {
+        R.drop |= m && (m->hctl.inject & 2);
+        refuse |= m && (m->hctl.inject & 4);
+    }
     R.wait_ns = R.drop ? kWaitNs / 20 : kWaitNs;
-    THY_CK(launch_resident(R, sms, st));
+    const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge : launch_resident(R, sms, st);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+        // fewer SMs than the device has are open to this process: nothing was
+        // launched, and this batch keeps to the launched kernels
+        cudaGetLastError();
+        res_refused = true;
+        return THY_OK;
+    }
+    THY_CK(e);
     lists_stale = true;
     return THY_OK;
 }
@@ -1274,6 +1288,7 @@ int Batch::run_chunk(bool timed, int len)
     if (timed) THY_CK(cudaEventRecord(ev0, st));
     if (res) {
         if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling()))) return rc;
+        if (res_refused) return run_chunk(timed, len);
     } else {
         for (int i = 0; i < len / chunk; i++) THY_CK(cudaGraphLaunch(gexec, st));
         for (int i = 0; i < len % chunk; i++) THY_CK(cudaGraphLaunch(one, st));
@@ -1716,7 +1731,7 @@ extern "C" double thy_session_time(const thy_session *S) { return S ? S->s.hctl.
 
 extern "C" int thy_session_inject(thy_session *S, int what)
 {
-    if (!S || what < 0 || what > 2) return THY_ERR_INVALID;
+    if (!S || what < 0 || (what > 2 && what != 4)) return THY_ERR_INVALID;
     // (a resident chunk that was given up has advanced nothing: it can be stepped again)
     if (S->s.hctl.inject == 2) S->s.hctl.errors &= ~2u;
     S->s.hctl.inject = what;

@@ -124,6 +124,7 @@ struct Batch {
     int *d_rorder = nullptr;
     ResidentSync *d_rsync = nullptr;
     int res_slots = 0, res_units = 0;  // of the current work list (0: too much work)
+    bool res_refused = false;          // the driver refused such a launch
     bool lists_stale = false;          // d_lists not made for the current states (made when a step is launched)
     ScenarioCtl *d_ctl = nullptr;      // slots
     ScenarioCtl *h_ctl = nullptr;      // pinned mirror
@@ -191,7 +192,7 @@ struct Batch {
     void reset_lists() { lists_stale = true; }   // classify again: after the host changed a member's state
     int fresh_lists();               // the classification, if it is due (before a launch of the stepping kernels)
     bool resident() const;           // the next chunk is one resident launch
-    int run_resident(int len, const Tiling &rows);
+    int run_resident(int len, const Tiling &rows);   // (a refused launch sets res_refused)
 };
 
 // Longest chunk that is no sample of the autotuner.  Between chunks the GPU waits
