@@ -252,15 +252,16 @@ int thy_session_inject(thy_session *s, int what);
 
 /* Autotuner of the warp tilings.  Every full chunk of a run (of any entry
    point) is timed as one sample of the tiling it ran with; the search, per
-   device and work of a step (ceil log2 of its deep units and of its general
-   units, estimated from each scenario's previous chunk), is coordinate
-   descent over deep phase 2, deep phase 1 and the general kernel.
+   device, kind of chunk (resident on the device, or steps launched one by one)
+   and work of a step (ceil log2 of its deep units and of its general units,
+   estimated from each scenario's previous chunk), is coordinate descent over
+   deep phase 2, deep phase 1 and the general kernel.
    Environment: THY_TILING="d1,d2,g" forces a tiling, THY_TUNE=0 keeps the
    default, THY_TUNE_CACHE=<file> keeps decided tilings across processes. */
 int thy_tiling_force(const thy_tiling *t);          /* NULL: autotune again */
 /* 1 when the tiling for steps of deep_units deep and general_units general
-   work units is decided on the current device (*best set), 0 while tuning
-   (*best: the incumbent) */
+   work units, in the kind of chunk that a run of that work takes, is decided on
+   the current device (*best set), 0 while tuning (*best: the incumbent) */
 int thy_tiling_tuned(double deep_units, double general_units, thy_tiling *best);
 void thy_tuner_clear(void);                         /* forget every decision of this process */
 

@@ -1243,7 +1243,7 @@ TuneKey Batch::tune_key(bool *known, bool all_members) const
             all = all && m->mix_known;
         }
     if (known) *known = all;
-    return TuneKey{device, tune_bucket(deep), tune_bucket(general)};
+    return TuneKey{device, tune_bucket(deep), tune_bucket(general), resident()};
 }
 
 int Batch::run_chunk(bool timed, int len)
@@ -1802,7 +1802,8 @@ extern "C" int thy_tiling_tuned(double deep_units, double general_units, thy_til
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) dev = 0;
     Tiling t;
-    const bool done = tuner_decided(TuneKey{dev, tune_bucket(deep_units), tune_bucket(general_units)}, &t);
+    const bool resident = dev < 64 && g_resident[dev] && deep_units + general_units <= resident_units(device_sm_count());
+    const bool done = tuner_decided(TuneKey{dev, tune_bucket(deep_units), tune_bucket(general_units), resident}, &t);
     if (best) *best = thy_tiling{t.deep1, t.deep2, t.general};
     return done ? 1 : 0;
 }

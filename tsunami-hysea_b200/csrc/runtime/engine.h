@@ -183,7 +183,7 @@ struct Batch {
     // of the tuner's, else kMaxChunk
     int chunk_for(long long steps) const;
     int max_chunk() const;
-    // the autotuner's key of the next chunk: this device, the deep and
+    // the autotuner's key of the next chunk: this device, its kind, the deep and
     // general units per step estimated from each stepping member's last
     // chunk (members with status running; every member when all_members);
     // *known: each of them has been measured

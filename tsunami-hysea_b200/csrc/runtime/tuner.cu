@@ -47,7 +47,7 @@ Tiling candidate(const Entry &e, int j)
 
 struct State {
     std::mutex mu;
-    std::map<std::tuple<int, int, int>, Entry> keys;
+    std::map<std::tuple<int, int, int, bool>, Entry> keys;
     bool env_read = false;
     bool forced = false;
     bool off = false;
@@ -88,15 +88,17 @@ void read_env(State &s)
     if (path && *path) s.cache_path = path;
 }
 
-// device identity written to the cache file: name (blanks replaced) and SM count
-std::string device_id(int device)
+// device identity written to the cache file: name (blanks replaced) with the kind
+// of chunk, and SM count
+std::string device_id(int device, bool resident)
 {
+    const char *kind = resident ? "/resident" : "/launched";
     cudaDeviceProp p;
-    if (cudaGetDeviceProperties(&p, device) != cudaSuccess) return "unknown 0";
+    if (cudaGetDeviceProperties(&p, device) != cudaSuccess) return std::string("unknown") + kind + " 0";
     std::string n = p.name;
     for (auto &ch : n)
         if (ch == ' ' || ch == '\t') ch = '_';
-    return n + " " + std::to_string(p.multiProcessorCount);
+    return n + kind + " " + std::to_string(p.multiProcessorCount);
 }
 
 void load_cache(State &s, int device)
@@ -105,13 +107,14 @@ void load_cache(State &s, int device)
     s.cache_loaded[device] = true;
     FILE *f = std::fopen(s.cache_path.c_str(), "r");
     if (!f) return;
-    const std::string id = device_id(device);
+    const std::string launched = device_id(device, false), resident = device_id(device, true);
     char name[256];
     int sms, bd, bg, a, b, c;
     while (std::fscanf(f, "%255s %d %d %d %d %d %d", name, &sms, &bd, &bg, &a, &b, &c) == 7) {
-        if (std::string(name) + " " + std::to_string(sms) != id) continue;
+        const std::string id = std::string(name) + " " + std::to_string(sms);
+        if (id != launched && id != resident) continue;
         if (a < 0 || b < 0 || c < 0 || a >= kTilingVariants || b >= kTilingVariants || c >= kTilingVariants) continue;
-        Entry &e = s.keys[std::make_tuple(device, bd, bg)];
+        Entry &e = s.keys[std::make_tuple(device, bd, bg, id == resident)];
         e.inc.deep1 = a;
         e.inc.deep2 = b;
         e.inc.general = c;
@@ -125,7 +128,7 @@ void store_cache(const State &s, const TuneKey &k, const Tiling &t)
     if (s.cache_path.empty()) return;
     FILE *f = std::fopen(s.cache_path.c_str(), "a");
     if (!f) return;
-    std::fprintf(f, "%s %d %d %d %d %d\n", device_id(k.device).c_str(), k.deep, k.general, t.deep1, t.deep2, t.general);
+    std::fprintf(f, "%s %d %d %d %d %d\n", device_id(k.device, k.resident).c_str(), k.deep, k.general, t.deep1, t.deep2, t.general);
     std::fclose(f);
 }
 
@@ -133,7 +136,7 @@ Entry &entry(State &s, const TuneKey &k)
 {
     read_env(s);
     load_cache(s, k.device);
-    return s.keys[std::make_tuple(k.device, k.deep, k.general)];
+    return s.keys[std::make_tuple(k.device, k.deep, k.general, k.resident)];
 }
 
 }  // namespace

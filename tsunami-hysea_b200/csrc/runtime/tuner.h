@@ -19,8 +19,9 @@
 //
 // Environment: THY_TILING="d1,d2,g" forces a tiling (variant indices);
 // THY_TUNE=0 keeps the default tiling; THY_TUNE_CACHE=<file> keeps decided
-// keys across processes (one line per key: device name, SM count, deep and
-// general buckets, tiling).
+// keys across processes (one line per key: device name and kind of chunk, SM
+// count, deep and general buckets, tiling; lines without a kind are of kernels
+// whose variants meant other row groups, and are left alone).
 #pragma once
 #include "../kernels/kernels.h"
 
@@ -28,11 +29,14 @@ namespace thy {
 
 // Key: the device and the work of a step, as ceil log2 buckets of its deep
 // units and of its general units (the best tiling of each kernel depends on
-// how many units it has to spread over the SMs).
+// how many units it has to spread over the SMs), and the kind of the chunk, in
+// which a variant means another thing: warps of a CTA's units where the steps are
+// launched, rows of a warp's tasks where the chunk is resident.
 struct TuneKey {
     int device;
     int deep;      // tune_bucket(deep units per step)
     int general;   // tune_bucket(general units per step)
+    bool resident = false;
 };
 
 int tune_bucket(double units);                       // ceil log2, 0 for units <= 1
