@@ -217,3 +217,32 @@ def test_refused_resident_launch_takes_the_launched_kernels(gpu):
         assert np.array_equal(got[key], want[key], equal_nan=True), key
     s.close()
     ref.close()
+
+
+def test_runs_of_several_threads_share_the_gpu(gpu):
+    """runs of several host threads at a time, each on its share of the SMs: the
+    results of each alone"""
+    import threading
+
+    sizes = [(96, 80, "file"), (256, 240, "late"), (500, 411, "open"), (113, 95, "late"), (1024, 700, "open"), (200, 640, "file")]
+    preps = [thysea.Prepared(_problem(nx, ny, kind, 400.0)) for nx, ny, kind in sizes]
+    alone = [_run(p) for p in preps]
+    out = [[] for _ in preps]
+    start = threading.Barrier(len(preps))
+
+    def work(k):
+        start.wait()
+        for _ in range(4):
+            out[k].append(_run(preps[k]))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(len(preps))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for (ref, r0), runs in zip(alone, out):
+        assert len(runs) == 4
+        for got, r in runs:
+            assert r["iterations"] == r0["iterations"] and r["deep_tiles"] == r0["deep_tiles"]
+            for k in FIELDS:
+                assert np.array_equal(got[k], ref[k], equal_nan=True), k

@@ -147,6 +147,18 @@ constexpr int resident_tasks_capacity(int warps) { return warps * 32; }         
 constexpr int kResidentUnits = 3712;
 constexpr int resident_units(int sms) { return sms < 148 ? kResidentUnits * sms / 148 : kResidentUnits; }
 static_assert(resident_units(1) * 8 <= resident_tasks_capacity(resident_warps(1)), "in rows of 8: 8 tasks a unit");
+// CTAs of a resident chunk of `units`, while the process steps all_units on the
+// device: its share of the SMs, at least an eighth of them and what holds its tasks.
+// A chunk on every SM would make the others wait for its end (one alone has them
+// all).  (Turns -> shares, ms for a run of each thread: 4 / 8 threads of 128^2 23.6 /
+// 48.1 -> 9.2 / 20.4, of 512^2 40 / 81 -> 29 / 59, of 1024^2 74 / 155 -> 64 / 142; a
+// 4096^2 run of 214 ms beside back-to-back runs of 128^2 to 1024^2 690..810 -> 247..257.)
+inline int resident_ctas(int units, int sms, long long all_units)
+{
+    const int per_cta = resident_tasks_capacity(kResidentWarps);
+    const int share = (int)((long long)sms * units / all_units);
+    return std::min(sms, std::max({share, (sms + 7) / 8, (8 * units + per_cta - 1) / per_cta}));
+}
 // Rows of the tasks of a resident chunk: r = 1, 2, 4 or 8 general rows, the
 // first with at most 3 r^2 / 64 units a warp, and twice as many deep rows.  Short
 // tasks shorten a step's chain while warps are idle; each evaluates one y edge
@@ -171,7 +183,7 @@ inline void resident_rows(int units, int warps, const Tiling &t, int *general, i
     }
 }
 cudaError_t configure_resident_kernel(int device, bool *usable);   // usable: the device takes such launches
-cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st);
+cudaError_t launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st);
 // init_extract.cu: the step controller of every slot (launch 5 of a step)
 void launch_controller(const StepLaunch &L, cudaStream_t st);
 // init_extract.cu: per-unit depth steps (ScenarioDev::unit_gmax), after the

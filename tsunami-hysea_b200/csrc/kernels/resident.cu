@@ -691,10 +691,10 @@ cudaError_t configure_resident_kernel(int device, bool *usable)
     return cudaSuccess;
 }
 
-cudaError_t launch_resident(const ResidentLaunch &L, int sms, cudaStream_t st)
+cudaError_t launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st)
 {
     void *args[] = {const_cast<ResidentLaunch *>(&L)};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(resident_kernel), dim3(sms), dim3(kResThreads), args,
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(resident_kernel), dim3(ctas), dim3(kResThreads), args,
                                        shared_bytes(L.nslots), st);
 }
 

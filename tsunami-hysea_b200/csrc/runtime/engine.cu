@@ -17,6 +17,7 @@
 #include <cuda.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdlib>
 #include <condition_variable>
@@ -71,6 +72,22 @@ int ensure_device()
         g_configured[g_device] = true;
     }
     return THY_OK;
+}
+
+// The units that the process's batches step on each device at the moment
+static std::atomic<long long> g_stepped[64];
+
+Stepping::Stepping(Batch &b) : b_(b) { b_.stepping = this; }
+Stepping::~Stepping()
+{
+    set(0);
+    b_.stepping = nullptr;
+}
+long long Stepping::set(long long units)
+{
+    const long long d = units - units_;
+    units_ = units;
+    return g_stepped[b_.device].fetch_add(d) + d;
 }
 
 int device_sm_count() { return g_sms[g_device] > 0 ? g_sms[g_device] : 148; }
@@ -1199,7 +1216,7 @@ bool Batch::resident() const
     return true;
 }
 
-int Batch::run_resident(int len, const Tiling &rows)
+int Batch::run_resident(int len, const Tiling &rows, long long all_units)
 {
     const int sms = device_sm_count();
     ResidentLaunch R;
@@ -1211,7 +1228,8 @@ int Batch::run_resident(int len, const Tiling &rows)
     R.nunits = res_units;
     R.cap = kResidentUnits;
     R.steps = len;
-    resident_rows(res_units, resident_warps(sms), rows, &R.rows_general, &R.rows_deep);
+    const int ctas = resident_ctas(res_units, sms, std::max<long long>(all_units, res_units));
+    resident_rows(res_units, resident_warps(ctas), rows, &R.rows_general, &R.rows_deep);
     R.drop = false;
     bool refuse = false;   // (test hook)
     for (auto *m : members) {
@@ -1219,7 +1237,7 @@ int Batch::run_resident(int len, const Tiling &rows)
         refuse |= m && (m->hctl.inject & 4);
     }
     R.wait_ns = R.drop ? kWaitNs / 20 : kWaitNs;
-    const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge : launch_resident(R, sms, st);
+    const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge : launch_resident(R, ctas, st);
     if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
         // fewer SMs than the device has are open to this process: nothing was
         // launched, and this batch keeps to the launched kernels
@@ -1273,21 +1291,24 @@ int Batch::run_chunk(bool timed, int len)
     }
     // a sample needs a chunk in which every running member steps `chunk`
     // times (no member reaches its end or an event before the chunk's last
-    // step, none fails) and whose work mix was known beforehand
+    // step, none fails), whose work mix was known beforehand and which no other
+    // batch of the process shared the device with
     struct Before {
         long long step;
         unsigned long long deep, dry;
     };
     std::vector<Before> b0(capacity, Before{-1, 0, 0});
-    long long running = 0;
+    long long running = 0, own_units = 0;
     for (int i = 0; i < capacity; i++)
         if (members[i] && members[i]->hctl.status == kRunning) {
+            own_units += members[i]->units();
             b0[i] = Before{members[i]->hctl.step, members[i]->hctl.units_deep, members[i]->hctl.units_dry};
             running++;
         }
+    const long long all_units = stepping ? stepping->set(own_units) : own_units;
     if (timed) THY_CK(cudaEventRecord(ev0, st));
     if (res) {
-        if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling()))) return rc;
+        if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling(), all_units))) return rc;
         if (res_refused) return run_chunk(timed, len);
     } else {
         for (int i = 0; i < len / chunk; i++) THY_CK(cudaGraphLaunch(gexec, st));
@@ -1296,6 +1317,7 @@ int Batch::run_chunk(bool timed, int len)
     if (timed) THY_CK(cudaEventRecord(ev1, st));
     THY_CK(cudaMemcpyAsync(h_ctl, d_ctl, capacity * sizeof(ScenarioCtl), cudaMemcpyDeviceToHost, st));
     THY_CK(cudaStreamSynchronize(st));
+    const bool shared = all_units != own_units || (stepping && stepping->set(own_units) != own_units);
     float ms = 0;
     if (timed) {
         THY_CK(cudaEventElapsedTime(&ms, ev0, ev1));
@@ -1303,7 +1325,7 @@ int Batch::run_chunk(bool timed, int len)
     }
     launches += res ? 1 : (long long)(kLaunchesPerStep - 1) * len;   // (the controller is part of phase 2)
     chunks_run++;
-    bool full = running > 0 && len == chunk;
+    bool full = running > 0 && len == chunk && !shared;
     double stepped = 0;   // deep + general units stepped in the chunk
     for (int i = 0; i < capacity; i++) {
         DevScenario *m = members[i];
@@ -1522,28 +1544,31 @@ extern "C" int thy_run(const thy_problem *p, const thy_outputs *o, thy_stats *st
         if (stats) stats->setup_seconds = std::chrono::duration<double>(t0 - t_start).count();
         if ((rc = initial_dt(b))) goto out;
         if (stats) stats->initial_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-        for (;;) {
-            if (!(s.hctl.t < s.t_end)) break;
-            if (s.max_steps >= 0 && s.hctl.step >= s.max_steps) break;
-            if (s.hctl.status == kFailed) { rc = failure_code(s.hctl); goto out; }
-            {
-                const auto te = std::chrono::steady_clock::now();
-                bool changed = false;
-                if ((rc = handle_events_ex(s, o, st, &changed))) goto out;
-                if (changed) b.reset_lists();
-                event_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - te).count();
+        {
+            Stepping loop(b);
+            for (;;) {
+                if (!(s.hctl.t < s.t_end)) break;
+                if (s.max_steps >= 0 && s.hctl.step >= s.max_steps) break;
+                if (s.hctl.status == kFailed) { rc = failure_code(s.hctl); goto out; }
+                {
+                    const auto te = std::chrono::steady_clock::now();
+                    bool changed = false;
+                    if ((rc = handle_events_ex(s, o, st, &changed))) goto out;
+                    if (changed) b.reset_lists();
+                    event_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - te).count();
+                }
+                s.hctl.status = kRunning;
+                s.hctl.events = 0;
+                if ((rc = s.upload_ctl(st))) goto out;
+                // chunks no longer than the steps left before the next event (as
+                // far as the current dt tells), so that few launches find the
+                // scenario paused
+                do {
+                    if ((rc = b.run_chunk(true, b.chunk_for(Batch::steps_to_event(s))))) goto out;
+                    if ((rc = s.read_device_gauges(o, st))) goto out;
+                } while (s.hctl.status == kRunning);
+                if (s.hctl.status == kFailed) { rc = failure_code(s.hctl); goto out; }
             }
-            s.hctl.status = kRunning;
-            s.hctl.events = 0;
-            if ((rc = s.upload_ctl(st))) goto out;
-            // chunks no longer than the steps left before the next event (as
-            // far as the current dt tells), so that few launches find the
-            // scenario paused
-            do {
-                if ((rc = b.run_chunk(true, b.chunk_for(Batch::steps_to_event(s))))) goto out;
-                if ((rc = s.read_device_gauges(o, st))) goto out;
-            } while (s.hctl.status == kRunning);
-            if (s.hctl.status == kFailed) { rc = failure_code(s.hctl); goto out; }
         }
         {
             auto t1 = std::chrono::steady_clock::now();
@@ -1641,6 +1666,7 @@ extern "C" int thy_session_steps(thy_session *S, long long steps, double *device
         // exactly `steps` steps' launches: full chunks, then power-of-two
         // chunks for the rest (a scenario that reaches its end or a fault
         // time earlier stops there)
+        Stepping loop(S->b);
         do {
             if ((rc = S->b.run_chunk(true, S->b.chunk_for(start + steps - s.hctl.step)))) return rc;
         } while (s.hctl.status == kRunning && s.hctl.step < start + steps);

@@ -191,8 +191,25 @@ struct Batch {
     StepLaunch params() const;
     void reset_lists() { lists_stale = true; }   // classify again: after the host changed a member's state
     int fresh_lists();               // the classification, if it is due (before a launch of the stepping kernels)
+    class Stepping *stepping = nullptr;   // while its owner steps it
     bool resident() const;           // the next chunk is one resident launch
-    int run_resident(int len, const Tiling &rows);   // (a refused launch sets res_refused)
+    int run_resident(int len, const Tiling &rows, long long all_units);   // (a refused launch sets res_refused)
+};
+
+// A batch that is being stepped, for as long as the object lives: its units count
+// among those that the process's batches step on the device, so that a resident
+// chunk takes its share of the SMs only (resident_ctas) and leaves room for the
+// others', and the tuner takes no sample of a device that is shared.
+class Stepping {
+public:
+    explicit Stepping(Batch &b);
+    ~Stepping();
+    Stepping(const Stepping &) = delete;
+    long long set(long long units);   // of the coming chunk; those of every batch on the device
+
+private:
+    Batch &b_;
+    long long units_ = 0;
 };
 
 // Longest chunk that is no sample of the autotuner.  Between chunks the GPU waits

@@ -343,6 +343,7 @@ extern "C" int thy_server_progress(thy_server *S, int *active)
         long long horizon = S->b.resident() ? S->b.max_chunk() : S->b.chunk;
         for (int i = 0; i < cap; i++)
             if (S->slots[i] && sel[i]) horizon = std::min(horizon, Batch::steps_to_event(*S->slots[i]->s));
+        Stepping loop(S->b);
         if ((rc = S->b.run_chunk(true, S->b.chunk_for(horizon)))) return rc;
         S->stats.chunks++;
         // hand on the gauge samples the chunk took; retire what finished in
