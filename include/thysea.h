@@ -245,8 +245,8 @@ void thy_session_close(thy_session *s);
    block of its resident chunks stays away from the barriers between the steps'
    phases, and the other blocks' waits (0.2 s) run out the same way; 0 turns it
    off (after 2 the session can step on: the chunk has advanced nothing).  With 4
-   the launch of its next resident chunk counts as refused by the driver, and the
-   session is stepped by separate launches from then on.
+   its resident chunks are left unstepped, as when too few of their blocks find a
+   free SM, and separate launches step the session.
    Nothing faults, traps or hangs. */
 int thy_session_inject(thy_session *s, int what);
 

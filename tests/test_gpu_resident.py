@@ -3,6 +3,10 @@ against the launched kernels: the same code of every cell, so bitwise the same
 fields, samples, step counts and unit counts, at sizes around the edges of
 strips (28 columns), tiles (112), units (16 rows) and of the task splits, up to
 the largest resident work."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -197,9 +201,9 @@ def test_barrier_timeout_is_reported_and_the_chunk_can_be_stepped_again(gpu):
     ref.close()
 
 
-def test_refused_resident_launch_takes_the_launched_kernels(gpu):
-    """a resident launch that the driver refuses (a partition of the GPU): the
-    chunk is stepped by separate launches, with the same results"""
+def test_unstepped_resident_chunk_takes_the_launched_kernels(gpu):
+    """a resident chunk that its blocks leave unstepped (too few of them found a
+    free SM): separate launches step it, with the same results"""
     prep = thysea.Prepared(_problem(500, 411, "open", 3600.0))
     ref, s = thysea.Session(prep), thysea.Session(prep)
     ref.steps(16)
@@ -217,6 +221,49 @@ def test_refused_resident_launch_takes_the_launched_kernels(gpu):
         assert np.array_equal(got[key], want[key], equal_nan=True), key
     s.close()
     ref.close()
+
+
+_BESIDE = """
+import sys, time
+import numpy as np
+import torch
+import thysea
+import test_gpu_resident as t
+
+prep = thysea.Prepared(t._problem(256, 240, "late", 900.0))
+ref, r0 = t._run(prep)
+streams, side = [torch.cuda.Stream() for _ in range(int(sys.argv[1]))], torch.cuda.Stream()
+x = torch.zeros(1024, device="cuda")
+x.add_(1.0)
+torch.cuda.synchronize()
+t0 = time.perf_counter()
+for st in streams:
+    with torch.cuda.stream(st):
+        torch.cuda._sleep(int(1.9e9))   # one block, a second
+got, r = t._run(prep)
+with torch.cuda.stream(side):
+    x.add_(1.0)
+side.synchronize()
+waited = time.perf_counter() - t0
+assert not any(st.query() for st in streams)   # they are still running
+torch.cuda.synchronize()
+assert waited < 0.5, waited
+assert r["iterations"] == r0["iterations"] and r["kernel_launches"] < r["iterations"]
+for k in t.FIELDS:
+    assert np.array_equal(got[k], ref[k], equal_nan=True), k
+"""
+
+
+@pytest.mark.parametrize("blocks", [1, 3])
+def test_resident_chunks_beside_another_streams_long_kernels(gpu, blocks):
+    """SMs held by other streams' kernels for a second: a run does not wait for
+    their end (its chunks are stepped by the blocks that find a free SM), other
+    kernels are not held back by it, and the results are the same.  (In a process
+    with a hardware queue for each of its streams.)"""
+    env = dict(os.environ, CUDA_DEVICE_MAX_CONNECTIONS="32",
+               PYTHONPATH=os.pathsep.join([os.path.dirname(os.path.abspath(__file__)), *sys.path]))
+    r = subprocess.run([sys.executable, "-c", _BESIDE, str(blocks)], env=env, capture_output=True, text=True, timeout=200)
+    assert r.returncode == 0, r.stderr[-3000:]
 
 
 def test_runs_of_several_threads_share_the_gpu(gpu):

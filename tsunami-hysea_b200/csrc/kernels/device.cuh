@@ -66,7 +66,7 @@ struct ScenarioCtl {
     unsigned int errors;       // bit 0 non-finite values, bit 1 a bounded wait ran out, bit 2 misaligned staging
     int inject;                // test hook: bit 0 = the deep kernels issue none of this scenario's copies,
                                // bit 1 = a CTA of its resident chunks stays away from the barriers,
-                               // bit 2 = the host takes its resident launches for refused
+                               // bit 2 = its resident chunks are not stepped
     const double *fault_times; // nfaults fault times (s), sorted, device memory
     unsigned long long units_deep;   // work units stepped by the deep-water kernels (phase 2)
     unsigned long long units_dry;    // work units skipped as dry land (classifications)

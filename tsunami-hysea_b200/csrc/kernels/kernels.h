@@ -110,7 +110,7 @@ void launch_initial_dt(const StepLaunch &L, cudaStream_t st);
 // lists for the current states of the work list's scenarios (from the host,
 // before a chunk: after the work list or a state changed)
 void launch_lists_current(const StepLaunch &L, cudaStream_t st);
-// resident.cu: a chunk of steps in one cooperative launch, one CTA per SM, for
+// resident.cu: a chunk of steps in one launch, at most one CTA per SM, for
 // work whose steps are bound by the latency of their launches
 constexpr int kResidentSlots = 64;      // scenarios of such a chunk at most
 // Barrier words, zero before the first launch and after one that gave up a wait
@@ -120,6 +120,8 @@ struct ResidentSync {
     struct alignas(128) Word {
         unsigned arrived, pad[31];
     };
+    Word team[3];                       // by launch modulo 3: CTAs that have started
+    unsigned team_size[3];              // of a team closed before all had
     Word start, phase1[3], phase2[3];   // by step modulo 3, counted on from launch to launch
     unsigned int dt_bits[3][kResidentSlots];
     int next;                           // the next launch's first step, modulo 3
@@ -133,7 +135,8 @@ struct ResidentLaunch {
     int nslots, nunits, cap, steps;
     int rows_general, rows_deep;   // rows of a task: 1, 2, 4 or 8
     unsigned long long wait_ns;    // limit of a barrier's wait
-    bool drop;                     // test hook: a CTA stays away from the steps' barriers
+    int launch;                    // counted from launch to launch, modulo 3
+    bool drop, decline;            // test hooks: a CTA stays away from the steps' barriers; the chunk is not stepped
 };
 constexpr int kResidentWarps = 16;       // warps of a CTA
 constexpr int resident_warps(int sms) { return sms * kResidentWarps; }           // of a launch
@@ -182,8 +185,8 @@ inline void resident_rows(int units, int warps, const Tiling &t, int *general, i
         *deep = std::min(8, 2 * *deep);
     }
 }
-cudaError_t configure_resident_kernel(int device, bool *usable);   // usable: the device takes such launches
-cudaError_t launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st);
+cudaError_t configure_resident_kernel(int device, bool *usable);   // usable: the device has room for its CTAs
+void launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st);
 // init_extract.cu: the step controller of every slot (launch 5 of a step)
 void launch_controller(const StepLaunch &L, cudaStream_t st);
 // init_extract.cu: per-unit depth steps (ScenarioDev::unit_gmax), after the

@@ -1,5 +1,4 @@
-// A chunk of time steps in one cooperative launch, for work that does not
-// fill the GPU.
+// A chunk of time steps in one launch, for work that does not fill the GPU.
 //
 // What bounds such work is latency, not throughput: as separate launches
 // (step.cu) a step is a chain of kernels, each of which reads
@@ -76,43 +75,22 @@ __device__ __forceinline__ int2 deep_rows(const Task &t)
     return make_int2(y, y < kHalfRows ? half : 0);
 }
 
-struct Shared {
-    ScenarioDev *tab;      // nslots
-    ScenarioCtl *ctl;      // nslots: every CTA advances its own copy
-    StepState *state;      // nslots
-    unsigned *dt_bits;     // nslots: the block's smallest dt bound of the step
-    Task *tasks;           // kResThreads: this CTA's tasks, one thread evaluates the class of each
-    unsigned char *cls;    // kResThreads
-    DeepRow *rows;         // kResWarps x kTaskRows
+// A scenario in shared memory.  (One array of them behind the CTA's tables, so that
+// every address is a constant, a slot and a field: pointers to an array each took
+// registers that the row loops need.)
+struct alignas(16) Slot {
+    ScenarioDev dev;
+    ScenarioCtl ctl;     // every CTA advances its own copy
+    StepState state;
+    unsigned dt_bits;    // the block's smallest dt bound of the step
 };
-
-constexpr size_t kTasksBytes = sizeof(Task) * kResThreads;
-constexpr size_t kClsBytes = kResThreads;
-constexpr size_t kRowsBytes = sizeof(DeepRow) * kResWarps * kTaskRows;
-__host__ __device__ constexpr size_t up16(size_t b) { return (b + 15) / 16 * 16; }
-__host__ __device__ inline size_t shared_bytes(int nslots)
-{
-    return kRowsBytes + kTasksBytes + up16(kClsBytes) + nslots * (up16(sizeof(ScenarioDev)) + up16(sizeof(ScenarioCtl)) +
-                                                                   sizeof(StepState)) + up16(nslots * sizeof(unsigned));
-}
-__device__ __forceinline__ Shared shared_layout(unsigned char *m, int nslots)
-{
-    Shared h;
-    h.rows = reinterpret_cast<DeepRow *>(m);
-    m += kRowsBytes;
-    h.tasks = reinterpret_cast<Task *>(m);
-    m += kTasksBytes;
-    h.cls = m;
-    m += up16(kClsBytes);
-    h.state = reinterpret_cast<StepState *>(m);
-    m += nslots * sizeof(StepState);
-    h.dt_bits = reinterpret_cast<unsigned *>(m);
-    m += up16(nslots * sizeof(unsigned));
-    h.tab = reinterpret_cast<ScenarioDev *>(m);
-    m += up16(nslots * sizeof(ScenarioDev));
-    h.ctl = reinterpret_cast<ScenarioCtl *>(m);
-    return h;
-}
+struct Shared {
+    DeepRow rows[kResWarps * kTaskRows];
+    Task tasks[kResThreads];           // this CTA's tasks, one thread evaluates the class of each
+    unsigned char cls[kResThreads];
+    Slot slots[1];                     // nslots
+};
+__host__ __device__ inline size_t shared_bytes(int nslots) { return sizeof(Shared) + (nslots - 1) * sizeof(Slot); }
 
 // ---------------------------------------------------------------------------
 // Grid barriers: one thread per CTA adds to a counter and polls it.  Arrivals
@@ -130,6 +108,10 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void st_release(unsigned *p, unsigned v)
+{
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
 // arrives at w and waits for n arrivals; false after wait_ns of global time (or
 // 2^28 polls), so that no wait is endless
 __device__ __forceinline__ bool arrive_and_wait(ResidentSync::Word &w, unsigned n, unsigned long long wait_ns)
@@ -145,6 +127,51 @@ __device__ __forceinline__ bool arrive_and_wait(ResidentSync::Word &w, unsigned 
         }
     }
     return false;
+}
+
+// ---------------------------------------------------------------------------
+// The team: the CTAs that step the chunk.  Each CTA counts itself in as it starts;
+// the team is all of the launch once they have, or those that have started kTeamNs
+// after the first one, which then closes it.  A CTA that comes later (its SM was
+// held by another stream's kernel) leaves, so a barrier waits for running CTAs only.
+// (A cooperative launch guarantees as much by starting only when every SM is free:
+// beside one block of a long kernel it waited for that kernel's end, and while it
+// was pending no other kernel of the process started.)
+// ---------------------------------------------------------------------------
+constexpr unsigned long long kTeamNs = 50000;   // all CTAs of a launch on a free GPU start within some us
+constexpr unsigned kTeamClosed = 0x80000000u;
+// this CTA's {rank, CTAs of the team}; {-, 0}: too late; {-, -1}: no answer within
+// wait_ns.  The ranks of a whole team are the block indices, which the device spreads
+// over its SMs (by arrival 1 % slower at 96 x 80 and 733 x 517).
+__device__ __forceinline__ int2 join_team(ResidentSync *sync, int launch, unsigned grid, unsigned long long wait_ns)
+{
+    ResidentSync::Word &w = sync->team[launch];
+    unsigned *size = &sync->team_size[launch];
+    const unsigned rank = atomicAdd(&w.arrived, 1u);   // by arrival
+    if (rank & kTeamClosed) return make_int2(0, 0);
+    if (rank == 0) {
+        // the next launch's words; the last one's are read by no one any more
+        const int next = launch == 2 ? 0 : launch + 1;
+        sync->team[next].arrived = 0u;
+        sync->team_size[next] = 0u;
+    }
+    const unsigned long long t0 = global_ns();
+    for (int i = 0; i < (1 << 28); i++) {
+        const unsigned v = ld_acquire(&w.arrived);
+        if (v == grid) return make_int2(blockIdx.x, grid);
+        if (v & kTeamClosed) {
+            const unsigned n = ld_acquire(size);
+            if (n) return make_int2(n == grid ? blockIdx.x : rank, n);
+        }
+        const unsigned long long waited = global_ns() - t0;
+        if (rank == 0 && waited > kTeamNs) {
+            const unsigned n = atomicOr(&w.arrived, kTeamClosed);
+            st_release(size, n);   // (all of them after all: some may have seen it)
+            return make_int2(n == grid ? blockIdx.x : rank, n);
+        }
+        if (waited > wait_ns) break;
+    }
+    return make_int2(rank, -1);
 }
 
 // ---------------------------------------------------------------------------
@@ -372,12 +399,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     extern __shared__ __align__(16) unsigned char dsm[];
     __shared__ bool s_ok;            // no wait has run out
     __shared__ int s_next[2];        // the CTA's next task of phase 1 and 2
-    __shared__ int s_sample[kResidentSlots];   // CTA 0: the step's gauge samples (ring slots)
+    __shared__ int s_sample[kResidentSlots];   // rank 0: the step's gauge samples (ring slots)
     __shared__ bool s_sampled, s_any;          // some; some scenario still runs
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int nblk = gridDim.x, NW = nblk * kResWarps;
-    const bool absent = L.drop && blockIdx.x == nblk - 1;   // test hook: this CTA takes part in no barrier of the steps
-    const Shared h = shared_layout(dsm, L.nslots);
+    __shared__ int s_rank, s_team;   // this CTA's place in the team, its CTAs
+    Shared &h = *reinterpret_cast<Shared *>(dsm);
+    Slot *slots = h.slots;
     ResidentSync *sync = L.sync;
     Task *tasks = h.tasks;
     unsigned char *cls = h.cls;
@@ -385,33 +412,42 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 
     // ---- the scenarios' descriptors and states ----
     {
-        const int words = L.nslots * (int)(sizeof(ScenarioDev) / 4);
+        constexpr int words = sizeof(ScenarioDev) / 4;
         const unsigned *src = reinterpret_cast<const unsigned *>(L.tab);
-        unsigned *dst = reinterpret_cast<unsigned *>(h.tab);
-        for (int k = tid; k < words; k += kResThreads) dst[k] = __ldg(src + k);
+        for (int k = tid; k < L.nslots * words; k += kResThreads)
+            reinterpret_cast<unsigned *>(&slots[k / words].dev)[k % words] = __ldg(src + k);
     }
     if (tid == 0) {
+        const int2 t = join_team(sync, L.launch, gridDim.x, L.wait_ns);
+        s_rank = t.x;
+        s_team = t.y;
         s_ok = true;
     }
     __syncthreads();
+    if (s_team <= 0) {
+        // (no answer: the others' waits for this CTA run out, too)
+        if (s_team < 0 && tid < L.nslots) atomicOr(&slots[tid].dev.ctl->errors, 2u);
+        return;
+    }
+    const bool absent = L.drop && s_rank == s_team - 1;   // test hook: this CTA takes part in no barrier of the steps
     for (int k = tid; k < L.nslots; k += kResThreads) {
-        h.ctl[k] = *h.tab[k].ctl;
-        h.state[k] = step_state(h.ctl[k]);
-        h.dt_bits[k] = 0x7f7fffffu;
+        slots[k].ctl = *slots[k].dev.ctl;
+        slots[k].state = step_state(slots[k].ctl);
+        slots[k].dt_bits = 0x7f7fffffu;
         s_sample[k] = -1;
-        if (blockIdx.x == 0) sync->dt_bits[0][k] = sync->dt_bits[1][k] = sync->dt_bits[2][k] = 0x7f7fffffu;
+        if (s_rank == 0) sync->dt_bits[0][k] = sync->dt_bits[1][k] = sync->dt_bits[2][k] = 0x7f7fffffu;
     }
     __syncthreads();
 
     // ---- the units by class (as the classification before a chunk) ----
-    for (int base = (blockIdx.x * kResWarps + warp) * 32; base < L.nunits; base += NW * 32) {
+    for (int base = (s_rank * kResWarps + warp) * 32; base < L.nunits; base += s_team * kResThreads) {
         const int u = base + lane;
         int c = -1;
         if (u < L.nunits) {
             const int2 item = L.units[u];
-            const ScenarioDev &s = h.tab[item.x];
+            const ScenarioDev &s = slots[item.x].dev;
             const int uy = item.y / s.tiles_x, tx = item.y - uy * s.tiles_x;
-            const int par = h.state[item.x].parity;
+            const int par = slots[item.x].state.parity;
             int age = s.dry_age[item.y];
             c = unit_class(s, s.usum[par], tx, uy, 0.f, false, age);
             // phase 1 folds its summary into the other parity's entry
@@ -430,7 +466,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     }
     int at = __ldcg(&sync->next);   // this launch's first barrier words
     __syncthreads();
-    if (tid == 0 && !arrive_and_wait(sync->start, nblk, L.wait_ns)) s_ok = false;
+    if (tid == 0 && !arrive_and_wait(sync->start, s_team, L.wait_ns)) s_ok = false;
     __syncthreads();
 
     // ---- this CTA's tasks, dealt in rounds: the shallow general units' first,
@@ -448,9 +484,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             per[k] = k == 2 ? 2 * (kHalfRows / L.rows_deep) : STRIPS * (kHalfRows / L.rows_general);
             total += n[k] * per[k];
         }
-        // round k gives this CTA task k nblk + (blockIdx.x + kDealStep k) mod nblk
-        const auto dealt = [&](int k) { return k * nblk + (int)((blockIdx.x + (unsigned)kDealStep * k) % nblk); };
-        ntask = total / nblk;
+        // a team too small for the tasks, or for their time, leaves the chunk to
+        // the launched kernels: the host finds that nothing was stepped
+        if (s_ok && (L.decline || total > s_team * kResThreads || 4 * s_team < (int)gridDim.x)) return;
+        // round k gives this CTA task k n + (rank + kDealStep k) mod n, n CTAs in the team
+        const auto dealt = [&](int k) { return k * s_team + (int)((s_rank + (unsigned)kDealStep * k) % s_team); };
+        ntask = total / s_team;
         ntask = min(kResThreads, ntask + (dealt(ntask) < total ? 1 : 0));
         if (s_ok && tid < ntask) {
             int i = dealt(tid), k = 0;
@@ -460,7 +499,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             }
             const int u = i % n[k], sub = i / n[k];
             const int2 item = L.units[L.order[k * L.cap + u]];
-            const ScenarioDev &s = h.tab[item.x];
+            const ScenarioDev &s = slots[item.x].dev;
             Task t;
             t.slot = (short)item.x;
             t.uy = (short)(item.y / s.tiles_x);
@@ -470,7 +509,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             tasks[tid] = t;
             age = s.dry_age[item.y];
             gmax = s.unit_gmax[item.y];
-            cls[tid] = (unsigned char)unit_class(s, s.usum[h.state[item.x].parity], t.tx, t.uy, gmax, false, age);
+            cls[tid] = (unsigned char)unit_class(s, s.usum[slots[item.x].state.parity], t.tx, t.uy, gmax, false, age);
         }
         if (tid < 2) s_next[tid] = kResWarps;
     }
@@ -480,10 +519,10 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
         // ---- phase 1 ----
         for (int j = warp; j < ntask; j = claim(&s_next[0])) {
             const Task t = tasks[j];
-            const StepState q = h.state[t.slot];
+            const StepState q = slots[t.slot].state;
             const int c = cls[j];
             if (q.status != kRunning || (c & 3) == kClsDry) continue;
-            const ScenarioDev &s = h.tab[t.slot];
+            const ScenarioDev &s = slots[t.slot].dev;
             UnitSum *dst = &s.usum[q.parity ^ 1][t.uy * s.tiles_x + t.tx];
             bool bad = false;
             if (c & kClsDeep) {
@@ -516,12 +555,12 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                     fold_unit_summary(hacc, cell, cell && gx < ux0 + 2, cell && gx >= ux1 - 2, dst);
                 }
             }
-            if (bad) fail(s, &h.dt_bits[t.slot]);
+            if (bad) fail(s, &slots[t.slot].dt_bits);
         }
         __syncthreads();
         if (tid == 0) {
             s_next[0] = kResWarps;
-            if (!arrive_and_wait(sync->phase1[at], nblk, L.wait_ns)) s_ok = false;
+            if (!arrive_and_wait(sync->phase1[at], s_team, L.wait_ns)) s_ok = false;
         }
         __syncthreads();
         if (!s_ok) break;
@@ -530,9 +569,9 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
         // step and phase 1 of the next), one thread per task ----
         if (tid < ntask) {
             const Task t = tasks[tid];
-            const StepState q = h.state[t.slot];
+            const StepState q = slots[t.slot].state;
             if (q.status == kRunning) {
-                const ScenarioDev &s = h.tab[t.slot];
+                const ScenarioDev &s = slots[t.slot].dev;
                 const int c = unit_class(s, s.usum[q.parity ^ 1], t.tx, t.uy, gmax, true, age);
                 cls[tid] = (unsigned char)c;
                 if (t.sub == 0) {
@@ -549,10 +588,10 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
         // ---- phase 2 ----
         for (int j = warp; j < ntask; j = claim(&s_next[1])) {
             const Task t = tasks[j];
-            const StepState q = h.state[t.slot];
+            const StepState q = slots[t.slot].state;
             const int c = cls[j];
             if (q.status != kRunning || (c & 3) == kClsDry) continue;
-            const ScenarioDev &s = h.tab[t.slot];
+            const ScenarioDev &s = slots[t.slot].dev;
             bool bad = false;
             float bound;
             if (c & kClsDeep) {
@@ -581,35 +620,35 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                     bound = fminf(bound, warp_min_bound(local_min));
                 }
             }
-            if (lane == 0) atomicMin(&h.dt_bits[t.slot], __float_as_uint(bound));
-            if (bad) fail(s, &h.dt_bits[t.slot]);
+            if (lane == 0) atomicMin(&slots[t.slot].dt_bits, __float_as_uint(bound));
+            if (bad) fail(s, &slots[t.slot].dt_bits);
         }
         __syncthreads();
         // the block's bounds into the step's words
         unsigned *gmin = sync->dt_bits[at];
         for (int k = tid; k < L.nslots; k += kResThreads)
-            if (h.dt_bits[k] != 0x7f7fffffu) {
-                atomicMin(gmin + k, h.dt_bits[k]);
-                h.dt_bits[k] = 0x7f7fffffu;
+            if (slots[k].dt_bits != 0x7f7fffffu) {
+                atomicMin(gmin + k, slots[k].dt_bits);
+                slots[k].dt_bits = 0x7f7fffffu;
             }
         if (L.nslots > 1) __syncthreads();   // (one scenario: the arriving thread's own)
 
         // ---- the step's control, by every CTA for itself: warp 0, a lane per
-        // scenario (the gauge samples by CTA 0) ----
+        // scenario (the gauge samples by rank 0) ----
         if (warp == 0) {
-            bool go = lane != 0 || arrive_and_wait(sync->phase2[at], nblk, L.wait_ns);
+            bool go = lane != 0 || arrive_and_wait(sync->phase2[at], s_team, L.wait_ns);
             go = __all_sync(0xffffffffu, go);
             __syncwarp();   // (the bounds are read after lane 0's wait)
             const int clear = at == 0 ? 2 : at - 1;   // the words every CTA is done with
             bool any = false, sampled = false;
             for (int k = lane; go && k < L.nslots; k += 32) {
-                ScenarioCtl &c = h.ctl[k];
+                ScenarioCtl &c = slots[k].ctl;
                 if (c.status != kRunning) continue;
-                const ScenarioDev &s = h.tab[k];
+                const ScenarioDev &s = slots[k].dev;
                 const int sample = advance_scenario(c, s, __uint_as_float(__ldcg(gmin + k)), 0u);
-                h.state[k] = step_state(c);
+                slots[k].state = step_state(c);
                 any |= c.status == kRunning;
-                if (blockIdx.x == 0) {
+                if (s_rank == 0) {
                     sync->dt_bits[clear][k] = 0x7f7fffffu;
                     s_sample[k] = sample;
                     if (sample >= 0) s.gauge_ring_t[sample] = c.t * c.T;
@@ -623,7 +662,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
                 s_ok = go;
                 s_any = any;
                 s_sampled = sampled;
-                if (blockIdx.x == 0 && go) {
+                if (s_rank == 0 && go) {
                     sync->phase1[clear].arrived = sync->phase2[clear].arrived = sync->start.arrived = 0u;
                     sync->counts[0] = sync->counts[1] = sync->counts[2] = sync->counts[3] = 0;
                     sync->next = at == 2 ? 0 : at + 1;
@@ -637,10 +676,10 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
             for (int k = 0; k < L.nslots; k++) {
                 const int sample = s_sample[k];
                 if (sample < 0) continue;
-                const ScenarioDev &s = h.tab[k];
+                const ScenarioDev &s = slots[k].dev;
                 float *dst = s.gauge_ring + (size_t)sample * 4 * s.ngauges;
                 for (int g = tid; g < s.ngauges; g += kResThreads)
-                    gauge_values(s, h.state[k].parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
+                    gauge_values(s, slots[k].state.parity, s.gauge_cells[g], dst + 4 * g, s.gauge_minmax + g);
             }
             __syncthreads();
             if (tid < kResidentSlots) s_sample[tid] = -1;
@@ -654,7 +693,7 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     if (whole && tid < ntask) {
         const Task t = tasks[tid];
         if (t.sub == 0) {
-            const ScenarioDev &s = h.tab[t.slot];
+            const ScenarioDev &s = slots[t.slot].dev;
             s.dry_age[t.uy * s.tiles_x + t.tx] = (unsigned char)age;
             if (counted_deep) atomicAdd(&s.ctl->units_deep, (unsigned long long)counted_deep);
             if (counted_dry) atomicAdd(&s.ctl->units_dry, (unsigned long long)counted_dry);
@@ -664,11 +703,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
     // whichever it is, it reports every scenario that it has not seen end, and the
     // host fails those and clears the barrier words.
     for (int k = tid; k < L.nslots; k += kResThreads) {
-        ScenarioCtl *c = h.tab[k].ctl;
-        const int status = h.state[k].status;
+        ScenarioCtl *c = slots[k].dev.ctl;
+        const int status = slots[k].state.status;
         const bool ended = status == kDone || status == kFailed;
         if (!whole && !ended) atomicOr(&c->errors, 2u);
-        if (blockIdx.x == 0 && (whole || ended)) store_advanced(c, h.ctl[k]);
+        if (s_rank == 0 && (whole || ended)) store_advanced(c, slots[k].ctl);
     }
 }
 
@@ -677,13 +716,11 @@ __global__ void __launch_bounds__(kResThreads, 1) resident_kernel(const Resident
 cudaError_t configure_resident_kernel(int device, bool *usable)
 {
     *usable = false;
-    int coop = 0, smem = 0, ctas = 0;
+    int smem = 0, ctas = 0;
     cudaError_t e;
-    if ((e = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device)) ||
-        (e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device)))
-        return e;
+    if ((e = cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, device))) return e;
     const size_t need = shared_bytes(kResidentSlots);
-    if (!coop || need > (size_t)smem) return cudaSuccess;
+    if (need > (size_t)smem) return cudaSuccess;
     if ((e = cudaFuncSetAttribute(resident_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need)) ||
         (e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctas, resident_kernel, kResThreads, need)))
         return e;
@@ -691,11 +728,9 @@ cudaError_t configure_resident_kernel(int device, bool *usable)
     return cudaSuccess;
 }
 
-cudaError_t launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st)
+void launch_resident(const ResidentLaunch &L, int ctas, cudaStream_t st)
 {
-    void *args[] = {const_cast<ResidentLaunch *>(&L)};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void *>(resident_kernel), dim3(ctas), dim3(kResThreads), args,
-                                       shared_bytes(L.nslots), st);
+    resident_kernel<<<ctas, kResThreads, shared_bytes(L.nslots), st>>>(L);
 }
 
 }  // namespace thy

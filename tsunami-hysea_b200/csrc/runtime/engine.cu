@@ -1210,7 +1210,7 @@ int Batch::fresh_lists()
 // nothing to withhold in a resident chunk.
 bool Batch::resident() const
 {
-    if (res_units == 0 || res_refused || !g_resident[device] || !tuner_free()) return false;
+    if (res_units == 0 || res_hold > 0 || !g_resident[device] || !tuner_free()) return false;
     for (auto *m : members)
         if (m && (m->hctl.inject & 1)) return false;
     return true;
@@ -1231,21 +1231,16 @@ int Batch::run_resident(int len, const Tiling &rows, long long all_units)
     const int ctas = resident_ctas(res_units, sms, std::max<long long>(all_units, res_units));
     resident_rows(res_units, resident_warps(ctas), rows, &R.rows_general, &R.rows_deep);
     R.drop = false;
-    bool refuse = false;   // (test hook)
+    R.decline = false;
     for (auto *m : members) {
         R.drop |= m && (m->hctl.inject & 2);
-        refuse |= m && (m->hctl.inject & 4);
+        R.decline |= m && (m->hctl.inject & 4);
     }
     R.wait_ns = R.drop ? kWaitNs / 20 : kWaitNs;
-    const cudaError_t e = refuse ? cudaErrorCooperativeLaunchTooLarge : launch_resident(R, ctas, st);
-    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
-        // fewer SMs than the device has are open to this process: nothing was
-        // launched, and this batch keeps to the launched kernels
-        cudaGetLastError();
-        res_refused = true;
-        return THY_OK;
-    }
-    THY_CK(e);
+    R.launch = res_launch;
+    res_launch = (res_launch + 1) % 3;
+    launch_resident(R, ctas, st);
+    THY_CK(cudaGetLastError());
     lists_stale = true;
     return THY_OK;
 }
@@ -1309,7 +1304,6 @@ int Batch::run_chunk(bool timed, int len)
     if (timed) THY_CK(cudaEventRecord(ev0, st));
     if (res) {
         if ((rc = run_resident(len, tuner_searches(key) ? tiling : Tiling(), all_units))) return rc;
-        if (res_refused) return run_chunk(timed, len);
     } else {
         for (int i = 0; i < len / chunk; i++) THY_CK(cudaGraphLaunch(gexec, st));
         for (int i = 0; i < len % chunk; i++) THY_CK(cudaGraphLaunch(one, st));
@@ -1322,6 +1316,20 @@ int Batch::run_chunk(bool timed, int len)
     if (timed) {
         THY_CK(cudaEventElapsedTime(&ms, ev0, ev1));
         device_ms += ms;
+    }
+    if (res) {
+        bool stepped = running == 0;
+        for (int i = 0; i < capacity; i++)
+            if (b0[i].step >= 0) stepped |= h_ctl[i].step != b0[i].step || h_ctl[i].status != kRunning || (h_ctl[i].errors & 2u);
+        if (!stepped) {
+            // too few of its CTAs found an SM: separate launches take this chunk
+            // and the next few
+            THY_CK(cudaMemsetAsync(d_rsync, 0, sizeof(ResidentSync), st));
+            res_hold = kResidentHold;
+            return run_chunk(timed, len);
+        }
+    } else if (res_hold > 0) {
+        res_hold--;
     }
     launches += res ? 1 : (long long)(kLaunchesPerStep - 1) * len;   // (the controller is part of phase 2)
     chunks_run++;

@@ -124,7 +124,8 @@ struct Batch {
     int *d_rorder = nullptr;
     ResidentSync *d_rsync = nullptr;
     int res_slots = 0, res_units = 0;  // of the current work list (0: too much work)
-    bool res_refused = false;          // the driver refused such a launch
+    int res_launch = 0;                // ResidentLaunch::launch
+    int res_hold = 0;                  // chunks to launch step by step, after a resident one that could not be stepped
     bool lists_stale = false;          // d_lists not made for the current states (made when a step is launched)
     ScenarioCtl *d_ctl = nullptr;      // slots
     ScenarioCtl *h_ctl = nullptr;      // pinned mirror
@@ -193,7 +194,7 @@ struct Batch {
     int fresh_lists();               // the classification, if it is due (before a launch of the stepping kernels)
     class Stepping *stepping = nullptr;   // while its owner steps it
     bool resident() const;           // the next chunk is one resident launch
-    int run_resident(int len, const Tiling &rows, long long all_units);   // (a refused launch sets res_refused)
+    int run_resident(int len, const Tiling &rows, long long all_units);
 };
 
 // A batch that is being stepped, for as long as the object lives: its units count
@@ -219,6 +220,7 @@ private:
 // admits and retires.  (Loop less device time of runs whose chunks after tuning have
 // 16 / 64 steps: 1024^2, 443 steps, 0.88 / 0.44 ms; 2048^2, 986 steps, 2.0 / 1.1 ms.)
 constexpr int kMaxChunk = 64;
+constexpr int kResidentHold = 4;   // Batch::res_hold after a chunk that was not stepped
 static_assert(kMaxChunk <= kGaugeRing, "at most one gauge sample a step");
 
 // Single-scenario batches of thy_run, kept per device between runs with

@@ -290,8 +290,8 @@ class Session:
         """Test hook (thy_session_inject): 1 = the deep-water kernels issue
         none of this session's staging copies, 2 = a block of its resident
         chunks stays away from the barriers, so that bounded waits run out and
-        the next steps fail with THY_ERR_TIMEOUT; 4 = its resident launches
-        count as refused, so that separate launches step it; 0 = off."""
+        the next steps fail with THY_ERR_TIMEOUT; 4 = its resident chunks
+        are left unstepped, so that separate launches step it; 0 = off."""
         _check(_ffi.lib().thy_session_inject(self._h, what), "thy_session_inject")
 
     def tuned(self):
