@@ -1030,14 +1030,24 @@ int Batch::update(const std::vector<char> *selected)
     }
     if ((int)work.size() > work_capacity) {
         // the captured graph holds the list pointers: grow, then recapture
+        // (without the memory for it the batch stays as it is)
+        int2 *w = nullptr, *w0 = nullptr;
+        int *l = nullptr;
+        cudaError_t e = cudaMallocAsync(&w, work.size() * sizeof(int2), st);
+        if (e == cudaSuccess) e = cudaMallocAsync(&w0, work.size() * sizeof(int2), st);
+        if (e == cudaSuccess) e = cudaMallocAsync(&l, (2 + 4 * work.size()) * sizeof(int), st);
+        if (e != cudaSuccess) {
+            if (w) cudaFreeAsync(w, st);
+            if (w0) cudaFreeAsync(w0, st);
+        }
+        THY_CK(e);
         cudaFreeAsync(d_work, st);
         cudaFreeAsync(d_work0, st);
         cudaFreeAsync(d_lists, st);
-        d_lists = nullptr;
+        d_work = w;
+        d_work0 = w0;
+        d_lists = l;
         work_capacity = (int)work.size();
-        THY_CK(cudaMallocAsync(&d_work, work_capacity * sizeof(int2), st));
-        THY_CK(cudaMallocAsync(&d_work0, work_capacity * sizeof(int2), st));
-        THY_CK(cudaMallocAsync(&d_lists, (2 + 4 * (size_t)work_capacity) * sizeof(int), st));
         drop_graphs();
     }
     nwork = (int)work.size();

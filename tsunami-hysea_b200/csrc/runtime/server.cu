@@ -140,18 +140,24 @@ static int admit(thy_server *S)
         }
         joining.push_back(slot);
     }
-    if (joining.empty()) return THY_OK;
-    std::vector<DevScenario *> who;
-    for (int slot : joining) who.push_back(S->slots[slot]->s.get());
-    int rc = S->b.update();
-    if (rc == THY_OK) rc = S->b.initial_dt_of(who);
-    if (rc != THY_OK) {
+    while (!joining.empty()) {
+        std::vector<DevScenario *> who;
+        for (int slot : joining) who.push_back(S->slots[slot]->s.get());
+        int rc = S->b.update();
+        if (rc == THY_OK) rc = S->b.initial_dt_of(who);
+        if (rc == THY_OK) {
+            S->members_changed = true;
+            break;
+        }
+        // the largest of them fails, and the others try again
         cudaGetLastError();
-        cudaStreamSynchronize(S->st);   // nothing reads the requests' problems any more
-        for (int slot : joining) complete(S, slot, rc);
-        return THY_OK;
+        cudaStreamSynchronize(S->st);   // nothing reads the request's problem any more
+        const auto largest = std::max_element(joining.begin(), joining.end(), [S](int a, int b) {
+            return S->slots[a]->r.bytes < S->slots[b]->r.bytes;
+        });
+        complete(S, *largest, rc);
+        joining.erase(largest);
     }
-    S->members_changed = true;
     return THY_OK;
 }
 
