@@ -172,13 +172,16 @@ def run(problem, max_steps: int = -1, snapshots: bool = True, series: bool = Tru
     snaps = {"time": [], "eta": [], "ux": [], "uy": []}
     ser = {"time": [], "eta": [], "ux": [], "uy": []}
     # the snapshots' stacks, filled as they arrive (pages of snapshots that do
-    # not come are never touched); of more than a GiB each, arrays stacked at the
-    # end
+    # not come are never touched); of more than a GiB each, or than there is address
+    # space for, arrays stacked at the end
     stack = {}
     if snapshots and pc.save_nc > 0.0:
         slots = pc.t_end / pc.save_nc + 2.0
-        if slots * ny * nx * 4 <= 1 << 30:
-            stack = {k: np.empty((int(slots), ny, nx), np.float32) for k in ("eta", "ux", "uy")}
+        if slots >= 1.0 and slots * ny * nx * 4 <= 1 << 30:
+            try:
+                stack = {k: np.empty((int(slots), ny, nx), np.float32) for k in ("eta", "ux", "uy")}
+            except MemoryError:
+                stack = {}
 
     def on_snap(user, idx, t, e, u, v):
         n = nx * ny
