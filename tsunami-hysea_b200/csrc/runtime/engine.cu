@@ -1618,6 +1618,7 @@ extern "C" int thy_run(const thy_problem *p, const thy_outputs *o, thy_stats *st
         }
     out:
         t_release = std::chrono::steady_clock::now();
+        if (rc) cudaStreamSynchronize(st);   // the set-up's copies may still read its host tables
         b.detach(&s);
     }
     {
@@ -1660,6 +1661,7 @@ extern "C" int thy_session_open(const thy_problem *p, thy_session **out)
         (rc = S->s.setup(&q, S->st)) || (rc = S->b.rebuild()) || (rc = initial_dt(S->b)) ||
         (rc = S->s.apply_due_faults(S->st))) {
         cudaStream_t st = S->st;
+        cudaStreamSynchronize(st);   // the set-up's copies may still read its host tables and the problem
         delete S;
         cudaStreamDestroy(st);
         return rc;
