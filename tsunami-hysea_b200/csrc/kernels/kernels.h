@@ -212,6 +212,20 @@ void launch_okada(const ScenarioDev *s_host, double *def, double lon0, double dl
 void launch_absmax(const double *def, long long n, unsigned int *max_bits, cudaStream_t st);
 void launch_apply_deformation(const ScenarioDev *s_host, const double *def, int crop_flag, double crop_value,
                               const unsigned int *max_bits, cudaStream_t st);
+// Split of a row over blocks of kOkadaThreads: `segs` blocks a row of `per` cells a
+// thread - up to 4, which share the row's sines, as long as every SM has its 5
+// blocks.  Unsigned: the first column behind a row may lie beyond the largest int.
+constexpr unsigned kOkadaThreads = 128;
+struct OkadaSplit {
+    unsigned per, segs;
+};
+inline OkadaSplit okada_split(int nx, int ny, int sms)
+{
+    const long long n = (long long)nx * ny;
+    const unsigned per = (unsigned)std::min(4ll, std::max(1ll, n / ((long long)sms * 5 * kOkadaThreads)));
+    return OkadaSplit{per, ((unsigned)nx + per * kOkadaThreads - 1) / (per * kOkadaThreads)};
+}
+__host__ __device__ inline unsigned okada_first_cell(const OkadaSplit &s, unsigned seg) { return seg * s.per * kOkadaThreads; }
 // the whole stage on the reference's device state; crop_flag 1 uses max_bits (one
 // word) and, if given, def (nx*ny doubles), otherwise both may be null
 void launch_okada_reference(int nx, int ny, int sms, double lon0, double dlon, double lat0, double dlat, const OkadaFault &f,

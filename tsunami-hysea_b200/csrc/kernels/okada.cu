@@ -365,24 +365,22 @@ struct OkadaCrop {
     static __device__ __forceinline__ double apply(double U, double limit) { return fabs(U) < limit ? 0.0 : U; }
 };
 
-constexpr int kOkadaThreads = 128;
-
-// A block takes `per` x kOkadaThreads cells of a row.  max_bits given: only the
+// A block takes `per` x kOkadaThreads cells of a row (OkadaSplit).  max_bits given: only the
 // largest (float)|U_Z| (non-negative floats order as unsigned) and, with def
 // given, U_Z itself; else U_Z is applied.  One kernel for all of them: a cell's
 // U_Z is the same bits in each.
-__global__ void __launch_bounds__(kOkadaThreads, 5) okada_reference_kernel(int nx, int segs, int per, OkadaConst c, ReferenceState out,
+__global__ void __launch_bounds__(kOkadaThreads, 5) okada_reference_kernel(unsigned nx, OkadaSplit split, OkadaConst c, ReferenceState out,
                                                                            OkadaCrop crop, unsigned int *max_bits,
                                                                            double *__restrict__ def)
 {
-    const int y = blockIdx.x / segs, x0 = (blockIdx.x - y * segs) * per * kOkadaThreads + threadIdx.x;
-    const OkadaRow row = okada_row(c, y);
+    const unsigned y = blockIdx.x / split.segs, x0 = okada_first_cell(split, blockIdx.x - y * split.segs) + threadIdx.x;
+    const OkadaRow row = okada_row(c, (int)y);
     const double limit = max_bits ? 0.0 : crop.limit();
     float m = 0.f;
 #pragma unroll 1
-    for (int k = 0, x = x0; k < per && x < nx; k++, x += kOkadaThreads) {
+    for (unsigned k = 0, x = x0; k < split.per && x < nx; k++, x += kOkadaThreads) {
         double px, py;
-        gauss_krueger(c, row, x, px, py);
+        gauss_krueger(c, row, (int)x, px, py);
         const double U = okada_uz(c, px * c.ss + py * c.cs, -px * c.cs + py * c.ss) * c.inv_scale;
         const size_t i = (size_t)y * nx + x;
         if (max_bits) {
@@ -414,21 +412,18 @@ void launch_okada_reference(int nx, int ny, int sms, double lon0, double dlon, d
     const OkadaConst c = okada_const(lon0, dlon, lat0, dlat, f, Hs);
     const ReferenceState out{state, eta_initial};
     const OkadaCrop crop{crop_flag, crop_value, max_bits};
-    // up to 4 cells a thread, which share the row's sines, as long as every SM has
-    // its 5 blocks
     const long long n = (long long)nx * ny;
-    const int per = (int)std::min(4ll, std::max(1ll, n / ((long long)sms * 5 * kOkadaThreads)));
-    const int segs = (nx + per * kOkadaThreads - 1) / (per * kOkadaThreads);
-    const unsigned blocks = (unsigned)segs * (unsigned)ny;
+    const OkadaSplit split = okada_split(nx, ny, sms);
+    const unsigned blocks = split.segs * (unsigned)ny;
     if (crop_flag == 1) {
         cudaMemsetAsync(max_bits, 0, sizeof(unsigned int), st);
-        okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, segs, per, c, out, crop, max_bits, def);
+        okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, split, c, out, crop, max_bits, def);
         if (def) {
             apply_reference_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>((size_t)n, def, out, crop);
             return;
         }
     }
-    okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, segs, per, c, out, crop, nullptr, nullptr);
+    okada_reference_kernel<<<blocks, kOkadaThreads, 0, st>>>(nx, split, c, out, crop, nullptr, nullptr);
 }
 
 cudaError_t preload_okada_kernels()
