@@ -17,8 +17,8 @@
  * Plus the pieces around it that a caller of the reference gets from its
  * main(): the problem-file loader (thy_load_problem_file), the
  * nondimensionalisation (thy_prepare), and the NetCDF writers
- * (thy_write_netcdf), and the batched / serving entry points that run many
- * scenarios in one persistent launch (thy_batch_*, thy_server_*).
+ * (thy_write_netcdf), and the batched / serving entry points that step many
+ * scenarios together (thy_server_*).
  *
  * Return codes 1 and 2 keep the meaning shallowWater() gives them
  * (src/GPU/ShallowWater.cu:262-353).
@@ -267,7 +267,7 @@ void thy_tuner_clear(void);                         /* forget every decision of 
 
 /* Multi-scenario runtime (batched and serving use): scenarios submitted at
    any time are admitted in order under an HBM budget and stepped together -
-   one work list over all their tiles, one CUDA graph per chunk of steps -
+   one work list over all their units, a chunk of steps at a time -
    and retired as they finish, each with its own dt, time and events.  A
    scenario's results are identical alone (thy_run) and in any mix.  A
    scenario whose state turns non-finite is retired with THY_ERR_NONFINITE

@@ -44,8 +44,9 @@ struct RowMetrics {
     const float *dlat;       // sponge dy
 };
 
-// Mutable per-scenario control block; written by the host between graph
-// launches and by the controller launch that ends each step.
+// Mutable per-scenario control block; written by the host between chunks and by
+// the step controller that ends each step (phase 2's last CTA, or a launch of its
+// own; a resident chunk's CTAs each advance a copy, stored at the chunk's end).
 struct ScenarioCtl {
     double t;            // simulated time (dimensionless)
     double dt;           // time step of the next step
@@ -326,9 +327,9 @@ __device__ __forceinline__ void swapf(float &a, float &b) { float t = a; a = b; 
 // Edges whose four stencil cells are all deeper than hpos and which lie at
 // least two cells from a boundary: the 2s blend weight is exactly 1, so the
 // flux is the 2s flux alone (the WAF part, the wet/dry tests and the limiter
-// drop out).  The general units and deep phase 1 call the mass fluxes; deep
-// phase 2 evaluates the momentum formulas two edges at a time in packed FP32x2
-// arithmetic (step_parts.cuh), which can round its last bit differently.
+// drop out).  The general units call these fluxes; the deep units evaluate the
+// formulas two edges at a time in packed FP32x2 arithmetic (mass_pair, pair_update in
+// step_parts.cuh), the momentum fluxes with roundings of their own.
 // ---------------------------------------------------------------------------
 
 // x edge: F = q0 len, outflow-limited (src/GPU/Arista_kernel.cu:118-219, alfa = 1)
@@ -406,8 +407,8 @@ __device__ __forceinline__ float fma2m(float a, float b, float c, float d) { ret
 __device__ __forceinline__ float fma2q(float a, float b, float c, float d) { return fma_(c, d, mul(a, b)); }
 __device__ __forceinline__ float fma2n(float a, float b, float c, float d) { return fma_(-c, d, mul(a, b)); }
 
-// Desingularised 1/h (src/GPU/Arista_kernel.cu:164): sqrt2 h / sqrt(h^4 + max(h,eps)^4),
-// which is exactly 1/h for h >= eps.
+// inv_depth with every rounding explicit: the general units' (inv_depth is the
+// initial dt's, one code copy).
 __device__ __forceinline__ float inv_depth_x(float h, float eps)
 {
     if (h >= eps) return __frcp_rn(h);

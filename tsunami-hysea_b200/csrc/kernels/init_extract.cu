@@ -110,7 +110,7 @@ void launch_gauges(const ScenarioDev *s_host, int parity, const int *cells, int 
 }
 
 // ---------------------------------------------------------------------------
-// Step controller (the last launch of every step), one block per scenario
+// Step controller as a launch of its own (the last one of a step), one block per scenario
 // slot (src/GPU/ShallowWater.cu:397-450 loop body after the step;
 // src/GPU/Timestep.cu:35-68 dt truncation to fault times).  Thread 0 reads
 // the control block once (plain loads see the step's atomics), advances time

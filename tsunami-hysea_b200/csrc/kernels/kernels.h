@@ -61,11 +61,7 @@ struct Tiling {
 // twice that many row groups; general {2, 1, 8} row groups (one warp task per strip
 // and row group; 8 groups of 2 rows for short chains).  (4096^2, us a launch: deep
 // phase 1 95 / 98 / 107, deep phase 2 86 / 98 / 146, general 48 / 51 / 59.)
-__host__ __device__ constexpr int deep_ng(int phase, int v)
-{
-    (void)phase;
-    return v == 0 ? 1 : v == 1 ? 2 : 4;
-}
+__host__ __device__ constexpr int deep_ng(int v) { return v == 0 ? 1 : v == 1 ? 2 : 4; }
 // resident CTAs per SM the deep kernels are compiled for: phase 1 is held to two
 // by its staging buffers (one of the largest variant, by its registers), phase 2
 // to three, two or one

@@ -136,10 +136,9 @@ __device__ __forceinline__ void tmap_acquire(const TmaMap *map)
     asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
 }
 
-// Warps of a deep-kernel CTA: 4 column strips x NG row groups (the tiling's
-// variant: by default phase 1, two CTAs per SM as its double-buffered staging
-// is larger, uses 3 row groups so that 24 warps per SM hide the latency;
-// phase 2 uses 2 at three CTAs per SM).
+// Compute warps of a deep-kernel CTA: 2 strips of column pairs x 2 NG row groups (the
+// tiling's variant: by default NG = 1 in both phases, 4 warps and the producer; two
+// CTAs per SM in phase 1, whose double-buffered staging is larger, three in phase 2).
 constexpr int SPLANE = (kStageRows * kStageW + 31) / 32 * 32;   // floats per staged plane (128-byte multiple)
 constexpr int DPLANE = kHalfRows * kTileX;          // floats per staged diagnostics plane
 constexpr uint32_t kStateBytes = kStageRows * kStageW * 4;
@@ -816,7 +815,7 @@ static StepEnds step_ends(const StepLaunch &L)
 template <int PHASE, int V>
 static void launch_deep(const StepLaunch &L, cudaStream_t st)
 {
-    constexpr int NG = deep_ng(PHASE, V);
+    constexpr int NG = deep_ng(V);
     deep_kernel<PHASE, NG, deep_minb(PHASE, V)>
         <<<L.deep_grid[PHASE - 1], 128 * NG + 32, deep_smem_bytes(PHASE, NG), st>>>(L.scen, L.work, L.lists,
                                                                             L.claims + (PHASE - 1), step_ends<PHASE>(L));
@@ -875,7 +874,7 @@ void launch_lists_current(const StepLaunch &L, cudaStream_t st)
 template <int PHASE, int V>
 static cudaError_t configure_deep()
 {
-    constexpr int NG = deep_ng(PHASE, V);
+    constexpr int NG = deep_ng(V);
     auto *f = deep_kernel<PHASE, NG, deep_minb(PHASE, V)>;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)deep_smem_bytes(PHASE, NG));
     if (e) return e;
@@ -920,7 +919,7 @@ int step_blocks_per_sm(int v)
 template <int PHASE, int V>
 static int deep_occupancy()
 {
-    constexpr int NG = deep_ng(PHASE, V);
+    constexpr int NG = deep_ng(V);
     int n = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, deep_kernel<PHASE, NG, deep_minb(PHASE, V)>, 128 * NG + 32,
                                                   deep_smem_bytes(PHASE, NG));

@@ -5,7 +5,7 @@
 //
 // The time loop stays on the device: dt, the simulated time and the event
 // checks live in a per-scenario control block updated by the controller
-// launch that ends each step, so steps are launched in graph chunks with one host
+// that ends each step, so steps are launched in graph chunks with one host
 // synchronisation per chunk instead of one blocking copy per step.  When an
 // event is due (fault time, snapshot time, gauge time) the controller pauses
 // the scenario; later launches of the chunk do nothing for it, and the host
@@ -1683,8 +1683,7 @@ extern "C" int thy_session_steps(thy_session *S, long long steps, double *device
         s.hctl.status = kRunning;
         s.hctl.events = 0;
         if ((rc = s.upload_ctl(S->st))) return rc;
-        // exactly `steps` steps' launches: full chunks, then power-of-two
-        // chunks for the rest (a scenario that reaches its end or a fault
+        // exactly `steps` steps (a scenario that reaches its end or a fault
         // time earlier stops there)
         Stepping loop(S->b);
         do {

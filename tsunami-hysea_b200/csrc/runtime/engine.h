@@ -1,7 +1,6 @@
-// Host-side engine: device state of scenarios, the graph-captured time loop
-// and its event handling.  Shared by thy_run (one scenario), the session
-// API (benchmarking) and the batch / server runtimes (many scenarios in one
-// persistent launch).
+// Host-side engine: device state of scenarios, the time loop in chunks and its
+// event handling.  Shared by thy_run (one scenario), the session API
+// (benchmarking) and the server runtime (many scenarios in one batch).
 #pragma once
 #include <cstdint>
 #include <memory>

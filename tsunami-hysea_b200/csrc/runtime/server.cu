@@ -1,5 +1,5 @@
 // Multi-scenario runtime: many scenarios stepped together by one batch (one
-// work list over all their tiles, one CUDA graph of step chunks), admitted
+// work list over all their units, resident chunks or CUDA graphs of steps), admitted
 // from a queue under an HBM budget, retired as they finish (continuous
 // batching).  Drives the same kernels and control blocks as thy_run; each
 // scenario's arithmetic is independent of the others, so a result is the
