@@ -3,6 +3,7 @@ against the launched kernels: the same code of every cell, so bitwise the same
 fields, samples, step counts and unit counts, at sizes around the edges of
 strips (28 columns), tiles (112), units (16 rows) and of the task splits, up to
 the largest resident work."""
+import dataclasses
 import os
 import subprocess
 import sys
@@ -169,6 +170,31 @@ def test_scenarios_that_fail_in_a_resident_batch(gpu):
             assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k
     # (launched chunks of a queue are 16 steps long)
     assert chunks < max(r["iterations"] for _, r in alone) / 16
+
+
+def test_scenario_that_fails_late_in_a_resident_batch(gpu):
+    """a second fault whose deformation overflows single precision, in mid-run: the
+    scenario ends at the same step alone and in a batch, whose other scenarios, one
+    that ends before and one after it, finish as alone"""
+    bad = _problem(200, 190, "late", 600.0)
+    bad.points, bad.series_time, bad.save_time = None, -1.0, -1.0
+    bad.faults[1] = dataclasses.replace(bad.faults[1], slip=1e300)
+    goods = [_problem(120, 100, "open", 200.0), _problem(230, 256, "file", 900.0)]
+    alone = [_run(thysea.Prepared(p)) for p in goods]
+    srv = thysea.Server(hbm_budget_bytes=2 << 30, max_scenarios=8)
+    first = srv.submit(bad)
+    srv.drain()
+    ids = [srv.submit(p) for p in (goods[0], bad, goods[1])]
+    srv.drain()
+    srv.close()
+    steps = srv.results[first]["stats"]["steps"]
+    assert srv.results[first]["status"] == srv.results[ids[1]]["status"] == thysea.THY_ERR_NONFINITE
+    assert steps > 64 and srv.results[ids[1]]["stats"]["steps"] == steps
+    for rid, (ref, r) in zip((ids[0], ids[2]), alone):
+        assert srv.results[rid]["status"] == 0
+        assert srv.results[rid]["stats"]["steps"] == r["iterations"]
+        for k in FIELDS:
+            assert np.array_equal(srv.results[rid]["outputs"][k], ref[k], equal_nan=True), k
 
 
 def test_barrier_timeout_is_reported_and_the_chunk_can_be_stepped_again(gpu):
