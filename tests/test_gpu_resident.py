@@ -265,7 +265,7 @@ torch.cuda.synchronize()
 t0 = time.perf_counter()
 for st in streams:
     with torch.cuda.stream(st):
-        torch.cuda._sleep(int(1.9e9))   # one block, a second
+        torch.cuda._sleep(int(7.6e9))   # one block, four seconds
 got, r = t._run(prep)
 with torch.cuda.stream(side):
     x.add_(1.0)
@@ -273,7 +273,7 @@ side.synchronize()
 waited = time.perf_counter() - t0
 assert not any(st.query() for st in streams)   # they are still running
 torch.cuda.synchronize()
-assert waited < 0.5, waited
+assert waited < 2.0, waited   # (a run takes 0.01 s; a host may stall)
 assert r["iterations"] == r0["iterations"] and r["kernel_launches"] < r["iterations"]
 for k in t.FIELDS:
     assert np.array_equal(got[k], ref[k], equal_nan=True), k
@@ -282,7 +282,7 @@ for k in t.FIELDS:
 
 @pytest.mark.parametrize("blocks", [1, 3])
 def test_resident_chunks_beside_another_streams_long_kernels(gpu, blocks):
-    """SMs held by other streams' kernels for a second: a run does not wait for
+    """SMs held by other streams' kernels for seconds: a run does not wait for
     their end (its chunks are stepped by the blocks that find a free SM), other
     kernels are not held back by it, and the results are the same.  (In a process
     with a hardware queue for each of its streams.)"""
